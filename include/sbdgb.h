@@ -152,7 +152,9 @@ int sbdgb_sigma_mixed_block(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev
  * time, every beta pair of the problem a lane's product with the row of C in
  * shared memory), with shape_a 0 = its persistent double-buffered form where
  * the row length and alignment allow it (one row per CTA of 512 threads
- * otherwise) or 1 = one row per CTA of 1024 threads.
+ * otherwise) or 1 = one row per CTA of 1024 threads;
+ * shape_b = 7 (reported, not settable) means the fixed-point kernels
+ * (sigma_slab.cu), taken without timing where a row has more than 8 nonzeros.
  * The first product of each precision tunes (and synchronises), so make it
  * before any stream capture. */
 int sbdgb_problem_tuning(const sbdgb_problem *p, int precision, int *shape_a, int *shape_b, float *ms_a,

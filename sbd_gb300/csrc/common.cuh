@@ -165,6 +165,7 @@ struct Problem {
   // count in slices of 32, each slice's beta singles interleaved by lane
   uint32_t *ab_rows = nullptr, *ab_cols = nullptr, *ab_slice = nullptr, *ab_ent = nullptr;
   uint64_t *ab_mask = nullptr;
+  size_t ab_entries = 0;
   uint32_t n_ab_rows = 0, n_ab_slices = 0;
   // the row kernel for sparse rows (sigma_stream.cu): every beta pair in
   // column order, runs padded not to cross 32 entries, and its row order
@@ -172,6 +173,19 @@ struct Problem {
   uint32_t *rp_rows = nullptr;
   uint32_t rp_n = 0, rp_maxrun = 0;
   bool rp_ready = false;
+  // the fixed-point kernels (sigma_slab.cu): per spin the rows sorted by
+  // doubles in slices of 32, their table entries interleaved by lane, the
+  // values' exponent, and the eta masks of the strings
+  struct Slab {
+    int state = -1;  // -1 not decided yet, 0 does not apply, 1 built
+    uint32_t *rows[2] = {}, *off[2] = {};
+    uint4 *ent_s[2] = {}, *ket_d[2] = {};
+    int4 *val_s[2] = {}, *val_d[2] = {};
+    uint64_t *mask[2] = {};
+    uint32_t *ab_ent = nullptr;  // the beta singles of ab_ent below, in this kernel's order
+    uint32_t nslices[2] = {};
+    int ev[2] = {}, ek = 0;
+  } slab;
   size_t bytes = 0;
   std::vector<void *> allocs;
   // host copies of strings
@@ -259,6 +273,10 @@ void build_row_pairs(Problem &p, const std::vector<uint32_t> &off_s, const std::
                      const std::vector<uint32_t> &rows, cudaStream_t s);
 template <typename T>
 bool rows_fit(const Problem &p);
+// sigma_slab.cu: the FP64 product in fixed point, where slab_prepare (which
+// builds its tables on first use) says that it applies.
+bool slab_prepare(Problem &p, cudaStream_t s);
+void sigma_slab(const Problem &p, const double *C, double *S, int accumulate, cudaStream_t s, bool block);
 // block: the block-ordering product (H_block = eta H eta, no opposite-spin
 // parities) that the solvers use on eta-signed vectors; false: the
 // reference's interleaved convention.

@@ -523,8 +523,9 @@ constexpr int kFusedShape = 4;   // tune_b value meaning "beta sweep fused into 
 constexpr int kSparseShape = 5;  // tune_b value meaning "k_sigma_sparse"; tune_a 0/1 = 8/16 rows per tile
 constexpr int kNumSparse = 2;
 constexpr int kStreamShape = 6;  // tune_b value meaning "the row kernel" (sigma_stream.cu); tune_a 0/1 = its two forms
+constexpr int kSlabShape = 7;    // tune_b value meaning "the fixed-point kernels" (sigma_slab.cu)
 inline bool needs_transpose(int shape_b) {
-  return shape_b != kFusedShape && shape_b != kSparseShape && shape_b != kStreamShape;
+  return shape_b != kFusedShape && shape_b != kSparseShape && shape_b != kStreamShape && shape_b != kSlabShape;
 }
 constexpr int kShapeTA[kNumShapes] = {8, 8, 8, 16};
 constexpr int kShapeCPT[kNumShapes] = {1, 2, 4, 2};
@@ -627,6 +628,12 @@ void launch_stream_or_sparse(const Problem &p, const Args<T> &a, int variant, cu
 // pairs and k_sigma_ab adds them afterwards.
 template <typename T, bool kB>
 void launch_shapes(Problem &p, const Args<T> &a, int sa, int sb, int split, cudaStream_t s) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (sb == kSlabShape) {
+      sigma_slab(p, a.C, a.S, a.accumulate, s, kB);
+      return;
+    }
+  }
   Args<T> b = a;
   b.skip_ab = split > 0 ? 1 : 0;
   if (sb == kSparseShape) {
@@ -820,15 +827,28 @@ inline double nnz_per_row(const Problem &p) {
   return (p.na ? (double)(p.A.ns + p.A.nd) / p.na : 0.0) + (p.nb ? (double)(p.B.ns + p.B.nd) / p.nb : 0.0) + sa * sb;
 }
 
+// Nonzeros per row above which the fixed-point kernels are taken without
+// timing: below it a product is a stream through memory, which they pass over
+// twice.
+constexpr double kSlabPerRow = 8.0;
+
 // Alpha x beta single pairs per determinant above which the untimed choice
 // gives them their own kernel (k_sigma_ab stages rows per alpha single; with
 // a few singles per string on both sides that staging is cheap per term).
 constexpr double kAbSplitPerElement = 4.0;
 
 template <typename T, bool kB>
-bool needs_tuning(Problem &p) {
+bool needs_tuning(Problem &p, cudaStream_t s) {
   const int prec = slot_of<T, kB>();
   if (p.tune_a[prec] >= 0 && p.tune_b[prec] >= 0) return false;
+  if constexpr (std::is_same<T, double>::value) {
+    if (nnz_per_row(p) > kSlabPerRow && slab_prepare(p, s)) {
+      p.tune_a[prec] = 0;
+      p.tune_b[prec] = kSlabShape;
+      p.split_ab[prec] = p.A.ns > 0 && p.B.ns > 0 ? 1 : 0;
+      return false;
+    }
+  }
   if (p.ctx->autotune) return true;
   p.split_ab[prec] =
       (ab_fits<T>(p) && (double)p.A.ns * (double)p.B.ns >= kAbSplitPerElement * (double)p.N) ? 1 : 0;
@@ -1389,7 +1409,7 @@ namespace {
 template <typename T, bool kB>
 void run_sigma(Problem &p, const Args<T> &a, T *CT, cudaStream_t s) {
   constexpr int ts = slot_of<T, kB>();
-  if (needs_tuning<T, kB>(p)) {
+  if (needs_tuning<T, kB>(p, s)) {
     transpose<T>(p, a.C, CT, p.na, p.nb, s);
     autotune<T, kB>(p, a, s);
   }
@@ -1403,8 +1423,10 @@ void run_sigma(Problem &p, const Args<T> &a, T *CT, cudaStream_t s) {
 
 void sigma_fp64(Problem &p, const double *C, double *S, int accumulate, cudaStream_t s, bool block) {
   if (!p.tables || !p.diag) throw Error(SBDGB_E_STATE, "sigma needs tables and diagonal");
-  if (!p.CT) p.CT = (double *)dev_alloc(p, sizeof(double) * p.N);
   if (p.N == 0) return;
+  const bool tuned = !(block ? needs_tuning<double, true>(p, s) : needs_tuning<double, false>(p, s));
+  if (!p.CT && (!tuned || needs_transpose(p.tune_b[block ? 3 : 0])))
+    p.CT = (double *)dev_alloc(p, sizeof(double) * p.N);
   Args<double> a = base_args<double>(p, C, S, accumulate);
   a.CT = p.CT;
   a.val_sa = p.A.val_s;
@@ -1526,7 +1548,7 @@ namespace {
 template <bool kB>
 void sigma_mixed_multi_impl(Problem &p, const float *C, float *S, int nvec, cudaStream_t s, double shift) {
   constexpr int ts = slot_of<float, kB>();
-  if (needs_tuning<float, kB>(p)) sigma_mixed(p, C, S, s, shift, kB);  // tunes the FP32 shapes on the first vector
+  if (needs_tuning<float, kB>(p, s)) sigma_mixed(p, C, S, s, shift, kB);  // tunes the FP32 shapes on the first vector
   ArgsMV m{};
   m.a = mixed_args(p, C, S, shift);
   const bool fused = !needs_transpose(p.tune_b[ts]);

@@ -232,6 +232,7 @@ void build_ab_order(Problem &p, const std::vector<uint32_t> &off_a, const std::v
   SBDGB_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
   p.n_ab_rows = (uint32_t)rows.size();
   p.n_ab_slices = nslices;
+  p.ab_entries = total;
 }
 
 template <typename T>

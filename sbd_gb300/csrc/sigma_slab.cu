@@ -1,0 +1,991 @@
+// sigma = H*C with the pair sums in fixed point and the gathered vector in
+// shared memory (FP64 products; replaces sbd::mult, chemistry/tpb/mult.h:
+// 440-558, like the kernels of sigma.cu, for problems with many nonzeros a row).
+//
+// What bounds it.  The kernels of sigma.cu spend one FP64 multiply-add per
+// nonzero and keep the FP64 pipe (2 a clock and SM) 89-91% busy.  Here a
+// nonzero costs three 32 x 32 + 64-bit integer multiply-adds (fx.cuh; 32 a
+// clock and SM), and its gather comes from shared memory instead of L2.  ncu on
+// the beta sweep of 3274 x 3935 strings (norb 24, 245 pairs a row): L1 data
+// pipe 79%, integer multiply-adds near 70% of their rate, shared loads at 1.2
+// wavefronts per 8 lanes.
+//
+// Measured (one product in the reference's convention, ms; FP64 kernels, here):
+// norb 12, 161 x 187: 0.374, 0.084; norb 16, 800 x 800: 1.91, 0.70; norb 24,
+// 3274 x 3935: 18.8, 8.2 (sweeps 2.1 and 1.8, alpha x beta 4.4); norb 36, 6000 x
+// 6000: 6.4, 3.6 (1.4, 1.4 and 0.9).  Error against FP64 sums of the
+// off-diagonal part kept apart from the diagonal (2-norm): 0.7-1.1e-16, where
+// the FP64 kernels have 3e-16 to 1.3e-15.
+//
+// k_slab (same-spin pairs; task types 1 and 2).  The sweep over one spin's
+// pairs never mixes columns (the opposite-spin index), so a CTA takes K
+// columns and stages all n rows of them (8 K n bytes: 192 KB at K = 4, n =
+// 6000).  Staging finds each column's largest |C|, which sets the column's
+// fixed-point scale, and converts in place.  Then a lane owns a row: per pair
+// it reads (ket, V) once, coalesced, and K staged values, and adds K terms.
+// Rows are sorted by their number of doubles and cut into slices of 32 that
+// the warps take in turn (longest first); a slice's lists are interleaved by
+// lane in groups of four and padded to its longest (the sliced ELLPACK form)
+// with entries that point at a zero row.  The beta sweep stages K rows of C
+// (contiguous) and needs no transposed copy; the alpha sweep stages K columns
+// (32-byte pieces at K = 4).  The beta sweep runs first and writes the diagonal
+// while it stages; the sums are then added with one reduction per element and
+// launch (fire and forget, and in the order of the launches).
+//
+// Phases.  Both sweeps and k_slab_ab work in the block ordering (no
+// opposite-spin parity; sigma_dev.cuh).  For the reference's interleaved
+// convention the sign eta of each determinant is applied while staging and
+// again to the result: two popcounts per determinant instead of one or two per
+// nonzero.
+//
+// A column (or ket row) with an infinity, a NaN or values beyond 2^+-800 is
+// summed in FP64 from the values as they are (slow, and the same results as
+// the FP64 kernels give).
+#include <algorithm>
+#include <cmath>
+#include <numeric>
+#include <type_traits>
+
+#include "common.cuh"
+#include "fx.cuh"
+#include "sigma_dev.cuh"
+
+namespace sbdgb {
+
+namespace {
+
+using namespace sdev;
+
+constexpr int kSlabThreads = 768, kSlabAbThreads = 512;
+constexpr int kGroup = 4;  // table entries of a lane that are read together
+constexpr uint32_t kSlabMaxRows = 1u << 15;  // ket index bits of a packed single
+constexpr uint32_t kSlabMaxPair = 1u << 12;  // pair index bits
+
+// ---- the vector formats ----------------------------------------------------------
+
+// key: monotone in |x|, 0 for 0 only; key_exponent(key): |x| < 2^exponent (fx.cuh).
+__device__ __forceinline__ uint32_t key_of(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+  return hi ? hi : (__double2loint(x) ? 1u : 0u);
+}
+__device__ __forceinline__ int2 raw_bits(double x) { return make_int2(__double2loint(x), __double2hiint(x)); }
+__device__ __forceinline__ double raw_of(int2 v) { return __hiloint2double(v.y, v.x); }
+// ---- the sweep over one spin's pairs -----------------------------------------------
+
+struct SlabSpin {
+  const uint32_t *rows;           // 32 per slice; ~0u pads the last
+  const uint32_t *off_s, *off_d;  // per slice: first group of its singles and doubles
+  const uint4 *ent_s;             // singles: ket << 4 | pair << 19 | phase << 31
+  const int4 *val_s;              // V of the same-spin part with the phase applied
+  const uint4 *ket_d;             // doubles: ket << 4
+  const int4 *val_d;
+  uint32_t nslices;
+};
+
+struct SlabArgs {
+  const double *C;
+  double *S;
+  const double *hii;
+  SlabSpin t;
+  SpinTables tables;        // the same entries as the FP64 kernels read them
+  const double *Jo;         // opposite-spin Coulomb table [npair][m]
+  const uint64_t *rowstr;   // this spin's strings
+  const uint64_t *colmask;  // per column: the orbitals whose parity on rowstr is eta
+  uint32_t n, m, nb;        // rows (this spin), columns (the other spin), row length of C and S
+  int npair;                // 0: no singles (J is not staged)
+  int ev;                   // |v| < 2^ev for every table value of this spin
+  int eta;                  // interleaved convention: eta on the way in and out
+  int add;                  // what S holds is kept
+  int diag;                 // the diagonal term is added here
+  int staged_diag;          // ... while staging, so that S is complete but for this spin's sums
+  uint32_t parts;           // CTAs that share a column group (gridDim.y)
+};
+
+// Staged values: K columns, two of a row side by side (16 bytes) in planes of
+// `rows` rows, so that a lane reads two columns with one load.
+template <int K>
+__device__ __forceinline__ size_t staged(uint32_t rows, uint32_t r, int c) {
+  return K == 1 ? r : ((size_t)(c >> 1) * rows + r) * 2 + (c & 1);
+}
+
+// Row `row` summed in FP64 as the kernels of sigma.cu do, from the raw staged
+// values (a column that is not finite, or out of the fixed-point range).
+template <int K>
+__device__ __noinline__ double slab_row_fp64(const SpinTables &T, uint32_t row, const int2 *X, uint32_t n1,
+                                             const double *Jo, uint32_t m, uint32_t col, int c) {
+  double sum = 0.0;
+  for (uint32_t p = ldg(T.off_s + row); p < ldg(T.off_s + row + 1); ++p) {
+    const uint32_t code = ldg(T.code_s + p);
+    const double v = ldg(T.val_s + p) + ldg(Jo + (size_t)((code >> 16) & 0x7fffu) * m + col);
+    sum = fma(flip(v, code >> 31), raw_of(X[staged<K>(n1, ldg(T.ket_s + p), c)]), sum);
+  }
+  for (uint32_t p = ldg(T.off_d + row); p < ldg(T.off_d + row + 1); ++p)
+    sum = fma(ldg(T.val_d + p), raw_of(X[staged<K>(n1, ldg(T.ket_d + p), c)]), sum);
+  return sum;
+}
+
+// Four table entries of a lane: three 16-byte loads.
+struct Group {
+  uint4 w;
+  int4 v0, v1;
+  __device__ __forceinline__ void load(const uint4 *__restrict__ ent, const int4 *__restrict__ val, uint32_t at) {
+    w = ldg(ent + at);
+    v0 = __ldg(val + 2 * at);
+    v1 = __ldg(val + 2 * at + 1);
+  }
+};
+
+template <int K, bool kSingles>
+__device__ __forceinline__ void slab_group(fx::Acc (&acc)[K], const Group &g, const char *X, uint32_t xplane,
+                                           const char *J, uint32_t jplane) {
+  constexpr int NQ = (K + 1) / 2;
+  const uint32_t w[kGroup] = {g.w.x, g.w.y, g.w.z, g.w.w};
+  const int vh[kGroup] = {g.v0.x, g.v0.z, g.v1.x, g.v1.z}, vl[kGroup] = {g.v0.y, g.v0.w, g.v1.y, g.v1.w};
+#pragma unroll
+  for (int u = 0; u < kGroup; ++u) {
+    const uint32_t x16 = kSingles ? w[u] & 0x7fff0u : w[u], j16 = (w[u] >> 15) & 0xfff0u;
+    const int sg = (int)w[u] >> 31;  // singles, -1: the Coulomb part is subtracted
+    if constexpr (K == 1) {
+      const int2 x = *reinterpret_cast<const int2 *>(X + (x16 >> 1));
+      if constexpr (kSingles) {
+        const int2 j = *reinterpret_cast<const int2 *>(J + (j16 >> 1));
+        fx::mac(acc[0], x.x, x.y, vh[u] + ((j.x ^ sg) - sg), vl[u] + ((j.y ^ sg) - sg));
+      } else {
+        fx::mac(acc[0], x.x, x.y, vh[u], vl[u]);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const int4 x = *reinterpret_cast<const int4 *>(X + q * xplane + x16);
+        if constexpr (kSingles) {
+          const int4 j = *reinterpret_cast<const int4 *>(J + q * jplane + j16);
+          fx::mac(acc[2 * q], x.x, x.y, vh[u] + ((j.x ^ sg) - sg), vl[u] + ((j.y ^ sg) - sg));
+          fx::mac(acc[2 * q + 1], x.z, x.w, vh[u] + ((j.z ^ sg) - sg), vl[u] + ((j.w ^ sg) - sg));
+        } else {
+          fx::mac(acc[2 * q], x.x, x.y, vh[u], vl[u]);
+          fx::mac(acc[2 * q + 1], x.z, x.w, vh[u], vl[u]);
+        }
+      }
+    }
+  }
+}
+
+// Adds one slice's singles or doubles to the lane's K sums, two groups a turn:
+// each is requested before the other is summed.
+template <int K, bool kSingles>
+__device__ __forceinline__ void slab_list(fx::Acc (&acc)[K], const uint4 *__restrict__ ent,
+                                          const int4 *__restrict__ val, uint32_t g, uint32_t end, uint32_t lane,
+                                          const char *X, uint32_t xplane, const char *J, uint32_t jplane) {
+  static_assert(fx::kChunkHigh == 4 * kGroup && fx::kChunk == 8 * kGroup, "carries every 4 and 8 groups");
+  if (g >= end) return;
+  uint32_t at = g * 32u + lane, left = end - g, turn = 0;
+  Group a, b;
+  a.load(ent, val, at);
+  while (true) {
+    if (left > 1) b.load(ent, val, at + 32u);
+    slab_group<K, kSingles>(acc, a, X, xplane, J, jplane);
+    if (left == 1) break;
+    if (left > 2) a.load(ent, val, at + 64u);
+    slab_group<K, kSingles>(acc, b, X, xplane, J, jplane);
+    if (left == 2) break;
+    left -= 2;
+    at += 64u;
+    ++turn;
+    if ((turn & 3u) == 0u) {
+#pragma unroll
+      for (int c = 0; c < K; ++c) fx::carry(acc[c]);
+    } else if ((turn & 1u) == 0u) {
+#pragma unroll
+      for (int c = 0; c < K; ++c) fx::carry_high(acc[c]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < K; ++c) fx::carry(acc[c]);
+}
+
+template <int K, bool kAlpha>
+__global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
+  constexpr int NQ = (K + 1) / 2;
+  extern __shared__ __align__(16) unsigned char slab_smem[];
+  int2 *X = reinterpret_cast<int2 *>(slab_smem);     // (n + 1) x K; row n is zero (padding entries)
+  int2 *J = X + (size_t)(a.n + 1) * K;               // (npair + 1) x K; row npair is zero
+  __shared__ uint32_t skey[K], snext;
+  const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
+  const uint32_t c0 = blockIdx.x * K;
+  if (tid < K) skey[tid] = 0u;
+  if (tid == 0) snext = 0u;
+  __syncthreads();
+  // stage the raw values and find each column's largest
+  if constexpr (kAlpha) {
+    const int c = (int)(tid % K);
+    const bool ok = c0 + c < a.m;
+    const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
+    uint32_t key = 0u;
+    for (uint32_t r = tid / K; r < a.n; r += nt / K) {
+      double x = ok ? ldg(a.C + (size_t)r * a.nb + (c0 + c)) : 0.0;
+      if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
+      key = max(key, key_of(x));
+      X[staged<K>(a.n + 1, r, c)] = raw_bits(x);
+    }
+    for (int o = 16; o >= K; o >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
+    if (lane < (uint32_t)K) atomicMax(&skey[c], key);
+  } else {
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      const bool ok = c0 + c < a.m;
+      const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
+      const double *row = a.C + (size_t)(c0 + c) * a.nb;
+      uint32_t key = 0u;
+      for (uint32_t r = tid; r < a.n; r += nt) {
+        double x = ok ? ldg(row + r) : 0.0;
+        if (a.staged_diag && ok) {
+          const size_t k = (size_t)(c0 + c) * a.nb + r;
+          const double d = ldg(a.hii + k) * x;
+          a.S[k] = a.add ? a.S[k] + d : d;
+        }
+        if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
+        key = max(key, key_of(x));
+        X[staged<K>(a.n + 1, r, c)] = raw_bits(x);
+      }
+      key = __reduce_max_sync(0xffffffffu, key);
+      if (lane == 0) atomicMax(&skey[c], key);
+    }
+  }
+  if (tid < K) X[staged<K>(a.n + 1, a.n, tid)] = make_int2(0, 0);
+  if (a.npair) {
+    for (uint32_t i = tid; i < (uint32_t)(a.npair + 1) * K; i += nt) {
+      const uint32_t P = i / K;
+      const int c = (int)(i % K);
+      const bool ok = P < (uint32_t)a.npair && c0 + c < a.m;
+      J[staged<K>(a.npair + 1, P, c)] =
+          ok ? fx::make(ldg(a.Jo + (size_t)P * a.m + (c0 + c)), fx::kVBits - a.ev) : make_int2(0, 0);
+    }
+  }
+  __syncthreads();
+  int ex[K];
+  bool bad = false;
+#pragma unroll
+  for (int c = 0; c < K; ++c) {
+    ex[c] = fx::exponent_of(skey[c], skey[c] != 0u);
+    bad = bad || ex[c] == fx::kBad;
+  }
+  if (!bad) {  // to fixed point, in place (an all-zero column has no scale and its sums are not read)
+    constexpr int kw = K == 1 ? 1 : 2;
+    const uint32_t plane = (a.n + 1) * kw;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      for (uint32_t i = tid; i < plane; i += nt) {
+        const int e = K == 1 || !(i & 1u) ? ex[q * kw] : ex[q * kw + kw - 1];
+        int2 &x = X[(size_t)q * plane + i];
+        if (e != fx::kZero) x = fx::vector_parts((uint32_t)x.x, (uint32_t)x.y, e);
+      }
+    __syncthreads();
+  }
+  const SlabSpin &t = a.t;
+  while (true) {
+    uint32_t sl = 0;
+    if (lane == 0) sl = atomicAdd(&snext, 1u);
+    sl = blockIdx.y + a.parts * __shfl_sync(0xffffffffu, sl, 0);
+    if (sl >= t.nslices) break;
+    const uint32_t row = ldg(t.rows + sl * 32u + lane);
+    double out[K];
+    if (!bad) {
+      fx::Acc acc[K];
+#pragma unroll
+      for (int c = 0; c < K; ++c) fx::zero(acc[c]);
+      const uint32_t xplane = 16u * (a.n + 1), jplane = 16u * (a.npair + 1);
+      slab_list<K, true>(acc, t.ent_s, t.val_s, ldg(t.off_s + sl), ldg(t.off_s + sl + 1), lane,
+                         reinterpret_cast<const char *>(X), xplane, reinterpret_cast<const char *>(J), jplane);
+      slab_list<K, false>(acc, t.ket_d, t.val_d, ldg(t.off_d + sl), ldg(t.off_d + sl + 1), lane,
+                          reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
+#pragma unroll
+      for (int c = 0; c < K; ++c)
+        out[c] = ex[c] == fx::kZero ? 0.0 : fx::value(acc[c], ex[c] + a.ev + fx::kUnit);
+    } else {
+#pragma unroll
+      for (int c = 0; c < K; ++c)
+        out[c] = row != ~0u && c0 + c < a.m ? slab_row_fp64<K>(a.tables, row, X, a.n + 1, a.Jo, a.m, c0 + c, c) : 0.0;
+    }
+    if (row == ~0u) continue;
+    const uint64_t str = a.eta ? ldg(a.rowstr + row) : 0ull;
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      if (c0 + c >= a.m) break;
+      double s = out[c];
+      if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c0 + c))));
+      const size_t k = kAlpha ? (size_t)row * a.nb + (c0 + c) : (size_t)(c0 + c) * a.nb + row;
+      if (a.diag && !a.staged_diag) s = fma(ldg(a.hii + k), ldg(a.C + k), s);
+      // one addition per element and launch: the order of the sum is that of the launches
+      if (a.add || a.staged_diag)
+        atomicAdd(a.S + k, s);
+      else
+        a.S[k] = s;
+    }
+  }
+}
+
+// ---- alpha single x beta single (task type 0) ---------------------------------------
+//
+// The layout of k_sigma_ab (sigma_ab.cu): a CTA owns one alpha row (with
+// gridDim.y > 1, every gridDim.y-th slice of its columns) and takes G of its
+// singles at a time, C rows and (P|Q) rows staged in shared memory; beta singles
+// in slices of 32 columns, their entries ordered against bank conflicts
+// (k_slab_ab_order).  Each (P|Q) value is staged with both signs, so that an
+// entry's phase is part of its index.
+//
+// kFixed: in fixed point.  The ket rows of a batch have scales of their own
+// (2^e_g); the batch's is the largest, and the (P|Q) values of a smaller row are
+// scaled down by the difference.  Otherwise FP64 multiply-adds on the values as
+// they are (few terms a column; slab_ab_fixed).
+// kSum: the row's sums stay in shared memory until the last batch; otherwise
+// each batch's go to sigma at once (rows with a batch or two; less shared
+// memory, so more CTAs an SM).
+
+struct SlabAbArgs {
+  const double *C;
+  double *S;
+  const uint64_t *astr;
+  const uint64_t *colmask;           // per beta string
+  const uint32_t *off, *ket, *code;  // alpha singles
+  const double *Kp;
+  const uint32_t *rows, *cols, *slice, *ent;
+  uint32_t nslices, nb;
+  int npair, ek, eta;
+};
+
+template <int G, bool kFixed, bool kSum>
+__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs a) {
+  constexpr int NP = G / 2;
+  extern __shared__ __align__(16) unsigned char slab_smem[];
+  const uint32_t kplane = 2 * (a.npair + 1);
+  int4 *Cs = reinterpret_cast<int4 *>(slab_smem);                // [G/2][nb]: two ket rows' values at jb
+  int4 *Ks = Cs + (size_t)NP * a.nb;                             // [G/2][2 Q + phase]
+  double *Ss = reinterpret_cast<double *>(Ks + NP * kplane);     // kSum: [nb]
+  __shared__ uint32_t skey[G];
+  const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
+  const uint32_t ia = ldg(a.rows + blockIdx.x);
+  const uint32_t p0 = ldg(a.off + ia), p1 = ldg(a.off + ia + 1);
+  const uint64_t str = a.eta ? ldg(a.astr + ia) : 0ull;
+  const uint32_t parts = gridDim.y, mine = (a.nslices - blockIdx.y + parts - 1) / parts;  // slices of this CTA
+  if (kSum)
+    for (uint32_t c = tid; c < a.nb; c += nt) Ss[c] = 0.0;
+  for (uint32_t pb = p0; pb < p1; pb += G) {
+    const uint32_t live = min((uint32_t)G, p1 - pb);
+    __syncthreads();  // the previous batch is applied
+    if (tid < G) skey[tid] = 0u;
+    __syncthreads();
+    uint32_t key[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) key[g] = 0u;
+#pragma unroll
+    for (int h = 0; h < NP; ++h) {
+      const bool ok0 = 2 * h < live, ok1 = 2 * h + 1 < live;
+      const uint32_t ja0 = ok0 ? ldg(a.ket + pb + 2 * h) : 0u, ja1 = ok1 ? ldg(a.ket + pb + 2 * h + 1) : 0u;
+      const uint64_t s0 = a.eta && ok0 ? ldg(a.astr + ja0) : 0ull, s1 = a.eta && ok1 ? ldg(a.astr + ja1) : 0ull;
+      const double *r0 = a.C + (size_t)ja0 * a.nb, *r1 = a.C + (size_t)ja1 * a.nb;
+      for (uint32_t c = tid; c < a.nb; c += nt) {
+        double x0 = ok0 ? ldg(r0 + c) : 0.0, x1 = ok1 ? ldg(r1 + c) : 0.0;
+        if (a.eta) {
+          const uint64_t m = ldg(a.colmask + c);
+          x0 = flip(x0, parity((unsigned long long)(s0 & m)));
+          x1 = flip(x1, parity((unsigned long long)(s1 & m)));
+        }
+        if (kFixed) {
+          key[2 * h] = max(key[2 * h], key_of(x0));
+          key[2 * h + 1] = max(key[2 * h + 1], key_of(x1));
+        }
+        const int2 b0 = raw_bits(x0), b1 = raw_bits(x1);
+        Cs[h * a.nb + c] = make_int4(b0.x, b0.y, b1.x, b1.y);
+      }
+    }
+    int e[G], es = fx::kZero;
+    bool fixed = kFixed;
+    if (kFixed) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        key[g] = __reduce_max_sync(0xffffffffu, key[g]);
+        if (lane == 0) atomicMax(&skey[g], key[g]);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        e[g] = fx::exponent_of(skey[g], skey[g] != 0u);
+        es = max(es, e[g]);
+      }
+      if (es == fx::kZero) continue;  // every row is zero
+      fixed = es != fx::kBad;
+    }
+    if (fixed) {  // to fixed point, in place: each thread the columns that it staged
+#pragma unroll
+      for (int h = 0; h < NP; ++h)
+        for (uint32_t c = tid; c < a.nb; c += nt) {
+          const int4 r = Cs[h * a.nb + c];
+          const int2 z = make_int2(0, 0);
+          const int2 x0 = e[2 * h] == fx::kZero ? z : fx::vector_parts((uint32_t)r.x, (uint32_t)r.y, e[2 * h]);
+          const int2 x1 = e[2 * h + 1] == fx::kZero ? z : fx::vector_parts((uint32_t)r.z, (uint32_t)r.w, e[2 * h + 1]);
+          Cs[h * a.nb + c] = make_int4(x0.x, x0.y, x1.x, x1.y);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < NP; ++h) {
+      const uint32_t c0 = 2 * h < live ? ldg(a.code + pb + 2 * h) : 0u;
+      const uint32_t c1 = 2 * h + 1 < live ? ldg(a.code + pb + 2 * h + 1) : 0u;
+      const double *k0 = a.Kp + (size_t)((c0 >> 16) & 0x7fffu) * a.npair, *k1 = a.Kp + (size_t)((c1 >> 16) & 0x7fffu) * a.npair;
+      for (uint32_t Q = tid; Q <= (uint32_t)a.npair; Q += nt) {
+        const bool ok = Q < (uint32_t)a.npair;
+        const double v0 = ok && 2 * h < live ? flip(ldg(k0 + Q), c0 >> 31) : 0.0;
+        const double v1 = ok && 2 * h + 1 < live ? flip(ldg(k1 + Q), c1 >> 31) : 0.0;
+        int2 f0, f1, n0, n1;
+        if (fixed) {
+          // (an all-zero row's values are not used, whatever its scale)
+          f0 = fx::make(v0, fx::kVBits - a.ek - min(es - e[2 * h], 100));
+          f1 = fx::make(v1, fx::kVBits - a.ek - min(es - e[2 * h + 1], 100));
+          n0 = make_int2(-f0.x, -f0.y);
+          n1 = make_int2(-f1.x, -f1.y);
+        } else {
+          f0 = raw_bits(v0);
+          f1 = raw_bits(v1);
+          n0 = raw_bits(-v0);
+          n1 = raw_bits(-v1);
+        }
+        Ks[h * kplane + 2 * Q] = make_int4(f0.x, f0.y, f1.x, f1.y);
+        Ks[h * kplane + 2 * Q + 1] = make_int4(n0.x, n0.y, n1.x, n1.y);
+      }
+    }
+    __syncthreads();
+    // this CTA's slices (longest first) dealt to the warps in snake order
+    for (uint32_t base = 0, round = 0; base < mine; base += nw, ++round) {
+      const uint32_t i = base + ((round & 1u) ? nw - 1u - warp : warp);
+      if (i >= mine) continue;
+      const uint32_t sl = blockIdx.y + parts * i, k = sl * 32u + lane;
+      uint32_t at = ldg(a.slice + sl) + lane;
+      const uint32_t end = ldg(a.slice + sl + 1) + lane;
+      if (at >= end) continue;
+      const uint32_t pad = (uint32_t)a.npair << 1;
+      uint32_t w[kGroup];  // four entries; the next four are requested before these are summed
+      auto load = [&](uint32_t from) {
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) w[u] = from + 32u * u < end ? ldg(a.ent + from + 32u * u) : pad;
+      };
+      load(at);
+      double sum = 0.0;
+      if (fixed) {
+        fx::Acc acc;
+        fx::zero(acc);
+        uint32_t since = 0;
+        for (; at < end; at += 32u * kGroup) {
+          uint32_t wc[kGroup];
+#pragma unroll
+          for (int u = 0; u < kGroup; ++u) wc[u] = w[u];
+          if (at + 32u * kGroup < end) load(at + 32u * kGroup);
+#pragma unroll
+          for (int u = 0; u < kGroup; ++u)
+#pragma unroll
+            for (int h = 0; h < NP; ++h) {
+              const int4 kv = Ks[h * kplane + (wc[u] & 0x1fffu)], cv = Cs[h * a.nb + (wc[u] >> 13)];
+              fx::mac(acc, cv.x, cv.y, kv.x, kv.y);
+              fx::mac(acc, cv.z, cv.w, kv.z, kv.w);
+            }
+          since += G * kGroup;
+          if (since >= fx::kChunkHigh) {
+            fx::carry(acc);
+            since = 0;
+          }
+        }
+        fx::carry(acc);
+        sum = fx::value(acc, es + a.ek + fx::kUnit);
+      } else {
+        for (; at < end; at += 32u * kGroup) {
+          uint32_t wc[kGroup];
+#pragma unroll
+          for (int u = 0; u < kGroup; ++u) wc[u] = w[u];
+          if (at + 32u * kGroup < end) load(at + 32u * kGroup);
+#pragma unroll
+          for (int u = 0; u < kGroup; ++u) {
+            if ((wc[u] & 0x1ffeu) == pad) continue;  // padding (its C value may not be finite)
+#pragma unroll
+            for (int h = 0; h < NP; ++h) {
+              const int4 kv = Ks[h * kplane + (wc[u] & 0x1fffu)], cv = Cs[h * a.nb + (wc[u] >> 13)];
+              sum = fma(raw_of(make_int2(kv.x, kv.y)), raw_of(make_int2(cv.x, cv.y)), sum);
+              if (2 * h + 1 < live) sum = fma(raw_of(make_int2(kv.z, kv.w)), raw_of(make_int2(cv.z, cv.w)), sum);
+            }
+          }
+        }
+      }
+      if (k >= a.nb) continue;
+      const uint32_t ib = ldg(a.cols + k);
+      if (kSum) {
+        Ss[ib] += sum;
+      } else {
+        if (a.eta) sum = flip(sum, parity((unsigned long long)(str & ldg(a.colmask + ib))));
+        atomicAdd(a.S + ((size_t)ia * a.nb + ib), sum);  // this thread's alone: batches add in their order
+      }
+    }
+  }
+  if (!kSum) return;
+  __syncthreads();
+  if (parts == 1) {
+    for (uint32_t c = tid; c < a.nb; c += nt) {
+      double s = Ss[c];
+      if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c))));
+      a.S[(size_t)ia * a.nb + c] += s;
+    }
+  } else {
+    for (uint32_t i = warp; i < mine; i += nw) {
+      const uint32_t k = (blockIdx.y + parts * i) * 32u + lane;
+      if (k >= a.nb) continue;
+      const uint32_t ib = ldg(a.cols + k);
+      double s = Ss[ib];
+      if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + ib))));
+      a.S[(size_t)ia * a.nb + ib] += s;
+    }
+  }
+}
+
+// ---- tables -----------------------------------------------------------------------
+
+// Largest |x| (as ordered bits) of n values, into out.
+__global__ void k_absmax(const double *__restrict__ x, size_t n, unsigned long long *out) {
+  unsigned long long b = 0ull;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
+    b = max(b, (unsigned long long)__double_as_longlong(x[e]) & ~(1ull << 63));
+  for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, b);
+}
+
+// The same over the rows P = (p, q), p != q, of an [npair][n] table (the others
+// belong to no excitation).
+__global__ void k_absmax_pairs(const double *__restrict__ x, uint32_t n, unsigned long long *out) {
+  const uint32_t P = blockIdx.y;
+  uint32_t p = (uint32_t)((sqrtf(8.f * (float)P + 1.f) - 1.f) * 0.5f);  // the p of P = p (p + 1) / 2 + q, or next to it
+  while (p * (p + 1) / 2 > P) --p;
+  while ((p + 1) * (p + 2) / 2 <= P) ++p;
+  if (P == p * (p + 1) / 2 + p) return;
+  unsigned long long b = 0ull;
+  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
+    b = max(b, (unsigned long long)__double_as_longlong(x[(size_t)P * n + e]) & ~(1ull << 63));
+  for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, b);
+}
+
+// Order in which each row's entries are taken: a lane's gather reads 16 bytes
+// of shared memory at 16 ket (mod 128), and the 8 lanes that one 128-byte
+// wavefront serves collide where their kets agree mod 8 (2.6 wavefronts for 8
+// random ones, 2.4 measured).  The order of a list is free, so one warp per
+// slice deals the entries out step by step: the lanes of an 8-lane group choose
+// one after another (a different one first each step), each taking a residue
+// that no earlier lane has, the one it has most entries of (simulated: 1.35
+// wavefronts for lists of 40, 1.14 for 228).  order: entry indices, row by row
+// as in the CSR lists; next: scratch of the same size.
+__global__ void __launch_bounds__(32) k_slab_order(const uint32_t *__restrict__ off, const uint32_t *__restrict__ ket,
+                                                   const uint32_t *__restrict__ rows, uint32_t *__restrict__ next,
+                                                   uint32_t *__restrict__ order) {
+  __shared__ uint32_t head[8][32];
+  const uint32_t lane = threadIdx.x;
+  const uint32_t row = rows[blockIdx.x * 32u + lane];
+  const uint32_t p0 = row == ~0u ? 0u : off[row], p1 = row == ~0u ? 0u : off[row + 1];
+  uint32_t cnt[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    cnt[r] = 0u;
+    head[r][lane] = ~0u;
+  }
+  for (uint32_t p = p1; p-- > p0;) {  // lists by residue, in ascending order
+    const uint32_t r = ket[p] & 7u;
+    next[p] = head[r][lane];
+    head[r][lane] = p;
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) cnt[q] += q == r;
+  }
+  const uint32_t steps = __reduce_max_sync(0xffffffffu, p1 - p0), group = lane & 24u;
+  for (uint32_t t = 0; t < steps; ++t) {
+    uint32_t used = 0u;  // residues taken at this step in this group of lanes
+    for (uint32_t i = 0; i < 8; ++i) {
+      uint32_t best = 0u, pick = 8u;
+#pragma unroll
+      for (uint32_t r = 0; r < 8; ++r) {
+        const uint32_t key = cnt[r] ? cnt[r] + ((used >> r & 1u) ? 0u : 1u << 16) : 0u;
+        if (key > best) {
+          best = key;
+          pick = r;
+        }
+      }
+      const uint32_t turn = group | ((i + t) & 7u);
+      const uint32_t taken = __shfl_sync(0xffffffffu, pick, turn);
+      used |= 1u << taken;  // bit 8: the lane's list is empty
+      if (lane == turn && pick < 8u) {
+        const uint32_t p = head[pick][lane];
+        head[pick][lane] = next[p];
+        order[p0 + t] = p;
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q) cnt[q] -= q == pick;
+      }
+    }
+  }
+}
+
+// The same for the beta singles of k_slab_ab, whose entries read two places of
+// shared memory (column w >> 13, pair and phase w & 0x1fff): in its turn a lane
+// takes, of the next 16 entries of its list, the one that collides least with
+// the lanes before it (simulated for lists of 18-25: 1.85 wavefronts per 8
+// lanes and read, 2.6 in list order).  One warp per slice, in place; real
+// entries stay ahead of the padding.
+__global__ void __launch_bounds__(32) k_slab_ab_order(const uint32_t *__restrict__ slice, uint32_t pad,
+                                                      uint32_t *__restrict__ ent) {
+  const uint32_t lane = threadIdx.x, e0 = slice[blockIdx.x] + lane, len = (slice[blockIdx.x + 1] - slice[blockIdx.x]) / 32u;
+  uint32_t cnt = 0;
+  while (cnt < len && (ent[e0 + 32u * cnt] & 0x1ffeu) != pad) ++cnt;
+  const uint32_t group = lane & 24u;
+  for (uint32_t t = 0; t < len; ++t) {
+    uint32_t used = 0u;  // residues taken in this group of lanes: columns in bits 0-7, pairs in 8-15
+    for (uint32_t i = 0; i < 8; ++i) {
+      const uint32_t turn = group | ((i + t) & 7u);
+      uint32_t take = 0u;
+      if (lane == turn && t < cnt) {
+        uint32_t best = 3u, at = t, word = 0u;
+        for (uint32_t j = t; j < min(t + 16u, cnt) && best; ++j) {
+          const uint32_t w = ent[e0 + 32u * j];
+          const uint32_t cost = (used >> ((w >> 13) & 7u) & 1u) + (used >> (8u + (w & 7u)) & 1u);
+          if (cost < best) {
+            best = cost;
+            at = j;
+            word = w;
+          }
+        }
+        if (at != t) {
+          ent[e0 + 32u * at] = ent[e0 + 32u * t];
+          ent[e0 + 32u * t] = word;
+        }
+        take = 1u << ((word >> 13) & 7u) | 1u << (8u + (word & 7u));
+      }
+      used |= __shfl_sync(0xffffffffu, take, turn);
+    }
+  }
+}
+
+// The sliced form of one spin's tables: one CTA per slice, thread (lane, y)
+// writes every 4th group of the lane's row.
+__global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t *__restrict__ rows,
+                                                   const uint32_t *__restrict__ off_s,
+                                                   const uint32_t *__restrict__ off_d,
+                                                   const uint32_t *__restrict__ order_s,
+                                                   const uint32_t *__restrict__ order_d, int npair, int ev,
+                                                   uint4 *__restrict__ ent_s, int4 *__restrict__ val_s,
+                                                   uint4 *__restrict__ ket_d, int4 *__restrict__ val_d) {
+  const uint32_t sl = blockIdx.x, lane = threadIdx.x & 31u, y = threadIdx.x >> 5;
+  const uint32_t row = rows[sl * 32u + lane];
+  for (int doubles = 0; doubles < 2; ++doubles) {
+    const uint32_t *off = doubles ? off_d : off_s, *rp = doubles ? T.off_d : T.off_s;
+    const uint32_t *order = doubles ? order_d : order_s;
+    const uint32_t p0 = row == ~0u ? 0u : rp[row], cnt = row == ~0u ? 0u : rp[row + 1] - p0;
+    for (uint32_t g = off[sl] + y; g < off[sl + 1]; g += 4) {
+      uint32_t w[kGroup];
+      int2 v[kGroup];
+#pragma unroll
+      for (int u = 0; u < kGroup; ++u) {
+        const uint32_t j = (g - off[sl]) * kGroup + u;
+        const bool ok = j < cnt;
+        const uint32_t p = ok ? order[p0 + j] : 0u;
+        if (doubles) {
+          w[u] = (ok ? T.ket_d[p] : T.n) << 4;
+          v[u] = ok ? fx::make(T.val_d[p], fx::kVBits - ev) : make_int2(0, 0);
+        } else {
+          const uint32_t code = ok ? T.code_s[p] : 0u;
+          w[u] = ok ? (T.ket_s[p] << 4 | ((code >> 16) & 0x7fffu) << 19 | (code & 0x80000000u))
+                    : (T.n << 4 | (uint32_t)npair << 19);
+          v[u] = ok ? fx::make(flip(T.val_s[p], code >> 31), fx::kVBits - ev) : make_int2(0, 0);
+        }
+      }
+      const size_t e = (size_t)g * 32u + lane;
+      (doubles ? ket_d : ent_s)[e] = make_uint4(w[0], w[1], w[2], w[3]);
+      (doubles ? val_d : val_s)[2 * e] = make_int4(v[0].x, v[0].y, v[1].x, v[1].y);
+      (doubles ? val_d : val_s)[2 * e + 1] = make_int4(v[2].x, v[2].y, v[3].x, v[3].y);
+    }
+  }
+}
+
+// Per string: the orbitals of the other spin's strings whose parity is eta
+// (sigma_dev.cuh:eta_parity): below a beta string's electrons for an alpha
+// string, above an alpha string's for a beta string.
+__global__ void k_slab_masks(const uint64_t *__restrict__ str, uint32_t n, int beta, uint64_t *__restrict__ mask) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  unsigned long long x = str[i];
+  if (beta) {
+    x <<= 1;
+    for (int k = 1; k < 64; k <<= 1) x ^= x << k;
+  } else {
+    x >>= 1;
+    for (int k = 1; k < 64; k <<= 1) x ^= x >> k;
+  }
+  mask[i] = x;
+}
+
+size_t max_smem() {
+  int dev = 0, optin = 0;
+  SBDGB_CUDA(cudaGetDevice(&dev));
+  SBDGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  return (size_t)optin - 1024;  // the kernels' static part
+}
+size_t slab_smem_bytes(int K, uint32_t n, int npair) {
+  return 8ull * K * ((size_t)n + 1 + (npair ? (size_t)npair + 1 : 0));
+}
+size_t slab_ab_smem_bytes(const Problem &p, int G, bool sum) {
+  return 8ull * G * ((size_t)p.nb + 2 * ((size_t)p.npair + 1)) + (sum ? 8ull * p.nb : 0);
+}
+
+// Whether the alpha x beta pairs are summed in fixed point too.  A batch of two
+// ket rows costs about 100 integer instructions a column to stage and to round
+// its sums; with few terms a column FP64 multiply-adds are cheaper.
+constexpr double kAbFixedPerElement = 8.0;
+bool slab_ab_fixed(const Problem &p) {
+  return (double)p.A.ns * (double)p.B.ns >= kAbFixedPerElement * (double)p.N;
+}
+
+}  // namespace
+
+// ---- host side ----------------------------------------------------------------------
+
+// Builds the sliced tables on first use.  False where the kernels do not apply
+// or their tables would not fit the memory that the transposed copy (8 N
+// bytes, which they do without) is budgeted for.
+bool slab_prepare(Problem &p, cudaStream_t s) {
+  if (p.slab.state >= 0) return p.slab.state == 1;
+  p.slab.state = 0;
+  const size_t limit = max_smem();
+  const uint32_t nmax = std::max(p.na, p.nb);
+  if (nmax >= kSlabMaxRows || (uint32_t)p.npair + 1 >= kSlabMaxPair) return false;
+  if (slab_smem_bytes(1, nmax, p.npair) > limit) return false;
+  const bool ab = p.A.ns > 0 && p.B.ns > 0;
+  if (ab && (p.n_ab_rows == 0 || slab_ab_smem_bytes(p, 2, slab_ab_fixed(p)) > limit)) return false;
+  // the largest table values
+  unsigned long long *mx = (unsigned long long *)workspace(p, WS_RED2, 8 * sizeof(unsigned long long));
+  SBDGB_CUDA(cudaMemsetAsync(mx, 0, 8 * sizeof(unsigned long long), s));
+  auto absmax = [&](const double *x, size_t n, int slot) {
+    if (n == 0) return;
+    k_absmax<<<(unsigned)std::min<size_t>((n + 1023) / 1024, 1024), 256, 0, s>>>(x, n, mx + slot);
+    count_launch(p.ctx);
+  };
+  auto pairmax = [&](const double *x, uint32_t n, int slot) {
+    k_absmax_pairs<<<dim3((n + 1023) / 1024, p.npair), 256, 0, s>>>(x, n, mx + slot);
+    count_launch(p.ctx);
+  };
+  absmax(p.A.val_s, p.A.ns, 0);
+  absmax(p.A.val_d, p.A.nd, 1);
+  pairmax(p.Jb, p.nb, 2);
+  absmax(p.B.val_s, p.B.ns, 3);
+  absmax(p.B.val_d, p.B.nd, 4);
+  pairmax(p.Ja, p.na, 5);
+  pairmax(p.Kp, (uint32_t)p.npair, 6);
+  SBDGB_CUDA(cudaGetLastError());
+  double v[8];
+  SBDGB_CUDA(cudaMemcpyAsync(v, mx, sizeof(v), cudaMemcpyDeviceToHost, s));
+  std::vector<uint32_t> os[2], od[2];
+  for (int sp = 0; sp < 2; ++sp) {
+    const SpinTables &T = sp == 0 ? p.A : p.B;
+    os[sp].resize(T.n + 1);
+    od[sp].resize(T.n + 1);
+    SBDGB_CUDA(cudaMemcpyAsync(os[sp].data(), T.off_s, sizeof(uint32_t) * (T.n + 1), cudaMemcpyDeviceToHost, s));
+    SBDGB_CUDA(cudaMemcpyAsync(od[sp].data(), T.off_d, sizeof(uint32_t) * (T.n + 1), cudaMemcpyDeviceToHost, s));
+  }
+  SBDGB_CUDA(cudaStreamSynchronize(s));
+  auto exponent = [](double x) {
+    int e = 0;
+    std::frexp(x, &e);
+    return e;
+  };
+  for (int i = 0; i < 7; ++i)
+    if (!(v[i] < 0x1p100)) return false;
+  std::vector<uint32_t> rows[2], ls[2], ld[2];
+  size_t bytes = 0;
+  for (int sp = 0; sp < 2; ++sp) {
+    const SpinTables &T = sp == 0 ? p.A : p.B;
+    p.slab.ev[sp] = std::max(-100, exponent(std::max(v[3 * sp] + v[3 * sp + 2], v[3 * sp + 1])));
+    auto ns = [&](uint32_t r) { return os[sp][r + 1] - os[sp][r]; };
+    auto nd = [&](uint32_t r) { return od[sp][r + 1] - od[sp][r]; };
+    rows[sp].resize((T.n + 31) / 32 * 32, ~0u);
+    std::iota(rows[sp].begin(), rows[sp].begin() + T.n, 0u);
+    std::stable_sort(rows[sp].begin(), rows[sp].begin() + T.n,
+                     [&](uint32_t x, uint32_t y) {  // lists of equal length in groups, then by singles
+                       const uint32_t gx = (nd(x) + kGroup - 1) / kGroup, gy = (nd(y) + kGroup - 1) / kGroup;
+                       return gx != gy ? gx > gy : ns(x) > ns(y);
+                     });
+    ls[sp].assign(1, 0u);
+    ld[sp].assign(1, 0u);
+    for (size_t b = 0; b < rows[sp].size(); b += 32) {
+      uint32_t ms = 0, md = 0;
+      for (size_t i = b; i < b + 32 && i < T.n; ++i) {
+        ms = std::max(ms, ns(rows[sp][i]));
+        md = std::max(md, nd(rows[sp][i]));
+        if (ns(rows[sp][i]) + nd(rows[sp][i]) > (uint32_t)fx::kMaxTerms) return false;
+      }
+      ls[sp].push_back(ls[sp].back() + (ms + kGroup - 1) / kGroup);
+      ld[sp].push_back(ld[sp].back() + (md + kGroup - 1) / kGroup);
+    }
+    if ((uint64_t)std::max(ls[sp].back(), ld[sp].back()) * 64u >= (1ull << 32)) return false;  // 32-bit group indices
+    bytes += 4 * rows[sp].size() + 8 * ls[sp].size() + 32ull * 12 * kGroup * (ls[sp].back() + ld[sp].back()) + 8ull * T.n;
+  }
+  for (uint32_t c = 0; ab && c < p.nb; ++c)  // two terms per beta single of a column
+    if (2 * (os[1][c + 1] - os[1][c]) > (uint32_t)fx::kMaxTerms) return false;
+  std::vector<void *> tmps;
+  p.slab.ek = std::max(-100, exponent(v[6]));
+  if (ab) bytes += 4 * p.ab_entries;
+  if (bytes > 8 * p.N + (1u << 20)) return false;
+  if (p.ctx->budget && p.ctx->in_use + bytes > p.ctx->budget) return false;
+  for (int sp = 0; sp < 2; ++sp) {
+    const SpinTables &T = sp == 0 ? p.A : p.B;
+    const size_t nrow = rows[sp].size(), nsl = ls[sp].size() - 1;
+    uint32_t *r = (uint32_t *)dev_alloc(p, 4 * nrow), *o = (uint32_t *)dev_alloc(p, 8 * (nsl + 1));
+    SBDGB_CUDA(cudaMemcpyAsync(r, rows[sp].data(), 4 * nrow, cudaMemcpyHostToDevice, s));
+    SBDGB_CUDA(cudaMemcpyAsync(o, ls[sp].data(), 4 * (nsl + 1), cudaMemcpyHostToDevice, s));
+    SBDGB_CUDA(cudaMemcpyAsync(o + nsl + 1, ld[sp].data(), 4 * (nsl + 1), cudaMemcpyHostToDevice, s));
+    p.slab.rows[sp] = r;
+    p.slab.off[sp] = o;
+    p.slab.nslices[sp] = (uint32_t)nsl;
+    p.slab.ent_s[sp] = (uint4 *)dev_alloc(p, 512ull * ls[sp].back());
+    p.slab.val_s[sp] = (int4 *)dev_alloc(p, 1024ull * ls[sp].back());
+    p.slab.ket_d[sp] = (uint4 *)dev_alloc(p, 512ull * ld[sp].back());
+    p.slab.val_d[sp] = (int4 *)dev_alloc(p, 1024ull * ld[sp].back());
+    p.slab.mask[sp] = (uint64_t *)dev_alloc(p, 8ull * T.n);
+    // the order of the entries (two scratch words each)
+    uint32_t *tmp = (uint32_t *)tmp_alloc(p.ctx, 8ull * (T.ns + T.nd));
+    uint32_t *order_s = tmp, *order_d = order_s + T.ns, *next = order_d + T.nd;
+    k_slab_order<<<(unsigned)nsl, 32, 0, s>>>(T.off_s, T.ket_s, r, next, order_s);
+    k_slab_order<<<(unsigned)nsl, 32, 0, s>>>(T.off_d, T.ket_d, r, next, order_d);
+    k_slab_fill<<<(unsigned)nsl, 128, 0, s>>>(T, r, o, o + nsl + 1, order_s, order_d, p.npair, p.slab.ev[sp],
+                                              p.slab.ent_s[sp], p.slab.val_s[sp], p.slab.ket_d[sp], p.slab.val_d[sp]);
+    tmps.push_back(tmp);
+    k_slab_masks<<<(T.n + 127) / 128, 128, 0, s>>>(sp == 0 ? p.astr : p.bstr, T.n, sp, p.slab.mask[sp]);
+    count_launch(p.ctx, 4);
+  }
+  if (ab) {
+    p.slab.ab_ent = (uint32_t *)dev_alloc(p, 4 * p.ab_entries);
+    SBDGB_CUDA(cudaMemcpyAsync(p.slab.ab_ent, p.ab_ent, 4 * p.ab_entries, cudaMemcpyDeviceToDevice, s));
+    k_slab_ab_order<<<p.n_ab_slices, 32, 0, s>>>(p.ab_slice, (uint32_t)p.npair << 1, p.slab.ab_ent);
+    count_launch(p.ctx);
+  }
+  SBDGB_CUDA(cudaGetLastError());
+  SBDGB_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
+  for (void *t : tmps) tmp_free(p.ctx, t);
+  p.slab.state = 1;
+  return true;
+}
+
+namespace {
+
+template <bool kAlpha>
+void launch_slab(const Problem &p, const double *C, double *S, int add, int diag, int eta, cudaStream_t s) {
+  constexpr int sp = kAlpha ? 0 : 1;
+  const SpinTables &T = kAlpha ? p.A : p.B;
+  SlabArgs a{};
+  a.C = C;
+  a.S = S;
+  a.hii = p.hii;
+  a.tables = T;
+  a.t.rows = p.slab.rows[sp];
+  a.t.off_s = p.slab.off[sp];
+  a.t.off_d = p.slab.off[sp] + p.slab.nslices[sp] + 1;
+  a.t.ent_s = p.slab.ent_s[sp];
+  a.t.val_s = p.slab.val_s[sp];
+  a.t.ket_d = p.slab.ket_d[sp];
+  a.t.val_d = p.slab.val_d[sp];
+  a.t.nslices = p.slab.nslices[sp];
+  a.Jo = kAlpha ? p.Jb : p.Ja;
+  a.rowstr = kAlpha ? p.astr : p.bstr;
+  a.colmask = p.slab.mask[1 - sp];
+  a.n = kAlpha ? p.na : p.nb;
+  a.m = kAlpha ? p.nb : p.na;
+  a.nb = p.nb;
+  a.npair = T.ns ? p.npair : 0;
+  a.ev = p.slab.ev[sp];
+  a.eta = eta;
+  a.add = add;
+  a.diag = diag;
+  // Columns a CTA: the most that fit in shared memory (fewer table reads per
+  // term), halved while the (column group, slice) pairs would not fill the
+  // warps that 80 registers a thread allow (24 an SM).  Warps a CTA: 8 where
+  // three CTAs fit an SM (small CTAs even out better), 12 where two do, else
+  // 24.  A group's slices are shared by several CTAs, each staging the group,
+  // while there are fewer than three CTAs for each that is resident.
+  const size_t limit = max_smem();
+  int sms = 0;
+  SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
+  int K = 4;
+  while (K > 1 && (slab_smem_bytes(K, a.n, a.npair) > limit ||
+                   (uint64_t)((a.m + K - 1) / K) * a.t.nslices < 36ull * sms))
+    K >>= 1;
+  const uint32_t groups = (a.m + K - 1) / K;
+  const size_t smem = slab_smem_bytes(K, a.n, a.npair);
+  const uint32_t resident = smem <= limit / 3 ? 3 : smem <= limit / 2 ? 2 : 1;
+  uint32_t warps = kSlabThreads / 32 / resident;
+  a.parts = 1;
+  if (groups < 3 * resident * sms)
+    a.parts = std::min((a.t.nslices + warps - 1) / warps, (3 * resident * sms + groups - 1) / groups);
+  warps = std::max<uint32_t>(2, std::min(warps, (a.t.nslices + a.parts - 1) / a.parts));
+  a.staged_diag = diag && !kAlpha && a.parts == 1;
+  const dim3 g(groups, a.parts);
+  auto go = [&](auto k) {
+    ensure_dynamic_smem((const void *)k, smem);
+    prefer_shared_carveout((const void *)k);
+    k<<<g, warps * 32, smem, s>>>(a);
+  };
+  switch (K) {
+    case 4: go(k_slab<4, kAlpha>); break;
+    case 2: go(k_slab<2, kAlpha>); break;
+    default: go(k_slab<1, kAlpha>); break;
+  }
+  count_launch(p.ctx);
+  SBDGB_CUDA(cudaGetLastError());
+}
+
+}  // namespace
+
+// One FP64 product (slab_prepare has returned true): no allocation and no
+// scratch, so products of one problem may overlap on several streams.
+void sigma_slab(const Problem &p, const double *C, double *S, int accumulate, cudaStream_t s, bool block) {
+  const int eta = block ? 0 : 1;
+  const bool beta = p.B.ns + p.B.nd > 0;
+  if (beta) launch_slab<false>(p, C, S, accumulate, 1, eta, s);
+  if (!beta || p.A.ns + p.A.nd > 0) launch_slab<true>(p, C, S, accumulate || beta, !beta, eta, s);
+  if (p.A.ns > 0 && p.B.ns > 0) {
+    SlabAbArgs a{};
+    a.C = C;
+    a.S = S;
+    a.astr = p.astr;
+    a.colmask = p.slab.mask[1];
+    a.off = p.A.off_s;
+    a.ket = p.A.ket_s;
+    a.code = p.A.code_s;
+    a.Kp = p.Kp;
+    a.rows = p.ab_rows;
+    a.cols = p.ab_cols;
+    a.slice = p.ab_slice;
+    a.ent = p.slab.ab_ent;
+    a.nslices = p.n_ab_slices;
+    a.nb = p.nb;
+    a.npair = p.npair;
+    a.ek = p.slab.ek;
+    a.eta = eta;
+    int sms = 0;
+    SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
+    // few rows: the columns of a row are shared by several CTAs
+    const uint32_t parts = std::min(a.nslices, std::max<uint32_t>(1, 4u * sms / p.n_ab_rows));
+    const uint32_t mine = (a.nslices + parts - 1) / parts, rounds = (mine + kSlabAbThreads / 32 - 1) / (kSlabAbThreads / 32);
+    const uint32_t warps = std::max<uint32_t>(4, (mine + rounds - 1) / rounds);
+    auto go = [&](auto k, size_t smem) {
+      ensure_dynamic_smem((const void *)k, smem);
+      prefer_shared_carveout((const void *)k);
+      k<<<dim3(p.n_ab_rows, parts), warps * 32, smem, s>>>(a);
+    };
+    if (!slab_ab_fixed(p))
+      go(k_slab_ab<2, false, false>, slab_ab_smem_bytes(p, 2, false));
+    else if (slab_ab_smem_bytes(p, 4, true) <= max_smem() / 2)
+      go(k_slab_ab<4, true, true>, slab_ab_smem_bytes(p, 4, true));
+    else
+      go(k_slab_ab<2, true, true>, slab_ab_smem_bytes(p, 2, true));
+    count_launch(p.ctx);
+    SBDGB_CUDA(cudaGetLastError());
+  }
+}
+
+}  // namespace sbdgb

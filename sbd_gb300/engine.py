@@ -316,9 +316,11 @@ class TPBProblem:
         self.engine.check(self.lib.sbdgb_problem_tuning(self.h, precision, C.byref(a), C.byref(b), ma, mb, 4))
         mf, ms, mt = (C.c_float * 4)(), (C.c_float * 2)(), (C.c_float * 2)()
         self.engine.check(self.lib.sbdgb_problem_tuning_times(self.h, precision, mf, ms, mt))
-        shapes = ["8x128", "8x256", "8x512", "16x256", "fused", "sparse", "stream"]
+        shapes = ["8x128", "8x256", "8x512", "16x256", "fused", "sparse", "stream", "slab"]
         alpha = shapes[a.value] if a.value >= 0 else None
-        if b.value >= 5:
+        if b.value == 7:
+            alpha = "slab"
+        elif b.value >= 5:
             alpha = ["8 rows", "16 rows"][a.value]
         return {"alpha_shape": alpha, "beta_shape": shapes[b.value] if b.value >= 0 else None,
                 "alpha_ms": [round(x, 4) for x in ma], "beta_ms": [round(x, 4) for x in mb],

@@ -1,0 +1,109 @@
+"""The fixed-point sigma kernels (sigma_slab.cu), which the engine takes by itself
+for FP64 products of problems with more than 8 nonzeros a row: edges of their
+slices of 32 rows, groups of 1, 2 and 4 columns and batches of ket rows, and the
+vectors that fixed point cannot hold.
+
+Tolerance: an element's error is at most 2^-55 times the number of its terms
+times the largest |v| and |x| of its sums (below 2^-46 of the largest sigma for
+the shapes here), plus a few FP64 roundings; 1e-13 of the largest sigma bounds
+both.
+"""
+import numpy as np
+import pytest
+
+from golden_io import max_rel
+from oracle.oracle import Oracle
+from sbd_gb300.engine import TPBProblem
+from sbd_gb300.generators import make_problem
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+SLAB = "slab"
+
+
+def _sigma(p, c, base=None):
+    s = torch.full_like(c, float("nan")) if base is None else base.clone()
+    p.sigma_device(c.data_ptr(), s.data_ptr(), accumulate=base is not None,
+                   stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return s
+
+
+def _problem(engine, *args, **kw):
+    prob = make_problem(*args, **kw)
+    p = TPBProblem.from_problem(engine, prob)
+    p.diag_terms()
+    return prob, p
+
+
+# (norb, na, nb, occupied): one slice and one column group, a slice's edges, odd
+# lengths on either side, two and four columns a group, one and both spins with
+# few electrons; the last has under 8 alpha x beta pairs a determinant (FP64
+# multiply-adds there), the one before it more than a batch of ket rows holds
+SHAPES = [(10, 31, 1, 2), (8, 28, 28, 2), (10, 33, 32, 3), (12, 32, 97, 4), (12, 495, 70, 4), (12, 100, 495, 4),
+          (16, 801, 799, 5), (16, 1500, 1237, 5), (24, 700, 733, 8), (36, 1401, 1333, 12)]
+
+
+@pytest.mark.parametrize("norb,na,nb,nocc", SHAPES)
+def test_products_against_oracle(engine, norb, na, nb, nocc):
+    prob, p = _problem(engine, norb, nocc, nocc, na, nb, seed=na + nb)
+    rng = np.random.default_rng(na)
+    # a weight for each string over six orders of magnitude, as in a solution
+    C = rng.normal(size=(na, nb)) * 10.0 ** rng.uniform(-3, 0, (na, 1)) * 10.0 ** rng.uniform(-3, 0, (1, nb))
+    ref = Oracle.from_problem(prob).mult(C.ravel())
+    c = torch.tensor(C.ravel(), device="cuda")
+    s = _sigma(p, c)
+    assert p.tuning(0)["beta_shape"] == SLAB
+    assert max_rel(s.cpu().numpy(), ref) <= 1e-13
+    assert torch.equal(_sigma(p, c), s)  # the same bits every time
+    base = torch.tensor(rng.uniform(-1, 1, C.size), device="cuda")
+    assert max_rel((_sigma(p, c, base) - base).cpu().numpy(), ref) <= 1e-13 * (1 + 1 / np.abs(ref).max())
+    p.close()
+
+
+@pytest.mark.parametrize("norb,na,nb,nocc", [(8, 28, 28, 2), (16, 801, 799, 5), (36, 1401, 1333, 12)])
+def test_vectors_out_of_range(engine, norb, na, nb, nocc):
+    """Infinities and NaN reach the same elements as in the FP64 kernels, and the
+    others are as without them; zero, tiny and huge vectors keep their scale."""
+    prob, p = _problem(engine, norb, nocc, nocc, na, nb, seed=5)
+    q = TPBProblem.from_problem(engine, prob)
+    q.diag_terms()
+    q.set_tuning(0, 1, 1)  # the FP64 sweeps
+    rng = np.random.default_rng(1)
+    x = torch.tensor(rng.uniform(-1, 1, prob.ndet), device="cuda")
+    _sigma(p, x)
+    assert p.tuning(0)["beta_shape"] == SLAB
+    for where in ([0], [prob.ndet // 2, 7], [prob.ndet - 1]):
+        for v in (float("nan"), float("inf"), -float("inf"), 1e305):
+            y = x.clone()
+            y[where] = v
+            s, r = _sigma(p, y), _sigma(q, y)
+            assert torch.equal(torch.isnan(s), torch.isnan(r)) and torch.equal(torch.isinf(s), torch.isinf(r))
+            ok = torch.isfinite(r)
+            assert torch.equal(s[~ok & ~torch.isnan(r)], r[~ok & ~torch.isnan(r)])
+            for part in (ok, ok & (r.abs() < 1e10)):
+                assert max_rel(s[part].cpu().numpy(), r[part].cpu().numpy()) <= 1e-13
+    assert not _sigma(p, torch.zeros_like(x)).any()
+    for scale in (1e-300, 1e-200, 1e200):
+        assert max_rel((_sigma(p, x * scale) / scale).cpu().numpy(), _sigma(q, x).cpu().numpy()) <= 1e-13
+    y = x.clone()  # a row and a column far from the others
+    y.reshape(na, nb)[na // 3] *= 1e-290
+    y.reshape(na, nb)[:, nb // 3] = 0.0
+    assert max_rel(_sigma(p, y).cpu().numpy(), _sigma(q, y).cpu().numpy()) <= 1e-13
+    p.close()
+    q.close()
+
+
+def test_solver_products_and_fp64_sweeps_agree(engine):
+    """The block-ordering product (the solvers') through a solve: energies as from
+    the FP64 sweeps."""
+    prob, p = _problem(engine, 16, 5, 5, 300, 280, seed=11)
+    q = TPBProblem.from_problem(engine, prob)
+    q.set_tuning(3, 1, 1)
+    kw = dict(nroots=2, max_nb=16, eps=1e-9, max_it=40, init=1, want_vectors=False)
+    a, b = p.davidson(**kw), q.davidson(**kw)
+    assert p.tuning(3)["beta_shape"] == SLAB and q.tuning(3)["beta_shape"] != SLAB
+    assert a.report["converged"] and np.abs(a.energies - b.energies).max() <= 1e-10
+    p.close()
+    q.close()
