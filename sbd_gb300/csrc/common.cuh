@@ -181,9 +181,13 @@ struct Problem {
     uint32_t *rows[2] = {}, *off[2] = {};
     uint4 *ent_s[2] = {}, *ket_d[2] = {};
     int4 *val_s[2] = {}, *val_d[2] = {};
+    float4 *valf_s[2] = {}, *valf_d[2] = {};
     uint64_t *mask[2] = {};
     uint32_t *ab_ent = nullptr;  // the beta singles of ab_ent below, in this kernel's order
-    uint32_t nslices[2] = {};
+    uint2 *ab_items = nullptr;   // its CTAs: (alpha row, part | parts << 16), most batches first
+    uint32_t n_ab_items = 0, ab_warps = 0;
+    int2 *Jfx[2] = {};
+    uint32_t nslices[2] = {}, groups[2] = {}, longest[2] = {};
     int ev[2] = {}, ek = 0;
   } slab;
   size_t bytes = 0;
@@ -273,10 +277,8 @@ void build_row_pairs(Problem &p, const std::vector<uint32_t> &off_s, const std::
                      const std::vector<uint32_t> &rows, cudaStream_t s);
 template <typename T>
 bool rows_fit(const Problem &p);
-// sigma_slab.cu: the FP64 product in fixed point, where slab_prepare (which
-// builds its tables on first use) says that it applies.
+// sigma_slab.cu: whether its kernels apply (their tables are built on first use).
 bool slab_prepare(Problem &p, cudaStream_t s);
-void sigma_slab(const Problem &p, const double *C, double *S, int accumulate, cudaStream_t s, bool block);
 // block: the block-ordering product (H_block = eta H eta, no opposite-spin
 // parities) that the solvers use on eta-signed vectors; false: the
 // reference's interleaved convention.

@@ -19,6 +19,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#ifdef __CUDACC__
+#include "df.cuh"
+#endif
+
 namespace sbdgb {
 namespace fx {
 
@@ -74,6 +78,21 @@ __device__ __forceinline__ int2 vector_parts(uint32_t lo, uint32_t hi, int ex) {
   return make_int2((h ^ s) - s, (l ^ s) - s);
 }
 
+#ifdef __CUDACC__
+// A double-float's, from the bits of hi and lo: their integers on the sum's
+// scale, added (|hi| + |lo| < 2^ex).
+__device__ __forceinline__ int2 vector_parts_df(uint32_t lo, uint32_t hi, int ex) {
+  auto fixed = [&](uint32_t b) {
+    const int e = (int)(b >> 23) & 0xff;
+    const unsigned long long m = (unsigned long long)((b & 0x7fffffu) | (e ? 0x800000u : 0u)) << 32;
+    const int d = min(ex + 126 - max(e, 1), 62);  // 2^32 m: 56 bits, the last one below the unit, for e = ex + 126
+    const long long v = (long long)(m >> d);
+    return (int)b < 0 ? -v : v;
+  };
+  return split((fixed(hi) + fixed(lo) + 1) >> 1);
+}
+#endif
+
 // A sum: (m + hh 2^27 + top 2^59) 2^27.
 struct Acc {
   long long m, hh, top;
@@ -97,34 +116,68 @@ __device__ __forceinline__ void carry(Acc &a) {
   a.m &= (1ll << kLow) - 1;
   carry_high(a);
 }
-// Its value times 2^e, rounded to FP64 (after carry(); integer instructions
-// only: a conversion of a 64-bit integer costs an FP64 issue).
-constexpr int kUnit = kLow - kXBits - kVBits;  // e of a sum: ex + ev + kUnit
-__device__ __forceinline__ double value(const Acc &a, int e) {
+constexpr int kUnit = kLow - kXBits - kVBits;  // a sum's value is its integer times 2^(ex + ev + kUnit)
+
+// |a| (after carry()) with its leading one in bit 63, the rest cut off: the sign
+// in neg, that bit's exponent in top.  0 for a zero sum.
+__device__ __forceinline__ unsigned long long normalised(const Acc &a, bool &neg, int &top) {
   // 128-bit two's complement (hi, lo)
   unsigned long long lo =
       (unsigned long long)a.m | ((unsigned long long)a.hh << kLow) | ((unsigned long long)a.top << (kLow + 32));
   unsigned long long hi = (unsigned long long)(a.top >> (32 - kLow));
-  const bool neg = (long long)hi < 0;
+  neg = (long long)hi < 0;
   if (neg) {
     lo = ~lo + 1ull;
     hi = ~hi + (lo == 0ull ? 1ull : 0ull);
   }
-  int top = 127;  // exponent of the leading bit once normalised
+  top = 127;
   if (hi == 0ull) {
     hi = lo;
     lo = 0ull;
     top = 63;
   }
-  if (hi == 0ull) return 0.0;
+  if (hi == 0ull) return 0ull;
   const int lz = __clzll((long long)hi);
   top -= lz;
-  unsigned long long t = hi << lz;
-  if (lz) t |= lo >> (64 - lz);
+  return lz ? hi << lz | lo >> (64 - lz) : hi;
+}
+// A sum's value times 2^e, rounded to FP64 (integer instructions only: a
+// conversion of a 64-bit integer costs an FP64 issue).
+__device__ __forceinline__ double value(const Acc &a, int e) {
+  bool neg;
+  int top;
+  const unsigned long long t = normalised(a, neg, top);
+  if (t == 0ull) return 0.0;
   const unsigned long long mant = (t >> 11) + ((t >> 10) & 1ull);  // 53 bits, or 2^53 after rounding up
   const unsigned long long bits = ((unsigned long long)(1022 + top + e) << 52) + mant;
   return __longlong_as_double((long long)(bits | (neg ? 1ull << 63 : 0ull)));
 }
+#ifdef __CUDACC__
+// x 2^k in two steps, so that no factor leaves FP32's range where the result does not.
+__device__ __forceinline__ float scaled(float x, int k) {
+  k = max(-250, min(250, k));
+  const int h = k >> 1;
+  return x * __int_as_float((h + 127) << 23) * __int_as_float((k - h + 127) << 23);
+}
+// The same as a double-float: 24 bits in hi, the next 31 in lo.
+__device__ __forceinline__ dfloat value_df(const Acc &a, int e) {
+  bool neg;
+  int top;
+  const unsigned long long t = normalised(a, neg, top);
+  if (t == 0ull) return dfloat(0.f, 0.f);
+  int h = (int)(t >> 40), l = (int)((uint32_t)(t >> 8) >> 1);  // l: 31 bits below h's last
+  if (l >> 30) {  // nearest: lo may be negative
+    h += 1;
+    l = -(int)((1u << 31) - (uint32_t)l);
+  }
+  if (neg) {
+    h = -h;
+    l = -l;
+  }
+  const int k = top + e - 23;
+  return dfloat(scaled((float)h, k), scaled((float)l, k - 31));
+}
+#endif
 
 }  // namespace fx
 }  // namespace sbdgb

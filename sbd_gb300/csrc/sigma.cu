@@ -628,11 +628,12 @@ void launch_stream_or_sparse(const Problem &p, const Args<T> &a, int variant, cu
 // pairs and k_sigma_ab adds them afterwards.
 template <typename T, bool kB>
 void launch_shapes(Problem &p, const Args<T> &a, int sa, int sb, int split, cudaStream_t s) {
-  if constexpr (std::is_same<T, double>::value) {
-    if (sb == kSlabShape) {
-      sigma_slab(p, a.C, a.S, a.accumulate, s, kB);
-      return;
-    }
+  if (sb == kSlabShape) {
+    if constexpr (std::is_same<T, float>::value)
+      sigma_slab_f32(p, a, &a.C, &a.S, 1, kB, s);
+    else
+      sigma_slab<T>(p, a, kB, s);
+    return;
   }
   Args<T> b = a;
   b.skip_ab = split > 0 ? 1 : 0;
@@ -827,10 +828,23 @@ inline double nnz_per_row(const Problem &p) {
   return (p.na ? (double)(p.A.ns + p.A.nd) / p.na : 0.0) + (p.nb ? (double)(p.B.ns + p.B.nd) / p.nb : 0.0) + sa * sb;
 }
 
-// Nonzeros per row above which the fixed-point kernels are taken without
-// timing: below it a product is a stream through memory, which they pass over
-// twice.
-constexpr double kSlabPerRow = 8.0;
+// Whether the kernels of sigma_slab.cu are taken, without timing.  Below about
+// 14 nonzeros a row a product is a stream through memory, which they pass over
+// twice (us, FP64 and FP32, the timed shapes and slab: 961 x 290 strings, 8.6 a
+// row, 40 and 55, 28 and 49; 1580 x 890, 16.6, 126 and 111, 104 and 95).  With
+// few strings of one spin their CTAs are few or their staging serves few columns
+// (3517 x 108, 64 a row, 196 and 223; 3070 x 180, 58, FP32 116 and 130), which
+// 100 a row outweigh (1914 x 225, 207 a row, 610 and 274).  In the block
+// ordering the double-float sweeps are not bound by phases and win up to about
+// 100 (ms, sweeps and slab: 2011 x 1703, 58 a row, 0.47 and 0.53; 6000 x 6000,
+// 78, 3.9 and 4.5; 800 x 800, 605, 1.33 and 0.71).
+template <typename T, bool kB>
+bool slab_pays(const Problem &p) {
+  const double nnz = nnz_per_row(p);
+  if (nnz >= 100.0) return true;
+  if (kB && std::is_same<T, dfloat>::value) return false;
+  return nnz >= 14.0 && std::min(p.na, p.nb) >= 256;
+}
 
 // Alpha x beta single pairs per determinant above which the untimed choice
 // gives them their own kernel (k_sigma_ab stages rows per alpha single; with
@@ -841,13 +855,11 @@ template <typename T, bool kB>
 bool needs_tuning(Problem &p, cudaStream_t s) {
   const int prec = slot_of<T, kB>();
   if (p.tune_a[prec] >= 0 && p.tune_b[prec] >= 0) return false;
-  if constexpr (std::is_same<T, double>::value) {
-    if (nnz_per_row(p) > kSlabPerRow && slab_prepare(p, s)) {
-      p.tune_a[prec] = 0;
-      p.tune_b[prec] = kSlabShape;
-      p.split_ab[prec] = p.A.ns > 0 && p.B.ns > 0 ? 1 : 0;
-      return false;
-    }
+  if (slab_pays<T, kB>(p) && slab_prepare(p, s)) {
+    p.tune_a[prec] = 0;
+    p.tune_b[prec] = kSlabShape;
+    p.split_ab[prec] = p.A.ns > 0 && p.B.ns > 0 ? 1 : 0;
+    return false;
   }
   if (p.ctx->autotune) return true;
   p.split_ab[prec] =
@@ -1471,8 +1483,10 @@ void prepare_df(Problem &p, cudaStream_t s) {
 // the FP64 form with double-float values, products and sums.
 void sigma_df(Problem &p, const dfloat *C, dfloat *S, int accumulate, cudaStream_t s, double shift, bool block) {
   prepare_df(p, s);
-  if (!p.CT) p.CT = (double *)dev_alloc(p, sizeof(double) * p.N);  // the FP64 transpose scratch, same size
   if (p.N == 0) return;
+  const bool tuned = !(block ? needs_tuning<dfloat, true>(p, s) : needs_tuning<dfloat, false>(p, s));
+  if (!p.CT && (!tuned || needs_transpose(p.tune_b[block ? 5 : 2])))
+    p.CT = (double *)dev_alloc(p, sizeof(double) * p.N);  // the FP64 transpose scratch, same size
   Args<dfloat> a = base_args<dfloat>(p, C, S, accumulate);
   a.shift_df = dfloat(shift);
   dfloat *CT = reinterpret_cast<dfloat *>(p.CT);
@@ -1535,8 +1549,10 @@ Args<float> mixed_args(Problem &p, const float *C, float *S, double shift) {
 
 void sigma_mixed(Problem &p, const float *C, float *S, cudaStream_t s, double shift, bool block) {
   prepare_mixed(p, s);
-  if (!p.CTf) p.CTf = (float *)dev_alloc(p, sizeof(float) * p.N);
   if (p.N == 0) return;
+  const bool tuned = !(block ? needs_tuning<float, true>(p, s) : needs_tuning<float, false>(p, s));
+  if (!p.CTf && (!tuned || needs_transpose(p.tune_b[block ? 4 : 1])))
+    p.CTf = (float *)dev_alloc(p, sizeof(float) * p.N);
   const Args<float> a = mixed_args(p, C, S, shift);
   if (block)
     run_sigma<float, true>(p, a, p.CTf, s);
@@ -1561,6 +1577,11 @@ void sigma_mixed_multi_impl(Problem &p, const float *C, float *S, int nvec, cuda
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   begin_timing(p, s, ev0, ev1);
+  if (p.tune_b[ts] == kSlabShape) {
+    sigma_slab_f32(p, m.a, m.Cv, m.Sv, nvec, kB, s);
+    end_timing(p, s, ev0, ev1);
+    return;
+  }
   switch (nvec) {
     case 2: launch_mv<2, kB>(p, m, s); break;
     case 3: launch_mv<3, kB>(p, m, s); break;
@@ -1583,7 +1604,6 @@ void sigma_mixed_multi(Problem &p, const float *C, float *S, int nvec, cudaStrea
   }
   SBDGB_REQUIRE(nvec <= kMaxNV, SBDGB_E_UNSUPPORTED, "at most 4 vectors per multi-vector sigma");
   prepare_mixed(p, s);
-  if (!p.CTf) p.CTf = (float *)dev_alloc(p, sizeof(float) * p.N);
   if (p.N == 0) return;
   if (block)
     sigma_mixed_multi_impl<true>(p, C, S, nvec, s, shift);

@@ -300,4 +300,11 @@ void launch_ab(const Problem &p, const sdev::Args<T> &a, bool block, cudaStream_
 template <typename T, bool kB>
 void launch_stream(const Problem &p, const sdev::Args<T> &a, int variant, cudaStream_t s);
 
+// sigma_slab.cu: a product from shared memory in fixed point (T double or
+// dfloat), and of nvec <= 4 vectors in FP32 (x.C and x.S are not read).
+template <typename T>
+void sigma_slab(const Problem &p, const sdev::Args<T> &x, bool block, cudaStream_t s);
+void sigma_slab_f32(const Problem &p, const sdev::Args<float> &x, const float *const *C, float *const *S, int nvec,
+                    bool block, cudaStream_t s);
+
 }  // namespace sbdgb

@@ -28,9 +28,11 @@
 // lane in groups of four and padded to its longest (the sliced ELLPACK form)
 // with entries that point at a zero row.  The beta sweep stages K rows of C
 // (contiguous) and needs no transposed copy; the alpha sweep stages K columns
-// (32-byte pieces at K = 4).  The beta sweep runs first and writes the diagonal
-// while it stages; the sums are then added with one reduction per element and
-// launch (fire and forget, and in the order of the launches).
+// (32-byte pieces at K = 4).  The alpha sweep and the alpha x beta pairs come
+// first; the beta sweep adds the diagonal, the largest term, while it stages, so
+// that the others' sums are not rounded at its size, and its own sums with one
+// reduction per element (fire and forget; the order of an element's sum is that
+// of the launches).
 //
 // Phases.  Both sweeps and k_slab_ab work in the block ordering (no
 // opposite-spin parity; sigma_dev.cuh).  For the reference's interleaved
@@ -63,13 +65,69 @@ constexpr uint32_t kSlabMaxPair = 1u << 12;  // pair index bits
 
 // ---- the vector formats ----------------------------------------------------------
 
-// key: monotone in |x|, 0 for 0 only; key_exponent(key): |x| < 2^exponent (fx.cuh).
-__device__ __forceinline__ uint32_t key_of(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
-  return hi ? hi : (__double2loint(x) ? 1u : 0u);
+// key: monotone in |x|, 0 for 0 only; exponent(key): |x| < 2^exponent (fx.cuh).
+// Staged as they are, and after parts() in fixed point, both 8 bytes.
+template <typename T>
+struct Format;
+template <>
+struct Format<double> {
+  static __device__ __forceinline__ uint32_t key(double x) {
+    const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    return hi ? hi : (__double2loint(x) ? 1u : 0u);
+  }
+  static __device__ __forceinline__ int exponent(uint32_t key) { return fx::exponent_of(key, key != 0u); }
+  static __device__ __forceinline__ int2 raw(double x) { return make_int2(__double2loint(x), __double2hiint(x)); }
+  static __device__ __forceinline__ double fp64(int2 v) { return __hiloint2double(v.y, v.x); }
+  static __device__ __forceinline__ int2 parts(int2 v, int ex) {
+    return fx::vector_parts((uint32_t)v.x, (uint32_t)v.y, ex);
+  }
+  static __device__ __forceinline__ double value(const fx::Acc &a, int e) { return fx::value(a, e); }
+};
+template <>
+struct Format<dfloat> {
+  static __device__ __forceinline__ uint32_t key(dfloat x) {
+    return __float_as_uint(fabsf(x.hi) + fabsf(x.lo));  // a NaN is above every number
+  }
+  static __device__ __forceinline__ int exponent(uint32_t key) {
+    return key == 0u ? fx::kZero : key >= 0x7f800000u ? fx::kBad : (int)(key >> 23) - 126;
+  }
+  static __device__ __forceinline__ int2 raw(dfloat x) { return make_int2(__float_as_int(x.lo), __float_as_int(x.hi)); }
+  static __device__ __forceinline__ double fp64(int2 v) {
+    return (double)__int_as_float(v.y) + (double)__int_as_float(v.x);
+  }
+  static __device__ __forceinline__ int2 parts(int2 v, int ex) {
+    return fx::vector_parts_df((uint32_t)v.x, (uint32_t)v.y, ex);
+  }
+  static __device__ __forceinline__ dfloat value(const fx::Acc &a, int e) { return fx::value_df(a, e); }
+};
+
+// How a lane adds to sigma.  FP64: one reduction per element (each element once
+// per launch, so the order of the sum is that of the launches).  FP32 and
+// double-float: what sigma holds is loaded before the lists are summed, so that
+// the loads do not stall the end of a slice, and stored with the sum (no other
+// lane of the launch touches it).
+template <typename T>
+constexpr bool kReduce = std::is_same<T, double>::value;
+__device__ __forceinline__ void add_to(double *s, double, double x) { atomicAdd(s, x); }
+__device__ __forceinline__ void add_to(dfloat *s, dfloat old, dfloat x) { *s = old + x; }
+
+// The K (4 or 8: 32 bytes) neighbouring elements of one row in 16-byte pieces.
+template <int K, typename T>
+__device__ __forceinline__ void load_row(const T *p, T (&x)[K]) {
+  const uint4 *q = reinterpret_cast<const uint4 *>(p);
+  uint4 u[sizeof(T) * K / 16];
+#pragma unroll
+  for (size_t i = 0; i < sizeof(T) * K / 16; ++i) u[i] = q[i];
+  memcpy(x, u, sizeof(T) * K);
 }
-__device__ __forceinline__ int2 raw_bits(double x) { return make_int2(__double2loint(x), __double2hiint(x)); }
-__device__ __forceinline__ double raw_of(int2 v) { return __hiloint2double(v.y, v.x); }
+template <int K, typename T>
+__device__ __forceinline__ void store_row(T *p, const T (&x)[K]) {
+  uint4 u[sizeof(T) * K / 16];
+  memcpy(u, x, sizeof(T) * K);
+#pragma unroll
+  for (size_t i = 0; i < sizeof(T) * K / 16; ++i) reinterpret_cast<uint4 *>(p)[i] = u[i];
+}
+
 // ---- the sweep over one spin's pairs -----------------------------------------------
 
 struct SlabSpin {
@@ -82,13 +140,16 @@ struct SlabSpin {
   uint32_t nslices;
 };
 
+template <typename T>
 struct SlabArgs {
-  const double *C;
-  double *S;
-  const double *hii;
+  const T *C;
+  T *S;
+  const T *hii;  // the diagonal in the vectors' format
+  T shift;       // taken off the diagonal (0 in FP64)
   SlabSpin t;
   SpinTables tables;        // the same entries as the FP64 kernels read them
   const double *Jo;         // opposite-spin Coulomb table [npair][m]
+  const int2 *Jfx;          // the same in fixed point, or null: converted here
   const uint64_t *rowstr;   // this spin's strings
   const uint64_t *colmask;  // per column: the orbitals whose parity on rowstr is eta
   uint32_t n, m, nb;        // rows (this spin), columns (the other spin), row length of C and S
@@ -98,6 +159,7 @@ struct SlabArgs {
   int add;                  // what S holds is kept
   int diag;                 // the diagonal term is added here
   int staged_diag;          // ... while staging, so that S is complete but for this spin's sums
+  int vec;                  // rows of S start on 16-byte boundaries
   uint32_t parts;           // CTAs that share a column group (gridDim.y)
 };
 
@@ -110,17 +172,17 @@ __device__ __forceinline__ size_t staged(uint32_t rows, uint32_t r, int c) {
 
 // Row `row` summed in FP64 as the kernels of sigma.cu do, from the raw staged
 // values (a column that is not finite, or out of the fixed-point range).
-template <int K>
-__device__ __noinline__ double slab_row_fp64(const SpinTables &T, uint32_t row, const int2 *X, uint32_t n1,
+template <typename T, int K>
+__device__ __noinline__ double slab_row_fp64(const SpinTables &t, uint32_t row, const int2 *X, uint32_t n1,
                                              const double *Jo, uint32_t m, uint32_t col, int c) {
   double sum = 0.0;
-  for (uint32_t p = ldg(T.off_s + row); p < ldg(T.off_s + row + 1); ++p) {
-    const uint32_t code = ldg(T.code_s + p);
-    const double v = ldg(T.val_s + p) + ldg(Jo + (size_t)((code >> 16) & 0x7fffu) * m + col);
-    sum = fma(flip(v, code >> 31), raw_of(X[staged<K>(n1, ldg(T.ket_s + p), c)]), sum);
+  for (uint32_t p = ldg(t.off_s + row); p < ldg(t.off_s + row + 1); ++p) {
+    const uint32_t code = ldg(t.code_s + p);
+    const double v = ldg(t.val_s + p) + ldg(Jo + (size_t)((code >> 16) & 0x7fffu) * m + col);
+    sum = fma(flip(v, code >> 31), Format<T>::fp64(X[staged<K>(n1, ldg(t.ket_s + p), c)]), sum);
   }
-  for (uint32_t p = ldg(T.off_d + row); p < ldg(T.off_d + row + 1); ++p)
-    sum = fma(ldg(T.val_d + p), raw_of(X[staged<K>(n1, ldg(T.ket_d + p), c)]), sum);
+  for (uint32_t p = ldg(t.off_d + row); p < ldg(t.off_d + row + 1); ++p)
+    sum = fma(ldg(t.val_d + p), Format<T>::fp64(X[staged<K>(n1, ldg(t.ket_d + p), c)]), sum);
   return sum;
 }
 
@@ -203,8 +265,9 @@ __device__ __forceinline__ void slab_list(fx::Acc (&acc)[K], const uint4 *__rest
   for (int c = 0; c < K; ++c) fx::carry(acc[c]);
 }
 
-template <int K, bool kAlpha>
-__global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
+template <typename T, int K, bool kAlpha>
+__global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
+  using F = Format<T>;
   constexpr int NQ = (K + 1) / 2;
   extern __shared__ __align__(16) unsigned char slab_smem[];
   int2 *X = reinterpret_cast<int2 *>(slab_smem);     // (n + 1) x K; row n is zero (padding entries)
@@ -212,6 +275,12 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
   __shared__ uint32_t skey[K], snext;
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
   const uint32_t c0 = blockIdx.x * K;
+  auto diag = [&](size_t k) {
+    if constexpr (std::is_same<T, double>::value)
+      return ldg(a.hii + k);
+    else
+      return ldg(a.hii + k) - a.shift;
+  };
   if (tid < K) skey[tid] = 0u;
   if (tid == 0) snext = 0u;
   __syncthreads();
@@ -222,10 +291,10 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
     const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
     uint32_t key = 0u;
     for (uint32_t r = tid / K; r < a.n; r += nt / K) {
-      double x = ok ? ldg(a.C + (size_t)r * a.nb + (c0 + c)) : 0.0;
+      T x = ok ? ldg(a.C + (size_t)r * a.nb + (c0 + c)) : T(0.0);
       if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
-      key = max(key, key_of(x));
-      X[staged<K>(a.n + 1, r, c)] = raw_bits(x);
+      key = max(key, F::key(x));
+      X[staged<K>(a.n + 1, r, c)] = F::raw(x);
     }
     for (int o = 16; o >= K; o >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
     if (lane < (uint32_t)K) atomicMax(&skey[c], key);
@@ -234,18 +303,17 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
     for (int c = 0; c < K; ++c) {
       const bool ok = c0 + c < a.m;
       const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
-      const double *row = a.C + (size_t)(c0 + c) * a.nb;
+      const T *row = a.C + (size_t)(c0 + c) * a.nb;
       uint32_t key = 0u;
       for (uint32_t r = tid; r < a.n; r += nt) {
-        double x = ok ? ldg(row + r) : 0.0;
+        T x = ok ? ldg(row + r) : T(0.0);
         if (a.staged_diag && ok) {
           const size_t k = (size_t)(c0 + c) * a.nb + r;
-          const double d = ldg(a.hii + k) * x;
-          a.S[k] = a.add ? a.S[k] + d : d;
+          a.S[k] = a.add ? fma(diag(k), x, a.S[k]) : diag(k) * x;
         }
         if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
-        key = max(key, key_of(x));
-        X[staged<K>(a.n + 1, r, c)] = raw_bits(x);
+        key = max(key, F::key(x));
+        X[staged<K>(a.n + 1, r, c)] = F::raw(x);
       }
       key = __reduce_max_sync(0xffffffffu, key);
       if (lane == 0) atomicMax(&skey[c], key);
@@ -257,8 +325,10 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
       const uint32_t P = i / K;
       const int c = (int)(i % K);
       const bool ok = P < (uint32_t)a.npair && c0 + c < a.m;
-      J[staged<K>(a.npair + 1, P, c)] =
-          ok ? fx::make(ldg(a.Jo + (size_t)P * a.m + (c0 + c)), fx::kVBits - a.ev) : make_int2(0, 0);
+      const size_t from = (size_t)P * a.m + (c0 + c);
+      J[staged<K>(a.npair + 1, P, c)] = !ok       ? make_int2(0, 0)
+                                        : a.Jfx ? __ldg(a.Jfx + from)
+                                                : fx::make(ldg(a.Jo + from), fx::kVBits - a.ev);
     }
   }
   __syncthreads();
@@ -266,7 +336,7 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
   bool bad = false;
 #pragma unroll
   for (int c = 0; c < K; ++c) {
-    ex[c] = fx::exponent_of(skey[c], skey[c] != 0u);
+    ex[c] = F::exponent(skey[c]);
     bad = bad || ex[c] == fx::kBad;
   }
   if (!bad) {  // to fixed point, in place (an all-zero column has no scale and its sums are not read)
@@ -277,7 +347,7 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
       for (uint32_t i = tid; i < plane; i += nt) {
         const int e = K == 1 || !(i & 1u) ? ex[q * kw] : ex[q * kw + kw - 1];
         int2 &x = X[(size_t)q * plane + i];
-        if (e != fx::kZero) x = fx::vector_parts((uint32_t)x.x, (uint32_t)x.y, e);
+        if (e != fx::kZero) x = F::parts(x, e);
       }
     __syncthreads();
   }
@@ -288,7 +358,19 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
     sl = blockIdx.y + a.parts * __shfl_sync(0xffffffffu, sl, 0);
     if (sl >= t.nslices) break;
     const uint32_t row = ldg(t.rows + sl * 32u + lane);
-    double out[K];
+    auto element = [&](int c) { return kAlpha ? (size_t)row * a.nb + (c0 + c) : (size_t)(c0 + c) * a.nb + row; };
+    const bool add = a.add || a.staged_diag;
+    const bool whole = kAlpha && K == 4 && a.vec && c0 + K <= a.m && !(kReduce<T> && add);  // 16-byte pieces
+    T out[K], old[K];
+    if (!kReduce<T> && add && row != ~0u) {
+      if (whole) {
+        if constexpr (K == 4) load_row<K>(a.S + element(0), old);
+      } else {
+#pragma unroll
+        for (int c = 0; c < K; ++c)
+          if (c0 + c < a.m) old[c] = a.S[element(c)];
+      }
+    }
     if (!bad) {
       fx::Acc acc[K];
 #pragma unroll
@@ -300,73 +382,260 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs a) {
                           reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
 #pragma unroll
       for (int c = 0; c < K; ++c)
-        out[c] = ex[c] == fx::kZero ? 0.0 : fx::value(acc[c], ex[c] + a.ev + fx::kUnit);
+        out[c] = ex[c] == fx::kZero ? T(0.0) : F::value(acc[c], ex[c] + a.ev + fx::kUnit);
     } else {
 #pragma unroll
       for (int c = 0; c < K; ++c)
-        out[c] = row != ~0u && c0 + c < a.m ? slab_row_fp64<K>(a.tables, row, X, a.n + 1, a.Jo, a.m, c0 + c, c) : 0.0;
+        out[c] = row != ~0u && c0 + c < a.m
+                     ? T(slab_row_fp64<T, K>(a.tables, row, X, a.n + 1, a.Jo, a.m, c0 + c, c))
+                     : T(0.0);
     }
     if (row == ~0u) continue;
     const uint64_t str = a.eta ? ldg(a.rowstr + row) : 0ull;
 #pragma unroll
     for (int c = 0; c < K; ++c) {
       if (c0 + c >= a.m) break;
-      double s = out[c];
+      T s = out[c];
       if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c0 + c))));
-      const size_t k = kAlpha ? (size_t)row * a.nb + (c0 + c) : (size_t)(c0 + c) * a.nb + row;
-      if (a.diag && !a.staged_diag) s = fma(ldg(a.hii + k), ldg(a.C + k), s);
-      // one addition per element and launch: the order of the sum is that of the launches
-      if (a.add || a.staged_diag)
-        atomicAdd(a.S + k, s);
-      else
+      const size_t k = element(c);
+      if (a.diag && !a.staged_diag) s = fma(diag(k), ldg(a.C + k), s);
+      if (whole) {
+        out[c] = add ? old[c] + s : s;
+      } else if (add) {
+        add_to(a.S + k, old[c], s);
+      } else {
         a.S[k] = s;
+      }
     }
+    if (whole) {
+      if constexpr (K == 4) store_row<K>(a.S + element(0), out);
+    }
+  }
+}
+
+// ---- the same sweep in FP32 -------------------------------------------------------
+//
+// FP32 vectors and table values, FP32 products and list sums, the diagonal added
+// in float-float as in the kernels of sigma.cu.  Four columns of a row are 16
+// bytes.  Bound: the L1 data pipe (3 bytes of table and 4 of shared memory a
+// term at K = 8).  gridDim.z vectors at once.
+struct SlabArgsF {
+  const float *C[4];
+  float *S[4];
+  const dfloat *hii_df;  // the diagonal as hi + lo, less shift ...
+  const float *hii_f;    // ... or rounded to FP32 where there is no shift
+  dfloat shift;
+  SlabSpin t;
+  const float4 *val_s, *val_d;  // four entries' values
+  const float *Jo;
+  const uint64_t *rowstr, *colmask;
+  uint32_t n, m, nb;
+  int npair, eta, add, diag;
+  int vec;  // rows of S start on 16-byte boundaries
+  uint32_t parts;
+};
+
+template <int K, bool kSingles>
+__device__ __forceinline__ void slab_group_f32(float (&acc)[K], const uint4 &g, const float4 &v, const char *X,
+                                               uint32_t xplane, const char *J, uint32_t jplane) {
+  const uint32_t w[kGroup] = {g.x, g.y, g.z, g.w};
+  const float vs[kGroup] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int u = 0; u < kGroup; ++u) {
+    const uint32_t x16 = kSingles ? w[u] & 0x7fff0u : w[u], j16 = (w[u] >> 15) & 0xfff0u;
+#pragma unroll
+    for (int q = 0; q < K / 4; ++q) {
+      const float4 x = *reinterpret_cast<const float4 *>(X + q * xplane + x16);
+      if constexpr (kSingles) {
+        const float4 j = *reinterpret_cast<const float4 *>(J + q * jplane + j16);
+        acc[4 * q] = fmaf(vs[u] + flip(j.x, w[u] >> 31), x.x, acc[4 * q]);
+        acc[4 * q + 1] = fmaf(vs[u] + flip(j.y, w[u] >> 31), x.y, acc[4 * q + 1]);
+        acc[4 * q + 2] = fmaf(vs[u] + flip(j.z, w[u] >> 31), x.z, acc[4 * q + 2]);
+        acc[4 * q + 3] = fmaf(vs[u] + flip(j.w, w[u] >> 31), x.w, acc[4 * q + 3]);
+      } else {
+        acc[4 * q] = fmaf(vs[u], x.x, acc[4 * q]);
+        acc[4 * q + 1] = fmaf(vs[u], x.y, acc[4 * q + 1]);
+        acc[4 * q + 2] = fmaf(vs[u], x.z, acc[4 * q + 2]);
+        acc[4 * q + 3] = fmaf(vs[u], x.w, acc[4 * q + 3]);
+      }
+    }
+  }
+}
+
+template <int K, bool kSingles>
+__device__ __forceinline__ void slab_list_f32(float (&acc)[K], const uint4 *__restrict__ ent,
+                                              const float4 *__restrict__ val, uint32_t g, uint32_t end, uint32_t lane,
+                                              const char *X, uint32_t xplane, const char *J, uint32_t jplane) {
+  if (g >= end) return;
+  uint32_t at = g * 32u + lane, left = end - g;
+  uint4 wa = ldg(ent + at), wb;
+  float4 va = __ldg(val + at), vb;
+  while (true) {
+    if (left > 1) {
+      wb = ldg(ent + at + 32u);
+      vb = __ldg(val + at + 32u);
+    }
+    slab_group_f32<K, kSingles>(acc, wa, va, X, xplane, J, jplane);
+    if (left == 1) break;
+    if (left > 2) {
+      wa = ldg(ent + at + 64u);
+      va = __ldg(val + at + 64u);
+    }
+    slab_group_f32<K, kSingles>(acc, wb, vb, X, xplane, J, jplane);
+    if (left == 2) break;
+    left -= 2;
+    at += 64u;
+  }
+}
+
+template <int K, bool kAlpha>
+__global__ void __launch_bounds__(kSlabThreads) k_slab_f32(SlabArgsF a) {
+  extern __shared__ __align__(16) unsigned char slab_smem[];
+  float *X = reinterpret_cast<float *>(slab_smem);  // planes of four columns, n + 1 rows; row n is zero
+  float *J = X + (size_t)(a.n + 1) * K;             // the same, npair + 1 rows
+  __shared__ uint32_t snext;
+  const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
+  const uint32_t c0 = blockIdx.x * K;
+  const float *C = a.C[blockIdx.z];
+  float *S = a.S[blockIdx.z];
+  auto place = [](uint32_t rows, uint32_t r, uint32_t c) { return ((size_t)(c >> 2) * rows + r) * 4 + (c & 3u); };
+  if (tid == 0) snext = 0u;
+  if constexpr (kAlpha) {
+    const uint32_t c = tid % K;
+    const bool ok = c0 + c < a.m;
+    const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
+    for (uint32_t r = tid / K; r < a.n; r += nt / K) {
+      float x = ok ? ldg(C + (size_t)r * a.nb + (c0 + c)) : 0.f;
+      if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
+      X[place(a.n + 1, r, c)] = x;
+    }
+  } else {
+#pragma unroll
+    for (uint32_t c = 0; c < K; ++c) {
+      const bool ok = c0 + c < a.m;
+      const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
+      for (uint32_t r = tid; r < a.n; r += nt) {
+        float x = ok ? ldg(C + (size_t)(c0 + c) * a.nb + r) : 0.f;
+        if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
+        X[place(a.n + 1, r, c)] = x;
+      }
+    }
+  }
+  if (tid < K) X[place(a.n + 1, a.n, tid)] = 0.f;
+  if (a.npair)
+    for (uint32_t i = tid; i < (uint32_t)(a.npair + 1) * K; i += nt) {
+      const uint32_t P = i / K, c = i % K;
+      J[place(a.npair + 1, P, c)] =
+          P < (uint32_t)a.npair && c0 + c < a.m ? ldg(a.Jo + (size_t)P * a.m + (c0 + c)) : 0.f;
+    }
+  __syncthreads();
+  const SlabSpin &t = a.t;
+  const uint32_t xplane = 16u * (a.n + 1), jplane = 16u * (a.npair + 1);
+  while (true) {
+    uint32_t sl = 0;
+    if (lane == 0) sl = atomicAdd(&snext, 1u);
+    sl = blockIdx.y + a.parts * __shfl_sync(0xffffffffu, sl, 0);
+    if (sl >= t.nslices) break;
+    const uint32_t row = ldg(t.rows + sl * 32u + lane);
+    auto element = [&](int c) { return kAlpha ? (size_t)row * a.nb + (c0 + c) : (size_t)(c0 + c) * a.nb + row; };
+    const bool whole = kAlpha && a.vec && c0 + K <= a.m;  // this row's K elements in 16-byte pieces
+    float acc[K], old[K], hi[K];
+#pragma unroll
+    for (int c = 0; c < K; ++c) acc[c] = old[c] = hi[c] = 0.f;
+    if (row != ~0u) {  // what the end of the slice needs, requested now
+      if (a.add && whole && !a.diag) {
+        load_row<K>(S + element(0), old);
+      } else {
+#pragma unroll
+        for (int c = 0; c < K; ++c)
+          if (c0 + c < a.m) {
+            if (a.add) old[c] = S[element(c)];
+            if (a.diag && a.hii_f) hi[c] = ldg(a.hii_f + element(c));
+          }
+      }
+    }
+    slab_list_f32<K, true>(acc, t.ent_s, a.val_s, ldg(t.off_s + sl), ldg(t.off_s + sl + 1), lane,
+                           reinterpret_cast<const char *>(X), xplane, reinterpret_cast<const char *>(J), jplane);
+    slab_list_f32<K, false>(acc, t.ket_d, a.val_d, ldg(t.off_d + sl), ldg(t.off_d + sl + 1), lane,
+                            reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
+    if (row == ~0u) continue;
+    const uint64_t str = a.eta ? ldg(a.rowstr + row) : 0ull;
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      if (c0 + c >= a.m) break;
+      float s = acc[c];
+      if (a.diag) {  // eta sigma = h (eta C) + the sums
+        const float x = X[place(a.n + 1, row, c)];
+        FF d;
+        if (a.hii_f) {
+          d = ff_prod(hi[c], x);
+        } else {
+          const dfloat h = ldg(a.hii_df + element(c));
+          d = ff_diag(h.hi, h.lo, a.shift.hi, a.shift.lo, x);
+        }
+        ff_add(d, s);
+        if (a.eta) d = parity((unsigned long long)(str & ldg(a.colmask + c0 + c))) ? FF{-d.hi, -d.lo} : d;
+        if (a.add) ff_add(d, old[c]);
+        acc[c] = ff_value(d);
+      } else {
+        if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c0 + c))));
+        acc[c] = a.add ? old[c] + s : s;
+      }
+      if (!whole) S[element(c)] = acc[c];
+    }
+    if (whole) store_row<K>(S + element(0), acc);
   }
 }
 
 // ---- alpha single x beta single (task type 0) ---------------------------------------
 //
-// The layout of k_sigma_ab (sigma_ab.cu): a CTA owns one alpha row (with
-// gridDim.y > 1, every gridDim.y-th slice of its columns) and takes G of its
+// The layout of k_sigma_ab (sigma_ab.cu): a CTA owns one alpha row (or every
+// parts-th slice of its columns: rows with many more batches than most, whose
+// batches follow one another, would end the launch alone) and takes G of its
 // singles at a time, C rows and (P|Q) rows staged in shared memory; beta singles
 // in slices of 32 columns, their entries ordered against bank conflicts
 // (k_slab_ab_order).  Each (P|Q) value is staged with both signs, so that an
 // entry's phase is part of its index.
 //
-// kFixed: in fixed point.  The ket rows of a batch have scales of their own
-// (2^e_g); the batch's is the largest, and the (P|Q) values of a smaller row are
-// scaled down by the difference.  Otherwise FP64 multiply-adds on the values as
-// they are (few terms a column; slab_ab_fixed).
+// The ket rows of a batch have scales of their own (2^e_g); the batch's is the
+// largest, and the (P|Q) values of a smaller row are scaled down by the
+// difference.
 // kSum: the row's sums stay in shared memory until the last batch; otherwise
 // each batch's go to sigma at once (rows with a batch or two; less shared
 // memory, so more CTAs an SM).
 
+template <typename T>
 struct SlabAbArgs {
-  const double *C;
-  double *S;
+  const T *C;
+  T *S;
   const uint64_t *astr;
   const uint64_t *colmask;           // per beta string
   const uint32_t *off, *ket, *code;  // alpha singles
   const double *Kp;
-  const uint32_t *rows, *cols, *slice, *ent;
+  const uint2 *items;  // (alpha row, part | parts << 16)
+  const uint32_t *cols, *slice, *ent;
   uint32_t nslices, nb;
   int npair, ek, eta;
 };
 
-template <int G, bool kFixed, bool kSum>
-__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs a) {
+template <typename T, int G, bool kSum>
+__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
+  using F = Format<T>;
   constexpr int NP = G / 2;
   extern __shared__ __align__(16) unsigned char slab_smem[];
-  const uint32_t kplane = 2 * (a.npair + 1);
-  int4 *Cs = reinterpret_cast<int4 *>(slab_smem);                // [G/2][nb]: two ket rows' values at jb
-  int4 *Ks = Cs + (size_t)NP * a.nb;                             // [G/2][2 Q + phase]
+  const uint32_t kplane = 2 * (a.npair + 1), cplane = a.nb + 1;
+  const uint32_t pad = a.nb << 13 | (uint32_t)a.npair << 1;  // padding entries: a zero column and a zero pair
+  int4 *Cs = reinterpret_cast<int4 *>(slab_smem);                // [G/2][nb + 1]: two ket rows' values at jb
+  int4 *Ks = Cs + (size_t)NP * cplane;                           // [G/2][2 Q + phase]
   double *Ss = reinterpret_cast<double *>(Ks + NP * kplane);     // kSum: [nb]
   __shared__ uint32_t skey[G];
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
-  const uint32_t ia = ldg(a.rows + blockIdx.x);
+  const uint2 item = __ldg(a.items + blockIdx.x);
+  const uint32_t ia = item.x, part = item.y & 0xffffu, parts = item.y >> 16;
   const uint32_t p0 = ldg(a.off + ia), p1 = ldg(a.off + ia + 1);
   const uint64_t str = a.eta ? ldg(a.astr + ia) : 0ull;
-  const uint32_t parts = gridDim.y, mine = (a.nslices - blockIdx.y + parts - 1) / parts;  // slices of this CTA
+  const uint32_t mine = (a.nslices - part + parts - 1) / parts;  // slices of this CTA
+  if (tid < NP) Cs[tid * cplane + a.nb] = make_int4(0, 0, 0, 0);
   if (kSum)
     for (uint32_t c = tid; c < a.nb; c += nt) Ss[c] = 0.0;
   for (uint32_t pb = p0; pb < p1; pb += G) {
@@ -382,48 +651,43 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs a) {
       const bool ok0 = 2 * h < live, ok1 = 2 * h + 1 < live;
       const uint32_t ja0 = ok0 ? ldg(a.ket + pb + 2 * h) : 0u, ja1 = ok1 ? ldg(a.ket + pb + 2 * h + 1) : 0u;
       const uint64_t s0 = a.eta && ok0 ? ldg(a.astr + ja0) : 0ull, s1 = a.eta && ok1 ? ldg(a.astr + ja1) : 0ull;
-      const double *r0 = a.C + (size_t)ja0 * a.nb, *r1 = a.C + (size_t)ja1 * a.nb;
+      const T *r0 = a.C + (size_t)ja0 * a.nb, *r1 = a.C + (size_t)ja1 * a.nb;
       for (uint32_t c = tid; c < a.nb; c += nt) {
-        double x0 = ok0 ? ldg(r0 + c) : 0.0, x1 = ok1 ? ldg(r1 + c) : 0.0;
+        T x0 = ok0 ? ldg(r0 + c) : T(0.0), x1 = ok1 ? ldg(r1 + c) : T(0.0);
         if (a.eta) {
           const uint64_t m = ldg(a.colmask + c);
           x0 = flip(x0, parity((unsigned long long)(s0 & m)));
           x1 = flip(x1, parity((unsigned long long)(s1 & m)));
         }
-        if (kFixed) {
-          key[2 * h] = max(key[2 * h], key_of(x0));
-          key[2 * h + 1] = max(key[2 * h + 1], key_of(x1));
-        }
-        const int2 b0 = raw_bits(x0), b1 = raw_bits(x1);
-        Cs[h * a.nb + c] = make_int4(b0.x, b0.y, b1.x, b1.y);
+        key[2 * h] = max(key[2 * h], F::key(x0));
+        key[2 * h + 1] = max(key[2 * h + 1], F::key(x1));
+        const int2 b0 = F::raw(x0), b1 = F::raw(x1);
+        Cs[h * cplane + c] = make_int4(b0.x, b0.y, b1.x, b1.y);
       }
     }
     int e[G], es = fx::kZero;
-    bool fixed = kFixed;
-    if (kFixed) {
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        key[g] = __reduce_max_sync(0xffffffffu, key[g]);
-        if (lane == 0) atomicMax(&skey[g], key[g]);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        e[g] = fx::exponent_of(skey[g], skey[g] != 0u);
-        es = max(es, e[g]);
-      }
-      if (es == fx::kZero) continue;  // every row is zero
-      fixed = es != fx::kBad;
+    for (int g = 0; g < G; ++g) {
+      key[g] = __reduce_max_sync(0xffffffffu, key[g]);
+      if (lane == 0) atomicMax(&skey[g], key[g]);
     }
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      e[g] = F::exponent(skey[g]);
+      es = max(es, e[g]);
+    }
+    if (es == fx::kZero) continue;  // every row is zero
+    const bool fixed = es != fx::kBad;  // otherwise FP64 sums of the values as they are
     if (fixed) {  // to fixed point, in place: each thread the columns that it staged
 #pragma unroll
       for (int h = 0; h < NP; ++h)
         for (uint32_t c = tid; c < a.nb; c += nt) {
-          const int4 r = Cs[h * a.nb + c];
+          const int4 r = Cs[h * cplane + c];
           const int2 z = make_int2(0, 0);
-          const int2 x0 = e[2 * h] == fx::kZero ? z : fx::vector_parts((uint32_t)r.x, (uint32_t)r.y, e[2 * h]);
-          const int2 x1 = e[2 * h + 1] == fx::kZero ? z : fx::vector_parts((uint32_t)r.z, (uint32_t)r.w, e[2 * h + 1]);
-          Cs[h * a.nb + c] = make_int4(x0.x, x0.y, x1.x, x1.y);
+          const int2 x0 = e[2 * h] == fx::kZero ? z : F::parts(make_int2(r.x, r.y), e[2 * h]);
+          const int2 x1 = e[2 * h + 1] == fx::kZero ? z : F::parts(make_int2(r.z, r.w), e[2 * h + 1]);
+          Cs[h * cplane + c] = make_int4(x0.x, x0.y, x1.x, x1.y);
         }
     }
 #pragma unroll
@@ -443,10 +707,10 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs a) {
           n0 = make_int2(-f0.x, -f0.y);
           n1 = make_int2(-f1.x, -f1.y);
         } else {
-          f0 = raw_bits(v0);
-          f1 = raw_bits(v1);
-          n0 = raw_bits(-v0);
-          n1 = raw_bits(-v1);
+          f0 = Format<double>::raw(v0);
+          f1 = Format<double>::raw(v1);
+          n0 = Format<double>::raw(-v0);
+          n1 = Format<double>::raw(-v1);
         }
         Ks[h * kplane + 2 * Q] = make_int4(f0.x, f0.y, f1.x, f1.y);
         Ks[h * kplane + 2 * Q + 1] = make_int4(n0.x, n0.y, n1.x, n1.y);
@@ -457,17 +721,19 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs a) {
     for (uint32_t base = 0, round = 0; base < mine; base += nw, ++round) {
       const uint32_t i = base + ((round & 1u) ? nw - 1u - warp : warp);
       if (i >= mine) continue;
-      const uint32_t sl = blockIdx.y + parts * i, k = sl * 32u + lane;
+      const uint32_t sl = part + parts * i, k = sl * 32u + lane;
       uint32_t at = ldg(a.slice + sl) + lane;
       const uint32_t end = ldg(a.slice + sl + 1) + lane;
       if (at >= end) continue;
-      const uint32_t pad = (uint32_t)a.npair << 1;
       uint32_t w[kGroup];  // four entries; the next four are requested before these are summed
       auto load = [&](uint32_t from) {
 #pragma unroll
         for (int u = 0; u < kGroup; ++u) w[u] = from + 32u * u < end ? ldg(a.ent + from + 32u * u) : pad;
       };
       load(at);
+      const uint32_t ib = k < a.nb ? ldg(a.cols + k) : 0u;
+      T *const to = a.S + ((size_t)ia * a.nb + ib);
+      const T old = !kSum && !kReduce<T> && k < a.nb ? *to : T(0.0);
       double sum = 0.0;
       if (fixed) {
         fx::Acc acc;
@@ -482,7 +748,7 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs a) {
           for (int u = 0; u < kGroup; ++u)
 #pragma unroll
             for (int h = 0; h < NP; ++h) {
-              const int4 kv = Ks[h * kplane + (wc[u] & 0x1fffu)], cv = Cs[h * a.nb + (wc[u] >> 13)];
+              const int4 kv = Ks[h * kplane + (wc[u] & 0x1fffu)], cv = Cs[h * cplane + (wc[u] >> 13)];
               fx::mac(acc, cv.x, cv.y, kv.x, kv.y);
               fx::mac(acc, cv.z, cv.w, kv.z, kv.w);
             }
@@ -502,42 +768,153 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs a) {
           if (at + 32u * kGroup < end) load(at + 32u * kGroup);
 #pragma unroll
           for (int u = 0; u < kGroup; ++u) {
-            if ((wc[u] & 0x1ffeu) == pad) continue;  // padding (its C value may not be finite)
+            if (at + 32u * u >= end) break;  // the same for the whole warp
 #pragma unroll
             for (int h = 0; h < NP; ++h) {
-              const int4 kv = Ks[h * kplane + (wc[u] & 0x1fffu)], cv = Cs[h * a.nb + (wc[u] >> 13)];
-              sum = fma(raw_of(make_int2(kv.x, kv.y)), raw_of(make_int2(cv.x, cv.y)), sum);
-              if (2 * h + 1 < live) sum = fma(raw_of(make_int2(kv.z, kv.w)), raw_of(make_int2(cv.z, cv.w)), sum);
+              const int4 kv = Ks[h * kplane + (wc[u] & 0x1fffu)], cv = Cs[h * cplane + (wc[u] >> 13)];
+              sum = fma(Format<double>::fp64(make_int2(kv.x, kv.y)), F::fp64(make_int2(cv.x, cv.y)), sum);
+              if (2 * h + 1 < live)
+                sum = fma(Format<double>::fp64(make_int2(kv.z, kv.w)), F::fp64(make_int2(cv.z, cv.w)), sum);
             }
           }
         }
       }
       if (k >= a.nb) continue;
-      const uint32_t ib = ldg(a.cols + k);
       if (kSum) {
         Ss[ib] += sum;
       } else {
         if (a.eta) sum = flip(sum, parity((unsigned long long)(str & ldg(a.colmask + ib))));
-        atomicAdd(a.S + ((size_t)ia * a.nb + ib), sum);  // this thread's alone: batches add in their order
+        add_to(to, old, T(sum));  // this thread's alone: batches add in their order
       }
     }
   }
   if (!kSum) return;
+  auto add_row = [](T *at, double x) { *at = *at + T(x); };
   __syncthreads();
   if (parts == 1) {
     for (uint32_t c = tid; c < a.nb; c += nt) {
       double s = Ss[c];
       if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c))));
-      a.S[(size_t)ia * a.nb + c] += s;
+      add_row(a.S + ((size_t)ia * a.nb + c), s);
     }
   } else {
     for (uint32_t i = warp; i < mine; i += nw) {
-      const uint32_t k = (blockIdx.y + parts * i) * 32u + lane;
+      const uint32_t k = (part + parts * i) * 32u + lane;
       if (k >= a.nb) continue;
       const uint32_t ib = ldg(a.cols + k);
       double s = Ss[ib];
       if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + ib))));
-      a.S[(size_t)ia * a.nb + ib] += s;
+      add_row(a.S + ((size_t)ia * a.nb + ib), s);
+    }
+  }
+}
+
+// FP32: four ket rows' values at a column are 16 bytes, four (P|Q) rows' at a
+// pair too; the sums of a row stay in shared memory.
+struct SlabAbArgsF {
+  const float *C[4];
+  float *S[4];
+  const uint64_t *astr, *colmask;
+  const uint32_t *off, *ket, *code;
+  const float *Kp;
+  const uint2 *items;
+  const uint32_t *cols, *slice, *ent;
+  uint32_t nslices, nb;
+  int npair, eta;
+};
+
+__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab_f32(SlabAbArgsF a) {
+  extern __shared__ __align__(16) unsigned char slab_smem[];
+  float4 *Cs = reinterpret_cast<float4 *>(slab_smem);               // [nb + 1]
+  float4 *Ks = Cs + a.nb + 1;                                       // [2 Q + phase]
+  float *Ss = reinterpret_cast<float *>(Ks + 2 * (a.npair + 1));    // [nb]
+  const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
+  const float *C = a.C[blockIdx.z];
+  const uint2 item = __ldg(a.items + blockIdx.x);
+  const uint32_t ia = item.x, part = item.y & 0xffffu, parts = item.y >> 16;
+  const uint32_t p0 = ldg(a.off + ia), p1 = ldg(a.off + ia + 1);
+  const uint32_t mine = (a.nslices - part + parts - 1) / parts;
+  const uint32_t pad = a.nb << 13 | (uint32_t)a.npair << 1;
+  for (uint32_t c = tid; c < a.nb; c += nt) Ss[c] = 0.f;
+  if (tid == 0) Cs[a.nb] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t pb = p0; pb < p1; pb += 4) {
+    const float *r[4], *kr[4];
+    uint64_t str[4];
+    uint32_t sg[4];
+    bool ok[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      ok[g] = pb + g < p1;
+      const uint32_t ja = ok[g] ? ldg(a.ket + pb + g) : 0u, code = ok[g] ? ldg(a.code + pb + g) : 0u;
+      str[g] = a.eta && ok[g] ? ldg(a.astr + ja) : 0ull;
+      r[g] = C + (size_t)ja * a.nb;
+      kr[g] = a.Kp + (size_t)((code >> 16) & 0x7fffu) * a.npair;
+      sg[g] = code >> 31;
+    }
+    __syncthreads();  // the previous batch is applied
+    for (uint32_t c = tid; c < a.nb; c += nt) {
+      float x[4];
+      const uint64_t m = a.eta ? ldg(a.colmask + c) : 0ull;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        x[g] = ok[g] ? ldg(r[g] + c) : 0.f;
+        if (a.eta) x[g] = flip(x[g], parity((unsigned long long)(str[g] & m)));
+      }
+      Cs[c] = make_float4(x[0], x[1], x[2], x[3]);
+    }
+    for (uint32_t Q = tid; Q <= (uint32_t)a.npair; Q += nt) {
+      float v[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) v[g] = ok[g] && Q < (uint32_t)a.npair ? flip(ldg(kr[g] + Q), sg[g]) : 0.f;
+      Ks[2 * Q] = make_float4(v[0], v[1], v[2], v[3]);
+      Ks[2 * Q + 1] = make_float4(-v[0], -v[1], -v[2], -v[3]);
+    }
+    __syncthreads();
+    for (uint32_t base = 0, round = 0; base < mine; base += nw, ++round) {
+      const uint32_t i = base + ((round & 1u) ? nw - 1u - warp : warp);
+      if (i >= mine) continue;
+      const uint32_t sl = part + parts * i, k = sl * 32u + lane;
+      uint32_t at = ldg(a.slice + sl) + lane;
+      const uint32_t end = ldg(a.slice + sl + 1) + lane;
+      if (at >= end) continue;
+      uint32_t w[kGroup];
+      auto load = [&](uint32_t from) {
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) w[u] = from + 32u * u < end ? ldg(a.ent + from + 32u * u) : pad;
+      };
+      load(at);
+      float sum = 0.f;
+      for (; at < end; at += 32u * kGroup) {
+        uint32_t wc[kGroup];
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) wc[u] = w[u];
+        if (at + 32u * kGroup < end) load(at + 32u * kGroup);
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) {
+          const float4 kv = Ks[wc[u] & 0x1fffu], cv = Cs[wc[u] >> 13];
+          sum = fmaf(kv.x, cv.x, sum);
+          sum = fmaf(kv.y, cv.y, sum);
+          sum = fmaf(kv.z, cv.z, sum);
+          sum = fmaf(kv.w, cv.w, sum);
+        }
+      }
+      if (k < a.nb) Ss[ldg(a.cols + k)] += sum;
+    }
+  }
+  __syncthreads();
+  const uint64_t istr = a.eta ? ldg(a.astr + ia) : 0ull;
+  float *srow = a.S[blockIdx.z] + (size_t)ia * a.nb;
+  auto add = [&](uint32_t c) {
+    float s = Ss[c];
+    if (a.eta) s = flip(s, parity((unsigned long long)(istr & ldg(a.colmask + c))));
+    srow[c] += s;
+  };
+  if (parts == 1) {
+    for (uint32_t c = tid; c < a.nb; c += nt) add(c);
+  } else {
+    for (uint32_t i = warp; i < mine; i += nw) {
+      const uint32_t k = (part + parts * i) * 32u + lane;
+      if (k < a.nb) add(ldg(a.cols + k));
     }
   }
 }
@@ -628,13 +1005,14 @@ __global__ void __launch_bounds__(32) k_slab_order(const uint32_t *__restrict__ 
 // shared memory (column w >> 13, pair and phase w & 0x1fff): in its turn a lane
 // takes, of the next 16 entries of its list, the one that collides least with
 // the lanes before it (simulated for lists of 18-25: 1.85 wavefronts per 8
-// lanes and read, 2.6 in list order).  One warp per slice, in place; real
-// entries stay ahead of the padding.
-__global__ void __launch_bounds__(32) k_slab_ab_order(const uint32_t *__restrict__ slice, uint32_t pad,
+// lanes and read, 2.6 in list order).  One warp per slice, in place; the
+// padding, behind the real entries, is pointed at the zero column nb.
+__global__ void __launch_bounds__(32) k_slab_ab_order(const uint32_t *__restrict__ slice, uint32_t npair, uint32_t nb,
                                                       uint32_t *__restrict__ ent) {
   const uint32_t lane = threadIdx.x, e0 = slice[blockIdx.x] + lane, len = (slice[blockIdx.x + 1] - slice[blockIdx.x]) / 32u;
   uint32_t cnt = 0;
-  while (cnt < len && (ent[e0 + 32u * cnt] & 0x1ffeu) != pad) ++cnt;
+  while (cnt < len && (ent[e0 + 32u * cnt] & 0x1ffeu) != npair << 1) ++cnt;
+  for (uint32_t t = cnt; t < len; ++t) ent[e0 + 32u * t] = nb << 13 | npair << 1;
   const uint32_t group = lane & 24u;
   for (uint32_t t = 0; t < len; ++t) {
     uint32_t used = 0u;  // residues taken in this group of lanes: columns in bits 0-7, pairs in 8-15
@@ -671,7 +1049,8 @@ __global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t 
                                                    const uint32_t *__restrict__ order_s,
                                                    const uint32_t *__restrict__ order_d, int npair, int ev,
                                                    uint4 *__restrict__ ent_s, int4 *__restrict__ val_s,
-                                                   uint4 *__restrict__ ket_d, int4 *__restrict__ val_d) {
+                                                   uint4 *__restrict__ ket_d, int4 *__restrict__ val_d,
+                                                   float4 *__restrict__ valf_s, float4 *__restrict__ valf_d) {
   const uint32_t sl = blockIdx.x, lane = threadIdx.x & 31u, y = threadIdx.x >> 5;
   const uint32_t row = rows[sl * 32u + lane];
   for (int doubles = 0; doubles < 2; ++doubles) {
@@ -681,6 +1060,7 @@ __global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t 
     for (uint32_t g = off[sl] + y; g < off[sl + 1]; g += 4) {
       uint32_t w[kGroup];
       int2 v[kGroup];
+      float f[kGroup];
 #pragma unroll
       for (int u = 0; u < kGroup; ++u) {
         const uint32_t j = (g - off[sl]) * kGroup + u;
@@ -689,19 +1069,27 @@ __global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t 
         if (doubles) {
           w[u] = (ok ? T.ket_d[p] : T.n) << 4;
           v[u] = ok ? fx::make(T.val_d[p], fx::kVBits - ev) : make_int2(0, 0);
+          f[u] = ok ? (float)T.val_d[p] : 0.f;
         } else {
           const uint32_t code = ok ? T.code_s[p] : 0u;
           w[u] = ok ? (T.ket_s[p] << 4 | ((code >> 16) & 0x7fffu) << 19 | (code & 0x80000000u))
                     : (T.n << 4 | (uint32_t)npair << 19);
           v[u] = ok ? fx::make(flip(T.val_s[p], code >> 31), fx::kVBits - ev) : make_int2(0, 0);
+          f[u] = ok ? flip((float)T.val_s[p], code >> 31) : 0.f;
         }
       }
       const size_t e = (size_t)g * 32u + lane;
       (doubles ? ket_d : ent_s)[e] = make_uint4(w[0], w[1], w[2], w[3]);
       (doubles ? val_d : val_s)[2 * e] = make_int4(v[0].x, v[0].y, v[1].x, v[1].y);
       (doubles ? val_d : val_s)[2 * e + 1] = make_int4(v[2].x, v[2].y, v[3].x, v[3].y);
+      (doubles ? valf_d : valf_s)[e] = make_float4(f[0], f[1], f[2], f[3]);
     }
   }
+}
+
+__global__ void k_slab_coulomb(const double *__restrict__ J, size_t n, int s, int2 *__restrict__ out) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
+    out[e] = fx::make(J[e], s);
 }
 
 // Per string: the orbitals of the other spin's strings whose parity is eta
@@ -731,24 +1119,22 @@ size_t slab_smem_bytes(int K, uint32_t n, int npair) {
   return 8ull * K * ((size_t)n + 1 + (npair ? (size_t)npair + 1 : 0));
 }
 size_t slab_ab_smem_bytes(const Problem &p, int G, bool sum) {
-  return 8ull * G * ((size_t)p.nb + 2 * ((size_t)p.npair + 1)) + (sum ? 8ull * p.nb : 0);
+  return 8ull * G * ((size_t)p.nb + 1 + 2 * ((size_t)p.npair + 1)) + (sum ? 8ull * p.nb : 0);
+}
+size_t slab_ab_smem_bytes_f32(const Problem &p) {
+  return 16ull * ((size_t)p.nb + 1 + 2 * ((size_t)p.npair + 1)) + 4ull * p.nb;
 }
 
-// Whether the alpha x beta pairs are summed in fixed point too.  A batch of two
-// ket rows costs about 100 integer instructions a column to stage and to round
-// its sums; with few terms a column FP64 multiply-adds are cheaper.
-constexpr double kAbFixedPerElement = 8.0;
-bool slab_ab_fixed(const Problem &p) {
-  return (double)p.A.ns * (double)p.B.ns >= kAbFixedPerElement * (double)p.N;
-}
+// Whether a row's alpha x beta sums stay in shared memory between batches: not
+// where rows have a batch or two.
+bool slab_ab_sum(const Problem &p) { return (double)p.A.ns * (double)p.B.ns >= 8.0 * (double)p.N; }
 
 }  // namespace
 
 // ---- host side ----------------------------------------------------------------------
 
 // Builds the sliced tables on first use.  False where the kernels do not apply
-// or their tables would not fit the memory that the transposed copy (8 N
-// bytes, which they do without) is budgeted for.
+// or a budget has no room for their tables.
 bool slab_prepare(Problem &p, cudaStream_t s) {
   if (p.slab.state >= 0) return p.slab.state == 1;
   p.slab.state = 0;
@@ -757,7 +1143,7 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
   if (nmax >= kSlabMaxRows || (uint32_t)p.npair + 1 >= kSlabMaxPair) return false;
   if (slab_smem_bytes(1, nmax, p.npair) > limit) return false;
   const bool ab = p.A.ns > 0 && p.B.ns > 0;
-  if (ab && (p.n_ab_rows == 0 || slab_ab_smem_bytes(p, 2, slab_ab_fixed(p)) > limit)) return false;
+  if (ab && (p.n_ab_rows == 0 || slab_ab_smem_bytes(p, 2, slab_ab_sum(p)) > limit)) return false;
   // the largest table values
   unsigned long long *mx = (unsigned long long *)workspace(p, WS_RED2, 8 * sizeof(unsigned long long));
   SBDGB_CUDA(cudaMemsetAsync(mx, 0, 8 * sizeof(unsigned long long), s));
@@ -823,15 +1209,16 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
       ld[sp].push_back(ld[sp].back() + (md + kGroup - 1) / kGroup);
     }
     if ((uint64_t)std::max(ls[sp].back(), ld[sp].back()) * 64u >= (1ull << 32)) return false;  // 32-bit group indices
-    bytes += 4 * rows[sp].size() + 8 * ls[sp].size() + 32ull * 12 * kGroup * (ls[sp].back() + ld[sp].back()) + 8ull * T.n;
+    bytes += 4 * rows[sp].size() + 8 * ls[sp].size() + 32ull * 16 * kGroup * (ls[sp].back() + ld[sp].back()) + 8ull * T.n;
   }
   for (uint32_t c = 0; ab && c < p.nb; ++c)  // two terms per beta single of a column
     if (2 * (os[1][c + 1] - os[1][c]) > (uint32_t)fx::kMaxTerms) return false;
   std::vector<void *> tmps;
   p.slab.ek = std::max(-100, exponent(v[6]));
-  if (ab) bytes += 4 * p.ab_entries;
-  if (bytes > 8 * p.N + (1u << 20)) return false;
-  if (p.ctx->budget && p.ctx->in_use + bytes > p.ctx->budget) return false;
+  if (ab) bytes += 4 * p.ab_entries + 16 * p.na;
+  // under a budget: within what the transposed copy, which this form does
+  // without, is counted for
+  if (p.ctx->budget && (bytes > 8 * p.N + (1u << 20) || p.ctx->in_use + bytes > p.ctx->budget)) return false;
   for (int sp = 0; sp < 2; ++sp) {
     const SpinTables &T = sp == 0 ? p.A : p.B;
     const size_t nrow = rows[sp].size(), nsl = ls[sp].size() - 1;
@@ -842,26 +1229,66 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
     p.slab.rows[sp] = r;
     p.slab.off[sp] = o;
     p.slab.nslices[sp] = (uint32_t)nsl;
+    p.slab.groups[sp] = ls[sp].back() + ld[sp].back();
+    p.slab.longest[sp] = 0;
+    for (size_t i = 0; i < nsl; ++i)
+      p.slab.longest[sp] =
+          std::max(p.slab.longest[sp], kGroup * (ls[sp][i + 1] - ls[sp][i] + ld[sp][i + 1] - ld[sp][i]));
     p.slab.ent_s[sp] = (uint4 *)dev_alloc(p, 512ull * ls[sp].back());
     p.slab.val_s[sp] = (int4 *)dev_alloc(p, 1024ull * ls[sp].back());
     p.slab.ket_d[sp] = (uint4 *)dev_alloc(p, 512ull * ld[sp].back());
     p.slab.val_d[sp] = (int4 *)dev_alloc(p, 1024ull * ld[sp].back());
+    p.slab.valf_s[sp] = (float4 *)dev_alloc(p, 512ull * ls[sp].back());
+    p.slab.valf_d[sp] = (float4 *)dev_alloc(p, 512ull * ld[sp].back());
     p.slab.mask[sp] = (uint64_t *)dev_alloc(p, 8ull * T.n);
+    if (T.ns && !p.ctx->budget) {  // the Coulomb table this spin's singles read, where memory is not counted
+      const size_t nj = (size_t)p.npair * (sp == 0 ? p.nb : p.na);
+      p.slab.Jfx[sp] = (int2 *)dev_alloc(p, 8 * nj);
+      k_slab_coulomb<<<(unsigned)std::min<size_t>((nj + 255) / 256, 4096), 256, 0, s>>>(
+          sp == 0 ? p.Jb : p.Ja, nj, fx::kVBits - p.slab.ev[sp], p.slab.Jfx[sp]);
+      count_launch(p.ctx);
+    }
     // the order of the entries (two scratch words each)
     uint32_t *tmp = (uint32_t *)tmp_alloc(p.ctx, 8ull * (T.ns + T.nd));
     uint32_t *order_s = tmp, *order_d = order_s + T.ns, *next = order_d + T.nd;
     k_slab_order<<<(unsigned)nsl, 32, 0, s>>>(T.off_s, T.ket_s, r, next, order_s);
     k_slab_order<<<(unsigned)nsl, 32, 0, s>>>(T.off_d, T.ket_d, r, next, order_d);
     k_slab_fill<<<(unsigned)nsl, 128, 0, s>>>(T, r, o, o + nsl + 1, order_s, order_d, p.npair, p.slab.ev[sp],
-                                              p.slab.ent_s[sp], p.slab.val_s[sp], p.slab.ket_d[sp], p.slab.val_d[sp]);
+                                              p.slab.ent_s[sp], p.slab.val_s[sp], p.slab.ket_d[sp], p.slab.val_d[sp],
+                                              p.slab.valf_s[sp], p.slab.valf_d[sp]);
     tmps.push_back(tmp);
     k_slab_masks<<<(T.n + 127) / 128, 128, 0, s>>>(sp == 0 ? p.astr : p.bstr, T.n, sp, p.slab.mask[sp]);
     count_launch(p.ctx, 4);
   }
+  std::vector<uint2> items;
   if (ab) {
+    // CTAs of the alpha x beta kernels: a row is shared by `base` of them where
+    // rows are few, and (while the rows are only a few waves, which the longest
+    // would otherwise end alone) by more the further its batches exceed the mean:
+    // 2011 x 1703 strings 0.166 ms, here 0.152; with 6000 x 6000, where it only
+    // adds staging, 0.89 and 0.99
+    int sms = 0;
+    SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
+    const uint32_t base = std::min(p.n_ab_slices, std::max<uint32_t>(1, 4u * sms / p.n_ab_rows));
+    const double mean = (double)p.A.ns / p.n_ab_rows;
+    std::vector<uint32_t> order(p.na);
+    std::iota(order.begin(), order.end(), 0u);
+    auto singles = [&](uint32_t r) { return os[0][r + 1] - os[0][r]; };
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return singles(x) > singles(y); });
+    for (uint32_t r : order) {
+      if (singles(r) == 0) break;
+      const uint32_t parts = std::min<uint32_t>(p.n_ab_slices, base * (uint32_t)std::ceil(p.n_ab_rows < 12u * sms ? singles(r) / (4.0 * mean) : 1.0));
+      for (uint32_t y = 0; y < parts; ++y) items.push_back(make_uint2(r, y | parts << 16));
+    }
+    const uint32_t mine = (p.n_ab_slices + base - 1) / base;
+    const uint32_t rounds = (mine + kSlabAbThreads / 32 - 1) / (kSlabAbThreads / 32);
+    p.slab.ab_warps = std::max<uint32_t>(4, (mine + rounds - 1) / rounds);
+    p.slab.n_ab_items = (uint32_t)items.size();
+    p.slab.ab_items = (uint2 *)dev_alloc(p, 8 * items.size());
+    SBDGB_CUDA(cudaMemcpyAsync(p.slab.ab_items, items.data(), 8 * items.size(), cudaMemcpyHostToDevice, s));
     p.slab.ab_ent = (uint32_t *)dev_alloc(p, 4 * p.ab_entries);
     SBDGB_CUDA(cudaMemcpyAsync(p.slab.ab_ent, p.ab_ent, 4 * p.ab_entries, cudaMemcpyDeviceToDevice, s));
-    k_slab_ab_order<<<p.n_ab_slices, 32, 0, s>>>(p.ab_slice, (uint32_t)p.npair << 1, p.slab.ab_ent);
+    k_slab_ab_order<<<p.n_ab_slices, 32, 0, s>>>(p.ab_slice, (uint32_t)p.npair, p.nb, p.slab.ab_ent);
     count_launch(p.ctx);
   }
   SBDGB_CUDA(cudaGetLastError());
@@ -873,119 +1300,239 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
 
 namespace {
 
-template <bool kAlpha>
-void launch_slab(const Problem &p, const double *C, double *S, int add, int diag, int eta, cudaStream_t s) {
+// Columns a CTA (K), CTAs that share a column group and its staging (parts) and
+// warps a CTA, by the cycles of the busiest SM.  Warp instructions: about 1.1 per
+// staged element and 0.5 per staged Coulomb value (a column, a row), 10 + 4 K per
+// step of a slice (4 + 1.25 K in FP32), 70 (20) per column and slice at its end;
+// 1.6 of them a cycle.  A CTA lasts at least as long as its longest slice, at
+// about 120 cycles a step.  An SM holds 24 warps (80 registers a thread) in CTAs
+// of 8, 12 or 24.  (Beta sweep, ms, against one rule for the K that fits and as
+// many parts as fill three waves: 2011 x 1703 strings double-float 0.228, here
+// 0.203; FP32 0.157, 0.103.)
+struct SlabShape {
+  int K;
+  uint32_t groups, parts, warps;
+  size_t smem;
+};
+SlabShape slab_shape(const Problem &p, int sp, uint32_t n, uint32_t m, int npair, int element, int Kmax, int Kmin,
+                     int nvec) {
+  SlabShape best{};
+  const size_t limit = max_smem();
+  int sms = 0;
+  SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
+  const uint32_t nslices = p.slab.nslices[sp];
+  double cost = 0.0;
+  for (int K = Kmax; K >= Kmin; K >>= 1) {
+    const size_t smem = (size_t)element * K * ((size_t)n + 1 + (npair ? (size_t)npair + 1 : 0));
+    if (smem > limit && K > Kmin) continue;
+    const uint32_t groups = (m + K - 1) / K;
+    const uint32_t resident = smem <= limit / 3 ? 3 : smem <= limit / 2 ? 2 : 1, slots = resident * sms;
+    const double stage = (1.1 * n + 0.5 * npair) * K * (element == 8 ? 1.0 : 0.5);
+    const double work = 4.0 * p.slab.groups[sp] * (element == 8 ? 10.0 + 4.0 * K : 4.0 + 1.25 * K) +
+                        nslices * K * (element == 8 ? 70.0 : 20.0);
+    for (uint32_t parts = 1; parts <= std::min<uint32_t>(nslices, 16); ++parts) {
+      const uint32_t full = kSlabThreads / 32 / resident;
+      const uint32_t warps = std::max<uint32_t>(2, std::min(full, (nslices + parts - 1) / parts));
+      const uint32_t ctas = groups * parts * nvec, waves = (ctas + slots - 1) / slots;
+      // rounds: the slices of a part that its warps take one after another
+      const double rounds = (double)((nslices + parts - 1) / parts + warps - 1) / warps;
+      const double even = std::max(1.0, std::floor(rounds) * warps * parts / nslices);
+      // CTAs of the busiest SM at once; few of them leave it waiting on latency
+      const double live = std::min<double>(resident, (double)((ctas + sms - 1) / sms));
+      const double busy = std::min(1.0, live * warps / 12.0);
+      // (a shared group's diagonal is gathered at the end instead of streamed while staging)
+      const double c = (parts > 1 ? 1.2 : 1.0) * waves * std::max(live * (stage + work / parts * even) / (1.6 * busy),
+                                        stage / (0.4 * warps) + 120.0 * p.slab.longest[sp]);
+      if (best.K == 0 || c < 0.97 * cost) {
+        cost = c;
+        best = {K, groups, parts, warps, smem};
+      }
+    }
+  }
+  return best;
+}
+
+template <typename K, typename A>
+void go_slab(K k, const A &a, dim3 grid, uint32_t warps, size_t smem, cudaStream_t s) {
+  ensure_dynamic_smem((const void *)k, smem);
+  prefer_shared_carveout((const void *)k);
+  k<<<grid, warps * 32, smem, s>>>(a);
+}
+
+SlabSpin slab_spin(const Problem &p, int sp) {
+  SlabSpin t{};
+  t.rows = p.slab.rows[sp];
+  t.off_s = p.slab.off[sp];
+  t.off_d = p.slab.off[sp] + p.slab.nslices[sp] + 1;
+  t.ent_s = p.slab.ent_s[sp];
+  t.val_s = p.slab.val_s[sp];
+  t.ket_d = p.slab.ket_d[sp];
+  t.val_d = p.slab.val_d[sp];
+  t.nslices = p.slab.nslices[sp];
+  return t;
+}
+
+template <typename T, bool kAlpha>
+void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta, cudaStream_t s) {
   constexpr int sp = kAlpha ? 0 : 1;
-  const SpinTables &T = kAlpha ? p.A : p.B;
-  SlabArgs a{};
-  a.C = C;
-  a.S = S;
-  a.hii = p.hii;
-  a.tables = T;
-  a.t.rows = p.slab.rows[sp];
-  a.t.off_s = p.slab.off[sp];
-  a.t.off_d = p.slab.off[sp] + p.slab.nslices[sp] + 1;
-  a.t.ent_s = p.slab.ent_s[sp];
-  a.t.val_s = p.slab.val_s[sp];
-  a.t.ket_d = p.slab.ket_d[sp];
-  a.t.val_d = p.slab.val_d[sp];
-  a.t.nslices = p.slab.nslices[sp];
+  SlabArgs<T> a{};
+  a.C = x.C;
+  a.S = x.S;
+  if constexpr (std::is_same<T, double>::value) {
+    a.hii = x.hii;
+  } else {
+    a.hii = x.hii_df;
+    a.shift = x.shift_df;
+  }
+  a.tables = kAlpha ? p.A : p.B;
+  a.t = slab_spin(p, sp);
   a.Jo = kAlpha ? p.Jb : p.Ja;
+  a.Jfx = p.slab.Jfx[sp];
   a.rowstr = kAlpha ? p.astr : p.bstr;
   a.colmask = p.slab.mask[1 - sp];
   a.n = kAlpha ? p.na : p.nb;
   a.m = kAlpha ? p.nb : p.na;
   a.nb = p.nb;
-  a.npair = T.ns ? p.npair : 0;
+  a.npair = a.tables.ns ? p.npair : 0;
   a.ev = p.slab.ev[sp];
   a.eta = eta;
   a.add = add;
   a.diag = diag;
-  // Columns a CTA: the most that fit in shared memory (fewer table reads per
-  // term), halved while the (column group, slice) pairs would not fill the
-  // warps that 80 registers a thread allow (24 an SM).  Warps a CTA: 8 where
-  // three CTAs fit an SM (small CTAs even out better), 12 where two do, else
-  // 24.  A group's slices are shared by several CTAs, each staging the group,
-  // while there are fewer than three CTAs for each that is resident.
-  const size_t limit = max_smem();
-  int sms = 0;
-  SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
-  int K = 4;
-  while (K > 1 && (slab_smem_bytes(K, a.n, a.npair) > limit ||
-                   (uint64_t)((a.m + K - 1) / K) * a.t.nslices < 36ull * sms))
-    K >>= 1;
-  const uint32_t groups = (a.m + K - 1) / K;
-  const size_t smem = slab_smem_bytes(K, a.n, a.npair);
-  const uint32_t resident = smem <= limit / 3 ? 3 : smem <= limit / 2 ? 2 : 1;
-  uint32_t warps = kSlabThreads / 32 / resident;
-  a.parts = 1;
-  if (groups < 3 * resident * sms)
-    a.parts = std::min((a.t.nslices + warps - 1) / warps, (3 * resident * sms + groups - 1) / groups);
-  warps = std::max<uint32_t>(2, std::min(warps, (a.t.nslices + a.parts - 1) / a.parts));
-  a.staged_diag = diag && !kAlpha && a.parts == 1;
-  const dim3 g(groups, a.parts);
-  auto go = [&](auto k) {
-    ensure_dynamic_smem((const void *)k, smem);
-    prefer_shared_carveout((const void *)k);
-    k<<<g, warps * 32, smem, s>>>(a);
-  };
-  switch (K) {
-    case 4: go(k_slab<4, kAlpha>); break;
-    case 2: go(k_slab<2, kAlpha>); break;
-    default: go(k_slab<1, kAlpha>); break;
+  const SlabShape c = slab_shape(p, sp, a.n, a.m, a.npair, 8, 4, 1, 1);
+  a.parts = c.parts;
+  a.staged_diag = diag && !kAlpha && c.parts == 1;
+  a.vec = p.nb % 2 == 0 && ((uintptr_t)x.S & 15u) == 0;
+  const dim3 g(c.groups, c.parts);
+  switch (c.K) {
+    case 4: go_slab(k_slab<T, 4, kAlpha>, a, g, c.warps, c.smem, s); break;
+    case 2: go_slab(k_slab<T, 2, kAlpha>, a, g, c.warps, c.smem, s); break;
+    default: go_slab(k_slab<T, 1, kAlpha>, a, g, c.warps, c.smem, s); break;
   }
+  count_launch(p.ctx);
+  SBDGB_CUDA(cudaGetLastError());
+}
+
+template <bool kAlpha>
+void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec, int add,
+                     int diag, int eta, cudaStream_t s) {
+  constexpr int sp = kAlpha ? 0 : 1;
+  SlabArgsF a{};
+  for (int v = 0; v < nvec; ++v) {
+    a.C[v] = C[v];
+    a.S[v] = S[v];
+  }
+  a.hii_df = x.hii_df;
+  a.hii_f = x.hii_f;
+  a.shift = x.shift_df;
+  a.t = slab_spin(p, sp);
+  a.val_s = p.slab.valf_s[sp];
+  a.val_d = p.slab.valf_d[sp];
+  a.Jo = kAlpha ? x.Jb : x.Ja;
+  a.rowstr = kAlpha ? p.astr : p.bstr;
+  a.colmask = p.slab.mask[1 - sp];
+  a.n = kAlpha ? p.na : p.nb;
+  a.m = kAlpha ? p.nb : p.na;
+  a.nb = p.nb;
+  a.npair = (kAlpha ? p.A.ns : p.B.ns) ? p.npair : 0;
+  a.eta = eta;
+  a.add = add;
+  a.diag = diag;
+  a.vec = p.nb % 4 == 0;
+  for (int v = 0; v < nvec; ++v) a.vec = a.vec && ((uintptr_t)S[v] & 15u) == 0;
+  const SlabShape c = slab_shape(p, sp, a.n, a.m, a.npair, 4, 8, 4, nvec);
+  a.parts = c.parts;
+  const dim3 g(c.groups, c.parts, nvec);
+  if (c.K == 8)
+    go_slab(k_slab_f32<8, kAlpha>, a, g, c.warps, c.smem, s);
+  else
+    go_slab(k_slab_f32<4, kAlpha>, a, g, c.warps, c.smem, s);
+  count_launch(p.ctx);
+  SBDGB_CUDA(cudaGetLastError());
+}
+
+template <typename T>
+void launch_slab_ab(const Problem &p, const Args<T> &x, int eta, cudaStream_t s) {
+  SlabAbArgs<T> a{};
+  a.C = x.C;
+  a.S = x.S;
+  a.astr = p.astr;
+  a.colmask = p.slab.mask[1];
+  a.off = p.A.off_s;
+  a.ket = p.A.ket_s;
+  a.code = p.A.code_s;
+  a.Kp = p.Kp;
+  a.items = p.slab.ab_items;
+  a.cols = p.ab_cols;
+  a.slice = p.ab_slice;
+  a.ent = p.slab.ab_ent;
+  a.nslices = p.n_ab_slices;
+  a.nb = p.nb;
+  a.npair = p.npair;
+  a.ek = p.slab.ek;
+  a.eta = eta;
+  const uint32_t warps = p.slab.ab_warps;
+  const dim3 g(p.slab.n_ab_items);
+  if (!slab_ab_sum(p))
+    go_slab(k_slab_ab<T, 2, false>, a, g, warps, slab_ab_smem_bytes(p, 2, false), s);
+  else if (slab_ab_smem_bytes(p, 4, true) <= max_smem() / 2)
+    go_slab(k_slab_ab<T, 4, true>, a, g, warps, slab_ab_smem_bytes(p, 4, true), s);
+  else
+    go_slab(k_slab_ab<T, 2, true>, a, g, warps, slab_ab_smem_bytes(p, 2, true), s);
+  count_launch(p.ctx);
+  SBDGB_CUDA(cudaGetLastError());
+}
+
+void launch_slab_ab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec,
+                        int eta, cudaStream_t s) {
+  SlabAbArgsF a{};
+  for (int v = 0; v < nvec; ++v) {
+    a.C[v] = C[v];
+    a.S[v] = S[v];
+  }
+  a.astr = p.astr;
+  a.colmask = p.slab.mask[1];
+  a.off = p.A.off_s;
+  a.ket = p.A.ket_s;
+  a.code = p.A.code_s;
+  a.Kp = x.Kp;
+  a.items = p.slab.ab_items;
+  a.cols = p.ab_cols;
+  a.slice = p.ab_slice;
+  a.ent = p.slab.ab_ent;
+  a.nslices = p.n_ab_slices;
+  a.nb = p.nb;
+  a.npair = p.npair;
+  a.eta = eta;
+  const uint32_t warps = p.slab.ab_warps;
+  go_slab(k_slab_ab_f32, a, dim3(p.slab.n_ab_items, 1, nvec), warps, slab_ab_smem_bytes_f32(p), s);
   count_launch(p.ctx);
   SBDGB_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
-// One FP64 product (slab_prepare has returned true): no allocation and no
-// scratch, so products of one problem may overlap on several streams.
-void sigma_slab(const Problem &p, const double *C, double *S, int accumulate, cudaStream_t s, bool block) {
+// One FP64 or double-float product (slab_prepare has returned true): no
+// allocation and no scratch, so products of one problem may overlap on several
+// streams.
+template <typename T>
+void sigma_slab(const Problem &p, const Args<T> &x, bool block, cudaStream_t s) {
   const int eta = block ? 0 : 1;
-  const bool beta = p.B.ns + p.B.nd > 0;
-  if (beta) launch_slab<false>(p, C, S, accumulate, 1, eta, s);
-  if (!beta || p.A.ns + p.A.nd > 0) launch_slab<true>(p, C, S, accumulate || beta, !beta, eta, s);
-  if (p.A.ns > 0 && p.B.ns > 0) {
-    SlabAbArgs a{};
-    a.C = C;
-    a.S = S;
-    a.astr = p.astr;
-    a.colmask = p.slab.mask[1];
-    a.off = p.A.off_s;
-    a.ket = p.A.ket_s;
-    a.code = p.A.code_s;
-    a.Kp = p.Kp;
-    a.rows = p.ab_rows;
-    a.cols = p.ab_cols;
-    a.slice = p.ab_slice;
-    a.ent = p.slab.ab_ent;
-    a.nslices = p.n_ab_slices;
-    a.nb = p.nb;
-    a.npair = p.npair;
-    a.ek = p.slab.ek;
-    a.eta = eta;
-    int sms = 0;
-    SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
-    // few rows: the columns of a row are shared by several CTAs
-    const uint32_t parts = std::min(a.nslices, std::max<uint32_t>(1, 4u * sms / p.n_ab_rows));
-    const uint32_t mine = (a.nslices + parts - 1) / parts, rounds = (mine + kSlabAbThreads / 32 - 1) / (kSlabAbThreads / 32);
-    const uint32_t warps = std::max<uint32_t>(4, (mine + rounds - 1) / rounds);
-    auto go = [&](auto k, size_t smem) {
-      ensure_dynamic_smem((const void *)k, smem);
-      prefer_shared_carveout((const void *)k);
-      k<<<dim3(p.n_ab_rows, parts), warps * 32, smem, s>>>(a);
-    };
-    if (!slab_ab_fixed(p))
-      go(k_slab_ab<2, false, false>, slab_ab_smem_bytes(p, 2, false));
-    else if (slab_ab_smem_bytes(p, 4, true) <= max_smem() / 2)
-      go(k_slab_ab<4, true, true>, slab_ab_smem_bytes(p, 4, true));
-    else
-      go(k_slab_ab<2, true, true>, slab_ab_smem_bytes(p, 2, true));
-    count_launch(p.ctx);
-    SBDGB_CUDA(cudaGetLastError());
-  }
+  const bool alpha = p.A.ns + p.A.nd > 0, beta = p.B.ns + p.B.nd > 0;
+  if (alpha || !beta) launch_slab<T, true>(p, x, x.accumulate, !beta, eta, s);
+  if (p.A.ns > 0 && p.B.ns > 0) launch_slab_ab<T>(p, x, eta, s);
+  if (beta) launch_slab<T, false>(p, x, x.accumulate || alpha, 1, eta, s);
+}
+template void sigma_slab<double>(const Problem &, const Args<double> &, bool, cudaStream_t);
+template void sigma_slab<dfloat>(const Problem &, const Args<dfloat> &, bool, cudaStream_t);
+
+// FP32 products of nvec <= 4 vectors.
+void sigma_slab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec,
+                    bool block, cudaStream_t s) {
+  const int eta = block ? 0 : 1;
+  const bool alpha = p.A.ns + p.A.nd > 0, beta = p.B.ns + p.B.nd > 0;
+  if (alpha || !beta) launch_slab_f32<true>(p, x, C, S, nvec, 0, !beta, eta, s);
+  if (p.A.ns > 0 && p.B.ns > 0) launch_slab_ab_f32(p, x, C, S, nvec, eta, s);
+  if (beta) launch_slab_f32<false>(p, x, C, S, nvec, alpha, 1, eta, s);
 }
 
 }  // namespace sbdgb

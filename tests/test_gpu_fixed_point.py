@@ -1,12 +1,13 @@
-"""The fixed-point sigma kernels (sigma_slab.cu), which the engine takes by itself
-for FP64 products of problems with more than 8 nonzeros a row: edges of their
+"""The sigma kernels of sigma_slab.cu, which the engine takes by itself according to
+the number of nonzeros and strings (sigma.cu:slab_pays): edges of their
 slices of 32 rows, groups of 1, 2 and 4 columns and batches of ket rows, and the
 vectors that fixed point cannot hold.
 
 Tolerance: an element's error is at most 2^-55 times the number of its terms
 times the largest |v| and |x| of its sums (below 2^-46 of the largest sigma for
 the shapes here), plus a few FP64 roundings; 1e-13 of the largest sigma bounds
-both.
+both.  Double-float results hold 48 bits (1e-12); FP32 sums of up to a few hundred
+terms are held to the 5e-6 of the other FP32 kernels' tests.
 """
 import numpy as np
 import pytest
@@ -41,7 +42,7 @@ def _problem(engine, *args, **kw):
 # lengths on either side, two and four columns a group, one and both spins with
 # few electrons; the last has under 8 alpha x beta pairs a determinant (FP64
 # multiply-adds there), the one before it more than a batch of ket rows holds
-SHAPES = [(10, 31, 1, 2), (8, 28, 28, 2), (10, 33, 32, 3), (12, 32, 97, 4), (12, 495, 70, 4), (12, 100, 495, 4),
+SHAPES = [(12, 300, 1, 4), (8, 28, 28, 2), (10, 33, 32, 5), (12, 32, 97, 4), (12, 495, 70, 4), (12, 100, 495, 4),
           (16, 801, 799, 5), (16, 1500, 1237, 5), (24, 700, 733, 8), (36, 1401, 1333, 12)]
 
 
@@ -59,6 +60,31 @@ def test_products_against_oracle(engine, norb, na, nb, nocc):
     assert torch.equal(_sigma(p, c), s)  # the same bits every time
     base = torch.tensor(rng.uniform(-1, 1, C.size), device="cuda")
     assert max_rel((_sigma(p, c, base) - base).cpu().numpy(), ref) <= 1e-13 * (1 + 1 / np.abs(ref).max())
+    # double-float (48 bits in, 48 out) and FP32, one vector and blocks
+    st = torch.cuda.current_stream().cuda_stream
+    hi = c.float()
+    x = torch.stack([hi, (c - hi.double()).float()], dim=-1).contiguous()
+    y = torch.full_like(x, float("nan"))
+    p.sigma_df_device(x.data_ptr(), y.data_ptr(), stream=st)
+    torch.cuda.synchronize()
+    assert p.tuning(2)["beta_shape"] == SLAB
+    assert max_rel(y.double().sum(-1).cpu().numpy(), ref) <= 1e-12
+    y = torch.stack([base.float(), (base - base.float().double()).float()], dim=-1).contiguous()
+    p.sigma_df_device(x.data_ptr(), y.data_ptr(), accumulate=True, stream=st)
+    torch.cuda.synchronize()
+    assert max_rel((y.double().sum(-1) - base).cpu().numpy(), ref) <= 1e-12 * (1 + 1 / np.abs(ref).max())
+    f = torch.stack([hi, -2 * hi, hi.flip(0), hi + 1]).contiguous()
+    one = torch.full_like(f, float("nan"))
+    for j in range(4):
+        p.sigma_mixed_device(f[j].data_ptr(), one[j].data_ptr(), stream=st)
+    torch.cuda.synchronize()
+    assert p.tuning(1)["beta_shape"] == SLAB
+    assert max_rel(one[0].double().cpu().numpy(), ref) <= 5e-6
+    for nvec in (2, 3, 4):
+        many = torch.full_like(f, float("nan"))
+        p.sigma_mixed_block_device(f.data_ptr(), many.data_ptr(), nvec, stream=st)
+        torch.cuda.synchronize()
+        assert torch.equal(many[:nvec], one[:nvec])
     p.close()
 
 
