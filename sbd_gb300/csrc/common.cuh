@@ -153,13 +153,14 @@ struct Problem {
   uint32_t *tile_start[2][2] = {}, *tile_order[2][2] = {};
   uint32_t n_tiles[2][2] = {};
   // autotuned sigma tile shapes: FP64, FP32, double-float, in the interleaved
-  // (0..2) and block (3..5) orderings
-  int tune_a[6] = {-1, -1, -1, -1, -1, -1}, tune_b[6] = {-1, -1, -1, -1, -1, -1};
-  float tune_ms[6][3][8] = {};  // timings the autotuner saw (A, B, fused + sparse)
+  // (0..2) and block (3..5) orderings; 6: the FP64 sweeps of the block ordering
+  // where the solver keeps to them (sigma_fp64_sweeps)
+  int tune_a[7] = {-1, -1, -1, -1, -1, -1, -1}, tune_b[7] = {-1, -1, -1, -1, -1, -1, -1};
+  float tune_ms[7][3][8] = {};  // timings the autotuner saw (A, B, fused + sparse)
   // 1: the alpha x beta single pairs run in their own kernel (sigma_ab.cu)
   // after the tuned shapes, which then skip them; -1 = not decided yet
-  int split_ab[6] = {-1, -1, -1, -1, -1, -1};
-  float tune_ab_ms[6][2] = {};  // the autotuner's time of the tuned shapes without and with the split
+  int split_ab[7] = {-1, -1, -1, -1, -1, -1, -1};
+  float tune_ab_ms[7][2] = {};  // the autotuner's time of the tuned shapes without and with the split
   // work order of the alpha x beta kernel (sigma_ab.cu): alpha rows with at
   // least one single (most singles first); beta columns by decreasing single
   // count in slices of 32, each slice's beta singles interleaved by lane
@@ -283,6 +284,9 @@ bool slab_prepare(Problem &p, cudaStream_t s);
 // parities) that the solvers use on eta-signed vectors; false: the
 // reference's interleaved convention.
 void sigma_fp64(Problem &p, const double *C, double *S, int accumulate, cudaStream_t s, bool block = false);
+// The block-ordering product by the FP64 kernels of sigma.cu alone: the solvers'
+// where a run is too ill-conditioned for another order of rounding (davidson.cu).
+void sigma_fp64_sweeps(Problem &p, const double *C, double *S, int accumulate, cudaStream_t s);
 void sigma_fp64_scratch(Problem &p, const double *C, double *S, int accumulate, double *CT, cudaStream_t s);
 // (H - shift) C in the mixed form: the diagonal term is formed in FP64 before
 // the result is rounded, so a shift near the spectrum keeps FP32 outputs small.

@@ -687,6 +687,14 @@ struct Solver {
   double *hs = nullptr;       // projected matrix on the device (kRR x kRR, ld kRR)
   double *rr = nullptr;       // Rayleigh-Ritz result on the device: n eigenvalues, n x n eigenvectors
   double *host = nullptr;     // pinned read-back buffer of the context
+  // FP64 solves from a start that is not the lowest determinants' (init 0 or 2)
+  // keep to the FP64 sweeps, with every rounding as it has always been.  The unit
+  // vector on determinant 0 can lie in the middle of the spectrum, where the
+  // preconditioner divides by differences of any size and sign: on 800 x 800 strings
+  // of norb 16 a last bit of a product grew to a different vector altogether in two
+  // cycles of 15 steps (also between the tile shapes that the autotuner picks from),
+  // so such a solve stopped after a number of steps keeps its result only this way.
+  bool ordered = false;
 
   Solver(Problem &pp, cudaStream_t ss) : p(pp), s(ss), N(pp.N) {
     int dev = p.ctx->device, sms = 0;
@@ -1103,6 +1111,7 @@ void davidson_core(Problem &p, const sbdgb_davidson_opts &o, const CorePhase &ph
   SBDGB_REQUIRE(max_nb <= 64, SBDGB_E_INPUT, "max_nb must be <= 64");
   cudaStream_t s = p.ctx->stream;
   Solver sv(p, s);
+  sv.ordered = kF64 && !ph.seed && o.init != 1;
   const int nstart = ph.seed ? ph.nseed : k;
   F *V = (F *)workspace(p, slot(WS_V, WS_VF, WS_VD), sizeof(F) * N * max_nb);
   F *HV = (F *)workspace(p, slot(WS_HV, WS_HVF, WS_HVD), sizeof(F) * N * max_nb);
@@ -1136,7 +1145,10 @@ void davidson_core(Problem &p, const sbdgb_davidson_opts &o, const CorePhase &ph
   auto extend = [&](int from, int to) {
     if constexpr (kF64) {
       for (int j = from; j < to; ++j) {
-        sigma_fp64(p, V + (size_t)j * N, HV + (size_t)j * N, 0, s, true);
+        if (sv.ordered)
+          sigma_fp64_sweeps(p, V + (size_t)j * N, HV + (size_t)j * N, 0, s);
+        else
+          sigma_fp64(p, V + (size_t)j * N, HV + (size_t)j * N, 0, s, true);
         r.sigma_fp64++;
       }
     } else if constexpr (kDF) {
@@ -1647,6 +1659,7 @@ void lanczos_fp64(Problem &p, const sbdgb_davidson_opts &o, double *E, double *X
   const int nb = std::max(2, std::min(o.max_nb, 64));
   cudaStream_t s = p.ctx->stream;
   Solver sv(p, s);
+  sv.ordered = o.init != 1;
   double *Cv = (double *)workspace(p, WS_V, sizeof(double) * N * nb);
   double *HC = (double *)workspace(p, WS_HV, sizeof(double) * N);
   double *W = (double *)workspace(p, WS_X, sizeof(double) * N);
@@ -1675,7 +1688,10 @@ void lanczos_fp64(Problem &p, const sbdgb_davidson_opts &o, double *E, double *X
     for (int ib = 0; ib < nb; ++ib) {
       ++n;
       double *Cb = Cv + (size_t)ib * N;
-      sigma_fp64(p, Cb, HC, 1, s, true);
+      if (sv.ordered)
+        sigma_fp64_sweeps(p, Cb, HC, 1, s);
+      else
+        sigma_fp64(p, Cb, HC, 1, s, true);
       r.sigma_calls++;
       r.sigma_fp64++;
       r.iterations++;

@@ -657,9 +657,9 @@ void launch_shapes(Problem &p, const Args<T> &a, int sa, int sb, int split, cuda
 
 // Tuning slot of a kernel family: precision (0 FP64, 1 FP32, 2 double-float)
 // in the interleaved (0..2) or block (3..5) ordering.
-template <typename T, bool kB>
+template <typename T, bool kB, bool kSweeps = false>
 constexpr int slot_of() {
-  return prec_of<T>() + (kB ? 3 : 0);
+  return kSweeps ? 6 : prec_of<T>() + (kB ? 3 : 0);
 }
 
 template <typename T>
@@ -667,9 +667,9 @@ void transpose(Problem &p, const T *in, T *out, uint32_t R, uint32_t Cn, cudaStr
 
 // Times every tile shape of both kernels once (after one untimed run) on the
 // problem's own vectors, writing into scratch, and keeps the fastest.
-template <typename T, bool kB>
+template <typename T, bool kB, bool kSweeps = false>
 void autotune(Problem &p, Args<T> a, cudaStream_t s) {
-  const int prec = slot_of<T, kB>();
+  const int prec = slot_of<T, kB, kSweeps>();
   if (p.tune_a[prec] >= 0 && p.tune_b[prec] >= 0) return;
   const std::array<uint64_t, 6> key{(uint64_t)prec, (uint64_t)p.norb, p.na, p.nb, p.A.ns + p.A.nd, p.B.ns + p.B.nd};
   const auto hit = p.ctx->tuned.find(key);
@@ -851,11 +851,11 @@ bool slab_pays(const Problem &p) {
 // a few singles per string on both sides that staging is cheap per term).
 constexpr double kAbSplitPerElement = 4.0;
 
-template <typename T, bool kB>
+template <typename T, bool kB, bool kSweeps = false>
 bool needs_tuning(Problem &p, cudaStream_t s) {
-  const int prec = slot_of<T, kB>();
+  const int prec = slot_of<T, kB, kSweeps>();
   if (p.tune_a[prec] >= 0 && p.tune_b[prec] >= 0) return false;
-  if (slab_pays<T, kB>(p) && slab_prepare(p, s)) {
+  if (!kSweeps && slab_pays<T, kB>(p) && slab_prepare(p, s)) {
     p.tune_a[prec] = 0;
     p.tune_b[prec] = kSlabShape;
     p.split_ab[prec] = p.A.ns > 0 && p.B.ns > 0 ? 1 : 0;
@@ -874,10 +874,10 @@ bool needs_tuning(Problem &p, cudaStream_t s) {
   return false;
 }
 
-template <typename T, bool kB>
+template <typename T, bool kB, bool kSweeps = false>
 void launch(Problem &p, const Args<T> &a, cudaStream_t s) {
-  const int prec = slot_of<T, kB>();
-  if (p.tune_a[prec] < 0 || p.tune_b[prec] < 0) autotune<T, kB>(p, a, s);
+  const int prec = slot_of<T, kB, kSweeps>();
+  if (p.tune_a[prec] < 0 || p.tune_b[prec] < 0) autotune<T, kB, kSweeps>(p, a, s);
   launch_shapes<T, kB>(p, a, p.tune_a[prec], p.tune_b[prec], p.split_ab[prec], s);
 }
 
@@ -1418,18 +1418,32 @@ void sigma_fp64_scratch(Problem &p, const double *C, double *S, int accumulate, 
 namespace {
 // One product with the problem's tuned shapes (tuning first if needed), timed
 // when the context records sigma timing; CT is the transpose scratch.
-template <typename T, bool kB>
+template <typename T, bool kB, bool kSweeps = false>
 void run_sigma(Problem &p, const Args<T> &a, T *CT, cudaStream_t s) {
-  constexpr int ts = slot_of<T, kB>();
-  if (needs_tuning<T, kB>(p, s)) {
+  constexpr int ts = slot_of<T, kB, kSweeps>();
+  if (needs_tuning<T, kB, kSweeps>(p, s)) {
     transpose<T>(p, a.C, CT, p.na, p.nb, s);
-    autotune<T, kB>(p, a, s);
+    autotune<T, kB, kSweeps>(p, a, s);
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   begin_timing(p, s, ev0, ev1);
   if (needs_transpose(p.tune_b[ts])) transpose<T>(p, a.C, CT, p.na, p.nb, s);
-  launch<T, kB>(p, a, s);
+  launch<T, kB, kSweeps>(p, a, s);
   end_timing(p, s, ev0, ev1);
+}
+}  // namespace
+
+namespace {
+Args<double> fp64_args(Problem &p, const double *C, double *S, int accumulate) {
+  Args<double> a = base_args<double>(p, C, S, accumulate);
+  a.val_sa = p.A.val_s;
+  a.val_da = p.A.val_d;
+  a.val_sb = p.B.val_s;
+  a.val_db = p.B.val_d;
+  a.Jb = p.Jb;
+  a.Ja = p.Ja;
+  a.Kp = p.Kp;
+  return a;
 }
 }  // namespace
 
@@ -1439,19 +1453,25 @@ void sigma_fp64(Problem &p, const double *C, double *S, int accumulate, cudaStre
   const bool tuned = !(block ? needs_tuning<double, true>(p, s) : needs_tuning<double, false>(p, s));
   if (!p.CT && (!tuned || needs_transpose(p.tune_b[block ? 3 : 0])))
     p.CT = (double *)dev_alloc(p, sizeof(double) * p.N);
-  Args<double> a = base_args<double>(p, C, S, accumulate);
+  Args<double> a = fp64_args(p, C, S, accumulate);
   a.CT = p.CT;
-  a.val_sa = p.A.val_s;
-  a.val_da = p.A.val_d;
-  a.val_sb = p.B.val_s;
-  a.val_db = p.B.val_d;
-  a.Jb = p.Jb;
-  a.Ja = p.Ja;
-  a.Kp = p.Kp;
   if (block)
     run_sigma<double, true>(p, a, p.CT, s);
   else
     run_sigma<double, false>(p, a, p.CT, s);
+}
+
+void sigma_fp64_sweeps(Problem &p, const double *C, double *S, int accumulate, cudaStream_t s) {
+  if (p.tune_b[3] >= 0 && p.tune_b[3] != kSlabShape) {  // shapes set by the caller, or timed: the sweeps already
+    sigma_fp64(p, C, S, accumulate, s, true);
+    return;
+  }
+  if (!p.tables || !p.diag) throw Error(SBDGB_E_STATE, "sigma needs tables and diagonal");
+  if (!p.CT) p.CT = (double *)dev_alloc(p, sizeof(double) * p.N);
+  if (p.N == 0) return;
+  Args<double> a = fp64_args(p, C, S, accumulate);
+  a.CT = p.CT;
+  run_sigma<double, true, true>(p, a, p.CT, s);
 }
 
 // Double-float copies of the table values and integral tables, for the

@@ -133,3 +133,17 @@ def test_solver_products_and_fp64_sweeps_agree(engine):
     assert a.report["converged"] and np.abs(a.energies - b.energies).max() <= 1e-10
     p.close()
     q.close()
+
+
+def test_unit_vector_starts_keep_the_fp64_sweeps(engine):
+    """A stopped FP64 solve from init 0 goes by the FP64 sweeps (davidson.cu,
+    Solver::ordered), with the same bits before and after a solve that does not."""
+    prob, p = _problem(engine, 16, 5, 5, 300, 280, seed=11)
+    kw = dict(nroots=2, max_nb=16, eps=1e-9)
+    a = p.davidson(max_it=1, init=0, **kw)
+    assert p.tuning(3)["beta_shape"] is None
+    b = p.davidson(max_it=40, init=1, **kw)
+    assert p.tuning(3)["beta_shape"] == SLAB and b.report["converged"]
+    c = p.davidson(max_it=1, init=0, **kw)
+    assert np.array_equal(a.vectors, c.vectors) and np.array_equal(a.energies, c.energies)
+    p.close()
