@@ -15,15 +15,19 @@
 //     s alone, those of the opposite-spin orbitals on u[q];
 //   - same-spin double: s alone (four entries);
 //   - alpha single x beta single: the sum over all pairs with the same four
-//     orbitals, accumulated per alpha pair in shared memory and then per
-//     orbital quadruple in a global L^4 array, scattered once at the end;
+//     orbitals (singles of both spins sorted by their two orbitals, so that a
+//     thread's sum is one quadruple's), scattered once at the end;
 //   - the diagonal (ZeroDiffCorrelation): string weights for the same-spin
 //     pairs and Y = (W o W) O_beta, M = O_alpha^T Y for the alpha-beta pairs.
 // Phases are the ones of the sigma kernels (same tables, same masks); the
 // same-spin doubles recompute theirs from the four orbitals.
 #include <algorithm>
 
+#include <numeric>
+
 #include "common.cuh"
+#include "fx.cuh"
+#include "sigma_dev.cuh"
 
 namespace sbdgb {
 
@@ -52,102 +56,173 @@ struct RdmArgs {
   SpinTables A, B;
 };
 
-// Same-spin singles of spin S, one CTA per bra string: for each pair, s and
-// u[q] over the spectators; for S = 0 also the alpha-beta sums of the pair.
+// Same-spin singles of spin S, one warp per pair: s and u[q] over the
+// spectators.  Of 32 spectators each lane forms one's product, on the fixed-point
+// scale of the largest (57 bits), and the lanes then add them all, lane q those
+// with orbital q: integer additions (62 a clock and SM) where FP64 ones take 16
+// clocks a warp.  Before, every spectator added to its orbitals' sums by FP64
+// atomics in shared memory (compare-and-swap loops on 8 of 24 places): 1.3 ms
+// a spin for 301 x 420 strings of norb 24, 22 us here.
 template <int S>
 __global__ void __launch_bounds__(kT) k_rdm_singles(RdmArgs a) {
   const SpinTables &T = S == 0 ? a.A : a.B;
-  const SpinTables &O = S == 0 ? a.B : a.A;  // opposite-spin tables (alpha-beta part)
   const uint64_t *same = S == 0 ? a.astr : a.bstr;
   const uint64_t *opp = S == 0 ? a.bstr : a.astr;
   const double *Wr = S == 0 ? a.W : a.WT;  // rows indexed by this spin's strings
   const uint32_t nopp = S == 0 ? a.nb : a.na;
   const int L = a.L;
-  const uint32_t bra = blockIdx.x;
-  __shared__ double su[kMaxL];
-  __shared__ double sR[S == 0 ? kMaxL * kMaxL : 1];
-  __shared__ double red[kT / 32];
+  __shared__ ulonglong2 sv[kT / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool two = a.two != nullptr;
-  const uint32_t p0 = T.off_s[bra], p1 = T.off_s[bra + 1];
-  const uint64_t bs = same[bra];
-  for (uint32_t p = p0; p < p1; ++p) {
-    const uint32_t ket = T.ket_s[p], code = T.code_s[p];
+  for (uint64_t p = (uint64_t)blockIdx.x * (kT / 32) + warp; p < T.ns; p += (uint64_t)gridDim.x * (kT / 32)) {
+    const uint32_t bra = T.bra_s[p], ket = T.ket_s[p], code = T.code_s[p];
     const uint64_t mask = T.mask_s[p];
     const int oi = code & 0xff, oa = (code >> 8) & 0xff;
-    for (int t = threadIdx.x; t < L; t += kT) su[t] = 0.0;
-    if (S == 0 && two)
-      for (int t = threadIdx.x; t < L * L; t += kT) sR[t] = 0.0;
-    __syncthreads();
     const double *rb = Wr + (size_t)bra * nopp, *rk = Wr + (size_t)ket * nopp;
-    const uint64_t kstr = same[ket];
-    double sacc = 0.0;
-    for (uint32_t o = threadIdx.x; o < nopp; o += kT) {
-      const uint64_t os = __ldg(opp + o);
-      const double wb = __ldg(rb + o);
-      const uint32_t ph = (__popcll(os & mask) ^ (code >> 31)) & 1u;
-      const double v = (ph ? -wb : wb) * __ldg(rk + o);
-      sacc += v;
-      if (two && v != 0.0) {
-        uint64_t bits = os;
-        while (bits) {
-          const int q = __ffsll((long long)bits) - 1;
-          bits &= bits - 1;
-          atomicAdd(&su[q], v);
+    double u0 = 0.0, u1 = 0.0, ssum = 0.0;  // orbitals lane and lane + 32, and all
+    for (uint32_t o0 = 0; o0 < nopp; o0 += 32) {
+      const uint32_t o = o0 + lane;
+      const uint64_t os = o < nopp ? __ldg(opp + o) : 0ull;
+      double v = o < nopp ? __ldg(rb + o) * __ldg(rk + o) : 0.0;
+      v = sdev::flip(v, (__popcll(os & mask) ^ (code >> 31)) & 1u);
+      const uint32_t hi = (uint32_t)__double2hiint(v) & 0x7fffffffu;
+      const uint32_t top = __reduce_max_sync(0xffffffffu, hi ? hi : (__double2loint(v) ? 1u : 0u));
+      if (top == 0u) continue;  // all zero
+      const int ex = fx::exponent_of(top, true);
+      const bool fixed = ex != fx::kBad;
+      const long long f = fixed ? fx::from_double(v, fx::kVBits - ex) : __double_as_longlong(v);
+      __syncwarp();
+      sv[warp][lane] = make_ulonglong2((unsigned long long)f, os);
+      __syncwarp();
+      if (fixed) {
+        long long a0 = 0, a1 = 0, as = 0;  // 32 terms of 57 bits
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) {
+          const ulonglong2 x = sv[warp][i];
+          const long long t = (long long)x.x;
+          as += t;
+          a0 += (x.y >> lane & 1ull) ? t : 0ll;
+          if (L > 32) a1 += (x.y >> (lane + 32) & 1ull) ? t : 0ll;
         }
-      }
-      if (S == 0 && two && wb != 0.0) {
-        // alpha single (bra -> ket) x beta singles of spectator o: element
-        // W[bra][o] W[ket][jb] with the sigma kernels' alpha-beta phase
-        const uint32_t q0 = O.off_s[o], q1 = O.off_s[o + 1];
-        const uint32_t pa = (__popcll(os & mask) ^ (code >> 31)) & 1u;
-        for (uint32_t q = q0; q < q1; ++q) {
-          const uint32_t jb = __ldg(O.ket_s + q), cb = __ldg(O.code_s + q);
-          const uint64_t mb = __ldg(O.mask_s + q);
-          const uint32_t f = (pa ^ __popcll(kstr & mb) ^ (cb >> 31)) & 1u;
-          const double x = wb * __ldg(rk + jb);
-          atomicAdd(&sR[(cb & 0xff) * L + ((cb >> 8) & 0xff)], f ? -x : x);
+        const double unit = scalbn(1.0, ex - fx::kVBits);
+        ssum = fma((double)as, unit, ssum);
+        u0 = fma((double)a0, unit, u0);
+        if (L > 32) u1 = fma((double)a1, unit, u1);
+      } else {
+        for (int i = 0; i < 32; ++i) {
+          const ulonglong2 x = sv[warp][i];
+          const double t = __longlong_as_double((long long)x.x);
+          ssum += t;
+          if (x.y >> lane & 1ull) u0 += t;
+          if (L > 32 && (x.y >> (lane + 32) & 1ull)) u1 += t;
         }
       }
     }
-    for (int off = 16; off > 0; off >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sacc;
+    if (lane == 0) atomicAdd(&a.one[(size_t)S * L * L + oi + (size_t)L * oa], ssum);
+    if (!two) continue;
+    const uint64_t bs = same[bra];
+    double *blk = a.two + (size_t)(3 * S) * L * L * L * L;  // s1 = s2 = S
+    double *b1 = a.two + (size_t)(S + 2 * (1 - S)) * L * L * L * L;
+    double *b2 = a.two + (size_t)((1 - S) + 2 * S) * L * L * L * L;
+    for (int h = 0; h < 2; ++h) {
+      const int q = lane + 32 * h;
+      if (q >= L) continue;
+      if ((bs >> q & 1ull) && q != oi && ssum != 0.0) {  // same-spin electrons (q = oi: its four terms cancel)
+        atomicAdd(&blk[q4(L, oa, q, oi, q)], ssum);
+        atomicAdd(&blk[q4(L, q, oa, q, oi)], ssum);
+        atomicAdd(&blk[q4(L, oa, q, q, oi)], -ssum);
+        atomicAdd(&blk[q4(L, q, oa, oi, q)], -ssum);
+      }
+      const double u = h ? u1 : u0;  // opposite-spin spectator orbitals
+      if (u != 0.0) {
+        atomicAdd(&b1[q4(L, oa, q, oi, q)], u);
+        atomicAdd(&b2[q4(L, q, oa, q, oi)], u);
+      }
+    }
+  }
+}
+
+// Singles counted by their orbital pair oi L + oa, and sorted by it: a[] = entry
+// index (alpha), (bra, ket | phase << 31) (beta).
+__global__ void k_rdm_types(SpinTables T, int L, uint32_t *__restrict__ count) {
+  for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < T.ns; p += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t code = T.code_s[p];
+    atomicAdd(&count[(code & 0xff) * L + ((code >> 8) & 0xff)], 1u);
+  }
+}
+__global__ void k_rdm_sort(SpinTables T, int L, uint32_t *__restrict__ next, uint2 *__restrict__ out) {
+  for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < T.ns; p += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t code = T.code_s[p];
+    const uint32_t at = atomicAdd(&next[(code & 0xff) * L + ((code >> 8) & 0xff)], 1u);
+    out[at] = make_uint2(T.bra_s[p], T.ket_s[p] | (code & 0x80000000u));
+  }
+}
+
+// Alpha single x beta single.  A CTA takes up to kAbPairs alpha singles of one
+// orbital pair, stages the bra and ket rows of W (signed by eta, so that an
+// element's phase is the two singles' own) and, where they fit, the sorted beta
+// singles; a thread then sums one beta orbital pair's entries over them: one
+// atomic addition per quadruple and CTA.  Beta orbital pairs are dealt by
+// decreasing length.
+constexpr uint32_t kAbPairs = 8;
+struct RdmAb {
+  const uint64_t *astr, *bstr;
+  const double *W;
+  double *R;
+  const uint2 *pa, *pb;        // sorted singles: (bra, ket | phase << 31)
+  const uint4 *chunks;         // (orbital pair, first, count, -) of pa
+  const uint4 *types;          // (orbital pair, first, count, -) of pb, longest first
+  uint32_t ntypes, npb, nb;
+  int L;
+  int rows_smem, ent_smem;     // rows and entries staged in shared memory
+};
+__device__ __forceinline__ double rdm_signed(const RdmAb &a, uint32_t row, uint32_t ib) {
+  return sdev::flip(__ldg(a.W + (size_t)row * a.nb + ib), sdev::eta_parity(__ldg(a.astr + row), __ldg(a.bstr + ib)));
+}
+__global__ void __launch_bounds__(kT) k_rdm_ab(RdmAb a) {
+  extern __shared__ __align__(16) unsigned char rdm_smem[];
+  double2 *rows = reinterpret_cast<double2 *>(rdm_smem);  // [nb]: bra and ket row
+  uint2 *sent = reinterpret_cast<uint2 *>(rows + (a.rows_smem ? a.nb : 0));
+  const uint4 ch = __ldg(a.chunks + blockIdx.x);
+  const uint2 *ent = a.pb;
+  if (a.ent_smem) {
+    for (uint32_t e = threadIdx.x; e < a.npb; e += kT) sent[e] = __ldg(a.pb + e);
+    ent = sent;
+  }
+  constexpr int kPer = 16;  // orbital pairs a thread holds: L^2 <= 4096
+  double acc[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) acc[i] = 0.0;
+  for (uint32_t k = 0; k < ch.z; ++k) {
+    const uint2 pr = __ldg(a.pa + ch.y + k);
+    const uint32_t bra = pr.x, ket = pr.y & 0x7fffffffu, sg = pr.y >> 31;
+    if (a.rows_smem) {
+      __syncthreads();
+      for (uint32_t c = threadIdx.x; c < a.nb; c += kT)
+        rows[c] = make_double2(sdev::flip(rdm_signed(a, bra, c), sg), rdm_signed(a, ket, c));
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int w = 0; w < kT / 32; ++w) s += red[w];
-      atomicAdd(&a.one[(size_t)S * L * L + oi + (size_t)L * oa], s);
-      if (two && s != 0.0) {
-        double *blk = a.two + (size_t)(3 * S) * L * L * L * L;  // s1 = s2 = S
-        uint64_t bits = bs;
-        while (bits) {
-          const int oj = __ffsll((long long)bits) - 1;
-          bits &= bits - 1;
-          if (oj == oi) continue;  // its four terms cancel
-          atomicAdd(&blk[q4(L, oa, oj, oi, oj)], s);
-          atomicAdd(&blk[q4(L, oj, oa, oj, oi)], s);
-          atomicAdd(&blk[q4(L, oa, oj, oj, oi)], -s);
-          atomicAdd(&blk[q4(L, oj, oa, oi, oj)], -s);
-        }
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const uint32_t t = threadIdx.x + kT * i;
+      if (t >= a.ntypes) break;
+      const uint4 ty = __ldg(a.types + t);
+      double s = acc[i];
+      for (uint32_t e = ty.y; e < ty.y + ty.z; ++e) {
+        const uint2 w = ent[e];
+        const uint32_t jb = w.y & 0x7fffffffu;
+        const double x = a.rows_smem ? rows[w.x].x : sdev::flip(rdm_signed(a, bra, w.x), sg);
+        const double y = a.rows_smem ? rows[jb].y : rdm_signed(a, ket, jb);
+        s = fma(sdev::flip(x, w.y >> 31), y, s);
       }
+      acc[i] = s;
     }
-    if (two) {
-      // opposite-spin spectator orbitals: blocks S + 2(1-S) and (1-S) + 2S
-      double *b1 = a.two + (size_t)(S + 2 * (1 - S)) * L * L * L * L;
-      double *b2 = a.two + (size_t)((1 - S) + 2 * S) * L * L * L * L;
-      for (int q = threadIdx.x; q < L; q += kT) {
-        const double u = su[q];
-        if (u != 0.0) {
-          atomicAdd(&b1[q4(L, oa, q, oi, q)], u);
-          atomicAdd(&b2[q4(L, q, oa, q, oi)], u);
-        }
-      }
-      if (S == 0) {
-        double *ab = a.R + (size_t)(oi * L + oa) * L * L;
-        for (int t = threadIdx.x; t < L * L; t += kT)
-          if (sR[t] != 0.0) atomicAdd(&ab[t], sR[t]);
-      }
-    }
-    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const uint32_t t = threadIdx.x + kT * i;
+    if (t >= a.ntypes) break;
+    if (acc[i] != 0.0) atomicAdd(&a.R[(size_t)ch.x * a.L * a.L + __ldg(a.types + t).x], acc[i]);
   }
 }
 
@@ -291,6 +366,67 @@ __global__ void k_rdm_scatter_ab(RdmArgs a) {
   }
 }
 
+// Sorts the singles of both spins by orbital pair and adds their alpha x beta
+// sums to a.R.
+void rdm_ab(Problem &p, const RdmArgs &a, cudaStream_t s) {
+  const int L = a.L;
+  const size_t L2 = (size_t)L * L;
+  const size_t words = 4 * (p.A.ns / kAbPairs + L2) + 4 * L2;
+  // counts and cursors of both spins, chunks and types, sorted singles
+  unsigned char *ws = (unsigned char *)workspace(p, WS_RED2, 16 * L2 + 4 * words + 8 * (p.A.ns + p.B.ns) + 64);
+  uint32_t *count = (uint32_t *)ws, *next = count + 2 * L2;
+  uint4 *lists = (uint4 *)(ws + ((16 * L2 + 15) & ~(size_t)15));
+  uint2 *pa = (uint2 *)((unsigned char *)lists + 4 * words), *pb = pa + p.A.ns;
+  SBDGB_CUDA(cudaMemsetAsync(count, 0, 8 * L2, s));
+  auto blocks = [](uint64_t n) { return (unsigned)std::min<uint64_t>((n + 255) / 256, 1024); };
+  k_rdm_types<<<blocks(p.A.ns), 256, 0, s>>>(p.A, L, count);
+  k_rdm_types<<<blocks(p.B.ns), 256, 0, s>>>(p.B, L, count + L2);
+  std::vector<uint32_t> h(2 * L2), first(2 * L2);
+  SBDGB_CUDA(cudaMemcpyAsync(h.data(), count, 8 * L2, cudaMemcpyDeviceToHost, s));
+  SBDGB_CUDA(cudaStreamSynchronize(s));
+  std::exclusive_scan(h.begin(), h.begin() + L2, first.begin(), 0u);
+  std::exclusive_scan(h.begin() + L2, h.end(), first.begin() + L2, 0u);
+  std::vector<uint4> out;
+  for (uint32_t t = 0; t < L2; ++t)
+    for (uint32_t k = 0; k < h[t]; k += kAbPairs)
+      out.push_back(make_uint4(t, first[t] + k, std::min(kAbPairs, h[t] - k), 0));
+  const uint32_t nchunks = (uint32_t)out.size();
+  std::vector<uint32_t> order;
+  for (uint32_t t = 0; t < L2; ++t)
+    if (h[L2 + t]) order.push_back(t);
+  std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return h[L2 + x] > h[L2 + y]; });
+  for (uint32_t t : order) out.push_back(make_uint4(t, first[L2 + t], h[L2 + t], 0));
+  SBDGB_CUDA(cudaMemcpyAsync(lists, out.data(), sizeof(uint4) * out.size(), cudaMemcpyHostToDevice, s));
+  SBDGB_CUDA(cudaMemcpyAsync(next, first.data(), 8 * L2, cudaMemcpyHostToDevice, s));
+  k_rdm_sort<<<blocks(p.A.ns), 256, 0, s>>>(p.A, L, next, pa);
+  k_rdm_sort<<<blocks(p.B.ns), 256, 0, s>>>(p.B, L, next + L2, pb);
+  int optin = 0;
+  SBDGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, p.ctx->device));
+  RdmAb b{};
+  b.astr = p.astr;
+  b.bstr = p.bstr;
+  b.W = a.W;
+  b.R = a.R;
+  b.pa = pa;
+  b.pb = pb;
+  b.chunks = lists;
+  b.types = lists + nchunks;
+  b.ntypes = (uint32_t)order.size();
+  b.npb = (uint32_t)p.B.ns;
+  b.nb = p.nb;
+  b.L = L;
+  const size_t rows = 16ull * p.nb, ent = 8ull * p.B.ns, limit = (size_t)optin - 1024;
+  b.rows_smem = rows <= limit;
+  b.ent_smem = (b.rows_smem ? rows : 0) + ent <= limit;
+  const size_t smem = (b.rows_smem ? rows : 0) + (b.ent_smem ? ent : 0);
+  ensure_dynamic_smem((const void *)k_rdm_ab, smem);
+  prefer_shared_carveout((const void *)k_rdm_ab);
+  k_rdm_ab<<<nchunks, kT, smem, s>>>(b);
+  count_launch(p.ctx, 5);
+  SBDGB_CUDA(cudaGetLastError());
+  SBDGB_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
+}
+
 }  // namespace
 
 void rdm(Problem &p, const double *W, double *one_host, double *two_host, cudaStream_t s) {
@@ -324,13 +460,15 @@ void rdm(Problem &p, const double *W, double *one_host, double *two_host, cudaSt
   string_norms(p, W, r, c, s);
   k_rdm_diag_same<0><<<(p.na + 127) / 128, 128, 0, s>>>(a, r);
   k_rdm_diag_same<1><<<(p.nb + 127) / 128, 128, 0, s>>>(a, c);
-  k_rdm_singles<0><<<p.na, kT, 0, s>>>(a);
-  k_rdm_singles<1><<<p.nb, kT, 0, s>>>(a);
+  int sms = 0;
+  SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
+  auto pair_blocks = [&](uint64_t n) { return (unsigned)std::min<uint64_t>((n + kT / 32 - 1) / (kT / 32), 8ull * sms); };
+  if (p.A.ns) k_rdm_singles<0><<<pair_blocks(p.A.ns), kT, 0, s>>>(a);
+  if (p.B.ns) k_rdm_singles<1><<<pair_blocks(p.B.ns), kT, 0, s>>>(a);
   count_launch(p.ctx, 5);
+  if (two_host && p.A.ns && p.B.ns) rdm_ab(p, a, s);
   if (two_host) {
     double *Y = (double *)workspace(p, WS_RED2, sizeof(double) * (size_t)p.na * L);
-    int sms = 0;
-    SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
     const uint32_t rb = (uint32_t)std::min<size_t>(((size_t)p.na + 7) / 8, (size_t)sms * 8);
     k_rdm_occ_rows<<<rb, kT, 0, s>>>(a, Y);
     k_rdm_diag_ab<<<(int)((L2 + 127) / 128), 128, 0, s>>>(a, Y);
