@@ -22,7 +22,8 @@
 //   - dot products leave one partial per chunk (no atomics) that a
 //     per-problem warp sums in chunk order, so results are deterministic;
 //   - the projected eigenproblem (n <= 32) is a parallel-order Jacobi by one
-//     warp per problem, which also does the small coefficient-space work;
+//     warp per problem (one block in the mixed form), which also does the small
+//     coefficient-space work;
 //   - sigma is the fused per-element form (diagonal, alpha pairs of the row,
 //     alpha x beta singles, beta pairs of the column) for up to 8 vectors at
 //     once, sharing the index, value and phase work between the vectors; the
@@ -44,6 +45,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "rr_dev.cuh"
 #include "sigma_dev.cuh"
 
 namespace sbdgb {
@@ -221,7 +223,8 @@ __device__ __forceinline__ bool sub_range(const BCommon &g, Chunk &ch, uint32_t 
 // Parallel-order Jacobi: each sweep is n' - 1 rounds (n' = n rounded up to
 // even) of the round-robin pairing, and the n'/2 rotations of a round act on
 // disjoint index pairs, so their parameters are computed by n'/2 lanes at once
-// and applied together (A <- J^T A J zeroes every pair of the round).  FP64
+// and applied together (A <- J^T A J zeroes every pair of the round).  (The plain
+// FP64 form's; the mixed form takes rrdev::jacobi.)  FP64
 // division and square root dominate a rotation on this GPU; the parallel
 // order takes them once per round instead of once per pair.
 __device__ void warp_eig(int n, const double *A, double *Aw, double *Wv, double *E) {
@@ -542,6 +545,58 @@ __global__ void __launch_bounds__(32) k_b_rr(BCommon g) {
   const int nv = to, kk = min(g.k, nv), kc = min(2 * g.k, nv);
   warp_eig(nv, S.A, Aw, Wv, E);
   for (int t = l; t < nv * kc; t += 32) S.c[t] = Wv[(t % nv) + kNB * (t / nv)];
+  if (l < kk) S.th[l] = E[l];
+  if (l == 0) {
+    S.nv = nv;
+    S.kk = kk;
+    S.kc = kc;
+    S.iter++;
+  }
+}
+
+// The same by one block per problem with the cheaper rotations of rr_dev.cuh, for
+// the mixed form (24 problems, three roots, n up to 24: 625 ms a solve by the warps
+// above, 505 here; 3 problems, one root: 134 and 103).  The plain FP64 form keeps
+// its roundings, on which the vectors of a batch stopped after a number of steps
+// depend.
+constexpr int kRRT = 256;
+__global__ void __launch_bounds__(kRRT) k_b_rr_fast(BCommon g) {
+  __shared__ double buf0[kNB * kNB], buf1[kNB * kNB], buf2[kNB * kNB], buf3[kNB * kNB], E[kNB];
+  __shared__ rrdev::Scratch<kNB, kRRT> work;
+  __shared__ int rank[kNB];
+  const BProb &P = g.P[blockIdx.x];
+  BState &S = g.S[blockIdx.x];
+  if (!S.active) return;
+  const int l = threadIdx.x, from = S.from, to = S.to, nr = to - from;
+  for (int v = l; v < to * nr; v += kRRT) {
+    const double t = chunk_total(g, P, v);
+    const int i = v % to, j = from + v / to;
+    S.A[i + kNB * j] = t;
+    if (i < from) S.A[j + kNB * i] = t;
+  }
+  __syncthreads();
+  const int nv = to, kk = min(g.k, nv), kc = min(2 * g.k, nv);
+  double *A = buf0, *An = buf1, *V = buf2, *Vn = buf3;
+  for (int t = l; t < nv * nv; t += kRRT) {
+    const int i = t % nv, j = t / nv;
+    A[t] = 0.5 * (S.A[i + kNB * j] + S.A[j + kNB * i]);
+    V[t] = i == j ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  rrdev::jacobi<kNB, kRRT>(nv, A, An, V, Vn, work);
+  if (l < nv) {  // ascending order (ties by index)
+    const double e = A[l + nv * l];
+    int r = 0;
+    for (int j = 0; j < nv; ++j) {
+      const double f = A[j + nv * j];
+      r += (f < e) || (f == e && j < l);
+    }
+    rank[l] = r;
+    E[r] = e;
+  }
+  __syncthreads();
+  for (int t = l; t < nv * nv; t += kRRT)
+    if (rank[t / nv] < kc) S.c[t % nv + nv * rank[t / nv]] = V[t];
   if (l < kk) S.th[l] = E[l];
   if (l == 0) {
     S.nv = nv;
@@ -1150,7 +1205,10 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
       };
       auto iteration = [&] {
         k_b_dots<T><<<nch, kT, 0, s>>>(g, 0);
-        k_b_rr<<<count, 32, 0, s>>>(g);
+        if (mixed)
+          k_b_rr_fast<<<count, kRRT, 0, s>>>(g);
+        else
+          k_b_rr<<<count, 32, 0, s>>>(g);
         k_b_combine<T><<<nch, kT, 0, s>>>(g);
         k_b_ctl<<<count, 32, 0, s>>>(g);
         k_b_apply<T><<<nsub, kT, 0, s>>>(g);

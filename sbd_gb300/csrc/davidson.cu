@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "rr_dev.cuh"
 #include "small_eig.h"
 
 namespace sbdgb {
@@ -118,13 +119,64 @@ __global__ void __launch_bounds__(kRed) k_dots(Ptrs<TV, kMaxV> V, Ptrs<TW, kMaxW
   }
 }
 
-// Sums the per-block partials in block order (deterministic).
-__global__ void k_sum_partials(const double *__restrict__ partial, int nblocks, int width, double *__restrict__ out) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= width) return;
-  double s = 0.0;
-  for (int b = 0; b < nblocks; ++b) s += partial[(size_t)b * width + t];
-  out[t] = s;
+// Sums of the per-block partials.  (One thread per value, loading as it added,
+// took 38-65 us for 608 blocks: longer, on 10^6 determinants, than the pass that
+// left them.)
+//
+// kOrdered (FP64 solves from a start that is not the lowest determinants', init 0
+// or 2: Solver::ordered): in block order, as they have always been formed.  The
+// unit vector on determinant 0 can lie in the middle of the spectrum, where the
+// preconditioner divides by differences of any size and sign: on 800 x 800 strings
+// of norb 16 a last bit in a product or a sum grew to a different vector altogether
+// in two cycles of 15 steps (also between the tile shapes that the autotuner picks
+// from).  Such a solve stopped after a number of steps keeps its result only if
+// every rounding stays, so it also keeps the FP64 sweeps and the Rayleigh-Ritz
+// iteration with FP64 angles.  The blocks are staged in shared memory and eight
+// lanes add eight values (an FP64 addition occupies a quarter of the SM's pipe for
+// 64 cycles, so the chain is what is left).
+// Otherwise: a CTA per value, thread sums and a tree, 2-3 us.
+constexpr int kSum = 128, kSumVals = 8, kSumStage = 640;
+template <bool kOrdered>
+__device__ __forceinline__ int sum_blocks(const double *__restrict__ partial, int nblocks, int width, double &sum) {
+  if constexpr (kOrdered) {
+    __shared__ double st[kSumStage * kSumVals];
+    const int t0 = blockIdx.x * kSumVals, nv = min(kSumVals, width - t0), l = threadIdx.x;
+    double s = 0.0;
+    for (int b0 = 0; b0 < nblocks; b0 += kSumStage) {
+      const int nb = min(kSumStage, nblocks - b0);
+      __syncthreads();
+      for (int i = l; i < nb * kSumVals; i += kSum) {
+        const int v = i % kSumVals;
+        if (v < nv) st[i] = partial[(size_t)(b0 + i / kSumVals) * width + t0 + v];
+      }
+      __syncthreads();
+      if (l < nv) {
+#pragma unroll 8
+        for (int b = 0; b < nb; ++b) s += st[b * kSumVals + l];
+      }
+    }
+    sum = s;
+    return l < nv ? t0 + l : -1;
+  } else {
+    __shared__ double red[kSum / 32];
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += kSum) s += partial[(size_t)b * width + blockIdx.x];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    sum = (red[0] + red[1]) + (red[2] + red[3]);
+    return threadIdx.x == 0 ? (int)blockIdx.x : -1;
+  }
+}
+inline unsigned sum_ctas(bool ordered, int width) {
+  return (unsigned)(ordered ? (width + kSumVals - 1) / kSumVals : width);
+}
+template <bool kOrdered>
+__global__ void __launch_bounds__(kSum) k_sum_partials(const double *__restrict__ partial, int nblocks, int width,
+                                                       double *__restrict__ out) {
+  double x;
+  const int t = sum_blocks<kOrdered>(partial, nblocks, width, x);
+  if (t >= 0) out[t] = x;
 }
 
 template <typename F>
@@ -533,12 +585,13 @@ __global__ void __launch_bounds__(kRed) k_lz_ritz(const double *__restrict__ C, 
 
 // M[(i0 + i) + ld (j0 + j)] = sum over blocks of partial[b][i * mw + j] (and the
 // transposed entry when sym): a dots pass written into the projected matrix.
-__global__ void k_sum_partials_mat(const double *__restrict__ partial, int nblocks, int mv, int mw,
-                                   double *__restrict__ M, int ld, int i0, int j0, int sym) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= mv * mw) return;
-  double x = 0.0;
-  for (int b = 0; b < nblocks; ++b) x += partial[(size_t)b * mv * mw + t];
+template <bool kOrdered>
+__global__ void __launch_bounds__(kSum) k_sum_partials_mat(const double *__restrict__ partial, int nblocks, int mv,
+                                                           int mw, double *__restrict__ M, int ld, int i0, int j0,
+                                                           int sym) {
+  double x;
+  const int t = sum_blocks<kOrdered>(partial, nblocks, mv * mw, x);
+  if (t < 0) return;
   const int i = i0 + t / mw, j = j0 + t % mw;
   M[i + (size_t)ld * j] = x;
   if (sym) M[j + (size_t)ld * i] = x;
@@ -547,40 +600,26 @@ __global__ void k_sum_partials_mat(const double *__restrict__ partial, int nbloc
 constexpr int kRR = 64;          // largest projected matrix (max_nb <= 64)
 constexpr int kRRThreads = 1024;  // one element of the n x n matrices per thread (n <= 32)
 
-// Sum over the block (kRRThreads threads) of one value per thread.
-__device__ __forceinline__ double rr_block_sum(double v, double *tmp) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) tmp[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double r = 0.0;
-  for (int w = 0; w < kRRThreads / 32; ++w) r += tmp[w];
-  __syncthreads();
-  return r;
-}
-
 // Eigenvalues (ascending) and eigenvectors of the symmetric part of the n x n
 // leading block of Hs (ld), n <= 64, by one block: out[0..n) the eigenvalues,
 // out[n + i + n j] the eigenvector matrix (column j).  The reference solves
 // this with LAPACK dsyev on the host (framework/hp_numeric.h:503-520).
 //
-// Parallel-order Jacobi: each sweep is n' - 1 rounds (n' = n rounded up to
-// even) of the round-robin pairing; the n'/2 rotations of a round act on
-// disjoint index pairs, so n'/2 threads compute them at once and every
-// element of A <- J^T A J and of V <- V J is then formed by its own thread
-// from four (two) elements of the previous round.
+// Parallel-order Jacobi, kFast by rrdev::jacobi; otherwise (Solver::ordered) the
+// form with FP64 angles and every element of the matrix formed for itself.
 //
 // Warm start: when the first nw basis columns are unchanged since the
 // previous call (the subspace only grew), that call's eigenvectors, still in
 // out (n = nw), diagonalise their block.  The iteration then starts from
 // Y^T A Y with Y = diag(those eigenvectors, identity): diagonal but for the
 // new rows and columns, so a few sweeps converge it.
+template <bool kFast>
 __global__ void __launch_bounds__(kRRThreads) k_rr(const double *__restrict__ Hs, int ld, int n, int nw,
                                                    double *__restrict__ out) {
   extern __shared__ double sm[];
   const int nn = n * n;
   double *Acur = sm, *Anext = sm + nn, *Vcur = sm + 2 * nn, *Vnext = sm + 3 * nn;
-  __shared__ double ca[kRR], cb[kRR], tmp[kRRThreads / 32];
-  __shared__ int partner[kRR];
+  __shared__ rrdev::Scratch<kRR, kRRThreads> work;
   const int tid = threadIdx.x;
   for (int t = tid; t < nn; t += kRRThreads) {
     const int i = t % n, j = t / n;
@@ -613,53 +652,57 @@ __global__ void __launch_bounds__(kRRThreads) k_rr(const double *__restrict__ Hs
     for (int t = tid; t < nn; t += kRRThreads) Acur[t] = Anext[t];
   }
   __syncthreads();
-  const int n2 = (n + 1) & ~1, np = n2 / 2;
-  auto idx = [&](int pos, int r) { return pos == 0 ? 0 : 1 + (pos - 1 + r) % (n2 - 1); };
-  for (int sweep = 0; sweep < 60 && n > 1; ++sweep) {
-    double off = 0.0, dg = 0.0;
-    for (int t = tid; t < nn; t += kRRThreads) {
-      const double x = Acur[t];
-      if (t % n == t / n) dg += x * x; else off += x * x;
-    }
-    off = rr_block_sum(off, tmp);
-    dg = rr_block_sum(dg, tmp);
-    if (off <= 1e-30 * (dg + 1e-300)) break;
-    for (int r = 0; r < n2 - 1; ++r) {
-      if (tid < np) {
-        const int a = idx(tid, r), b = idx(n2 - 1 - tid, r);
-        const int pp = min(a, b), q = max(a, b);
-        double c = 1.0, sn = 0.0;
-        if (q < n) {  // q == n is the padding index of odd n
-          const double apq = Acur[pp + n * q];
-          if (fabs(apq) >= 1e-300) {
-            const double th = (Acur[q + n * q] - Acur[pp + n * pp]) / (2.0 * apq);
-            const double tt = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-            c = 1.0 / sqrt(tt * tt + 1.0);
-            sn = tt * c;
-          }
-          // new column p = c col_p - s col_q, new column q = s col_p + c col_q
-          partner[q] = pp;
-          ca[q] = c;
-          cb[q] = sn;
-        }
-        partner[pp] = q < n ? q : pp;
-        ca[pp] = c;
-        cb[pp] = q < n ? -sn : 0.0;
-      }
-      __syncthreads();
+  if constexpr (kFast) {
+    rrdev::jacobi<kRR, kRRThreads>(n, Acur, Anext, Vcur, Vnext, work);
+  } else {
+    const int n2 = (n + 1) & ~1, np = n2 / 2;
+    auto idx = [&](int pos, int r) { return pos == 0 ? 0 : 1 + (pos - 1 + r) % (n2 - 1); };
+    for (int sweep = 0; sweep < 60 && n > 1; ++sweep) {
+      double off = 0.0, dg = 0.0;
       for (int t = tid; t < nn; t += kRRThreads) {
-        const int i = t % n, j = t / n, pi = partner[i], pj = partner[j];
-        const double ci = ca[i], si = cb[i], cj = ca[j], sj = cb[j];
-        Anext[t] = ci * (cj * Acur[i + n * j] + sj * Acur[i + n * pj]) + si * (cj * Acur[pi + n * j] + sj * Acur[pi + n * pj]);
-        Vnext[t] = cj * Vcur[i + n * j] + sj * Vcur[i + n * pj];
+        const double x = Acur[t];
+        if (t % n == t / n) dg += x * x; else off += x * x;
       }
-      __syncthreads();
-      double *x = Acur;
-      Acur = Anext;
-      Anext = x;
-      x = Vcur;
-      Vcur = Vnext;
-      Vnext = x;
+      off = rrdev::block_sum<kRRThreads>(off, work.tmp, nn);
+      dg = rrdev::block_sum<kRRThreads>(dg, work.tmp, nn);
+      if (off <= 1e-30 * (dg + 1e-300)) break;
+      for (int r = 0; r < n2 - 1; ++r) {
+        if (tid < np) {
+          const int a = idx(tid, r), b = idx(n2 - 1 - tid, r);
+          const int pp = min(a, b), q = max(a, b);
+          double c = 1.0, sn = 0.0;
+          if (q < n) {  // q == n is the padding index of odd n
+            const double apq = Acur[pp + n * q];
+            if (fabs(apq) >= 1e-300) {
+              const double th = (Acur[q + n * q] - Acur[pp + n * pp]) / (2.0 * apq);
+              const double tt = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
+              c = 1.0 / sqrt(tt * tt + 1.0);
+              sn = tt * c;
+            }
+            // new column p = c col_p - s col_q, new column q = s col_p + c col_q
+            work.partner[q] = pp;
+            work.c[q] = c;
+            work.s[q] = sn;
+          }
+          work.partner[pp] = q < n ? q : pp;
+          work.c[pp] = c;
+          work.s[pp] = q < n ? -sn : 0.0;
+        }
+        __syncthreads();
+        for (int t = tid; t < nn; t += kRRThreads) {
+          const int i = t % n, j = t / n, pi = work.partner[i], pj = work.partner[j];
+          const double ci = work.c[i], si = work.s[i], cj = work.c[j], sj = work.s[j];
+          Anext[t] = ci * (cj * Acur[i + n * j] + sj * Acur[i + n * pj]) + si * (cj * Acur[pi + n * j] + sj * Acur[pi + n * pj]);
+          Vnext[t] = cj * Vcur[i + n * j] + sj * Vcur[i + n * pj];
+        }
+        __syncthreads();
+        double *x = Acur;
+        Acur = Anext;
+        Anext = x;
+        x = Vcur;
+        Vcur = Vnext;
+        Vnext = x;
+      }
     }
   }
   // ascending order: rank of each eigenvalue (ties by index), then scatter
@@ -687,14 +730,13 @@ struct Solver {
   double *hs = nullptr;       // projected matrix on the device (kRR x kRR, ld kRR)
   double *rr = nullptr;       // Rayleigh-Ritz result on the device: n eigenvalues, n x n eigenvectors
   double *host = nullptr;     // pinned read-back buffer of the context
-  // FP64 solves from a start that is not the lowest determinants' (init 0 or 2)
-  // keep to the FP64 sweeps, with every rounding as it has always been.  The unit
-  // vector on determinant 0 can lie in the middle of the spectrum, where the
-  // preconditioner divides by differences of any size and sign: on 800 x 800 strings
-  // of norb 16 a last bit of a product grew to a different vector altogether in two
-  // cycles of 15 steps (also between the tile shapes that the autotuner picks from),
-  // so such a solve stopped after a number of steps keeps its result only this way.
-  bool ordered = false;
+  bool ordered = false;       // every rounding as it has always been (k_sum_partials)
+
+  void sum_partials(const double *part, int width, double *out) {
+    (ordered ? k_sum_partials<true> : k_sum_partials<false>)<<<sum_ctas(ordered, width), kSum, 0, s>>>(part, blocks,
+                                                                                                     width, out);
+    count_launch(p.ctx);
+  }
 
   Solver(Problem &pp, cudaStream_t ss) : p(pp), s(ss), N(pp.N) {
     int dev = p.ctx->device, sms = 0;
@@ -724,7 +766,8 @@ struct Solver {
         for (int i = 0; i < kMaxV; ++i) vp.p[i] = V0 + (size_t)(i0 + std::min(i, mv - 1)) * N;
         double *part = partial + (size_t)(batch % kMaxChunks) * blocks * kMaxV * kMaxW;
         launch_dots<TV, TW>(vp, wp, mv, mw, part);
-        k_sum_partials_mat<<<(mv * mw + 63) / 64, 64, 0, s>>>(part, blocks, mv, mw, hs, kRR, i0, j0 + jb, 1);
+        (ordered ? k_sum_partials_mat<true> : k_sum_partials_mat<false>)<<<sum_ctas(ordered, mv * mw), kSum, 0, s>>>(
+            part, blocks, mv, mw, hs, kRR, i0, j0 + jb, 1);
         count_launch(p.ctx);
         ++batch;
       }
@@ -740,8 +783,9 @@ struct Solver {
     SBDGB_REQUIRE(n >= 1 && n <= kRR, SBDGB_E_UNSUPPORTED, "projected matrix larger than 64");
     if (nw > n) nw = 0;
     const size_t smem = sizeof(double) * 4 * (size_t)n * n;
-    ensure_dynamic_smem((const void *)k_rr, smem);
-    k_rr<<<1, kRRThreads, smem, s>>>(hs, kRR, n, nw, rr);
+    const auto k = ordered ? k_rr<false> : k_rr<true>;
+    ensure_dynamic_smem((const void *)k, smem);
+    k<<<1, kRRThreads, smem, s>>>(hs, kRR, n, nw, rr);
     count_launch(p.ctx);
     SBDGB_CUDA(cudaGetLastError());
   }
@@ -801,8 +845,7 @@ struct Solver {
         for (int i = 0; i < kMaxV; ++i) vp.p[i] = V0 + (size_t)(i0 + std::min(i, mv - 1)) * N;
         double *part = partial + (size_t)batch.size() * blocks * kMaxV * kMaxW;
         launch_dots<TV, TW>(vp, wp, mv, mw, part);
-        k_sum_partials<<<(mv * mw + 63) / 64, 64, 0, s>>>(part, blocks, mv * mw, red + width);
-        count_launch(p.ctx);
+        sum_partials(part, mv * mw, red + width);
         batch.push_back({i0, j0, mv, mw, width});
         width += mv * mw;
         if ((int)batch.size() == kMaxChunks) flush();
@@ -872,8 +915,8 @@ struct Solver {
       default: throw Error(SBDGB_E_UNSUPPORTED, "at most 16 roots");
     }
     const int width = U ? 3 * k : k;
-    k_sum_partials<<<1, 64, 0, s>>>(partial, blocks, width, red);
-    count_launch(p.ctx, 2);
+    sum_partials(partial, width, red);
+    count_launch(p.ctx);
     SBDGB_CUDA(cudaGetLastError());
     const int nrr = rr_host ? nv + nv * nv : 0;
     if (nrr) SBDGB_CUDA(cudaMemcpyAsync(host + width, rr, sizeof(double) * nrr, cudaMemcpyDeviceToHost, s));
@@ -937,8 +980,7 @@ struct Solver {
   }
 
   double reduce_partials(int width, std::vector<double> *out = nullptr) {
-    k_sum_partials<<<1, 64, 0, s>>>(partial, blocks, width, red);
-    count_launch(p.ctx);
+    sum_partials(partial, width, red);
     const double *h = read_back(width);
     if (out) out->assign(h, h + width);
     return h[0];
