@@ -1060,6 +1060,26 @@ __global__ void k_b_results(const BState *S, int count, int k, double *out) {
   o[2 * k + 4] = s.sigma_calls;
 }
 
+// Whether the products go through the kernels of sigma_slab.cu (three launches a
+// step instead of one): the fused per-element kernel is bound by the FP64 pipe
+// (97.8% busy) and gathers from L2; with few nonzeros a row it is a stream.
+// (Mixed solves, ms, fused and here: 3 problems, one root, 103 and 80; 24, one
+// root, 368 and 279; 24, three roots, 505 and 474.)
+// Asked of the mixed form only: a plain FP64 batch may be stopped after a number
+// of steps, and its higher roots' vectors then depend on every rounding (1e-16 in
+// the products grew to 5e-9 in 16 steps), so it keeps the fused kernel and the
+// Rayleigh-Ritz warps.
+bool slab_batch_pays(Problem **ps, int count) {
+  double work = 0.0, total = 0.0;
+  for (int i = 0; i < count; ++i) {
+    const Problem &p = *ps[i];
+    const double sa = (double)p.A.ns / p.na, sb = (double)p.B.ns / p.nb;
+    work += (double)p.N * (sa + sb + (double)p.A.nd / p.na + (double)p.B.nd / p.nb + sa * sb);
+    total += (double)p.N;
+  }
+  return work >= 32.0 * total;
+}
+
 }  // namespace
 
 // Solves every problem of the batch with the same options, all problems in
@@ -1098,6 +1118,7 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
     if (!p.diag) build_diag(p, s);
     if (mixed) prepare_mixed(p, s);
   }
+  const bool slab = mixed && slab_batch_pays(ps, count) && slab_batch_fits(ps, count, s);
   std::vector<BProb> hp(count);
   std::vector<Chunk> chunks;
   double *arena = (double *)tmp_alloc(&c, bytes);
@@ -1183,7 +1204,44 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
   Chunk *dch = (Chunk *)(dres + nres);
   int *dcount = (int *)(((uintptr_t)(dch + nch) + 7) & ~(uintptr_t)7);
   cudaGraphExec_t exec = nullptr;
+  SlabBatch slab64, slab32;
+  void *lists = nullptr;  // per problem: V, HV (FP64), V, HV (FP32), N
+  auto cleanup = [&] {
+    for (SlabBatch *b : {&slab64, &slab32})
+      for (void *d : b->tmps) tmp_free(&c, d);
+    if (lists) tmp_free(&c, lists);
+    tmp_free(&c, mb);
+    tmp_free(&c, arena);
+  };
   try {
+    if (slab) {
+      std::vector<void *> ptr(4 * (size_t)count);
+      std::vector<uint32_t> n(count);
+      std::vector<Args<double>> a64(count);
+      std::vector<Args<float>> a32(count);
+      for (int i = 0; i < count; ++i) {
+        ptr[i] = hp[i].V;
+        ptr[count + i] = hp[i].HV;
+        ptr[2 * count + i] = hp[i].Vf;
+        ptr[3 * count + i] = hp[i].HVf;
+        n[i] = hp[i].N;
+        a64[i] = hp[i].a;
+        a32[i] = hp[i].af;
+        a32[i].hii_f = ps[i]->hii_f;
+      }
+      lists = tmp_alloc(&c, sizeof(void *) * ptr.size() + sizeof(uint32_t) * count);
+      void **dptr = (void **)lists;
+      uint32_t *dn = (uint32_t *)(dptr + ptr.size());
+      SBDGB_CUDA(cudaMemcpyAsync(dptr, ptr.data(), sizeof(void *) * ptr.size(), cudaMemcpyHostToDevice, s));
+      SBDGB_CUDA(cudaMemcpyAsync(dn, n.data(), sizeof(uint32_t) * count, cudaMemcpyHostToDevice, s));
+      const SlabBatchState st{&dS->active, &dS->from, &dS->to, sizeof(BState), dptr, dptr + count, dn};
+      const int nvec = mixed ? nseed : k;  // the FP64 phase of the mixed form starts on nseed vectors
+      slab_batch_plan<double>(slab64, &c, ps, a64.data(), count, st, nvec, s);
+      SlabBatchState sf = st;
+      sf.V = dptr + 2 * count;
+      sf.HV = dptr + 3 * count;
+      if (mixed) slab_batch_plan<float>(slab32, &c, ps, a32.data(), count, sf, k, s);
+    }
     SBDGB_CUDA(cudaMemcpyAsync(dP, hp.data(), sizeof(BProb) * count, cudaMemcpyHostToDevice, s));
     SBDGB_CUDA(cudaMemcpyAsync(dch, chunks.data(), sizeof(Chunk) * nch, cudaMemcpyHostToDevice, s));
     int *pin = (int *)pinned_buffer(&c);
@@ -1201,7 +1259,10 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
         k_b_dots<T><<<nch, kT, 0, s>>>(g, 1);
         k_b_gs2<<<count, 32, 0, s>>>(g);
         k_b_newcols<T><<<nsub, kT, 0, s>>>(g);
-        k_b_sigma<T><<<nsub, kT, g.kp_smem ? sizeof(T) * npp_max : 0, s>>>(g);
+        if (slab)
+          slab_batch_sigma<T>(std::is_same<T, float>::value ? slab32 : slab64, s);
+        else
+          k_b_sigma<T><<<nsub, kT, g.kp_smem ? sizeof(T) * npp_max : 0, s>>>(g);
       };
       auto iteration = [&] {
         k_b_dots<T><<<nch, kT, 0, s>>>(g, 0);
@@ -1215,7 +1276,7 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
         ortho_sigma();
       };
       ortho_sigma();
-      count_launch(&c, 7);
+      count_launch(&c, slab ? 9 : 7);
       SBDGB_CUDA(cudaGetLastError());
       // the legacy default stream cannot be captured: launch directly there
       if (s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread) {
@@ -1234,7 +1295,7 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
             SBDGB_CUDA(cudaGraphLaunch(exec, s));
           else
             iteration();
-          count_launch(&c, kStepLaunches);
+          count_launch(&c, kStepLaunches + (slab ? 2 : 0));
         }
         SBDGB_CUDA(cudaGetLastError());
         k_b_count<<<1, 1024, 0, s>>>(dS, count, dcount);
@@ -1295,12 +1356,10 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
     }
   } catch (...) {
     if (exec) cudaGraphExecDestroy(exec);
-    tmp_free(&c, mb);
-    tmp_free(&c, arena);
+    cleanup();
     throw;
   }
-  tmp_free(&c, mb);
-  tmp_free(&c, arena);
+  cleanup();
 }
 
 }  // namespace sbdgb

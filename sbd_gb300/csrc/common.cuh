@@ -187,6 +187,7 @@ struct Problem {
     uint32_t *ab_ent = nullptr;  // the beta singles of ab_ent below, in this kernel's order
     uint2 *ab_items = nullptr;   // its CTAs: (alpha row, part | parts << 16), most batches first
     uint32_t n_ab_items = 0, ab_warps = 0;
+    std::vector<uint2> h_items;  // host copy of ab_items (the batched solver's grids)
     int2 *Jfx[2] = {};
     uint32_t nslices[2] = {}, groups[2] = {}, longest[2] = {};
     int ev[2] = {}, ek = 0;

@@ -307,4 +307,29 @@ void sigma_slab(const Problem &p, const sdev::Args<T> &x, bool block, cudaStream
 void sigma_slab_f32(const Problem &p, const sdev::Args<float> &x, const float *const *C, float *const *S, int nvec,
                     bool block, cudaStream_t s);
 
+// The batched solver's products by the same kernels, every problem's in one
+// grid.  State of problem i at i * stride bytes from the pointers (products only
+// where active: of basis columns [from, to)); V, HV: its basis and products.
+struct SlabBatchState {
+  const int *active, *from, *to;
+  size_t stride;
+  void *const *V, *const *HV;
+  const uint32_t *N;
+};
+struct SlabBatch {
+  void *args[3] = {};  // alpha, beta, alpha x beta
+  const uint4 *items[3] = {};
+  uint32_t n[3] = {};
+  size_t smem[3] = {};
+  int nvec = 0;
+  SlabBatchState state{};
+  std::vector<void *> tmps;  // its device memory (tmp_alloc)
+};
+bool slab_batch_fits(Problem **ps, int count, cudaStream_t s);
+template <typename T>
+void slab_batch_plan(SlabBatch &b, Ctx *c, Problem **ps, const sdev::Args<T> *args, int count,
+                     const SlabBatchState &state, int nvec, cudaStream_t s);
+template <typename T>
+void slab_batch_sigma(const SlabBatch &b, cudaStream_t s);
+
 }  // namespace sbdgb

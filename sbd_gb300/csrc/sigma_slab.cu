@@ -265,8 +265,10 @@ __device__ __forceinline__ void slab_list(fx::Acc (&acc)[K], const uint4 *__rest
   for (int c = 0; c < K; ++c) fx::carry(acc[c]);
 }
 
+// One CTA: column group `group`, every a.parts-th slice from `part`, of C into S.
 template <typename T, int K, bool kAlpha>
-__global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
+__device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restrict__ C, T *S, uint32_t group,
+                                         uint32_t part) {
   using F = Format<T>;
   constexpr int NQ = (K + 1) / 2;
   extern __shared__ __align__(16) unsigned char slab_smem[];
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
   int2 *J = X + (size_t)(a.n + 1) * K;               // (npair + 1) x K; row npair is zero
   __shared__ uint32_t skey[K], snext;
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
-  const uint32_t c0 = blockIdx.x * K;
+  const uint32_t c0 = group * K;
   auto diag = [&](size_t k) {
     if constexpr (std::is_same<T, double>::value)
       return ldg(a.hii + k);
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
     const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
     uint32_t key = 0u;
     for (uint32_t r = tid / K; r < a.n; r += nt / K) {
-      T x = ok ? ldg(a.C + (size_t)r * a.nb + (c0 + c)) : T(0.0);
+      T x = ok ? ldg(C + (size_t)r * a.nb + (c0 + c)) : T(0.0);
       if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
       key = max(key, F::key(x));
       X[staged<K>(a.n + 1, r, c)] = F::raw(x);
@@ -303,13 +305,13 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
     for (int c = 0; c < K; ++c) {
       const bool ok = c0 + c < a.m;
       const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
-      const T *row = a.C + (size_t)(c0 + c) * a.nb;
+      const T *row = C + (size_t)(c0 + c) * a.nb;
       uint32_t key = 0u;
       for (uint32_t r = tid; r < a.n; r += nt) {
         T x = ok ? ldg(row + r) : T(0.0);
         if (a.staged_diag && ok) {
           const size_t k = (size_t)(c0 + c) * a.nb + r;
-          a.S[k] = a.add ? fma(diag(k), x, a.S[k]) : diag(k) * x;
+          S[k] = a.add ? fma(diag(k), x, S[k]) : diag(k) * x;
         }
         if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
         key = max(key, F::key(x));
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
   while (true) {
     uint32_t sl = 0;
     if (lane == 0) sl = atomicAdd(&snext, 1u);
-    sl = blockIdx.y + a.parts * __shfl_sync(0xffffffffu, sl, 0);
+    sl = part + a.parts * __shfl_sync(0xffffffffu, sl, 0);
     if (sl >= t.nslices) break;
     const uint32_t row = ldg(t.rows + sl * 32u + lane);
     auto element = [&](int c) { return kAlpha ? (size_t)row * a.nb + (c0 + c) : (size_t)(c0 + c) * a.nb + row; };
@@ -364,11 +366,11 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
     T out[K], old[K];
     if (!kReduce<T> && add && row != ~0u) {
       if (whole) {
-        if constexpr (K == 4) load_row<K>(a.S + element(0), old);
+        if constexpr (K == 4) load_row<K>(S + element(0), old);
       } else {
 #pragma unroll
         for (int c = 0; c < K; ++c)
-          if (c0 + c < a.m) old[c] = a.S[element(c)];
+          if (c0 + c < a.m) old[c] = S[element(c)];
       }
     }
     if (!bad) {
@@ -398,19 +400,24 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
       T s = out[c];
       if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c0 + c))));
       const size_t k = element(c);
-      if (a.diag && !a.staged_diag) s = fma(diag(k), ldg(a.C + k), s);
+      if (a.diag && !a.staged_diag) s = fma(diag(k), ldg(C + k), s);
       if (whole) {
         out[c] = add ? old[c] + s : s;
       } else if (add) {
-        add_to(a.S + k, old[c], s);
+        add_to(S + k, old[c], s);
       } else {
-        a.S[k] = s;
+        S[k] = s;
       }
     }
     if (whole) {
-      if constexpr (K == 4) store_row<K>(a.S + element(0), out);
+      if constexpr (K == 4) store_row<K>(S + element(0), out);
     }
   }
+}
+
+template <typename T, int K, bool kAlpha>
+__global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
+  slab_cta<T, K, kAlpha>(a, a.C, a.S, blockIdx.x, blockIdx.y);
 }
 
 // ---- the same sweep in FP32 -------------------------------------------------------
@@ -489,15 +496,14 @@ __device__ __forceinline__ void slab_list_f32(float (&acc)[K], const uint4 *__re
 }
 
 template <int K, bool kAlpha>
-__global__ void __launch_bounds__(kSlabThreads) k_slab_f32(SlabArgsF a) {
+__device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__restrict__ C, float *S, uint32_t group,
+                                             uint32_t part) {
   extern __shared__ __align__(16) unsigned char slab_smem[];
   float *X = reinterpret_cast<float *>(slab_smem);  // planes of four columns, n + 1 rows; row n is zero
   float *J = X + (size_t)(a.n + 1) * K;             // the same, npair + 1 rows
   __shared__ uint32_t snext;
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
-  const uint32_t c0 = blockIdx.x * K;
-  const float *C = a.C[blockIdx.z];
-  float *S = a.S[blockIdx.z];
+  const uint32_t c0 = group * K;
   auto place = [](uint32_t rows, uint32_t r, uint32_t c) { return ((size_t)(c >> 2) * rows + r) * 4 + (c & 3u); };
   if (tid == 0) snext = 0u;
   if constexpr (kAlpha) {
@@ -534,7 +540,7 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab_f32(SlabArgsF a) {
   while (true) {
     uint32_t sl = 0;
     if (lane == 0) sl = atomicAdd(&snext, 1u);
-    sl = blockIdx.y + a.parts * __shfl_sync(0xffffffffu, sl, 0);
+    sl = part + a.parts * __shfl_sync(0xffffffffu, sl, 0);
     if (sl >= t.nslices) break;
     const uint32_t row = ldg(t.rows + sl * 32u + lane);
     auto element = [&](int c) { return kAlpha ? (size_t)row * a.nb + (c0 + c) : (size_t)(c0 + c) * a.nb + row; };
@@ -587,6 +593,11 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab_f32(SlabArgsF a) {
   }
 }
 
+template <int K, bool kAlpha>
+__global__ void __launch_bounds__(kSlabThreads) k_slab_f32(SlabArgsF a) {
+  slab_cta_f32<K, kAlpha>(a, a.C[blockIdx.z], a.S[blockIdx.z], blockIdx.x, blockIdx.y);
+}
+
 // ---- alpha single x beta single (task type 0) ---------------------------------------
 //
 // The layout of k_sigma_ab (sigma_ab.cu): a CTA owns one alpha row (or every
@@ -619,7 +630,7 @@ struct SlabAbArgs {
 };
 
 template <typename T, int G, bool kSum>
-__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
+__device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__restrict__ C, T *S, uint2 item) {
   using F = Format<T>;
   constexpr int NP = G / 2;
   extern __shared__ __align__(16) unsigned char slab_smem[];
@@ -630,7 +641,6 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
   double *Ss = reinterpret_cast<double *>(Ks + NP * kplane);     // kSum: [nb]
   __shared__ uint32_t skey[G];
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
-  const uint2 item = __ldg(a.items + blockIdx.x);
   const uint32_t ia = item.x, part = item.y & 0xffffu, parts = item.y >> 16;
   const uint32_t p0 = ldg(a.off + ia), p1 = ldg(a.off + ia + 1);
   const uint64_t str = a.eta ? ldg(a.astr + ia) : 0ull;
@@ -651,7 +661,7 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
       const bool ok0 = 2 * h < live, ok1 = 2 * h + 1 < live;
       const uint32_t ja0 = ok0 ? ldg(a.ket + pb + 2 * h) : 0u, ja1 = ok1 ? ldg(a.ket + pb + 2 * h + 1) : 0u;
       const uint64_t s0 = a.eta && ok0 ? ldg(a.astr + ja0) : 0ull, s1 = a.eta && ok1 ? ldg(a.astr + ja1) : 0ull;
-      const T *r0 = a.C + (size_t)ja0 * a.nb, *r1 = a.C + (size_t)ja1 * a.nb;
+      const T *r0 = C + (size_t)ja0 * a.nb, *r1 = C + (size_t)ja1 * a.nb;
       for (uint32_t c = tid; c < a.nb; c += nt) {
         T x0 = ok0 ? ldg(r0 + c) : T(0.0), x1 = ok1 ? ldg(r1 + c) : T(0.0);
         if (a.eta) {
@@ -732,7 +742,7 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
       };
       load(at);
       const uint32_t ib = k < a.nb ? ldg(a.cols + k) : 0u;
-      T *const to = a.S + ((size_t)ia * a.nb + ib);
+      T *const to = S + ((size_t)ia * a.nb + ib);
       const T old = !kSum && !kReduce<T> && k < a.nb ? *to : T(0.0);
       double sum = 0.0;
       if (fixed) {
@@ -795,7 +805,7 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
     for (uint32_t c = tid; c < a.nb; c += nt) {
       double s = Ss[c];
       if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c))));
-      add_row(a.S + ((size_t)ia * a.nb + c), s);
+      add_row(S + ((size_t)ia * a.nb + c), s);
     }
   } else {
     for (uint32_t i = warp; i < mine; i += nw) {
@@ -804,9 +814,14 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
       const uint32_t ib = ldg(a.cols + k);
       double s = Ss[ib];
       if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + ib))));
-      add_row(a.S + ((size_t)ia * a.nb + ib), s);
+      add_row(S + ((size_t)ia * a.nb + ib), s);
     }
   }
+}
+
+template <typename T, int G, bool kSum>
+__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab(SlabAbArgs<T> a) {
+  slab_ab_cta<T, G, kSum>(a, a.C, a.S, __ldg(a.items + blockIdx.x));
 }
 
 // FP32: four ket rows' values at a column are 16 bytes, four (P|Q) rows' at a
@@ -823,14 +838,13 @@ struct SlabAbArgsF {
   int npair, eta;
 };
 
-__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab_f32(SlabAbArgsF a) {
+__device__ __forceinline__ void slab_ab_cta_f32(const SlabAbArgsF &a, const float *__restrict__ C, float *S,
+                                                uint2 item) {
   extern __shared__ __align__(16) unsigned char slab_smem[];
   float4 *Cs = reinterpret_cast<float4 *>(slab_smem);               // [nb + 1]
   float4 *Ks = Cs + a.nb + 1;                                       // [2 Q + phase]
   float *Ss = reinterpret_cast<float *>(Ks + 2 * (a.npair + 1));    // [nb]
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
-  const float *C = a.C[blockIdx.z];
-  const uint2 item = __ldg(a.items + blockIdx.x);
   const uint32_t ia = item.x, part = item.y & 0xffffu, parts = item.y >> 16;
   const uint32_t p0 = ldg(a.off + ia), p1 = ldg(a.off + ia + 1);
   const uint32_t mine = (a.nslices - part + parts - 1) / parts;
@@ -903,7 +917,7 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab_f32(SlabAbArgsF a) {
   }
   __syncthreads();
   const uint64_t istr = a.eta ? ldg(a.astr + ia) : 0ull;
-  float *srow = a.S[blockIdx.z] + (size_t)ia * a.nb;
+  float *srow = S + (size_t)ia * a.nb;
   auto add = [&](uint32_t c) {
     float s = Ss[c];
     if (a.eta) s = flip(s, parity((unsigned long long)(istr & ldg(a.colmask + c))));
@@ -917,6 +931,62 @@ __global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab_f32(SlabAbArgsF a) {
       if (k < a.nb) add(ldg(a.cols + k));
     }
   }
+}
+
+__global__ void __launch_bounds__(kSlabAbThreads) k_slab_ab_f32(SlabAbArgsF a) {
+  slab_ab_cta_f32(a, a.C[blockIdx.z], a.S[blockIdx.z], __ldg(a.items + blockIdx.x));
+}
+
+// ---- many problems at once (batch.cu) ----------------------------------------------
+//
+// The CTAs of every problem's sweep in one grid; blockIdx.y numbers the new
+// vectors of a problem's step (columns from + y of its basis), whose count and
+// activity each CTA reads from the solver's state.
+template <typename A>
+struct SlabMany {
+  const A *args;        // per problem
+  const uint4 *items;   // (problem, group or row, part or part | parts << 16, -)
+  SlabBatchState state;
+};
+constexpr int kManyThreads = 256;
+
+template <typename T, typename A>
+__device__ __forceinline__ bool many_vector(const SlabMany<A> &m, uint32_t prob, const T *&C, T *&S) {
+  const SlabBatchState &st = m.state;
+  auto field = [&](const int *f) { return *reinterpret_cast<const int *>(reinterpret_cast<const char *>(f) + prob * st.stride); };
+  const int from = field(st.from), to = field(st.to);
+  if (!field(st.active) || from + (int)blockIdx.y >= to) return false;
+  const size_t at = (size_t)st.N[prob] * (from + blockIdx.y);
+  C = reinterpret_cast<const T *>(st.V[prob]) + at;
+  S = reinterpret_cast<T *>(st.HV[prob]) + at;
+  return true;
+}
+template <int K, bool kAlpha>
+__global__ void __launch_bounds__(kManyThreads, 3) k_slab_many(SlabMany<SlabArgs<double>> m) {
+  const uint4 it = __ldg(m.items + blockIdx.x);
+  const double *C;
+  double *S;
+  if (many_vector(m, it.x, C, S)) slab_cta<double, K, kAlpha>(m.args[it.x], C, S, it.y, it.z);
+}
+template <int K, bool kAlpha>
+__global__ void __launch_bounds__(kManyThreads, 3) k_slab_many_f32(SlabMany<SlabArgsF> m) {
+  const uint4 it = __ldg(m.items + blockIdx.x);
+  const float *C;
+  float *S;
+  if (many_vector(m, it.x, C, S)) slab_cta_f32<K, kAlpha>(m.args[it.x], C, S, it.y, it.z);
+}
+template <int G>
+__global__ void __launch_bounds__(kManyThreads, 3) k_slab_ab_many(SlabMany<SlabAbArgs<double>> m) {
+  const uint4 it = __ldg(m.items + blockIdx.x);
+  const double *C;
+  double *S;
+  if (many_vector(m, it.x, C, S)) slab_ab_cta<double, G, true>(m.args[it.x], C, S, make_uint2(it.y, it.z));
+}
+__global__ void __launch_bounds__(kManyThreads, 3) k_slab_ab_many_f32(SlabMany<SlabAbArgsF> m) {
+  const uint4 it = __ldg(m.items + blockIdx.x);
+  const float *C;
+  float *S;
+  if (many_vector(m, it.x, C, S)) slab_ab_cta_f32(m.args[it.x], C, S, make_uint2(it.y, it.z));
 }
 
 // ---- tables -----------------------------------------------------------------------
@@ -1284,6 +1354,7 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
     const uint32_t rounds = (mine + kSlabAbThreads / 32 - 1) / (kSlabAbThreads / 32);
     p.slab.ab_warps = std::max<uint32_t>(4, (mine + rounds - 1) / rounds);
     p.slab.n_ab_items = (uint32_t)items.size();
+    p.slab.h_items = items;
     p.slab.ab_items = (uint2 *)dev_alloc(p, 8 * items.size());
     SBDGB_CUDA(cudaMemcpyAsync(p.slab.ab_items, items.data(), 8 * items.size(), cudaMemcpyHostToDevice, s));
     p.slab.ab_ent = (uint32_t *)dev_alloc(p, 4 * p.ab_entries);
@@ -1373,7 +1444,7 @@ SlabSpin slab_spin(const Problem &p, int sp) {
 }
 
 template <typename T, bool kAlpha>
-void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta, cudaStream_t s) {
+SlabArgs<T> slab_args(const Problem &p, const Args<T> &x, int add, int diag, int eta) {
   constexpr int sp = kAlpha ? 0 : 1;
   SlabArgs<T> a{};
   a.C = x.C;
@@ -1398,10 +1469,18 @@ void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta,
   a.eta = eta;
   a.add = add;
   a.diag = diag;
-  const SlabShape c = slab_shape(p, sp, a.n, a.m, a.npair, 8, 4, 1, 1);
-  a.parts = c.parts;
-  a.staged_diag = diag && !kAlpha && c.parts == 1;
+  a.parts = 1;
+  a.staged_diag = diag && !kAlpha;
   a.vec = p.nb % 2 == 0 && ((uintptr_t)x.S & 15u) == 0;
+  return a;
+}
+
+template <typename T, bool kAlpha>
+void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta, cudaStream_t s) {
+  SlabArgs<T> a = slab_args<T, kAlpha>(p, x, add, diag, eta);
+  const SlabShape c = slab_shape(p, kAlpha ? 0 : 1, a.n, a.m, a.npair, 8, 4, 1, 1);
+  a.parts = c.parts;
+  a.staged_diag = a.staged_diag && c.parts == 1;
   const dim3 g(c.groups, c.parts);
   switch (c.K) {
     case 4: go_slab(k_slab<T, 4, kAlpha>, a, g, c.warps, c.smem, s); break;
@@ -1413,14 +1492,9 @@ void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta,
 }
 
 template <bool kAlpha>
-void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec, int add,
-                     int diag, int eta, cudaStream_t s) {
+SlabArgsF slab_args_f32(const Problem &p, const Args<float> &x, int add, int diag, int eta) {
   constexpr int sp = kAlpha ? 0 : 1;
   SlabArgsF a{};
-  for (int v = 0; v < nvec; ++v) {
-    a.C[v] = C[v];
-    a.S[v] = S[v];
-  }
   a.hii_df = x.hii_df;
   a.hii_f = x.hii_f;
   a.shift = x.shift_df;
@@ -1437,9 +1511,21 @@ void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const 
   a.eta = eta;
   a.add = add;
   a.diag = diag;
+  a.parts = 1;
+  return a;
+}
+
+template <bool kAlpha>
+void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec, int add,
+                     int diag, int eta, cudaStream_t s) {
+  SlabArgsF a = slab_args_f32<kAlpha>(p, x, add, diag, eta);
   a.vec = p.nb % 4 == 0;
-  for (int v = 0; v < nvec; ++v) a.vec = a.vec && ((uintptr_t)S[v] & 15u) == 0;
-  const SlabShape c = slab_shape(p, sp, a.n, a.m, a.npair, 4, 8, 4, nvec);
+  for (int v = 0; v < nvec; ++v) {
+    a.C[v] = C[v];
+    a.S[v] = S[v];
+    a.vec = a.vec && ((uintptr_t)S[v] & 15u) == 0;
+  }
+  const SlabShape c = slab_shape(p, kAlpha ? 0 : 1, a.n, a.m, a.npair, 4, 8, 4, nvec);
   a.parts = c.parts;
   const dim3 g(c.groups, c.parts, nvec);
   if (c.K == 8)
@@ -1451,7 +1537,7 @@ void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const 
 }
 
 template <typename T>
-void launch_slab_ab(const Problem &p, const Args<T> &x, int eta, cudaStream_t s) {
+SlabAbArgs<T> slab_ab_args(const Problem &p, const Args<T> &x, int eta) {
   SlabAbArgs<T> a{};
   a.C = x.C;
   a.S = x.S;
@@ -1470,6 +1556,12 @@ void launch_slab_ab(const Problem &p, const Args<T> &x, int eta, cudaStream_t s)
   a.npair = p.npair;
   a.ek = p.slab.ek;
   a.eta = eta;
+  return a;
+}
+
+template <typename T>
+void launch_slab_ab(const Problem &p, const Args<T> &x, int eta, cudaStream_t s) {
+  const SlabAbArgs<T> a = slab_ab_args<T>(p, x, eta);
   const uint32_t warps = p.slab.ab_warps;
   const dim3 g(p.slab.n_ab_items);
   if (!slab_ab_sum(p))
@@ -1482,13 +1574,8 @@ void launch_slab_ab(const Problem &p, const Args<T> &x, int eta, cudaStream_t s)
   SBDGB_CUDA(cudaGetLastError());
 }
 
-void launch_slab_ab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec,
-                        int eta, cudaStream_t s) {
+SlabAbArgsF slab_ab_args_f32(const Problem &p, const Args<float> &x, int eta) {
   SlabAbArgsF a{};
-  for (int v = 0; v < nvec; ++v) {
-    a.C[v] = C[v];
-    a.S[v] = S[v];
-  }
   a.astr = p.astr;
   a.colmask = p.slab.mask[1];
   a.off = p.A.off_s;
@@ -1503,6 +1590,16 @@ void launch_slab_ab_f32(const Problem &p, const Args<float> &x, const float *con
   a.nb = p.nb;
   a.npair = p.npair;
   a.eta = eta;
+  return a;
+}
+
+void launch_slab_ab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec,
+                        int eta, cudaStream_t s) {
+  SlabAbArgsF a = slab_ab_args_f32(p, x, eta);
+  for (int v = 0; v < nvec; ++v) {
+    a.C[v] = C[v];
+    a.S[v] = S[v];
+  }
   const uint32_t warps = p.slab.ab_warps;
   go_slab(k_slab_ab_f32, a, dim3(p.slab.n_ab_items, 1, nvec), warps, slab_ab_smem_bytes_f32(p), s);
   count_launch(p.ctx);
@@ -1534,5 +1631,114 @@ void sigma_slab_f32(const Problem &p, const Args<float> &x, const float *const *
   if (p.A.ns > 0 && p.B.ns > 0) launch_slab_ab_f32(p, x, C, S, nvec, eta, s);
   if (beta) launch_slab_f32<false>(p, x, C, S, nvec, alpha, 1, eta, s);
 }
+
+// ---- the batched solver's products ----------------------------------------------------
+
+namespace {
+constexpr int kManyK = 4, kManyKF = 8;
+
+template <typename A>
+A *to_device(Ctx *c, std::vector<void *> &tmps, const std::vector<A> &v, cudaStream_t s) {
+  A *d = (A *)tmp_alloc(c, sizeof(A) * v.size());
+  tmps.push_back(d);
+  SBDGB_CUDA(cudaMemcpyAsync(d, v.data(), sizeof(A) * v.size(), cudaMemcpyHostToDevice, s));
+  return d;
+}
+}  // namespace
+
+// False when some problem's tables do not apply or the CTAs would not fit.
+bool slab_batch_fits(Problem **ps, int count, cudaStream_t s) {
+  const size_t limit = max_smem();
+  for (int i = 0; i < count; ++i) {
+    Problem &p = *ps[i];
+    const uint32_t n = std::max(p.na, p.nb);
+    if (p.A.ns + p.A.nd == 0 || p.B.ns + p.B.nd == 0) return false;
+    if ((size_t)8 * kManyK * (n + 1 + p.npair + 1) > limit || slab_ab_smem_bytes(p, 4, true) > limit) return false;
+    if (!slab_prepare(p, s)) return false;
+  }
+  return true;
+}
+
+template <typename T>
+void slab_batch_plan(SlabBatch &b, Ctx *c, Problem **ps, const sdev::Args<T> *args, int count,
+                     const SlabBatchState &state, int nvec, cudaStream_t s) {
+  constexpr bool kF32 = std::is_same<T, float>::value;
+  using S = typename std::conditional<kF32, SlabArgsF, SlabArgs<double>>::type;
+  using AB = typename std::conditional<kF32, SlabAbArgsF, SlabAbArgs<double>>::type;
+  std::vector<S> sa, sb;
+  std::vector<AB> ab;
+  std::vector<uint4> ia, ib, iab;
+  b.state = state;
+  b.nvec = nvec;
+  for (int i = 0; i < count; ++i) {
+    const Problem &p = *ps[i];
+    if constexpr (kF32) {
+      sa.push_back(slab_args_f32<true>(p, args[i], 0, 0, 1));
+      sb.push_back(slab_args_f32<false>(p, args[i], 1, 1, 1));
+      ab.push_back(slab_ab_args_f32(p, args[i], 1));
+    } else {
+      sa.push_back(slab_args<double, true>(p, args[i], 0, 0, 1));
+      sb.push_back(slab_args<double, false>(p, args[i], 1, 1, 1));
+      ab.push_back(slab_ab_args<double>(p, args[i], 1));
+      sa.back().vec = sb.back().vec = 0;  // a column of the basis may start anywhere
+    }
+    const int K = kF32 ? kManyKF : kManyK, el = kF32 ? 4 : 8;
+    for (uint32_t g = 0; g < (p.nb + K - 1) / K; ++g) ia.push_back(make_uint4(i, g, 0, 0));
+    for (uint32_t g = 0; g < (p.na + K - 1) / K; ++g) ib.push_back(make_uint4(i, g, 0, 0));
+    for (const uint2 &it : p.slab.h_items) iab.push_back(make_uint4(i, it.x, it.y, 0));
+    auto smem = [&](uint32_t n, uint64_t ns) { return (size_t)el * K * (n + 1 + (ns ? p.npair + 1 : 0)); };
+    b.smem[0] = std::max(b.smem[0], smem(p.na, p.A.ns));
+    b.smem[1] = std::max(b.smem[1], smem(p.nb, p.B.ns));
+    b.smem[2] = std::max(b.smem[2], kF32 ? slab_ab_smem_bytes_f32(p) : slab_ab_smem_bytes(p, 4, true));
+  }
+  b.args[0] = to_device(c, b.tmps, sa, s);
+  b.args[1] = to_device(c, b.tmps, sb, s);
+  b.args[2] = to_device(c, b.tmps, ab, s);
+  b.items[0] = to_device(c, b.tmps, ia, s);
+  b.items[1] = to_device(c, b.tmps, ib, s);
+  b.items[2] = to_device(c, b.tmps, iab, s);
+  b.n[0] = (uint32_t)ia.size();
+  b.n[1] = (uint32_t)ib.size();
+  b.n[2] = (uint32_t)iab.size();
+  SBDGB_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
+  auto limit = [&](auto k, int i) {
+    ensure_dynamic_smem((const void *)k, b.smem[i]);
+    prefer_shared_carveout((const void *)k);
+  };
+  if constexpr (kF32) {
+    limit(k_slab_many_f32<kManyKF, true>, 0);
+    limit(k_slab_many_f32<kManyKF, false>, 1);
+    limit(k_slab_ab_many_f32, 2);
+  } else {
+    limit(k_slab_many<kManyK, true>, 0);
+    limit(k_slab_many<kManyK, false>, 1);
+    limit(k_slab_ab_many<4>, 2);
+  }
+}
+template void slab_batch_plan<double>(SlabBatch &, Ctx *, Problem **, const sdev::Args<double> *, int,
+                                      const SlabBatchState &, int, cudaStream_t);
+template void slab_batch_plan<float>(SlabBatch &, Ctx *, Problem **, const sdev::Args<float> *, int,
+                                     const SlabBatchState &, int, cudaStream_t);
+
+template <typename T>
+void slab_batch_sigma(const SlabBatch &b, cudaStream_t s) {
+  constexpr bool kF32 = std::is_same<T, float>::value;
+  using S = typename std::conditional<kF32, SlabArgsF, SlabArgs<double>>::type;
+  using AB = typename std::conditional<kF32, SlabAbArgsF, SlabAbArgs<double>>::type;
+  auto sweep = [&](int i) { return SlabMany<S>{(const S *)b.args[i], b.items[i], b.state}; };
+  const SlabMany<AB> ab{(const AB *)b.args[2], b.items[2], b.state};
+  const dim3 ga(b.n[0], b.nvec), gb(b.n[1], b.nvec), gab(b.n[2], b.nvec);
+  if constexpr (kF32) {
+    k_slab_many_f32<kManyKF, true><<<ga, kManyThreads, b.smem[0], s>>>(sweep(0));
+    if (b.n[2]) k_slab_ab_many_f32<<<gab, kManyThreads, b.smem[2], s>>>(ab);
+    k_slab_many_f32<kManyKF, false><<<gb, kManyThreads, b.smem[1], s>>>(sweep(1));
+  } else {
+    k_slab_many<kManyK, true><<<ga, kManyThreads, b.smem[0], s>>>(sweep(0));
+    if (b.n[2]) k_slab_ab_many<4><<<gab, kManyThreads, b.smem[2], s>>>(ab);
+    k_slab_many<kManyK, false><<<gb, kManyThreads, b.smem[1], s>>>(sweep(1));
+  }
+}
+template void slab_batch_sigma<double>(const SlabBatch &, cudaStream_t);
+template void slab_batch_sigma<float>(const SlabBatch &, cudaStream_t);
 
 }  // namespace sbdgb

@@ -75,3 +75,30 @@ def test_mixed_batch_moves_sigma_products_to_fp32(engine):
     finally:
         for t in tps:
             t.close()
+
+
+# shapes whose products go by the kernels of sigma_slab.cu (32 nonzeros a row or more
+# over the batch): a slice's edges, odd lengths, one problem, a sparse one among others
+@pytest.mark.parametrize("shapes,nroots", [([(97, 33)], 1), ([(33, 31), (300, 64), (65, 300)], 3),
+                                           ([(495, 130), (60, 60), (201, 495), (64, 32)], 2)])
+def test_mixed_batch_of_dense_problems(engine, shapes, nroots):
+    """Eigenpairs of the oracle's H: with a residual r an energy is off by at most
+    r^2 over its gap and r; 1e-9 and twice the tolerance of 1e-8 for r."""
+    from oracle.oracle import Oracle
+    from sbd_gb300.engine import TPBProblem, batch_davidson
+    from sbd_gb300.generators import make_problem
+    probs = [make_problem(12, 4, 4, na, nb, seed=na * nb) for na, nb in shapes]
+    tps = [TPBProblem.from_problem(engine, p) for p in probs]
+    try:
+        a = batch_davidson(engine, tps, nroots=nroots, max_nb=20, eps=1e-8)
+        b = batch_davidson(engine, tps, nroots=nroots, max_nb=20, eps=1e-8, precision=1, want_vectors=True)
+        for p, x, y in zip(probs, a, b):
+            assert x.report["converged"] and y.report["converged"]
+            assert np.abs(x.energies - y.energies).max() <= 1e-9
+            o = Oracle.from_problem(p)
+            for e, v in zip(y.energies, y.vectors):
+                assert abs(np.linalg.norm(v) - 1) <= 1e-10
+                assert np.linalg.norm(o.mult(v) - e * v) <= 2e-8
+    finally:
+        for t in tps:
+            t.close()
