@@ -16,8 +16,9 @@ diagonal resident, starting from the lowest diagonal entries).
           stream during the timed region; algorithmic bytes per product are
           24*N + 8*nnz_off (read C and hii, write sigma, one 8-byte C read per
           off-diagonal element).  roofline.fp64 gives the same product against
-          the measured FP64 FMA rate (one FMA per nonzero), which is what
-          bounds these kernels on this GPU
+          the measured FP64 FMA rate (one FMA per nonzero): the roof of the
+          FP64 kernels; the fixed-point ones (k_slab) add in integers and may
+          pass it
   cpu_baseline : the CPU oracle port of the reference's TRADMODE sigma (OpenMP,
           all host cores) timed on a bounded sample of alpha rows and scaled to
           the solve's sigma count
@@ -555,8 +556,8 @@ def run_gpu(args):
     sigma_ms_per = sigma_ms / max(ncalls, 1)
     achieved = bytes_sigma / (sigma_ms_per * 1e-3) / 1e9
     peak, peak_kind = peaks()
-    # the sigma kernels are bound by the FP64 FMA pipe: one FMA per off-diagonal
-    # element and per diagonal element, against the measured FP64 FMA rate
+    # one FMA per off-diagonal element and per diagonal element against the measured
+    # FP64 FMA rate, the roof of the FP64 kernels (k_slab adds in integers)
     rates = measure_fp64_rates(local)
     fp64_achieved = 2.0 * (nnz_off + N) / (sigma_ms_per * 1e-3) / 1e12
     tiles = p.tuning(3)  # the solver's products: FP64 in the block ordering
@@ -598,9 +599,9 @@ def run_gpu(args):
     if rank == 0 and not args.no_config3:
         config3 = config3_block(eng, peak, peak_kind)
 
-    traffic = None
+    traffic = None  # the capture is of the FP64 kernels
     prof_path = os.path.join(ROOT, "profiles", "sigma_traffic.json")
-    if os.path.exists(prof_path):
+    if os.path.exists(prof_path) and tiles.get("beta_shape") != "slab":
         try:
             with open(prof_path) as f:
                 traffic = float(json.load(f)["bytes_per_sigma_config1"])
@@ -675,7 +676,8 @@ def run_gpu(args):
             "sigma_tiles": tiles,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": ("sigma operator (fused k_sigma_alpha)" if tiles.get("beta_shape") == "fused"
+                         "kernel": ("sigma operator (k_slab + k_slab_ab)" if tiles.get("beta_shape") == "slab"
+                                    else "sigma operator (fused k_sigma_alpha)" if tiles.get("beta_shape") == "fused"
                                     else "sigma operator (k_transpose + k_sigma_alpha + k_sigma_beta)"),
                          "algorithmic_bytes": bytes_sigma, "peak_kind": f"{peak_kind} hbm_gbs",
                          "fp64": {"unit": "TFLOP/s", "achieved": fp64_achieved, "peak": rates["dfma_tflops"],
