@@ -279,7 +279,9 @@ void build_row_pairs(Problem &p, const std::vector<uint32_t> &off_s, const std::
                      const std::vector<uint32_t> &rows, cudaStream_t s);
 template <typename T>
 bool rows_fit(const Problem &p);
-// sigma_slab.cu: whether its kernels apply (their tables are built on first use).
+// sigma_slab.cu: whether its kernels apply (their tables are built on first use),
+// and whether those of a form (8-byte elements, or FP32) fit in shared memory.
+bool slab_fits(const Problem &p, int element);
 bool slab_prepare(Problem &p, cudaStream_t s);
 // block: the block-ordering product (H_block = eta H eta, no opposite-spin
 // parities) that the solvers use on eta-signed vectors; false: the

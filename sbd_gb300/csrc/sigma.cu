@@ -838,8 +838,10 @@ inline double nnz_per_row(const Problem &p) {
 // ordering the double-float sweeps are not bound by phases and win up to about
 // 100 (ms, sweeps and slab: 2011 x 1703, 58 a row, 0.47 and 0.53; 6000 x 6000,
 // 78, 3.9 and 4.5; 800 x 800, 605, 1.33 and 0.71).
+// Where a form's kernels need more shared memory than there is, it keeps the others.
 template <typename T, bool kB>
 bool slab_pays(const Problem &p) {
+  if (!slab_fits(p, sizeof(T))) return false;
   const double nnz = nnz_per_row(p);
   if (nnz >= 100.0) return true;
   if (kB && std::is_same<T, dfloat>::value) return false;

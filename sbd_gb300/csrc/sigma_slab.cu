@@ -51,6 +51,7 @@
 #include "common.cuh"
 #include "fx.cuh"
 #include "sigma_dev.cuh"
+#include "slab_fit.h"
 
 namespace sbdgb {
 
@@ -1185,35 +1186,26 @@ size_t max_smem() {
   SBDGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   return (size_t)optin - 1024;  // the kernels' static part
 }
-size_t slab_smem_bytes(int K, uint32_t n, int npair) {
-  return 8ull * K * ((size_t)n + 1 + (npair ? (size_t)npair + 1 : 0));
-}
-size_t slab_ab_smem_bytes(const Problem &p, int G, bool sum) {
-  return 8ull * G * ((size_t)p.nb + 1 + 2 * ((size_t)p.npair + 1)) + (sum ? 8ull * p.nb : 0);
-}
-size_t slab_ab_smem_bytes_f32(const Problem &p) {
-  return 16ull * ((size_t)p.nb + 1 + 2 * ((size_t)p.npair + 1)) + 4ull * p.nb;
-}
-
-// Whether a row's alpha x beta sums stay in shared memory between batches: not
-// where rows have a batch or two.
-bool slab_ab_sum(const Problem &p) { return (double)p.A.ns * (double)p.B.ns >= 8.0 * (double)p.N; }
+SlabSize slab_size(const Problem &p) { return {p.na, p.nb, p.npair, {p.A.ns, p.B.ns}}; }
+size_t slab_ab_smem_bytes(const Problem &p, int G, bool sum) { return sbdgb::slab_ab_smem_bytes(p.nb, p.npair, G, sum); }
+bool slab_ab_sum(const Problem &p) { return slab_size(p).ab_sum(); }
 
 }  // namespace
 
 // ---- host side ----------------------------------------------------------------------
 
+// Whether the kernels of a form (element: 8 bytes, or 4 in FP32) have the shared
+// memory that this problem takes.
+bool slab_fits(const Problem &p, int element) { return slab_fits(slab_size(p), element, max_smem()); }
+
 // Builds the sliced tables on first use.  False where the kernels do not apply
-// or a budget has no room for their tables.
+// to 8-byte elements or a budget has no room for their tables.
 bool slab_prepare(Problem &p, cudaStream_t s) {
   if (p.slab.state >= 0) return p.slab.state == 1;
   p.slab.state = 0;
-  const size_t limit = max_smem();
-  const uint32_t nmax = std::max(p.na, p.nb);
-  if (nmax >= kSlabMaxRows || (uint32_t)p.npair + 1 >= kSlabMaxPair) return false;
-  if (slab_smem_bytes(1, nmax, p.npair) > limit) return false;
+  if (std::max(p.na, p.nb) >= kSlabMaxRows || (uint32_t)p.npair + 1 >= kSlabMaxPair) return false;
   const bool ab = p.A.ns > 0 && p.B.ns > 0;
-  if (ab && (p.n_ab_rows == 0 || slab_ab_smem_bytes(p, 2, slab_ab_sum(p)) > limit)) return false;
+  if (!slab_fits(p, 8) || (ab && p.n_ab_rows == 0)) return false;
   // the largest table values
   unsigned long long *mx = (unsigned long long *)workspace(p, WS_RED2, 8 * sizeof(unsigned long long));
   SBDGB_CUDA(cudaMemsetAsync(mx, 0, 8 * sizeof(unsigned long long), s));
@@ -1394,8 +1386,8 @@ SlabShape slab_shape(const Problem &p, int sp, uint32_t n, uint32_t m, int npair
   const uint32_t nslices = p.slab.nslices[sp];
   double cost = 0.0;
   for (int K = Kmax; K >= Kmin; K >>= 1) {
-    const size_t smem = (size_t)element * K * ((size_t)n + 1 + (npair ? (size_t)npair + 1 : 0));
-    if (smem > limit && K > Kmin) continue;
+    const size_t smem = slab_smem_bytes(element, K, n, npair);
+    if (smem > limit) continue;
     const uint32_t groups = (m + K - 1) / K;
     const uint32_t resident = smem <= limit / 3 ? 3 : smem <= limit / 2 ? 2 : 1, slots = resident * sms;
     const double stage = (1.1 * n + 0.5 * npair) * K * (element == 8 ? 1.0 : 0.5);
@@ -1420,6 +1412,7 @@ SlabShape slab_shape(const Problem &p, int sp, uint32_t n, uint32_t m, int npair
       }
     }
   }
+  SBDGB_REQUIRE(best.K > 0, SBDGB_E_UNSUPPORTED, "sigma's columns do not fit in shared memory");  // slab_fits
   return best;
 }
 
@@ -1478,7 +1471,7 @@ SlabArgs<T> slab_args(const Problem &p, const Args<T> &x, int add, int diag, int
 template <typename T, bool kAlpha>
 void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta, cudaStream_t s) {
   SlabArgs<T> a = slab_args<T, kAlpha>(p, x, add, diag, eta);
-  const SlabShape c = slab_shape(p, kAlpha ? 0 : 1, a.n, a.m, a.npair, 8, 4, 1, 1);
+  const SlabShape c = slab_shape(p, kAlpha ? 0 : 1, a.n, a.m, a.npair, 8, 4, kSlabMinK, 1);
   a.parts = c.parts;
   a.staged_diag = a.staged_diag && c.parts == 1;
   const dim3 g(c.groups, c.parts);
@@ -1525,7 +1518,7 @@ void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const 
     a.S[v] = S[v];
     a.vec = a.vec && ((uintptr_t)S[v] & 15u) == 0;
   }
-  const SlabShape c = slab_shape(p, kAlpha ? 0 : 1, a.n, a.m, a.npair, 4, 8, 4, nvec);
+  const SlabShape c = slab_shape(p, kAlpha ? 0 : 1, a.n, a.m, a.npair, 4, 8, kSlabMinKF, nvec);
   a.parts = c.parts;
   const dim3 g(c.groups, c.parts, nvec);
   if (c.K == 8)
@@ -1601,7 +1594,7 @@ void launch_slab_ab_f32(const Problem &p, const Args<float> &x, const float *con
     a.S[v] = S[v];
   }
   const uint32_t warps = p.slab.ab_warps;
-  go_slab(k_slab_ab_f32, a, dim3(p.slab.n_ab_items, 1, nvec), warps, slab_ab_smem_bytes_f32(p), s);
+  go_slab(k_slab_ab_f32, a, dim3(p.slab.n_ab_items, 1, nvec), warps, slab_ab_smem_bytes_f32(p.nb, p.npair), s);
   count_launch(p.ctx);
   SBDGB_CUDA(cudaGetLastError());
 }
@@ -1689,7 +1682,7 @@ void slab_batch_plan(SlabBatch &b, Ctx *c, Problem **ps, const sdev::Args<T> *ar
     auto smem = [&](uint32_t n, uint64_t ns) { return (size_t)el * K * (n + 1 + (ns ? p.npair + 1 : 0)); };
     b.smem[0] = std::max(b.smem[0], smem(p.na, p.A.ns));
     b.smem[1] = std::max(b.smem[1], smem(p.nb, p.B.ns));
-    b.smem[2] = std::max(b.smem[2], kF32 ? slab_ab_smem_bytes_f32(p) : slab_ab_smem_bytes(p, 4, true));
+    b.smem[2] = std::max(b.smem[2], kF32 ? slab_ab_smem_bytes_f32(p.nb, p.npair) : slab_ab_smem_bytes(p, 4, true));
   }
   b.args[0] = to_device(c, b.tmps, sa, s);
   b.args[1] = to_device(c, b.tmps, sb, s);

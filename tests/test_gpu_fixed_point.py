@@ -14,7 +14,7 @@ import pytest
 
 from golden_io import max_rel
 from oracle.oracle import Oracle
-from sbd_gb300.engine import TPBProblem
+from sbd_gb300.engine import MIXED, TPBProblem
 from sbd_gb300.generators import make_problem
 
 torch = pytest.importorskip("torch")
@@ -147,3 +147,35 @@ def test_unit_vector_starts_keep_the_fp64_sweeps(engine):
     c = p.davidson(max_it=1, init=0, **kw)
     assert np.array_equal(a.vectors, c.vectors) and np.array_equal(a.energies, c.energies)
     p.close()
+
+
+# alpha sweep, beta sweep, alpha x beta of FP32: the longest list that its shared
+# memory holds, and one more string (the 8-byte forms go on to twice that)
+@pytest.mark.parametrize("na,nb,seed,fits", [(14252, 12, 1, True), (14253, 12, 1, False), (1, 14252, 1, True),
+                                             (1, 14253, 1, False), (12, 11232, 5, True), (12, 11233, 5, False)])
+def test_fp32_at_its_shared_memory_limit(engine, na, nb, seed, fits):
+    prob, p = _problem(engine, 20, 8, 8, na, nb, seed=seed)
+    q = TPBProblem.from_problem(engine, prob)
+    q.diag_terms()
+    q.set_tuning(0, 1, 1)  # the FP64 sweeps
+    st = torch.cuda.current_stream().cuda_stream
+    f = torch.tensor(np.random.default_rng(nb).normal(size=(3, prob.ndet)), device="cuda").float()
+    many, one = torch.full_like(f, float("nan")), torch.full_like(f, float("nan"))
+    for j in range(3):
+        p.sigma_mixed_device(f[j].data_ptr(), one[j].data_ptr(), stream=st)
+    p.sigma_mixed_block_device(f.data_ptr(), many.data_ptr(), 3, stream=st)
+    torch.cuda.synchronize()
+    assert (p.tuning(1)["beta_shape"] == SLAB) == fits
+    for j in range(3):
+        ref = _sigma(q, f[j].double()).cpu().numpy()
+        assert max_rel(one[j].double().cpu().numpy(), ref) <= 5e-6
+        assert max_rel(many[j].double().cpu().numpy(), ref) <= 5e-6
+    assert max_rel(_sigma(p, f[0].double()).cpu().numpy(), _sigma(q, f[0].double()).cpu().numpy()) <= 1e-13
+    assert p.tuning(0)["beta_shape"] == SLAB
+    if not fits:
+        kw = dict(nroots=1, max_nb=16, eps=1e-7, max_it=40, init=1, want_vectors=False)
+        a, b = p.davidson(precision=MIXED, **kw), q.davidson(**kw)
+        assert a.report["converged"] and b.report["converged"]
+        assert abs(a.energies[0] - b.energies[0]) <= 1e-8
+    p.close()
+    q.close()
