@@ -25,11 +25,15 @@ struct Error : std::runtime_error {
   Error(int s, const std::string &m) : std::runtime_error(m), status(s) {}
 };
 
+// Throws where a CUDA call fails, and clears the runtime's record of it: the next
+// call's check of cudaGetLastError() would otherwise report it again.
 #define SBDGB_CUDA(call)                                                                         \
   do {                                                                                            \
     cudaError_t _e = (call);                                                                      \
-    if (_e != cudaSuccess)                                                                        \
+    if (_e != cudaSuccess) {                                                                      \
+      cudaGetLastError();                                                                         \
       throw ::sbdgb::Error(SBDGB_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e));     \
+    }                                                                                             \
   } while (0)
 
 #define SBDGB_REQUIRE(cond, status, msg)                      \
