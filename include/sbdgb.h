@@ -155,6 +155,8 @@ int sbdgb_sigma_mixed_block(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev
  * otherwise) or 1 = one row per CTA of 1024 threads;
  * shape_b = 7 (reported, not settable) means the fixed-point kernels
  * (sigma_slab.cu), taken without timing where a row has more than 8 nonzeros.
+ * precision 6 reads the FP64 sweeps that solves from init 0 or 2 keep to where the
+ * other block-ordering products (3) go by the fixed-point kernels.
  * The first product of each precision tunes (and synchronises), so make it
  * before any stream capture. */
 int sbdgb_problem_tuning(const sbdgb_problem *p, int precision, int *shape_a, int *shape_b, float *ms_a,

@@ -459,7 +459,7 @@ int sbdgb_sigma_mixed_block(sbdgb_problem *pr, const float *Wk_dev, float *Wb_de
 
 int sbdgb_problem_tuning(const sbdgb_problem *pr, int precision, int *shape_a, int *shape_b, float *ms_a,
                          float *ms_b, int n_shapes) {
-  if (!pr || precision < 0 || precision > 5) return SBDGB_E_INPUT;
+  if (!pr || precision < 0 || precision > 6) return SBDGB_E_INPUT;
   const sbdgb::Problem &p = pr->p;
   if (shape_a) *shape_a = p.tune_a[precision];
   if (shape_b) *shape_b = p.tune_b[precision];
@@ -472,7 +472,7 @@ int sbdgb_problem_tuning(const sbdgb_problem *pr, int precision, int *shape_a, i
 
 int sbdgb_problem_tuning_times(const sbdgb_problem *pr, int precision, float *ms_fused, float *ms_sparse,
                                float *ms_stream) {
-  if (!pr || precision < 0 || precision > 5) return SBDGB_E_INPUT;
+  if (!pr || precision < 0 || precision > 6) return SBDGB_E_INPUT;
   const sbdgb::Problem &p = pr->p;
   for (int i = 0; i < 4; ++i)
     if (ms_fused) ms_fused[i] = p.tune_ms[precision][2][i];
@@ -492,7 +492,7 @@ int sbdgb_problem_set_tuning(sbdgb_problem *pr, int precision, int shape_a, int 
 }
 
 int sbdgb_problem_split(const sbdgb_problem *pr, int precision, int *split, float *ms) {
-  if (!pr || precision < 0 || precision > 5) return SBDGB_E_INPUT;
+  if (!pr || precision < 0 || precision > 6) return SBDGB_E_INPUT;
   if (split) *split = pr->p.split_ab[precision];
   if (ms) {
     ms[0] = pr->p.tune_ab_ms[precision][0];

@@ -158,7 +158,8 @@ struct Problem {
   uint32_t n_tiles[2][2] = {};
   // autotuned sigma tile shapes: FP64, FP32, double-float, in the interleaved
   // (0..2) and block (3..5) orderings; 6: the FP64 sweeps of the block ordering
-  // where the solver keeps to them (sigma_fp64_sweeps)
+  // where the solver keeps to them and slot 3 has the fixed-point kernels
+  // (sigma_fp64_sweeps)
   int tune_a[7] = {-1, -1, -1, -1, -1, -1, -1}, tune_b[7] = {-1, -1, -1, -1, -1, -1, -1};
   float tune_ms[7][3][8] = {};  // timings the autotuner saw (A, B, fused + sparse)
   // 1: the alpha x beta single pairs run in their own kernel (sigma_ab.cu)

@@ -671,7 +671,8 @@ template <typename T, bool kB, bool kSweeps = false>
 void autotune(Problem &p, Args<T> a, cudaStream_t s) {
   const int prec = slot_of<T, kB, kSweeps>();
   if (p.tune_a[prec] >= 0 && p.tune_b[prec] >= 0) return;
-  const std::array<uint64_t, 6> key{(uint64_t)prec, (uint64_t)p.norb, p.na, p.nb, p.A.ns + p.A.nd, p.B.ns + p.B.nd};
+  // (the FP64 sweeps of the block ordering are the same kernels whichever slot they are tuned for)
+  const std::array<uint64_t, 6> key{kSweeps ? 3u : (uint64_t)prec, (uint64_t)p.norb, p.na, p.nb, p.A.ns + p.A.nd, p.B.ns + p.B.nd};
   const auto hit = p.ctx->tuned.find(key);
   if (hit != p.ctx->tuned.end()) {
     p.tune_a[prec] = hit->second.a;
@@ -853,6 +854,15 @@ bool slab_pays(const Problem &p) {
 // a few singles per string on both sides that staging is cheap per term).
 constexpr double kAbSplitPerElement = 4.0;
 
+constexpr int kSweepSlot = slot_of<double, true, true>();
+void copy_tuning(Problem &p, int from, int to) {
+  p.tune_a[to] = p.tune_a[from];
+  p.tune_b[to] = p.tune_b[from];
+  p.split_ab[to] = p.split_ab[from];
+  std::copy(&p.tune_ms[from][0][0], &p.tune_ms[from][0][0] + 3 * 8, &p.tune_ms[to][0][0]);
+  std::copy(p.tune_ab_ms[from], p.tune_ab_ms[from] + 2, p.tune_ab_ms[to]);
+}
+
 template <typename T, bool kB, bool kSweeps = false>
 bool needs_tuning(Problem &p, cudaStream_t s) {
   const int prec = slot_of<T, kB, kSweeps>();
@@ -861,6 +871,10 @@ bool needs_tuning(Problem &p, cudaStream_t s) {
     p.tune_a[prec] = 0;
     p.tune_b[prec] = kSlabShape;
     p.split_ab[prec] = p.A.ns > 0 && p.B.ns > 0 ? 1 : 0;
+    return false;
+  }
+  if (prec == 3 && p.tune_b[kSweepSlot] >= 0) {  // the sweeps that a solve has gone by stay its sweeps
+    copy_tuning(p, kSweepSlot, prec);
     return false;
   }
   if (p.ctx->autotune) return true;
@@ -1464,7 +1478,11 @@ void sigma_fp64(Problem &p, const double *C, double *S, int accumulate, cudaStre
 }
 
 void sigma_fp64_sweeps(Problem &p, const double *C, double *S, int accumulate, cudaStream_t s) {
-  if (p.tune_b[3] >= 0 && p.tune_b[3] != kSlabShape) {  // shapes set by the caller, or timed: the sweeps already
+  // One choice of sweeps a problem, whatever was called before: slot 3's, and one of
+  // their own only beside the fixed-point kernels (taken already, or by the next
+  // product that does not come this way).
+  const bool slab = p.tune_b[3] >= 0 ? p.tune_b[3] == kSlabShape : p.slab.state != 0 && slab_pays<double, true>(p);
+  if (!slab) {
     sigma_fp64(p, C, S, accumulate, s, true);
     return;
   }

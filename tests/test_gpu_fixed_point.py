@@ -179,3 +179,24 @@ def test_fp32_at_its_shared_memory_limit(engine, na, nb, seed, fits):
         assert abs(a.energies[0] - b.energies[0]) <= 1e-8
     p.close()
     q.close()
+
+
+@pytest.mark.parametrize("norb,na,nb,nocc,slab", [(40, 900, 700, 13, False), (16, 300, 280, 5, True)])
+def test_one_choice_of_sweeps_a_problem(engine, norb, na, nb, nocc, slab):
+    """A stopped solve returns the same vectors before and after calls that are not
+    its own, and on a new problem of the same sizes, whether the other products go
+    by the sweeps or by the fixed-point kernels; the shapes can be read."""
+    kw = dict(nroots=2, max_nb=16, eps=1e-9)
+    first = None
+    for order in ("solve first", "solve last"):
+        prob, p = _problem(engine, norb, nocc, nocc, na, nb, seed=3)
+        if order == "solve first":
+            first = p.davidson(max_it=1, init=0, **kw)
+            assert (p.tuning(3)["beta_shape"] is None) == slab
+        p.davidson(max_it=2, init=1, **kw)
+        assert (p.tuning(3)["beta_shape"] == SLAB) == slab
+        again = p.davidson(max_it=1, init=0, **kw)
+        sweeps = p.tuning(6 if slab else 3)["beta_shape"]
+        assert sweeps not in (None, SLAB) and (p.tuning(6)["beta_shape"] is None) == (not slab)
+        assert np.array_equal(first.vectors, again.vectors) and np.array_equal(first.energies, again.energies)
+        p.close()
