@@ -183,7 +183,9 @@ int sbdgb_problem_set_tuning(sbdgb_problem *p, int precision, int shape_a, int s
  * interleaved and the block determinant).  No counterpart in the reference. */
 int sbdgb_problem_split(const sbdgb_problem *p, int precision, int *split, float *ms);
 /* Sets that choice (0 or 1) for one precision; 1 is refused with
- * SBDGB_E_UNSUPPORTED when the staging does not fit in shared memory. */
+ * SBDGB_E_UNSUPPORTED when the staging does not fit in shared memory.  The
+ * fixed-point kernels (shape_b = 7) have the pairs in a kernel of their own
+ * (split = 1); 0 takes the precision from them to the untimed sweeps. */
 int sbdgb_problem_set_split(sbdgb_problem *p, int precision, int split);
 
 /* sigma that makes no device allocation.  No counterpart in the reference:

@@ -511,7 +511,7 @@ int sbdgb_problem_set_split(sbdgb_problem *pr, int precision, int split) {
                       : prec == 1 ? sbdgb::ab_fits<float>(p)
                                   : sbdgb::ab_fits<sbdgb::dfloat>(p);
     SBDGB_REQUIRE(split == 0 || fits, SBDGB_E_UNSUPPORTED, "alpha x beta staging does not fit in shared memory");
-    p.split_ab[precision] = split;
+    sbdgb::set_split(p, precision, split);
   });
 }
 

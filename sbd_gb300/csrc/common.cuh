@@ -295,6 +295,8 @@ void sigma_fp64(Problem &p, const double *C, double *S, int accumulate, cudaStre
 // The block-ordering product by the FP64 kernels of sigma.cu alone: the solvers'
 // where a run is too ill-conditioned for another order of rounding (davidson.cu).
 void sigma_fp64_sweeps(Problem &p, const double *C, double *S, int accumulate, cudaStream_t s);
+// split_ab of a precision, on the caller's word.
+void set_split(Problem &p, int precision, int split);
 void sigma_fp64_scratch(Problem &p, const double *C, double *S, int accumulate, double *CT, cudaStream_t s);
 // (H - shift) C in the mixed form: the diagonal term is formed in FP64 before
 // the result is rounded, so a shift near the spectrum keeps FP32 outputs small.

@@ -854,6 +854,19 @@ bool slab_pays(const Problem &p) {
 // a few singles per string on both sides that staging is cheap per term).
 constexpr double kAbSplitPerElement = 4.0;
 
+template <typename T>
+void untimed_shapes(Problem &p, int prec) {
+  p.split_ab[prec] =
+      (ab_fits<T>(p) && (double)p.A.ns * (double)p.B.ns >= kAbSplitPerElement * (double)p.N) ? 1 : 0;
+  if (nnz_per_row(p) <= 8.0) {
+    p.tune_a[prec] = 0;
+    p.tune_b[prec] = rows_fit<T>(p) ? kStreamShape : kSparseShape;
+    return;
+  }
+  p.tune_a[prec] = size_shape(p.nb);
+  p.tune_b[prec] = (p.B.ns + p.B.nd) <= 8ull * p.nb ? kFusedShape : size_shape(p.na);
+}
+
 constexpr int kSweepSlot = slot_of<double, true, true>();
 void copy_tuning(Problem &p, int from, int to) {
   p.tune_a[to] = p.tune_a[from];
@@ -878,15 +891,7 @@ bool needs_tuning(Problem &p, cudaStream_t s) {
     return false;
   }
   if (p.ctx->autotune) return true;
-  p.split_ab[prec] =
-      (ab_fits<T>(p) && (double)p.A.ns * (double)p.B.ns >= kAbSplitPerElement * (double)p.N) ? 1 : 0;
-  if (nnz_per_row(p) <= 8.0) {
-    p.tune_a[prec] = 0;
-    p.tune_b[prec] = rows_fit<T>(p) ? kStreamShape : kSparseShape;
-    return false;
-  }
-  p.tune_a[prec] = size_shape(p.nb);
-  p.tune_b[prec] = (p.B.ns + p.B.nd) <= 8ull * p.nb ? kFusedShape : size_shape(p.na);
+  untimed_shapes<T>(p, prec);
   return false;
 }
 
@@ -1475,6 +1480,19 @@ void sigma_fp64(Problem &p, const double *C, double *S, int accumulate, cudaStre
     run_sigma<double, true>(p, a, p.CT, s);
   else
     run_sigma<double, false>(p, a, p.CT, s);
+}
+
+void set_split(Problem &p, int precision, int split) {
+  // The fixed-point kernels always have the pairs in a kernel of their own: without
+  // one the products are those of the sweeps.
+  if (p.tune_b[precision] == kSlabShape && split == 0 && p.split_ab[precision] > 0) {
+    switch (precision % 3) {
+      case 0: untimed_shapes<double>(p, precision); break;
+      case 1: untimed_shapes<float>(p, precision); break;
+      default: untimed_shapes<dfloat>(p, precision); break;
+    }
+  }
+  p.split_ab[precision] = split;
 }
 
 void sigma_fp64_sweeps(Problem &p, const double *C, double *S, int accumulate, cudaStream_t s) {

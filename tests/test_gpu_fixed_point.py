@@ -200,3 +200,19 @@ def test_one_choice_of_sweeps_a_problem(engine, norb, na, nb, nocc, slab):
         assert sweeps not in (None, SLAB) and (p.tuning(6)["beta_shape"] is None) == (not slab)
         assert np.array_equal(first.vectors, again.vectors) and np.array_equal(first.energies, again.energies)
         p.close()
+
+
+def test_split_choice_is_kept(engine):
+    """set_split on a precision that has taken the fixed-point kernels: 1 is what they
+    do, 0 leads to the sweeps with the pairs inside."""
+    prob, p = _problem(engine, 16, 5, 5, 300, 280, seed=11)
+    x = torch.tensor(np.random.default_rng(0).normal(size=prob.ndet), device="cuda")
+    a = _sigma(p, x)
+    p.set_split(0, 1)
+    assert p.tuning(0)["beta_shape"] == SLAB and torch.equal(_sigma(p, x), a)
+    p.set_split(0, 0)
+    b = _sigma(p, x)
+    t = p.tuning(0)
+    assert t["beta_shape"] not in (None, SLAB) and t["alpha_beta"]["split"] == 0
+    assert max_rel(b.cpu().numpy(), a.cpu().numpy()) <= 1e-13
+    p.close()
