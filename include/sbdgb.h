@@ -126,7 +126,8 @@ int sbdgb_sigma(sbdgb_problem *p, const double *Wk_dev, double *Wb_dev, int accu
 /* Mixed-precision sigma: FP32 vectors, FP32 products and pair-list sums, a
  * float-float accumulator per element (an FP32 sum and the rounding errors of
  * the additions into it, about 48 bits; FP32 instructions only) and the FP64
- * diagonal as FP32 hi + lo parts; FP32 result. */
+ * diagonal as FP32 hi + lo parts; FP32 result.  Where a product takes several
+ * kernels (the tile shapes below), their results are added in FP32. */
 int sbdgb_sigma_mixed(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev, void *stream);
 /* Double-float sigma: each element of Wk_dev and Wb_dev is a pair of FP32
  * numbers (hi, lo) whose sum is the value (2N floats, hi first; 48 significand

@@ -423,8 +423,10 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
 
 // ---- the same sweep in FP32 -------------------------------------------------------
 //
-// FP32 vectors and table values, FP32 products and list sums, the diagonal added
-// in float-float as in the kernels of sigma.cu.  Four columns of a row are 16
+// FP32 vectors and table values, FP32 products and list sums; a lane's two list sums,
+// the diagonal and what sigma holds are added in float-float as in the kernels of
+// sigma.cu, and the launches' results in FP32 (as there where the alpha x beta pairs
+// or the beta sweep have a launch of their own).  Four columns of a row are 16
 // bytes.  Bound: the L1 data pipe (3 bytes of table and 4 of shared memory a
 // term at K = 8).  gridDim.z vectors at once.
 struct SlabArgsF {
@@ -563,6 +565,12 @@ __device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__
     }
     slab_list_f32<K, true>(acc, t.ent_s, a.val_s, ldg(t.off_s + sl), ldg(t.off_s + sl + 1), lane,
                            reinterpret_cast<const char *>(X), xplane, reinterpret_cast<const char *>(J), jplane);
+    float singles[K];
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      singles[c] = acc[c];
+      acc[c] = 0.f;
+    }
     slab_list_f32<K, false>(acc, t.ket_d, a.val_d, ldg(t.off_d + sl), ldg(t.off_d + sl + 1), lane,
                             reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
     if (row == ~0u) continue;
@@ -570,7 +578,7 @@ __device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__
 #pragma unroll
     for (int c = 0; c < K; ++c) {
       if (c0 + c >= a.m) break;
-      float s = acc[c];
+      const uint32_t ph = a.eta ? parity((unsigned long long)(str & ldg(a.colmask + c0 + c))) : 0u;
       if (a.diag) {  // eta sigma = h (eta C) + the sums
         const float x = X[place(a.n + 1, row, c)];
         FF d;
@@ -580,13 +588,18 @@ __device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__
           const dfloat h = ldg(a.hii_df + element(c));
           d = ff_diag(h.hi, h.lo, a.shift.hi, a.shift.lo, x);
         }
-        ff_add(d, s);
-        if (a.eta) d = parity((unsigned long long)(str & ldg(a.colmask + c0 + c))) ? FF{-d.hi, -d.lo} : d;
+        ff_add(d, singles[c]);
+        ff_add(d, acc[c]);
+        if (ph) d = FF{-d.hi, -d.lo};
         if (a.add) ff_add(d, old[c]);
         acc[c] = ff_value(d);
+      } else if (a.add) {
+        FF d{flip(singles[c], ph), 0.f};
+        ff_add(d, flip(acc[c], ph));
+        ff_add(d, old[c]);
+        acc[c] = ff_value(d);
       } else {
-        if (a.eta) s = flip(s, parity((unsigned long long)(str & ldg(a.colmask + c0 + c))));
-        acc[c] = a.add ? old[c] + s : s;
+        acc[c] = flip(singles[c] + acc[c], ph);
       }
       if (!whole) S[element(c)] = acc[c];
     }

@@ -216,3 +216,50 @@ def test_split_choice_is_kept(engine):
     assert t["beta_shape"] not in (None, SLAB) and t["alpha_beta"]["split"] == 0
     assert max_rel(b.cpu().numpy(), a.cpu().numpy()) <= 1e-13
     p.close()
+
+
+def test_fp32_list_sums_join_in_float_float(engine):
+    """A beta single's term of 2^24 |V| that the diagonal's cancels, and doubles of
+    order 1 beside it: what the doubles add survives.  The two products share every
+    rounding of a table value, so their difference at the bra is the doubles' FP32
+    sum, off by its own roundings and one rounding of each result."""
+    prob, p = _problem(engine, 16, 5, 5, 300, 280, seed=11)
+    o = Oracle.from_problem(prob)
+    b = prob.bstr.astype(np.uint64)
+    nb, ia = b.size, 7
+    found = False
+    for ib in range(nb):
+        dist = np.array([bin(int(x)).count("1") for x in b ^ b[ib]])
+        singles, doubles = np.nonzero(dist == 2)[0], np.nonzero(dist == 4)[0]
+        if len(singles) == 0 or len(doubles) < 20:
+            continue
+        e = np.zeros(prob.ndet)
+        e[ia * nb + singles[0]] = 1.0
+        v, h = o.mult(e)[ia * nb + ib], o.hii()[ia * nb + ib]
+        if abs(v) > 1e-3:
+            found = True
+            break
+    assert found
+    c = np.zeros(prob.ndet, dtype=np.float32)
+    c[ia * nb + singles[0]] = 2.0 ** 24
+    c[ia * nb + ib] = -v * 2.0 ** 24 / h
+    d = c.copy()
+    d[ia * nb + doubles] = np.random.default_rng(0).uniform(0.5, 1.0, len(doubles)).astype(np.float32)
+    only = np.where(d != c, d, 0).astype(np.float64)
+    want, size = o.mult(only)[ia * nb + ib], 0.0
+    for k in doubles:
+        e[:] = 0.0
+        e[ia * nb + k] = d[ia * nb + k]
+        size += abs(o.mult(e)[ia * nb + ib])
+    out = []
+    for x in (c, d):
+        f = torch.tensor(x, device="cuda")
+        s = torch.empty_like(f)
+        p.sigma_mixed_device(f.data_ptr(), s.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        out.append(float(s[ia * nb + ib]))
+    assert p.tuning(1)["beta_shape"] == SLAB
+    bound = 2.0 ** -24 * (len(doubles) * size + abs(out[0]) + abs(out[1]))
+    assert bound < 0.05 * abs(want)
+    assert abs(out[1] - out[0] - want) <= 2 * bound
+    p.close()
