@@ -121,7 +121,13 @@ int sbdgb_diag_terms(sbdgb_problem *p, double *hii_out);
  * chemistry/basic/mult.h:19-103).  Wk_dev, Wb_dev: N = na*nb doubles of
  * device memory.  accumulate != 0 gives the reference's Wb += H*Wk,
  * accumulate == 0 writes Wb = H*Wk.  stream: a cudaStream_t, or NULL for the
- * context's stream (pass cudaStreamLegacy for the legacy default stream). */
+ * context's stream (pass cudaStreamLegacy for the legacy default stream).
+ * Where the fixed-point kernels are taken (shape_b = 7 below) the terms of a sum
+ * are added exactly on one scale: an element of Wk is held to 2^-56 of the largest
+ * of its sum's (one row or column of Wk), a matrix element to 2^-58 of the largest
+ * of its spin's.  A row or column of Wk whose nonzeros lie too far apart for that
+ * (more than one in 16 below 2^-14 of the largest, or any below 2^-40), or that is
+ * not finite or beyond 2^+-800, is summed in FP64 instead. */
 int sbdgb_sigma(sbdgb_problem *p, const double *Wk_dev, double *Wb_dev, int accumulate, void *stream);
 /* Mixed-precision sigma: FP32 vectors, FP32 products and pair-list sums, a
  * float-float accumulator per element (an FP32 sum and the rounding errors of
@@ -131,10 +137,12 @@ int sbdgb_sigma(sbdgb_problem *p, const double *Wk_dev, double *Wb_dev, int accu
 int sbdgb_sigma_mixed(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev, void *stream);
 /* Double-float sigma: each element of Wk_dev and Wb_dev is a pair of FP32
  * numbers (hi, lo) whose sum is the value (2N floats, hi first; 48 significand
- * bits), and every product and sum is a double-float operation on the FP32
- * pipe.  This is the sigma of the second phase of the mixed solver: about
- * 2^-47 relative rounding per operation, several times the FP64 FMA rate of
- * this GPU.  accumulate as for sbdgb_sigma. */
+ * bits).  This is the sigma of the second phase of the mixed solver: double-float
+ * operations on the FP32 pipe (about 2^-47 relative rounding per operation, several
+ * times the FP64 FMA rate of this GPU), or the fixed-point sums of sbdgb_sigma
+ * rounded to 48 bits, with double-float sums where the nonzeros lie too far apart
+ * (more than one in 16 below 2^-20 of the largest, or any below 2^-46).  accumulate
+ * as for sbdgb_sigma. */
 int sbdgb_sigma_df(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev, int accumulate, void *stream);
 /* sbdgb_sigma_mixed for nvec vectors stored one after another (nvec*N floats
  * in and out).  Up to four vectors share each element's phase and address,

@@ -188,6 +188,7 @@ struct Problem {
     uint4 *ent_s[2] = {}, *ket_d[2] = {};
     int4 *val_s[2] = {}, *val_d[2] = {};
     float4 *valf_s[2] = {}, *valf_d[2] = {};
+    double2 *fp_s[2] = {}, *fp_d[2] = {};
     uint64_t *mask[2] = {};
     uint32_t *ab_ent = nullptr;  // the beta singles of ab_ent below, in this kernel's order
     uint2 *ab_items = nullptr;   // its CTAs: (alpha row, part | parts << 16), most batches first

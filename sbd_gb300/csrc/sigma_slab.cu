@@ -40,9 +40,10 @@
 // again to the result: two popcounts per determinant instead of one or two per
 // nonzero.
 //
-// A column (or ket row) with an infinity, a NaN or values beyond 2^+-800 is
-// summed in FP64 from the values as they are (slow, and the same results as
-// the FP64 kernels give).
+// A column (or ket row) with an infinity, a NaN or values beyond 2^+-800, and in
+// the caller's products one whose values lie far apart (Format), is summed in
+// floating point from the values as they are, bound by the FP64 pipe as the kernels
+// of sigma.cu are.
 #include <algorithm>
 #include <cmath>
 #include <numeric>
@@ -67,7 +68,16 @@ constexpr uint32_t kSlabMaxPair = 1u << 12;  // pair index bits
 // ---- the vector formats ----------------------------------------------------------
 
 // key: monotone in |x|, 0 for 0 only; exponent(key): |x| < 2^exponent (fx.cuh).
-// Staged as they are, and after parts() in fixed point, both 8 bytes.
+// Staged as they are (raw, of), and after parts() in fixed point, both 8 bytes.
+//
+// Wide vectors (a.guard).  An element is held to 2^-56 of the largest of its sum,
+// so what only small elements feed is held to fewer bits than floating point keeps:
+// with weights over 12 decades on the strings of each spin (norb 24, 700 x 733) 1%
+// of sigma's elements were off by 6e-9 of their terms' magnitudes or more, FP64 sums
+// by 1e-15; with 3 decades no element is off by more than the FP64 sums' worst, and
+// the norm of the error is a fifth of theirs.  So a column (ket row) goes by
+// floating-point sums where more than a 16th of its nonzeros lie below 2^-kWide of
+// its largest, or any below 2^-kTiny.
 template <typename T>
 struct Format;
 template <>
@@ -78,7 +88,12 @@ struct Format<double> {
   }
   static __device__ __forceinline__ int exponent(uint32_t key) { return fx::exponent_of(key, key != 0u); }
   static __device__ __forceinline__ int2 raw(double x) { return make_int2(__double2loint(x), __double2hiint(x)); }
-  static __device__ __forceinline__ double fp64(int2 v) { return __hiloint2double(v.y, v.x); }
+  static __device__ __forceinline__ double of(int2 v) { return __hiloint2double(v.y, v.x); }
+  // x is below 2^-d of the largest for d = top_field - field, and above half of that.
+  static __device__ __forceinline__ int field(int2 v) { return (v.y >> 20) & 0x7ff; }
+  static __device__ __forceinline__ int top_field(int ex) { return ex + 1022; }
+  static constexpr int kWide = 14, kTiny = 40;
+  static __device__ __forceinline__ double table(int lo, int hi) { return __hiloint2double(hi, lo); }
   static __device__ __forceinline__ int2 parts(int2 v, int ex) {
     return fx::vector_parts((uint32_t)v.x, (uint32_t)v.y, ex);
   }
@@ -93,8 +108,17 @@ struct Format<dfloat> {
     return key == 0u ? fx::kZero : key >= 0x7f800000u ? fx::kBad : (int)(key >> 23) - 126;
   }
   static __device__ __forceinline__ int2 raw(dfloat x) { return make_int2(__float_as_int(x.lo), __float_as_int(x.hi)); }
-  static __device__ __forceinline__ double fp64(int2 v) {
-    return (double)__int_as_float(v.y) + (double)__int_as_float(v.x);
+  static __device__ __forceinline__ dfloat of(int2 v) { return dfloat(__int_as_float(v.y), __int_as_float(v.x)); }
+  static __device__ __forceinline__ int field(int2 v) { return (v.y >> 23) & 0xff; }
+  static __device__ __forceinline__ int top_field(int ex) { return ex + 126; }
+  static constexpr int kWide = 20, kTiny = 46;  // five bits fewer to keep than in FP64
+  // An FP64 table value: 24 bits in hi, the other 29 in lo (no FP64 instruction).
+  static __device__ __forceinline__ dfloat table(int lo, int hi) {
+    const int e = (hi >> 20) & 0x7ff, sign = hi & (int)0x80000000;
+    if (e < 1023 - 70 || e > 1023 + 126) return e ? dfloat(__hiloint2double(hi, lo)) : dfloat(0.f, 0.f);
+    const int h = sign | (e - 896) << 23 | (hi & 0xfffff) << 3 | (int)((uint32_t)lo >> 29);
+    const float unit = __int_as_float(sign | (e - 948) << 23);  // 2^(e - 1075)
+    return dfloat(__int_as_float(h), (float)(lo & 0x1fffffff) * unit);
   }
   static __device__ __forceinline__ int2 parts(int2 v, int ex) {
     return fx::vector_parts_df((uint32_t)v.x, (uint32_t)v.y, ex);
@@ -138,6 +162,7 @@ struct SlabSpin {
   const int4 *val_s;              // V of the same-spin part with the phase applied
   const uint4 *ket_d;             // doubles: ket << 4
   const int4 *val_d;
+  const int4 *fp_s, *fp_d;        // V in FP64 (the pairs of words that val_* has in fixed point)
   uint32_t nslices;
 };
 
@@ -148,8 +173,8 @@ struct SlabArgs {
   const T *hii;  // the diagonal in the vectors' format
   T shift;       // taken off the diagonal (0 in FP64)
   SlabSpin t;
-  SpinTables tables;        // the same entries as the FP64 kernels read them
   const double *Jo;         // opposite-spin Coulomb table [npair][m]
+  const T *Jt;              // the same in the vectors' format
   const int2 *Jfx;          // the same in fixed point, or null: converted here
   const uint64_t *rowstr;   // this spin's strings
   const uint64_t *colmask;  // per column: the orbitals whose parity on rowstr is eta
@@ -157,6 +182,7 @@ struct SlabArgs {
   int npair;                // 0: no singles (J is not staged)
   int ev;                   // |v| < 2^ev for every table value of this spin
   int eta;                  // interleaved convention: eta on the way in and out
+  int guard;                // wide columns are summed in floating point
   int add;                  // what S holds is kept
   int diag;                 // the diagonal term is added here
   int staged_diag;          // ... while staging, so that S is complete but for this spin's sums
@@ -171,21 +197,18 @@ __device__ __forceinline__ size_t staged(uint32_t rows, uint32_t r, int c) {
   return K == 1 ? r : ((size_t)(c >> 1) * rows + r) * 2 + (c & 1);
 }
 
-// Row `row` summed in FP64 as the kernels of sigma.cu do, from the raw staged
-// values (a column that is not finite, or out of the fixed-point range).
-template <typename T, int K>
-__device__ __noinline__ double slab_row_fp64(const SpinTables &t, uint32_t row, const int2 *X, uint32_t n1,
-                                             const double *Jo, uint32_t m, uint32_t col, int c) {
-  double sum = 0.0;
-  for (uint32_t p = ldg(t.off_s + row); p < ldg(t.off_s + row + 1); ++p) {
-    const uint32_t code = ldg(t.code_s + p);
-    const double v = ldg(t.val_s + p) + ldg(Jo + (size_t)((code >> 16) & 0x7fffu) * m + col);
-    sum = fma(flip(v, code >> 31), Format<T>::fp64(X[staged<K>(n1, ldg(t.ket_s + p), c)]), sum);
-  }
-  for (uint32_t p = ldg(t.off_d + row); p < ldg(t.off_d + row + 1); ++p)
-    sum = fma(ldg(t.val_d + p), Format<T>::fp64(X[staged<K>(n1, ldg(t.ket_d + p), c)]), sum);
-  return sum;
+// Whether a sum's elements lie too far apart for fixed point: how many of them are
+// small, of how many nonzeros (a tiny one counts as kManySmall, which is enough).
+constexpr uint32_t kManySmall = 1u << 16;
+template <typename T>
+__device__ __forceinline__ void count_small(int2 v, int top, uint32_t &small, uint32_t &nonzero) {
+  using F = Format<T>;
+  if (((uint32_t)v.x | (uint32_t)v.y) << 1 == 0u) return;
+  const int d = top - F::field(v);
+  ++nonzero;
+  small += d > F::kTiny ? kManySmall : d > F::kWide ? 1u : 0u;
 }
+__device__ __forceinline__ bool is_wide(uint32_t small, uint32_t nonzero) { return small > nonzero >> 4; }
 
 // Four table entries of a lane: three 16-byte loads.
 struct Group {
@@ -266,6 +289,51 @@ __device__ __forceinline__ void slab_list(fx::Acc (&acc)[K], const uint4 *__rest
   for (int c = 0; c < K; ++c) fx::carry(acc[c]);
 }
 
+// The same from the raw staged values (X, and J the raw Coulomb values), in the
+// vectors' format.
+template <typename T, int K, bool kSingles>
+__device__ __forceinline__ void slab_list_fp(T (&acc)[K], const uint4 *__restrict__ ent, const int4 *__restrict__ val,
+                                             uint32_t g, uint32_t end, uint32_t lane, const char *X, uint32_t xplane,
+                                             const char *J, uint32_t jplane) {
+  using F = Format<T>;
+  if (g >= end) return;
+  const uint32_t pad = xplane - 16u;  // the zero row, which padding entries point at
+  Group a;
+  a.load(ent, val, g * 32u + lane);
+  while (true) {
+    const Group b = a;
+    if (g + 1 < end) a.load(ent, val, (g + 1) * 32u + lane);
+    const uint32_t w[kGroup] = {b.w.x, b.w.y, b.w.z, b.w.w};
+    const T v[kGroup] = {F::table(b.v0.x, b.v0.y), F::table(b.v0.z, b.v0.w), F::table(b.v1.x, b.v1.y),
+                         F::table(b.v1.z, b.v1.w)};
+#pragma unroll
+    for (int u = 0; u < kGroup; ++u) {
+      const uint32_t x16 = kSingles ? w[u] & 0x7fff0u : w[u], j16 = (w[u] >> 15) & 0xfff0u;
+      if (!__any_sync(0xffffffffu, x16 != pad)) break;  // the rest of the group is padding in every lane
+      const uint32_t sg = w[u] >> 31;
+      if constexpr (K == 1) {
+        T m = v[u];
+        if constexpr (kSingles) m = m + flip(F::of(*reinterpret_cast<const int2 *>(J + (j16 >> 1))), sg);
+        acc[0] = fma(m, F::of(*reinterpret_cast<const int2 *>(X + (x16 >> 1))), acc[0]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < K / 2; ++q) {
+          const int4 x = *reinterpret_cast<const int4 *>(X + q * xplane + x16);
+          T m0 = v[u], m1 = v[u];
+          if constexpr (kSingles) {
+            const int4 j = *reinterpret_cast<const int4 *>(J + q * jplane + j16);
+            m0 = m0 + flip(F::of(make_int2(j.x, j.y)), sg);
+            m1 = m1 + flip(F::of(make_int2(j.z, j.w)), sg);
+          }
+          acc[2 * q] = fma(m0, F::of(make_int2(x.x, x.y)), acc[2 * q]);
+          acc[2 * q + 1] = fma(m1, F::of(make_int2(x.z, x.w)), acc[2 * q + 1]);
+        }
+      }
+    }
+    if (++g == end) return;
+  }
+}
+
 // One CTA: column group `group`, every a.parts-th slice from `part`, of C into S.
 template <typename T, int K, bool kAlpha>
 __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restrict__ C, T *S, uint32_t group,
@@ -275,16 +343,18 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
   extern __shared__ __align__(16) unsigned char slab_smem[];
   int2 *X = reinterpret_cast<int2 *>(slab_smem);     // (n + 1) x K; row n is zero (padding entries)
   int2 *J = X + (size_t)(a.n + 1) * K;               // (npair + 1) x K; row npair is zero
-  __shared__ uint32_t skey[K], snext;
+  __shared__ uint32_t skey[K], snext, ssmall[K], snonzero[K];
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
   const uint32_t c0 = group * K;
+  constexpr int kw = K == 1 ? 1 : 2;  // columns side by side in a plane of X
+  const uint32_t plane = (a.n + 1) * kw;
   auto diag = [&](size_t k) {
     if constexpr (std::is_same<T, double>::value)
       return ldg(a.hii + k);
     else
       return ldg(a.hii + k) - a.shift;
   };
-  if (tid < K) skey[tid] = 0u;
+  if (tid < K) skey[tid] = ssmall[tid] = snonzero[tid] = 0u;
   if (tid == 0) snext = 0u;
   __syncthreads();
   // stage the raw values and find each column's largest
@@ -342,9 +412,27 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
     ex[c] = F::exponent(skey[c]);
     bad = bad || ex[c] == fx::kBad;
   }
+  if (!bad && a.guard) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int c = q * kw + (kw == 1 ? 0 : (int)(tid & 1u));  // nt is even: a thread's elements are of one column
+      const int top = F::top_field(tid & 1u ? ex[q * kw + kw - 1] : ex[q * kw]);
+      uint32_t small = 0u, nonzero = 0u;
+      for (uint32_t i = tid; i < plane; i += nt) count_small<T>(X[(size_t)q * plane + i], top, small, nonzero);
+      for (int o = 16; o >= kw; o >>= 1) {
+        small += __shfl_xor_sync(0xffffffffu, small, o);
+        nonzero += __shfl_xor_sync(0xffffffffu, nonzero, o);
+      }
+      if (lane < (uint32_t)kw) {
+        atomicAdd(&ssmall[c], small);
+        atomicAdd(&snonzero[c], nonzero);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < K; ++c) bad = bad || is_wide(ssmall[c], snonzero[c]);
+  }
   if (!bad) {  // to fixed point, in place (an all-zero column has no scale and its sums are not read)
-    constexpr int kw = K == 1 ? 1 : 2;
-    const uint32_t plane = (a.n + 1) * kw;
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
       for (uint32_t i = tid; i < plane; i += nt) {
@@ -352,8 +440,14 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
         int2 &x = X[(size_t)q * plane + i];
         if (e != fx::kZero) x = F::parts(x, e);
       }
-    __syncthreads();
+  } else if (a.npair) {
+    for (uint32_t i = tid; i < (uint32_t)a.npair * K; i += nt) {
+      const uint32_t P = i / K;
+      const int c = (int)(i % K);
+      if (c0 + c < a.m) J[staged<K>(a.npair + 1, P, c)] = F::raw(ldg(a.Jt + ((size_t)P * a.m + (c0 + c))));
+    }
   }
+  __syncthreads();
   const SlabSpin &t = a.t;
   while (true) {
     uint32_t sl = 0;
@@ -388,10 +482,12 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
         out[c] = ex[c] == fx::kZero ? T(0.0) : F::value(acc[c], ex[c] + a.ev + fx::kUnit);
     } else {
 #pragma unroll
-      for (int c = 0; c < K; ++c)
-        out[c] = row != ~0u && c0 + c < a.m
-                     ? T(slab_row_fp64<T, K>(a.tables, row, X, a.n + 1, a.Jo, a.m, c0 + c, c))
-                     : T(0.0);
+      for (int c = 0; c < K; ++c) out[c] = T(0.0);
+      const uint32_t xplane = 16u * (a.n + 1), jplane = 16u * (a.npair + 1);
+      slab_list_fp<T, K, true>(out, t.ent_s, t.fp_s, ldg(t.off_s + sl), ldg(t.off_s + sl + 1), lane,
+                               reinterpret_cast<const char *>(X), xplane, reinterpret_cast<const char *>(J), jplane);
+      slab_list_fp<T, K, false>(out, t.ket_d, t.fp_d, ldg(t.off_d + sl), ldg(t.off_d + sl + 1), lane,
+                                reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
     }
     if (row == ~0u) continue;
     const uint64_t str = a.eta ? ldg(a.rowstr + row) : 0ull;
@@ -637,10 +733,11 @@ struct SlabAbArgs {
   const uint64_t *colmask;           // per beta string
   const uint32_t *off, *ket, *code;  // alpha singles
   const double *Kp;
+  const T *Kt;         // the same in the vectors' format
   const uint2 *items;  // (alpha row, part | parts << 16)
   const uint32_t *cols, *slice, *ent;
   uint32_t nslices, nb;
-  int npair, ek, eta;
+  int npair, ek, eta, guard;
 };
 
 template <typename T, int G, bool kSum>
@@ -653,7 +750,7 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
   int4 *Cs = reinterpret_cast<int4 *>(slab_smem);                // [G/2][nb + 1]: two ket rows' values at jb
   int4 *Ks = Cs + (size_t)NP * cplane;                           // [G/2][2 Q + phase]
   double *Ss = reinterpret_cast<double *>(Ks + NP * kplane);     // kSum: [nb]
-  __shared__ uint32_t skey[G];
+  __shared__ uint32_t skey[G], ssmall[G], snonzero[G];
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
   const uint32_t ia = item.x, part = item.y & 0xffffu, parts = item.y >> 16;
   const uint32_t p0 = ldg(a.off + ia), p1 = ldg(a.off + ia + 1);
@@ -665,7 +762,7 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
   for (uint32_t pb = p0; pb < p1; pb += G) {
     const uint32_t live = min((uint32_t)G, p1 - pb);
     __syncthreads();  // the previous batch is applied
-    if (tid < G) skey[tid] = 0u;
+    if (tid < G) skey[tid] = ssmall[tid] = snonzero[tid] = 0u;
     __syncthreads();
     uint32_t key[G];
 #pragma unroll
@@ -702,7 +799,32 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
       es = max(es, e[g]);
     }
     if (es == fx::kZero) continue;  // every row is zero
-    const bool fixed = es != fx::kBad;  // otherwise FP64 sums of the values as they are
+    bool fixed = es != fx::kBad;  // otherwise floating-point sums of the values as they are
+    if (fixed && a.guard) {
+#pragma unroll
+      for (int h = 0; h < NP; ++h) {
+        uint32_t small0 = 0u, nonzero0 = 0u, small1 = 0u, nonzero1 = 0u;
+        for (uint32_t c = tid; c < a.nb; c += nt) {
+          const int4 r = Cs[h * cplane + c];
+          count_small<T>(make_int2(r.x, r.y), F::top_field(e[2 * h]), small0, nonzero0);
+          count_small<T>(make_int2(r.z, r.w), F::top_field(e[2 * h + 1]), small1, nonzero1);
+        }
+        small0 = __reduce_add_sync(0xffffffffu, small0);
+        small1 = __reduce_add_sync(0xffffffffu, small1);
+        nonzero0 = __reduce_add_sync(0xffffffffu, nonzero0);
+        nonzero1 = __reduce_add_sync(0xffffffffu, nonzero1);
+        if (lane == 0) {
+          atomicAdd(&ssmall[2 * h], small0);
+          atomicAdd(&ssmall[2 * h + 1], small1);
+          atomicAdd(&snonzero[2 * h], nonzero0);
+          atomicAdd(&snonzero[2 * h + 1], nonzero1);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        fixed = fixed && !is_wide(ssmall[g], snonzero[g]) && (e[g] == fx::kZero || es - e[g] <= F::kTiny);
+    }
     if (fixed) {  // to fixed point, in place: each thread the columns that it staged
 #pragma unroll
       for (int h = 0; h < NP; ++h)
@@ -718,23 +840,25 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
     for (int h = 0; h < NP; ++h) {
       const uint32_t c0 = 2 * h < live ? ldg(a.code + pb + 2 * h) : 0u;
       const uint32_t c1 = 2 * h + 1 < live ? ldg(a.code + pb + 2 * h + 1) : 0u;
-      const double *k0 = a.Kp + (size_t)((c0 >> 16) & 0x7fffu) * a.npair, *k1 = a.Kp + (size_t)((c1 >> 16) & 0x7fffu) * a.npair;
+      const size_t k0 = (size_t)((c0 >> 16) & 0x7fffu) * a.npair, k1 = (size_t)((c1 >> 16) & 0x7fffu) * a.npair;
       for (uint32_t Q = tid; Q <= (uint32_t)a.npair; Q += nt) {
-        const bool ok = Q < (uint32_t)a.npair;
-        const double v0 = ok && 2 * h < live ? flip(ldg(k0 + Q), c0 >> 31) : 0.0;
-        const double v1 = ok && 2 * h + 1 < live ? flip(ldg(k1 + Q), c1 >> 31) : 0.0;
+        const bool ok0 = Q < (uint32_t)a.npair && 2 * h < live, ok1 = Q < (uint32_t)a.npair && 2 * h + 1 < live;
         int2 f0, f1, n0, n1;
         if (fixed) {
           // (an all-zero row's values are not used, whatever its scale)
+          const double v0 = ok0 ? flip(ldg(a.Kp + k0 + Q), c0 >> 31) : 0.0;
+          const double v1 = ok1 ? flip(ldg(a.Kp + k1 + Q), c1 >> 31) : 0.0;
           f0 = fx::make(v0, fx::kVBits - a.ek - min(es - e[2 * h], 100));
           f1 = fx::make(v1, fx::kVBits - a.ek - min(es - e[2 * h + 1], 100));
           n0 = make_int2(-f0.x, -f0.y);
           n1 = make_int2(-f1.x, -f1.y);
         } else {
-          f0 = Format<double>::raw(v0);
-          f1 = Format<double>::raw(v1);
-          n0 = Format<double>::raw(-v0);
-          n1 = Format<double>::raw(-v1);
+          const T v0 = ok0 ? flip(ldg(a.Kt + k0 + Q), c0 >> 31) : T(0.0);
+          const T v1 = ok1 ? flip(ldg(a.Kt + k1 + Q), c1 >> 31) : T(0.0);
+          f0 = F::raw(v0);
+          f1 = F::raw(v1);
+          n0 = F::raw(-v0);
+          n1 = F::raw(-v1);
         }
         Ks[h * kplane + 2 * Q] = make_int4(f0.x, f0.y, f1.x, f1.y);
         Ks[h * kplane + 2 * Q + 1] = make_int4(n0.x, n0.y, n1.x, n1.y);
@@ -785,6 +909,7 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
         fx::carry(acc);
         sum = fx::value(acc, es + a.ek + fx::kUnit);
       } else {
+        T acc = T(0.0);
         for (; at < end; at += 32u * kGroup) {
           uint32_t wc[kGroup];
 #pragma unroll
@@ -795,13 +920,15 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
             if (at + 32u * u >= end) break;  // the same for the whole warp
 #pragma unroll
             for (int h = 0; h < NP; ++h) {
+              if (2 * h >= live) break;
               const int4 kv = Ks[h * kplane + (wc[u] & 0x1fffu)], cv = Cs[h * cplane + (wc[u] >> 13)];
-              sum = fma(Format<double>::fp64(make_int2(kv.x, kv.y)), F::fp64(make_int2(cv.x, cv.y)), sum);
+              acc = fma(F::of(make_int2(kv.x, kv.y)), F::of(make_int2(cv.x, cv.y)), acc);
               if (2 * h + 1 < live)
-                sum = fma(Format<double>::fp64(make_int2(kv.z, kv.w)), F::fp64(make_int2(cv.z, cv.w)), sum);
+                acc = fma(F::of(make_int2(kv.z, kv.w)), F::of(make_int2(cv.z, cv.w)), acc);
             }
           }
         }
+        sum = (double)acc;
       }
       if (k >= a.nb) continue;
       if (kSum) {
@@ -1134,7 +1261,8 @@ __global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t 
                                                    const uint32_t *__restrict__ order_d, int npair, int ev,
                                                    uint4 *__restrict__ ent_s, int4 *__restrict__ val_s,
                                                    uint4 *__restrict__ ket_d, int4 *__restrict__ val_d,
-                                                   float4 *__restrict__ valf_s, float4 *__restrict__ valf_d) {
+                                                   float4 *__restrict__ valf_s, float4 *__restrict__ valf_d,
+                                                   double2 *__restrict__ fp_s, double2 *__restrict__ fp_d) {
   const uint32_t sl = blockIdx.x, lane = threadIdx.x & 31u, y = threadIdx.x >> 5;
   const uint32_t row = rows[sl * 32u + lane];
   for (int doubles = 0; doubles < 2; ++doubles) {
@@ -1145,6 +1273,7 @@ __global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t 
       uint32_t w[kGroup];
       int2 v[kGroup];
       float f[kGroup];
+      double d[kGroup];
 #pragma unroll
       for (int u = 0; u < kGroup; ++u) {
         const uint32_t j = (g - off[sl]) * kGroup + u;
@@ -1152,21 +1281,24 @@ __global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t 
         const uint32_t p = ok ? order[p0 + j] : 0u;
         if (doubles) {
           w[u] = (ok ? T.ket_d[p] : T.n) << 4;
-          v[u] = ok ? fx::make(T.val_d[p], fx::kVBits - ev) : make_int2(0, 0);
-          f[u] = ok ? (float)T.val_d[p] : 0.f;
+          d[u] = ok ? T.val_d[p] : 0.0;
+          f[u] = (float)d[u];
         } else {
           const uint32_t code = ok ? T.code_s[p] : 0u;
           w[u] = ok ? (T.ket_s[p] << 4 | ((code >> 16) & 0x7fffu) << 19 | (code & 0x80000000u))
                     : (T.n << 4 | (uint32_t)npair << 19);
-          v[u] = ok ? fx::make(flip(T.val_s[p], code >> 31), fx::kVBits - ev) : make_int2(0, 0);
+          d[u] = ok ? flip(T.val_s[p], code >> 31) : 0.0;
           f[u] = ok ? flip((float)T.val_s[p], code >> 31) : 0.f;
         }
+        v[u] = fx::make(d[u], fx::kVBits - ev);
       }
       const size_t e = (size_t)g * 32u + lane;
       (doubles ? ket_d : ent_s)[e] = make_uint4(w[0], w[1], w[2], w[3]);
       (doubles ? val_d : val_s)[2 * e] = make_int4(v[0].x, v[0].y, v[1].x, v[1].y);
       (doubles ? val_d : val_s)[2 * e + 1] = make_int4(v[2].x, v[2].y, v[3].x, v[3].y);
       (doubles ? valf_d : valf_s)[e] = make_float4(f[0], f[1], f[2], f[3]);
+      (doubles ? fp_d : fp_s)[2 * e] = make_double2(d[0], d[1]);
+      (doubles ? fp_d : fp_s)[2 * e + 1] = make_double2(d[2], d[3]);
     }
   }
 }
@@ -1284,7 +1416,7 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
       ld[sp].push_back(ld[sp].back() + (md + kGroup - 1) / kGroup);
     }
     if ((uint64_t)std::max(ls[sp].back(), ld[sp].back()) * 64u >= (1ull << 32)) return false;  // 32-bit group indices
-    bytes += 4 * rows[sp].size() + 8 * ls[sp].size() + 32ull * 16 * kGroup * (ls[sp].back() + ld[sp].back()) + 8ull * T.n;
+    bytes += 4 * rows[sp].size() + 8 * ls[sp].size() + 32ull * 24 * kGroup * (ls[sp].back() + ld[sp].back()) + 8ull * T.n;
   }
   for (uint32_t c = 0; ab && c < p.nb; ++c)  // two terms per beta single of a column
     if (2 * (os[1][c + 1] - os[1][c]) > (uint32_t)fx::kMaxTerms) return false;
@@ -1315,6 +1447,8 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
     p.slab.val_d[sp] = (int4 *)dev_alloc(p, 1024ull * ld[sp].back());
     p.slab.valf_s[sp] = (float4 *)dev_alloc(p, 512ull * ls[sp].back());
     p.slab.valf_d[sp] = (float4 *)dev_alloc(p, 512ull * ld[sp].back());
+    p.slab.fp_s[sp] = (double2 *)dev_alloc(p, 1024ull * ls[sp].back());
+    p.slab.fp_d[sp] = (double2 *)dev_alloc(p, 1024ull * ld[sp].back());
     p.slab.mask[sp] = (uint64_t *)dev_alloc(p, 8ull * T.n);
     if (T.ns && !p.ctx->budget) {  // the Coulomb table this spin's singles read, where memory is not counted
       const size_t nj = (size_t)p.npair * (sp == 0 ? p.nb : p.na);
@@ -1330,7 +1464,8 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
     k_slab_order<<<(unsigned)nsl, 32, 0, s>>>(T.off_d, T.ket_d, r, next, order_d);
     k_slab_fill<<<(unsigned)nsl, 128, 0, s>>>(T, r, o, o + nsl + 1, order_s, order_d, p.npair, p.slab.ev[sp],
                                               p.slab.ent_s[sp], p.slab.val_s[sp], p.slab.ket_d[sp], p.slab.val_d[sp],
-                                              p.slab.valf_s[sp], p.slab.valf_d[sp]);
+                                              p.slab.valf_s[sp], p.slab.valf_d[sp], p.slab.fp_s[sp],
+                                              p.slab.fp_d[sp]);
     tmps.push_back(tmp);
     k_slab_masks<<<(T.n + 127) / 128, 128, 0, s>>>(sp == 0 ? p.astr : p.bstr, T.n, sp, p.slab.mask[sp]);
     count_launch(p.ctx, 4);
@@ -1445,12 +1580,14 @@ SlabSpin slab_spin(const Problem &p, int sp) {
   t.val_s = p.slab.val_s[sp];
   t.ket_d = p.slab.ket_d[sp];
   t.val_d = p.slab.val_d[sp];
+  t.fp_s = reinterpret_cast<const int4 *>(p.slab.fp_s[sp]);
+  t.fp_d = reinterpret_cast<const int4 *>(p.slab.fp_d[sp]);
   t.nslices = p.slab.nslices[sp];
   return t;
 }
 
 template <typename T, bool kAlpha>
-SlabArgs<T> slab_args(const Problem &p, const Args<T> &x, int add, int diag, int eta) {
+SlabArgs<T> slab_args(const Problem &p, const Args<T> &x, int add, int diag, int eta, int guard) {
   constexpr int sp = kAlpha ? 0 : 1;
   SlabArgs<T> a{};
   a.C = x.C;
@@ -1461,18 +1598,19 @@ SlabArgs<T> slab_args(const Problem &p, const Args<T> &x, int add, int diag, int
     a.hii = x.hii_df;
     a.shift = x.shift_df;
   }
-  a.tables = kAlpha ? p.A : p.B;
   a.t = slab_spin(p, sp);
   a.Jo = kAlpha ? p.Jb : p.Ja;
+  a.Jt = kAlpha ? x.Jb : x.Ja;
   a.Jfx = p.slab.Jfx[sp];
   a.rowstr = kAlpha ? p.astr : p.bstr;
   a.colmask = p.slab.mask[1 - sp];
   a.n = kAlpha ? p.na : p.nb;
   a.m = kAlpha ? p.nb : p.na;
   a.nb = p.nb;
-  a.npair = a.tables.ns ? p.npair : 0;
+  a.npair = (kAlpha ? p.A.ns : p.B.ns) ? p.npair : 0;
   a.ev = p.slab.ev[sp];
   a.eta = eta;
+  a.guard = guard;
   a.add = add;
   a.diag = diag;
   a.parts = 1;
@@ -1482,8 +1620,8 @@ SlabArgs<T> slab_args(const Problem &p, const Args<T> &x, int add, int diag, int
 }
 
 template <typename T, bool kAlpha>
-void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta, cudaStream_t s) {
-  SlabArgs<T> a = slab_args<T, kAlpha>(p, x, add, diag, eta);
+void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta, int guard, cudaStream_t s) {
+  SlabArgs<T> a = slab_args<T, kAlpha>(p, x, add, diag, eta, guard);
   const SlabShape c = slab_shape(p, kAlpha ? 0 : 1, a.n, a.m, a.npair, 8, 4, kSlabMinK, 1);
   a.parts = c.parts;
   a.staged_diag = a.staged_diag && c.parts == 1;
@@ -1543,7 +1681,7 @@ void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const 
 }
 
 template <typename T>
-SlabAbArgs<T> slab_ab_args(const Problem &p, const Args<T> &x, int eta) {
+SlabAbArgs<T> slab_ab_args(const Problem &p, const Args<T> &x, int eta, int guard) {
   SlabAbArgs<T> a{};
   a.C = x.C;
   a.S = x.S;
@@ -1553,6 +1691,7 @@ SlabAbArgs<T> slab_ab_args(const Problem &p, const Args<T> &x, int eta) {
   a.ket = p.A.ket_s;
   a.code = p.A.code_s;
   a.Kp = p.Kp;
+  a.Kt = x.Kp;
   a.items = p.slab.ab_items;
   a.cols = p.ab_cols;
   a.slice = p.ab_slice;
@@ -1562,12 +1701,13 @@ SlabAbArgs<T> slab_ab_args(const Problem &p, const Args<T> &x, int eta) {
   a.npair = p.npair;
   a.ek = p.slab.ek;
   a.eta = eta;
+  a.guard = guard;
   return a;
 }
 
 template <typename T>
-void launch_slab_ab(const Problem &p, const Args<T> &x, int eta, cudaStream_t s) {
-  const SlabAbArgs<T> a = slab_ab_args<T>(p, x, eta);
+void launch_slab_ab(const Problem &p, const Args<T> &x, int eta, int guard, cudaStream_t s) {
+  const SlabAbArgs<T> a = slab_ab_args<T>(p, x, eta, guard);
   const uint32_t warps = p.slab.ab_warps;
   const dim3 g(p.slab.n_ab_items);
   if (!slab_ab_sum(p))
@@ -1619,11 +1759,13 @@ void launch_slab_ab_f32(const Problem &p, const Args<float> &x, const float *con
 // streams.
 template <typename T>
 void sigma_slab(const Problem &p, const Args<T> &x, bool block, cudaStream_t s) {
-  const int eta = block ? 0 : 1;
+  // The solvers' products (the block ordering) need no guard: what a solve returns is
+  // held to a norm, and the norm of the error is below the FP64 sums'.
+  const int eta = block ? 0 : 1, guard = eta;
   const bool alpha = p.A.ns + p.A.nd > 0, beta = p.B.ns + p.B.nd > 0;
-  if (alpha || !beta) launch_slab<T, true>(p, x, x.accumulate, !beta, eta, s);
-  if (p.A.ns > 0 && p.B.ns > 0) launch_slab_ab<T>(p, x, eta, s);
-  if (beta) launch_slab<T, false>(p, x, x.accumulate || alpha, 1, eta, s);
+  if (alpha || !beta) launch_slab<T, true>(p, x, x.accumulate, !beta, eta, guard, s);
+  if (p.A.ns > 0 && p.B.ns > 0) launch_slab_ab<T>(p, x, eta, guard, s);
+  if (beta) launch_slab<T, false>(p, x, x.accumulate || alpha, 1, eta, guard, s);
 }
 template void sigma_slab<double>(const Problem &, const Args<double> &, bool, cudaStream_t);
 template void sigma_slab<dfloat>(const Problem &, const Args<dfloat> &, bool, cudaStream_t);
@@ -1683,9 +1825,9 @@ void slab_batch_plan(SlabBatch &b, Ctx *c, Problem **ps, const sdev::Args<T> *ar
       sb.push_back(slab_args_f32<false>(p, args[i], 1, 1, 1));
       ab.push_back(slab_ab_args_f32(p, args[i], 1));
     } else {
-      sa.push_back(slab_args<double, true>(p, args[i], 0, 0, 1));
-      sb.push_back(slab_args<double, false>(p, args[i], 1, 1, 1));
-      ab.push_back(slab_ab_args<double>(p, args[i], 1));
+      sa.push_back(slab_args<double, true>(p, args[i], 0, 0, 1, 0));
+      sb.push_back(slab_args<double, false>(p, args[i], 1, 1, 1, 0));
+      ab.push_back(slab_ab_args<double>(p, args[i], 1, 0));
       sa.back().vec = sb.back().vec = 0;  // a column of the basis may start anywhere
     }
     const int K = kF32 ? kManyKF : kManyK, el = kF32 ? 4 : 8;

@@ -263,3 +263,39 @@ def test_fp32_list_sums_join_in_float_float(engine):
     assert bound < 0.05 * abs(want)
     assert abs(out[1] - out[0] - want) <= 2 * bound
     p.close()
+
+
+# weights over `decades` orders of magnitude on the strings of each spin; every fourth
+# alpha string's at the size of rounding noise; one beta string's
+@pytest.mark.parametrize("kind", ["3 decades", "6 decades", "12 decades", "noise", "one string"])
+@pytest.mark.parametrize("norb,na,nb,nocc", [(12, 161, 187, 4), (24, 300, 280, 8), (16, 60, 300, 5)])
+def test_elements_of_wide_vectors(engine, norb, na, nb, nocc, kind):
+    """Every element of sigma to the bound of its own terms, k terms of relative
+    error 2^-53 (2^-46 in double-float), whatever else its vector holds; twice
+    that, for the reference's sums have it too."""
+    prob, p = _problem(engine, norb, nocc, nocc, na, nb, seed=na + nb)
+    H = Oracle.from_problem(prob).hamiltonian()
+    rng = np.random.default_rng(nb)
+    d = int(kind.split()[0]) if "decades" in kind else 2
+    C = rng.normal(size=(na, nb)) * 10.0 ** rng.uniform(-d, 0, (na, 1)) * 10.0 ** rng.uniform(-d, 0, (1, nb))
+    if kind == "noise":
+        C[::4] *= 1e-17
+    elif kind == "one string":
+        C[:, nb // 2] *= 1e-17
+    x = C.ravel()
+    ref, size, k = H @ x, abs(H) @ np.abs(x), np.diff(H.indptr).max() + 8
+    c = torch.tensor(x, device="cuda")
+    s = _sigma(p, c)
+    assert p.tuning(0)["beta_shape"] == SLAB
+    assert (np.abs(s.cpu().numpy() - ref) / size).max() <= 2 * k * 2.0 ** -53
+    assert torch.equal(_sigma(p, c), s)
+    hi = c.float()
+    pair = torch.stack([hi, (c - hi.double()).float()], dim=-1).contiguous()
+    y = torch.empty_like(pair)
+    p.sigma_df_device(pair.data_ptr(), y.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert p.tuning(2)["beta_shape"] == SLAB
+    # (FP32's exponents: below 1e-25 a value's low part, or a product's, is subnormal)
+    err = np.abs(y.double().sum(-1).cpu().numpy() - ref) / (size + 1e-25)
+    assert err.max() <= 2 * k * 2.0 ** -46
+    p.close()
