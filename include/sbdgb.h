@@ -126,8 +126,8 @@ int sbdgb_diag_terms(sbdgb_problem *p, double *hii_out);
  * are added exactly on one scale: an element of Wk is held to 2^-56 of the largest
  * of its sum's (one row or column of Wk), a matrix element to 2^-58 of the largest
  * of its spin's.  A row or column of Wk whose nonzeros lie too far apart for that
- * (more than one in 16 below 2^-14 of the largest, or any below 2^-40), or that is
- * not finite or beyond 2^+-800, is summed in FP64 instead. */
+ * (more than 9 binary orders below the largest on average, or any more than 36), or
+ * that is not finite or beyond 2^+-800, is summed in FP64 instead. */
 int sbdgb_sigma(sbdgb_problem *p, const double *Wk_dev, double *Wb_dev, int accumulate, void *stream);
 /* Mixed-precision sigma: FP32 vectors, FP32 products and pair-list sums, a
  * float-float accumulator per element (an FP32 sum and the rounding errors of
@@ -141,8 +141,7 @@ int sbdgb_sigma_mixed(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev, void
  * operations on the FP32 pipe (about 2^-47 relative rounding per operation, several
  * times the FP64 FMA rate of this GPU), or the fixed-point sums of sbdgb_sigma
  * rounded to 48 bits, with double-float sums where the nonzeros lie too far apart
- * (more than one in 16 below 2^-20 of the largest, or any below 2^-46).  accumulate
- * as for sbdgb_sigma. */
+ * (15 orders on average, 42 any).  accumulate as for sbdgb_sigma. */
 int sbdgb_sigma_df(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev, int accumulate, void *stream);
 /* sbdgb_sigma_mixed for nvec vectors stored one after another (nvec*N floats
  * in and out).  Up to four vectors share each element's phase and address,

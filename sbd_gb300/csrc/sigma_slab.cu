@@ -76,8 +76,10 @@ constexpr uint32_t kSlabMaxPair = 1u << 12;  // pair index bits
 // of sigma's elements were off by 6e-9 of their terms' magnitudes or more, FP64 sums
 // by 1e-15; with 3 decades no element is off by more than the FP64 sums' worst, and
 // the norm of the error is a fifth of theirs.  So a column (ket row) goes by
-// floating-point sums where more than a 16th of its nonzeros lie below 2^-kWide of
-// its largest, or any below 2^-kTiny.
+// floating-point sums where its nonzeros lie on average more than kWide binary
+// orders below its largest, or any more than kTiny.  (3 decades of weights and
+// normal variates: 7 orders on average, 8.4 at most, hardly one beyond 36; 4
+// decades: 8.9.)
 template <typename T>
 struct Format;
 template <>
@@ -89,10 +91,8 @@ struct Format<double> {
   static __device__ __forceinline__ int exponent(uint32_t key) { return fx::exponent_of(key, key != 0u); }
   static __device__ __forceinline__ int2 raw(double x) { return make_int2(__double2loint(x), __double2hiint(x)); }
   static __device__ __forceinline__ double of(int2 v) { return __hiloint2double(v.y, v.x); }
-  // x is below 2^-d of the largest for d = top_field - field, and above half of that.
-  static __device__ __forceinline__ int field(int2 v) { return (v.y >> 20) & 0x7ff; }
-  static __device__ __forceinline__ int top_field(int ex) { return ex + 1022; }
-  static constexpr int kWide = 14, kTiny = 40;
+  static constexpr int kField = 20;  // key >> kField: the exponent's field
+  static constexpr int kWide = 9, kTiny = 36;
   static __device__ __forceinline__ double table(int lo, int hi) { return __hiloint2double(hi, lo); }
   static __device__ __forceinline__ int2 parts(int2 v, int ex) {
     return fx::vector_parts((uint32_t)v.x, (uint32_t)v.y, ex);
@@ -109,9 +109,8 @@ struct Format<dfloat> {
   }
   static __device__ __forceinline__ int2 raw(dfloat x) { return make_int2(__float_as_int(x.lo), __float_as_int(x.hi)); }
   static __device__ __forceinline__ dfloat of(int2 v) { return dfloat(__int_as_float(v.y), __int_as_float(v.x)); }
-  static __device__ __forceinline__ int field(int2 v) { return (v.y >> 23) & 0xff; }
-  static __device__ __forceinline__ int top_field(int ex) { return ex + 126; }
-  static constexpr int kWide = 20, kTiny = 46;  // five bits fewer to keep than in FP64
+  static constexpr int kField = 23;
+  static constexpr int kWide = 15, kTiny = 42;  // five bits fewer to keep than in FP64
   // An FP64 table value: 24 bits in hi, the other 29 in lo (no FP64 instruction).
   static __device__ __forceinline__ dfloat table(int lo, int hi) {
     const int e = (hi >> 20) & 0x7ff, sign = hi & (int)0x80000000;
@@ -197,18 +196,57 @@ __device__ __forceinline__ size_t staged(uint32_t rows, uint32_t r, int c) {
   return K == 1 ? r : ((size_t)(c >> 1) * rows + r) * 2 + (c & 1);
 }
 
-// Whether a sum's elements lie too far apart for fixed point: how many of them are
-// small, of how many nonzeros (a tiny one counts as kManySmall, which is enough).
-constexpr uint32_t kManySmall = 1u << 16;
+// How far apart a sum's elements lie, from their keys: in shared memory the largest
+// key, the smallest of a nonzero less 1, the number of nonzeros and the sum of their
+// exponents' fields.
+struct Keys {
+  uint32_t top, low, nonzero, fields;
+};
 template <typename T>
-__device__ __forceinline__ void count_small(int2 v, int top, uint32_t &small, uint32_t &nonzero) {
-  using F = Format<T>;
-  if (((uint32_t)v.x | (uint32_t)v.y) << 1 == 0u) return;
-  const int d = top - F::field(v);
-  ++nonzero;
-  small += d > F::kTiny ? kManySmall : d > F::kWide ? 1u : 0u;
-}
-__device__ __forceinline__ bool is_wide(uint32_t small, uint32_t nonzero) { return small > nonzero >> 4; }
+struct Spread {
+  uint32_t top = 0u, low = ~0u, nonzero = 0u, fields = 0u;
+  __device__ __forceinline__ void count(T x, int guard) {
+    const uint32_t key = Format<T>::key(x);
+    top = max(top, key);
+    if (guard) {
+      low = min(low, key - 1u);
+      nonzero += key != 0u;
+      fields += key >> Format<T>::kField;
+    }
+  }
+  // Adds the counts of every `step`-th lane to `at`.
+  __device__ __forceinline__ void add_to(Keys *at, int guard, int step = 1) {
+    const bool one = (threadIdx.x & 31u) < (uint32_t)step;
+    if (step == 1) {
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (guard) {
+        low = __reduce_min_sync(0xffffffffu, low);
+        nonzero = __reduce_add_sync(0xffffffffu, nonzero);
+        fields = __reduce_add_sync(0xffffffffu, fields);
+      }
+    } else {
+      for (int o = 16; o >= step; o >>= 1) {
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        if (guard) {
+          low = min(low, __shfl_xor_sync(0xffffffffu, low, o));
+          nonzero += __shfl_xor_sync(0xffffffffu, nonzero, o);
+          fields += __shfl_xor_sync(0xffffffffu, fields, o);
+        }
+      }
+    }
+    if (one) atomicMax(&at->top, top);
+    if (one && guard) {
+      atomicMin(&at->low, low);
+      atomicAdd(&at->nonzero, nonzero);
+      atomicAdd(&at->fields, fields);
+    }
+  }
+  static __device__ __forceinline__ bool wide(const Keys &k) {
+    const uint32_t top = k.top >> Format<T>::kField, low = (k.low + 1u) >> Format<T>::kField;
+    return k.nonzero && (top - low > (uint32_t)Format<T>::kTiny ||
+                         k.nonzero * top - k.fields > k.nonzero * (uint32_t)Format<T>::kWide);
+  }
+};
 
 // Four table entries of a lane: three 16-byte loads.
 struct Group {
@@ -343,7 +381,8 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
   extern __shared__ __align__(16) unsigned char slab_smem[];
   int2 *X = reinterpret_cast<int2 *>(slab_smem);     // (n + 1) x K; row n is zero (padding entries)
   int2 *J = X + (size_t)(a.n + 1) * K;               // (npair + 1) x K; row npair is zero
-  __shared__ uint32_t skey[K], snext, ssmall[K], snonzero[K];
+  __shared__ Keys skey[K];
+  __shared__ uint32_t snext;
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
   const uint32_t c0 = group * K;
   constexpr int kw = K == 1 ? 1 : 2;  // columns side by side in a plane of X
@@ -354,7 +393,7 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
     else
       return ldg(a.hii + k) - a.shift;
   };
-  if (tid < K) skey[tid] = ssmall[tid] = snonzero[tid] = 0u;
+  if (tid < K) skey[tid] = Keys{0u, ~0u, 0u, 0u};
   if (tid == 0) snext = 0u;
   __syncthreads();
   // stage the raw values and find each column's largest
@@ -362,22 +401,21 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
     const int c = (int)(tid % K);
     const bool ok = c0 + c < a.m;
     const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
-    uint32_t key = 0u;
+    Spread<T> keys;
     for (uint32_t r = tid / K; r < a.n; r += nt / K) {
       T x = ok ? ldg(C + (size_t)r * a.nb + (c0 + c)) : T(0.0);
       if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
-      key = max(key, F::key(x));
+      keys.count(x, a.guard);
       X[staged<K>(a.n + 1, r, c)] = F::raw(x);
     }
-    for (int o = 16; o >= K; o >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
-    if (lane < (uint32_t)K) atomicMax(&skey[c], key);
+    keys.add_to(&skey[c], a.guard, K);
   } else {
 #pragma unroll
     for (int c = 0; c < K; ++c) {
       const bool ok = c0 + c < a.m;
       const uint64_t mask = ok && a.eta ? ldg(a.colmask + c0 + c) : 0ull;
       const T *row = C + (size_t)(c0 + c) * a.nb;
-      uint32_t key = 0u;
+      Spread<T> keys;
       for (uint32_t r = tid; r < a.n; r += nt) {
         T x = ok ? ldg(row + r) : T(0.0);
         if (a.staged_diag && ok) {
@@ -385,11 +423,10 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
           S[k] = a.add ? fma(diag(k), x, S[k]) : diag(k) * x;
         }
         if (a.eta) x = flip(x, parity((unsigned long long)(mask & ldg(a.rowstr + r))));
-        key = max(key, F::key(x));
+        keys.count(x, a.guard);
         X[staged<K>(a.n + 1, r, c)] = F::raw(x);
       }
-      key = __reduce_max_sync(0xffffffffu, key);
-      if (lane == 0) atomicMax(&skey[c], key);
+      keys.add_to(&skey[c], a.guard);
     }
   }
   if (tid < K) X[staged<K>(a.n + 1, a.n, tid)] = make_int2(0, 0);
@@ -409,28 +446,8 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
   bool bad = false;
 #pragma unroll
   for (int c = 0; c < K; ++c) {
-    ex[c] = F::exponent(skey[c]);
-    bad = bad || ex[c] == fx::kBad;
-  }
-  if (!bad && a.guard) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      const int c = q * kw + (kw == 1 ? 0 : (int)(tid & 1u));  // nt is even: a thread's elements are of one column
-      const int top = F::top_field(tid & 1u ? ex[q * kw + kw - 1] : ex[q * kw]);
-      uint32_t small = 0u, nonzero = 0u;
-      for (uint32_t i = tid; i < plane; i += nt) count_small<T>(X[(size_t)q * plane + i], top, small, nonzero);
-      for (int o = 16; o >= kw; o >>= 1) {
-        small += __shfl_xor_sync(0xffffffffu, small, o);
-        nonzero += __shfl_xor_sync(0xffffffffu, nonzero, o);
-      }
-      if (lane < (uint32_t)kw) {
-        atomicAdd(&ssmall[c], small);
-        atomicAdd(&snonzero[c], nonzero);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < K; ++c) bad = bad || is_wide(ssmall[c], snonzero[c]);
+    ex[c] = F::exponent(skey[c].top);
+    bad = bad || ex[c] == fx::kBad || (a.guard && Spread<T>::wide(skey[c]));
   }
   if (!bad) {  // to fixed point, in place (an all-zero column has no scale and its sums are not read)
 #pragma unroll
@@ -440,7 +457,7 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
         int2 &x = X[(size_t)q * plane + i];
         if (e != fx::kZero) x = F::parts(x, e);
       }
-  } else if (a.npair) {
+  } else {  // the Coulomb values as they are too
     for (uint32_t i = tid; i < (uint32_t)a.npair * K; i += nt) {
       const uint32_t P = i / K;
       const int c = (int)(i % K);
@@ -671,6 +688,17 @@ __device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__
                             reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
     if (row == ~0u) continue;
     const uint64_t str = a.eta ? ldg(a.rowstr + row) : 0ull;
+    if (!a.diag && !a.add) {  // (two sums in float-float round to their FP32 sum)
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        if (c0 + c >= a.m) break;
+        acc[c] += singles[c];
+        if (a.eta) acc[c] = flip(acc[c], parity((unsigned long long)(str & ldg(a.colmask + c0 + c))));
+        if (!whole) S[element(c)] = acc[c];
+      }
+      if (whole) store_row<K>(S + element(0), acc);
+      continue;
+    }
 #pragma unroll
     for (int c = 0; c < K; ++c) {
       if (c0 + c >= a.m) break;
@@ -689,13 +717,11 @@ __device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__
         if (ph) d = FF{-d.hi, -d.lo};
         if (a.add) ff_add(d, old[c]);
         acc[c] = ff_value(d);
-      } else if (a.add) {
+      } else {
         FF d{flip(singles[c], ph), 0.f};
         ff_add(d, flip(acc[c], ph));
         ff_add(d, old[c]);
         acc[c] = ff_value(d);
-      } else {
-        acc[c] = flip(singles[c] + acc[c], ph);
       }
       if (!whole) S[element(c)] = acc[c];
     }
@@ -750,7 +776,7 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
   int4 *Cs = reinterpret_cast<int4 *>(slab_smem);                // [G/2][nb + 1]: two ket rows' values at jb
   int4 *Ks = Cs + (size_t)NP * cplane;                           // [G/2][2 Q + phase]
   double *Ss = reinterpret_cast<double *>(Ks + NP * kplane);     // kSum: [nb]
-  __shared__ uint32_t skey[G], ssmall[G], snonzero[G];
+  __shared__ Keys skey[G];
   const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
   const uint32_t ia = item.x, part = item.y & 0xffffu, parts = item.y >> 16;
   const uint32_t p0 = ldg(a.off + ia), p1 = ldg(a.off + ia + 1);
@@ -762,11 +788,9 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
   for (uint32_t pb = p0; pb < p1; pb += G) {
     const uint32_t live = min((uint32_t)G, p1 - pb);
     __syncthreads();  // the previous batch is applied
-    if (tid < G) skey[tid] = ssmall[tid] = snonzero[tid] = 0u;
+    if (tid < G) skey[tid] = Keys{0u, ~0u, 0u, 0u};
     __syncthreads();
-    uint32_t key[G];
-#pragma unroll
-    for (int g = 0; g < G; ++g) key[g] = 0u;
+    Spread<T> keys[G];
 #pragma unroll
     for (int h = 0; h < NP; ++h) {
       const bool ok0 = 2 * h < live, ok1 = 2 * h + 1 < live;
@@ -780,50 +804,27 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
           x0 = flip(x0, parity((unsigned long long)(s0 & m)));
           x1 = flip(x1, parity((unsigned long long)(s1 & m)));
         }
-        key[2 * h] = max(key[2 * h], F::key(x0));
-        key[2 * h + 1] = max(key[2 * h + 1], F::key(x1));
+        keys[2 * h].count(x0, a.guard);
+        keys[2 * h + 1].count(x1, a.guard);
         const int2 b0 = F::raw(x0), b1 = F::raw(x1);
         Cs[h * cplane + c] = make_int4(b0.x, b0.y, b1.x, b1.y);
       }
     }
     int e[G], es = fx::kZero;
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      key[g] = __reduce_max_sync(0xffffffffu, key[g]);
-      if (lane == 0) atomicMax(&skey[g], key[g]);
-    }
+    for (int g = 0; g < G; ++g) keys[g].add_to(&skey[g], a.guard);
     __syncthreads();
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      e[g] = F::exponent(skey[g]);
+      e[g] = F::exponent(skey[g].top);
       es = max(es, e[g]);
     }
     if (es == fx::kZero) continue;  // every row is zero
-    bool fixed = es != fx::kBad;  // otherwise floating-point sums of the values as they are
-    if (fixed && a.guard) {
-#pragma unroll
-      for (int h = 0; h < NP; ++h) {
-        uint32_t small0 = 0u, nonzero0 = 0u, small1 = 0u, nonzero1 = 0u;
-        for (uint32_t c = tid; c < a.nb; c += nt) {
-          const int4 r = Cs[h * cplane + c];
-          count_small<T>(make_int2(r.x, r.y), F::top_field(e[2 * h]), small0, nonzero0);
-          count_small<T>(make_int2(r.z, r.w), F::top_field(e[2 * h + 1]), small1, nonzero1);
-        }
-        small0 = __reduce_add_sync(0xffffffffu, small0);
-        small1 = __reduce_add_sync(0xffffffffu, small1);
-        nonzero0 = __reduce_add_sync(0xffffffffu, nonzero0);
-        nonzero1 = __reduce_add_sync(0xffffffffu, nonzero1);
-        if (lane == 0) {
-          atomicAdd(&ssmall[2 * h], small0);
-          atomicAdd(&ssmall[2 * h + 1], small1);
-          atomicAdd(&snonzero[2 * h], nonzero0);
-          atomicAdd(&snonzero[2 * h + 1], nonzero1);
-        }
-      }
-      __syncthreads();
+    bool fixed = es != fx::kBad;    // otherwise floating-point sums of the values as they are
+    if (a.guard) {
 #pragma unroll
       for (int g = 0; g < G; ++g)
-        fixed = fixed && !is_wide(ssmall[g], snonzero[g]) && (e[g] == fx::kZero || es - e[g] <= F::kTiny);
+        fixed = fixed && !Spread<T>::wide(skey[g]) && (e[g] == fx::kZero || es - e[g] <= F::kTiny);
     }
     if (fixed) {  // to fixed point, in place: each thread the columns that it staged
 #pragma unroll
