@@ -183,7 +183,7 @@ struct Problem {
   // doubles in slices of 32, their table entries interleaved by lane, the
   // values' exponent, and the eta masks of the strings
   struct Slab {
-    int state = -1;  // -1 not decided yet, 0 does not apply, 1 built
+    int state = -1;  // -1 not decided yet, 0 does not apply or no room, 1 built
     uint32_t *rows[2] = {}, *off[2] = {};
     uint4 *ent_s[2] = {}, *ket_d[2] = {};
     int4 *val_s[2] = {}, *val_d[2] = {};

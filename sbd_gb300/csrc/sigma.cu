@@ -880,7 +880,8 @@ template <typename T, bool kB, bool kSweeps = false>
 bool needs_tuning(Problem &p, cudaStream_t s) {
   const int prec = slot_of<T, kB, kSweeps>();
   if (p.tune_a[prec] >= 0 && p.tune_b[prec] >= 0) return false;
-  if (!kSweeps && slab_pays<T, kB>(p) && slab_prepare(p, s)) {
+  // (a caller's 8-byte vector may need FP64 sums, which a budget may leave no room for)
+  if (!kSweeps && slab_pays<T, kB>(p) && slab_prepare(p, s) && (kB || sizeof(T) == 4 || p.slab.fp_s[0])) {
     p.tune_a[prec] = 0;
     p.tune_b[prec] = kSlabShape;
     p.split_ab[prec] = p.A.ns > 0 && p.B.ns > 0 ? 1 : 0;

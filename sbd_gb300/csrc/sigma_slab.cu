@@ -161,7 +161,7 @@ struct SlabSpin {
   const int4 *val_s;              // V of the same-spin part with the phase applied
   const uint4 *ket_d;             // doubles: ket << 4
   const int4 *val_d;
-  const int4 *fp_s, *fp_d;        // V in FP64 (the pairs of words that val_* has in fixed point)
+  const int4 *fp_s, *fp_d;        // V in FP64 (the pairs of words that val_* has in fixed point), or null
   uint32_t nslices;
 };
 
@@ -328,22 +328,28 @@ __device__ __forceinline__ void slab_list(fx::Acc (&acc)[K], const uint4 *__rest
 }
 
 // The same from the raw staged values (X, and J the raw Coulomb values), in the
-// vectors' format.
+// vectors' format.  Where there are no FP64 values (fp null: a solve that met a
+// vector which is not finite) they come from the fixed-point ones, |v| < 2^ev.
 template <typename T, int K, bool kSingles>
-__device__ __forceinline__ void slab_list_fp(T (&acc)[K], const uint4 *__restrict__ ent, const int4 *__restrict__ val,
-                                             uint32_t g, uint32_t end, uint32_t lane, const char *X, uint32_t xplane,
-                                             const char *J, uint32_t jplane) {
+__device__ __forceinline__ void slab_list_fp(T (&acc)[K], const uint4 *__restrict__ ent, const int4 *__restrict__ fp,
+                                             const int4 *__restrict__ fixed, int ev, uint32_t g, uint32_t end,
+                                             uint32_t lane, const char *X, uint32_t xplane, const char *J,
+                                             uint32_t jplane) {
   using F = Format<T>;
   if (g >= end) return;
   const uint32_t pad = xplane - 16u;  // the zero row, which padding entries point at
+  const int4 *val = fp ? fp : fixed;
+  auto value = [&](int x, int y) {
+    return fp ? F::table(x, y) : T(scalbn((double)x * (double)(1 << fx::kLow) + (double)y, ev - fx::kVBits));
+  };
   Group a;
   a.load(ent, val, g * 32u + lane);
   while (true) {
     const Group b = a;
     if (g + 1 < end) a.load(ent, val, (g + 1) * 32u + lane);
     const uint32_t w[kGroup] = {b.w.x, b.w.y, b.w.z, b.w.w};
-    const T v[kGroup] = {F::table(b.v0.x, b.v0.y), F::table(b.v0.z, b.v0.w), F::table(b.v1.x, b.v1.y),
-                         F::table(b.v1.z, b.v1.w)};
+    const T v[kGroup] = {value(b.v0.x, b.v0.y), value(b.v0.z, b.v0.w), value(b.v1.x, b.v1.y),
+                         value(b.v1.z, b.v1.w)};
 #pragma unroll
     for (int u = 0; u < kGroup; ++u) {
       const uint32_t x16 = kSingles ? w[u] & 0x7fff0u : w[u], j16 = (w[u] >> 15) & 0xfff0u;
@@ -501,9 +507,9 @@ __device__ __forceinline__ void slab_cta(const SlabArgs<T> &a, const T *__restri
 #pragma unroll
       for (int c = 0; c < K; ++c) out[c] = T(0.0);
       const uint32_t xplane = 16u * (a.n + 1), jplane = 16u * (a.npair + 1);
-      slab_list_fp<T, K, true>(out, t.ent_s, t.fp_s, ldg(t.off_s + sl), ldg(t.off_s + sl + 1), lane,
+      slab_list_fp<T, K, true>(out, t.ent_s, t.fp_s, t.val_s, a.ev, ldg(t.off_s + sl), ldg(t.off_s + sl + 1), lane,
                                reinterpret_cast<const char *>(X), xplane, reinterpret_cast<const char *>(J), jplane);
-      slab_list_fp<T, K, false>(out, t.ket_d, t.fp_d, ldg(t.off_d + sl), ldg(t.off_d + sl + 1), lane,
+      slab_list_fp<T, K, false>(out, t.ket_d, t.fp_d, t.val_d, a.ev, ldg(t.off_d + sl), ldg(t.off_d + sl + 1), lane,
                                 reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
     }
     if (row == ~0u) continue;
@@ -1298,8 +1304,10 @@ __global__ void __launch_bounds__(128) k_slab_fill(SpinTables T, const uint32_t 
       (doubles ? val_d : val_s)[2 * e] = make_int4(v[0].x, v[0].y, v[1].x, v[1].y);
       (doubles ? val_d : val_s)[2 * e + 1] = make_int4(v[2].x, v[2].y, v[3].x, v[3].y);
       (doubles ? valf_d : valf_s)[e] = make_float4(f[0], f[1], f[2], f[3]);
-      (doubles ? fp_d : fp_s)[2 * e] = make_double2(d[0], d[1]);
-      (doubles ? fp_d : fp_s)[2 * e + 1] = make_double2(d[2], d[3]);
+      if (fp_s) {
+        (doubles ? fp_d : fp_s)[2 * e] = make_double2(d[0], d[1]);
+        (doubles ? fp_d : fp_s)[2 * e + 1] = make_double2(d[2], d[3]);
+      }
     }
   }
 }
@@ -1344,11 +1352,78 @@ bool slab_ab_sum(const Problem &p) { return slab_size(p).ab_sum(); }
 // memory that this problem takes.
 bool slab_fits(const Problem &p, int element) { return slab_fits(slab_size(p), element, max_smem()); }
 
-// Builds the sliced tables on first use.  False where the kernels do not apply
-// to 8-byte elements or a budget has no room for their tables.
-bool slab_prepare(Problem &p, cudaStream_t s) {
-  if (p.slab.state >= 0) return p.slab.state == 1;
-  p.slab.state = 0;
+namespace {
+
+// What building the tables holds until it is done: temporaries, and how to give
+// back the tables themselves where memory runs out half way.
+struct SlabBuild {
+  Problem &p;
+  cudaStream_t s;
+  size_t first, bytes = 0;  // of p.allocs; bytes allocated since
+  std::vector<void *> tmps;
+  bool done = false;
+  SlabBuild(Problem &pp, cudaStream_t ss) : p(pp), s(ss), first(pp.allocs.size()) {}
+  void *alloc(size_t n) {
+    void *d = dev_alloc(p, n);
+    bytes += n ? n : 8;
+    return d;
+  }
+  ~SlabBuild() {
+    if (!done && p.allocs.size() > first) cudaStreamSynchronize(s);  // they may still be written
+    for (void *t : tmps) tmp_free(p.ctx, t);
+    if (done) return;
+    for (size_t i = first; i < p.allocs.size(); ++i) tmp_free(p.ctx, p.allocs[i]);
+    p.allocs.resize(first);
+    p.bytes -= bytes;
+    p.ctx->in_use -= bytes;
+    p.slab = Problem::Slab{};
+    p.slab.state = 0;
+  }
+};
+
+// Bytes that a budget leaves for the tables.  A serving context's reservation counts
+// a transposed copy, which these kernels do without, and half a MB of its slack is
+// theirs too; they serve solves alone there and go without the FP64 values (24 bytes
+// an entry otherwise, 16).  Under a caller's budget, whose other uses are not known,
+// they must leave room for that copy and the largest solve (64 basis vectors and 16
+// roots): what fits without them fits with them.
+size_t slab_room(const Problem &p) {
+  const Ctx &c = *p.ctx;
+  const size_t left = c.in_use < c.budget ? c.budget - c.in_use : 0;
+  if (c.pool) return std::min(left, 8 * p.N + (1u << 19));
+  const size_t solve = 8 * p.N + 16 * 64 * p.N + 64 * 16 * p.N;
+  return left > solve ? left - solve : 0;
+}
+
+// CTAs of the alpha x beta kernels: a row is shared by `base` of them where
+// rows are few, and (while the rows are only a few waves, which the longest
+// would otherwise end alone) by more the further its batches exceed the mean:
+// 2011 x 1703 strings 0.166 ms, here 0.152; with 6000 x 6000, where it only
+// adds staging, 0.89 and 0.99
+uint32_t slab_ab_base(const Problem &p) {
+  int sms = 0;
+  SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
+  return std::min(p.n_ab_slices, std::max<uint32_t>(1, 4u * sms / p.n_ab_rows));
+}
+std::vector<uint2> slab_ab_items(const Problem &p, const std::vector<uint32_t> &off_a) {
+  std::vector<uint2> items;
+  int sms = 0;
+  SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
+  const uint32_t base = slab_ab_base(p);
+  const double mean = (double)p.A.ns / p.n_ab_rows;
+  std::vector<uint32_t> order(p.na);
+  std::iota(order.begin(), order.end(), 0u);
+  auto singles = [&](uint32_t r) { return off_a[r + 1] - off_a[r]; };
+  std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return singles(x) > singles(y); });
+  for (uint32_t r : order) {
+    if (singles(r) == 0) break;
+    const uint32_t parts = std::min<uint32_t>(p.n_ab_slices, base * (uint32_t)std::ceil(p.n_ab_rows < 12u * sms ? singles(r) / (4.0 * mean) : 1.0));
+    for (uint32_t y = 0; y < parts; ++y) items.push_back(make_uint2(r, y | parts << 16));
+  }
+  return items;
+}
+
+bool slab_build(Problem &p, SlabBuild &build, cudaStream_t s) {
   if (std::max(p.na, p.nb) >= kSlabMaxRows || (uint32_t)p.npair + 1 >= kSlabMaxPair) return false;
   const bool ab = p.A.ns > 0 && p.B.ns > 0;
   if (!slab_fits(p, 8) || (ab && p.n_ab_rows == 0)) return false;
@@ -1391,6 +1466,7 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
   for (int i = 0; i < 7; ++i)
     if (!(v[i] < 0x1p100)) return false;
   std::vector<uint32_t> rows[2], ls[2], ld[2];
+  const bool budget = p.ctx->budget != 0, fp = !(budget && p.ctx->pool);
   size_t bytes = 0;
   for (int sp = 0; sp < 2; ++sp) {
     const SpinTables &T = sp == 0 ? p.A : p.B;
@@ -1417,20 +1493,22 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
       ld[sp].push_back(ld[sp].back() + (md + kGroup - 1) / kGroup);
     }
     if ((uint64_t)std::max(ls[sp].back(), ld[sp].back()) * 64u >= (1ull << 32)) return false;  // 32-bit group indices
-    bytes += 4 * rows[sp].size() + 8 * ls[sp].size() + 32ull * 24 * kGroup * (ls[sp].back() + ld[sp].back()) + 8ull * T.n;
+    bytes += 4 * rows[sp].size() + 8 * ls[sp].size() +
+             32ull * (fp ? 24 : 16) * kGroup * (ls[sp].back() + ld[sp].back()) + 8ull * T.n;
   }
-  for (uint32_t c = 0; ab && c < p.nb; ++c)  // two terms per beta single of a column
-    if (2 * (os[1][c + 1] - os[1][c]) > (uint32_t)fx::kMaxTerms) return false;
-  std::vector<void *> tmps;
+  for (uint32_t c = 0; ab && c < p.nb; ++c)  // up to four terms per beta single of a column
+    if (4 * (os[1][c + 1] - os[1][c]) > (uint32_t)fx::kMaxTerms) return false;
   p.slab.ek = std::max(-100, exponent(v[6]));
-  if (ab) bytes += 4 * p.ab_entries + 16 * p.na;
-  // under a budget: within what the transposed copy, which this form does
-  // without, is counted for
-  if (p.ctx->budget && (bytes > 8 * p.N + (1u << 20) || p.ctx->in_use + bytes > p.ctx->budget)) return false;
+  std::vector<uint2> items;
+  if (ab) {
+    items = slab_ab_items(p, os[0]);
+    bytes += 4 * p.ab_entries + 8 * items.size();
+  }
+  if (budget && bytes > slab_room(p)) return false;
   for (int sp = 0; sp < 2; ++sp) {
     const SpinTables &T = sp == 0 ? p.A : p.B;
     const size_t nrow = rows[sp].size(), nsl = ls[sp].size() - 1;
-    uint32_t *r = (uint32_t *)dev_alloc(p, 4 * nrow), *o = (uint32_t *)dev_alloc(p, 8 * (nsl + 1));
+    uint32_t *r = (uint32_t *)build.alloc(4 * nrow), *o = (uint32_t *)build.alloc(8 * (nsl + 1));
     SBDGB_CUDA(cudaMemcpyAsync(r, rows[sp].data(), 4 * nrow, cudaMemcpyHostToDevice, s));
     SBDGB_CUDA(cudaMemcpyAsync(o, ls[sp].data(), 4 * (nsl + 1), cudaMemcpyHostToDevice, s));
     SBDGB_CUDA(cudaMemcpyAsync(o + nsl + 1, ld[sp].data(), 4 * (nsl + 1), cudaMemcpyHostToDevice, s));
@@ -1442,24 +1520,27 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
     for (size_t i = 0; i < nsl; ++i)
       p.slab.longest[sp] =
           std::max(p.slab.longest[sp], kGroup * (ls[sp][i + 1] - ls[sp][i] + ld[sp][i + 1] - ld[sp][i]));
-    p.slab.ent_s[sp] = (uint4 *)dev_alloc(p, 512ull * ls[sp].back());
-    p.slab.val_s[sp] = (int4 *)dev_alloc(p, 1024ull * ls[sp].back());
-    p.slab.ket_d[sp] = (uint4 *)dev_alloc(p, 512ull * ld[sp].back());
-    p.slab.val_d[sp] = (int4 *)dev_alloc(p, 1024ull * ld[sp].back());
-    p.slab.valf_s[sp] = (float4 *)dev_alloc(p, 512ull * ls[sp].back());
-    p.slab.valf_d[sp] = (float4 *)dev_alloc(p, 512ull * ld[sp].back());
-    p.slab.fp_s[sp] = (double2 *)dev_alloc(p, 1024ull * ls[sp].back());
-    p.slab.fp_d[sp] = (double2 *)dev_alloc(p, 1024ull * ld[sp].back());
-    p.slab.mask[sp] = (uint64_t *)dev_alloc(p, 8ull * T.n);
-    if (T.ns && !p.ctx->budget) {  // the Coulomb table this spin's singles read, where memory is not counted
+    p.slab.ent_s[sp] = (uint4 *)build.alloc(512ull * ls[sp].back());
+    p.slab.val_s[sp] = (int4 *)build.alloc(1024ull * ls[sp].back());
+    p.slab.ket_d[sp] = (uint4 *)build.alloc(512ull * ld[sp].back());
+    p.slab.val_d[sp] = (int4 *)build.alloc(1024ull * ld[sp].back());
+    p.slab.valf_s[sp] = (float4 *)build.alloc(512ull * ls[sp].back());
+    p.slab.valf_d[sp] = (float4 *)build.alloc(512ull * ld[sp].back());
+    if (fp) {
+      p.slab.fp_s[sp] = (double2 *)build.alloc(1024ull * ls[sp].back());
+      p.slab.fp_d[sp] = (double2 *)build.alloc(1024ull * ld[sp].back());
+    }
+    p.slab.mask[sp] = (uint64_t *)build.alloc(8ull * T.n);
+    if (T.ns && !budget) {  // the Coulomb table this spin's singles read, where memory is not counted
       const size_t nj = (size_t)p.npair * (sp == 0 ? p.nb : p.na);
-      p.slab.Jfx[sp] = (int2 *)dev_alloc(p, 8 * nj);
+      p.slab.Jfx[sp] = (int2 *)build.alloc(8 * nj);
       k_slab_coulomb<<<(unsigned)std::min<size_t>((nj + 255) / 256, 4096), 256, 0, s>>>(
           sp == 0 ? p.Jb : p.Ja, nj, fx::kVBits - p.slab.ev[sp], p.slab.Jfx[sp]);
       count_launch(p.ctx);
     }
     // the order of the entries (two scratch words each)
     uint32_t *tmp = (uint32_t *)tmp_alloc(p.ctx, 8ull * (T.ns + T.nd));
+    build.tmps.push_back(tmp);
     uint32_t *order_s = tmp, *order_d = order_s + T.ns, *next = order_d + T.nd;
     k_slab_order<<<(unsigned)nsl, 32, 0, s>>>(T.off_s, T.ket_s, r, next, order_s);
     k_slab_order<<<(unsigned)nsl, 32, 0, s>>>(T.off_d, T.ket_d, r, next, order_d);
@@ -1467,47 +1548,42 @@ bool slab_prepare(Problem &p, cudaStream_t s) {
                                               p.slab.ent_s[sp], p.slab.val_s[sp], p.slab.ket_d[sp], p.slab.val_d[sp],
                                               p.slab.valf_s[sp], p.slab.valf_d[sp], p.slab.fp_s[sp],
                                               p.slab.fp_d[sp]);
-    tmps.push_back(tmp);
     k_slab_masks<<<(T.n + 127) / 128, 128, 0, s>>>(sp == 0 ? p.astr : p.bstr, T.n, sp, p.slab.mask[sp]);
     count_launch(p.ctx, 4);
   }
-  std::vector<uint2> items;
   if (ab) {
-    // CTAs of the alpha x beta kernels: a row is shared by `base` of them where
-    // rows are few, and (while the rows are only a few waves, which the longest
-    // would otherwise end alone) by more the further its batches exceed the mean:
-    // 2011 x 1703 strings 0.166 ms, here 0.152; with 6000 x 6000, where it only
-    // adds staging, 0.89 and 0.99
-    int sms = 0;
-    SBDGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.ctx->device));
-    const uint32_t base = std::min(p.n_ab_slices, std::max<uint32_t>(1, 4u * sms / p.n_ab_rows));
-    const double mean = (double)p.A.ns / p.n_ab_rows;
-    std::vector<uint32_t> order(p.na);
-    std::iota(order.begin(), order.end(), 0u);
-    auto singles = [&](uint32_t r) { return os[0][r + 1] - os[0][r]; };
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return singles(x) > singles(y); });
-    for (uint32_t r : order) {
-      if (singles(r) == 0) break;
-      const uint32_t parts = std::min<uint32_t>(p.n_ab_slices, base * (uint32_t)std::ceil(p.n_ab_rows < 12u * sms ? singles(r) / (4.0 * mean) : 1.0));
-      for (uint32_t y = 0; y < parts; ++y) items.push_back(make_uint2(r, y | parts << 16));
-    }
+    const uint32_t base = slab_ab_base(p);
     const uint32_t mine = (p.n_ab_slices + base - 1) / base;
     const uint32_t rounds = (mine + kSlabAbThreads / 32 - 1) / (kSlabAbThreads / 32);
     p.slab.ab_warps = std::max<uint32_t>(4, (mine + rounds - 1) / rounds);
     p.slab.n_ab_items = (uint32_t)items.size();
     p.slab.h_items = items;
-    p.slab.ab_items = (uint2 *)dev_alloc(p, 8 * items.size());
+    p.slab.ab_items = (uint2 *)build.alloc(8 * items.size());
     SBDGB_CUDA(cudaMemcpyAsync(p.slab.ab_items, items.data(), 8 * items.size(), cudaMemcpyHostToDevice, s));
-    p.slab.ab_ent = (uint32_t *)dev_alloc(p, 4 * p.ab_entries);
+    p.slab.ab_ent = (uint32_t *)build.alloc(4 * p.ab_entries);
     SBDGB_CUDA(cudaMemcpyAsync(p.slab.ab_ent, p.ab_ent, 4 * p.ab_entries, cudaMemcpyDeviceToDevice, s));
     k_slab_ab_order<<<p.n_ab_slices, 32, 0, s>>>(p.ab_slice, (uint32_t)p.npair, p.nb, p.slab.ab_ent);
     count_launch(p.ctx);
   }
   SBDGB_CUDA(cudaGetLastError());
   SBDGB_CUDA(cudaStreamSynchronize(s));  // the host vectors go out of scope
-  for (void *t : tmps) tmp_free(p.ctx, t);
-  p.slab.state = 1;
   return true;
+}
+
+}  // namespace
+
+// Builds the sliced tables on first use.  False where the kernels do not apply
+// to 8-byte elements or there is no room for their tables.
+bool slab_prepare(Problem &p, cudaStream_t s) {
+  if (p.slab.state >= 0) return p.slab.state == 1;
+  SlabBuild build(p, s);
+  try {
+    build.done = slab_build(p, build, s);
+  } catch (const Error &e) {
+    if (e.status != SBDGB_E_NOMEM) throw;
+  }
+  if (build.done) p.slab.state = 1;
+  return build.done;
 }
 
 namespace {

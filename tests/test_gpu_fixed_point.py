@@ -14,7 +14,7 @@ import pytest
 
 from golden_io import max_rel
 from oracle.oracle import Oracle
-from sbd_gb300.engine import MIXED, TPBProblem
+from sbd_gb300.engine import MIXED, Engine, TPBProblem
 from sbd_gb300.generators import make_problem
 
 torch = pytest.importorskip("torch")
@@ -299,3 +299,35 @@ def test_elements_of_wide_vectors(engine, norb, na, nb, nocc, kind):
     err = np.abs(y.double().sum(-1).cpu().numpy() - ref) / (size + 1e-25)
     assert err.max() <= 2 * k * 2.0 ** -46
     p.close()
+
+
+@pytest.mark.parametrize("norb,na,nb,nocc", [(16, 300, 280, 5), (24, 300, 280, 8)])
+def test_a_budget_holds_what_it_held_without_the_tables(norb, na, nb, nocc):
+    """Products and solves within a budget that the sweeps need: what they hold at the
+    end of the same calls, and the vector that choosing their shapes takes."""
+    prob = make_problem(norb, nocc, nocc, na, nb, seed=11)
+    kw = dict(nroots=2, max_nb=16, eps=1e-9, max_it=1, want_vectors=False)
+
+    def calls(e, sweeps):
+        p = TPBProblem.from_problem(e, prob)
+        p.diag_terms()
+        if sweeps:
+            p.set_tuning(0, 1, 1)
+            p.set_tuning(3, 1, 1)
+        x = torch.ones(prob.ndet, dtype=torch.float64, device="cuda")
+        _sigma(p, x)
+        for init in (0, 1):
+            p.davidson(init=init, **kw)
+        used, shape = e.bytes_in_use, p.tuning(0)["beta_shape"]
+        p.close()
+        return used, shape
+
+    e = Engine(0)
+    used, _ = calls(e, True)
+    e.close()
+    e = Engine(0, hbm_budget=used + 8 * prob.ndet + 4096)
+    calls(e, False)
+    e.close()
+    e = Engine(0, hbm_budget=1 << 36)  # with room for the tables
+    assert calls(e, False)[1] == SLAB
+    e.close()
