@@ -57,12 +57,27 @@ struct RdmArgs {
 };
 
 // Same-spin singles of spin S, one warp per pair: s and u[q] over the
-// spectators.  Of 32 spectators each lane forms one's product, on the fixed-point
-// scale of the largest (57 bits), and the lanes then add them all, lane q those
+// spectators.  Of 32 spectators each lane forms one's product, as an integer of
+// twice 57 bits on the scale of the largest (exact for products down to 2^-61 of
+// it; further apart, FP64 sums), and the lanes then add them all, lane q those
 // with orbital q: integer additions (62 a clock and SM) where FP64 ones take 16
 // clocks a warp.  Before, every spectator added to its orbitals' sums by FP64
 // atomics in shared memory (compare-and-swap loops on 8 of 24 places): 1.3 ms
-// a spin for 301 x 420 strings of norb 24, 22 us here.
+// a spin for 301 x 420 strings of norb 24, 22 us with one word, 34 here.
+struct Wide57 {
+  unsigned long long hi, lo;  // hi 2^57 + lo on the scale of the second word, both with the sign
+};
+// x 2^s in two words: |x 2^s| <= 2^57, and exact for s + (x's exponent) >= -4.
+__device__ __forceinline__ Wide57 two_words(double x, int s) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)(b >> 52) & 0x7ff;
+  const unsigned long long m = (b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+  const int sh = max((e ? e : 1) - 1075 + s, -57);  // (zero: anything); at most 4
+  const long long h = (long long)(sh >= 0 ? m << sh : m >> -sh);
+  const long long l = (long long)(sh >= 0 ? 0ull : m << (57 + sh) & ((1ull << 57) - 1ull));
+  const long long sg = (long long)b >> 63;
+  return {(unsigned long long)((h ^ sg) - sg), (unsigned long long)((l ^ sg) - sg)};
+}
 template <int S>
 __global__ void __launch_bounds__(kT) k_rdm_singles(RdmArgs a) {
   const SpinTables &T = S == 0 ? a.A : a.B;
@@ -72,6 +87,7 @@ __global__ void __launch_bounds__(kT) k_rdm_singles(RdmArgs a) {
   const uint32_t nopp = S == 0 ? a.nb : a.na;
   const int L = a.L;
   __shared__ ulonglong2 sv[kT / 32][32];
+  __shared__ unsigned long long svl[kT / 32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool two = a.two != nullptr;
   for (uint64_t p = (uint64_t)blockIdx.x * (kT / 32) + warp; p < T.ns; p += (uint64_t)gridDim.x * (kT / 32)) {
@@ -85,29 +101,39 @@ __global__ void __launch_bounds__(kT) k_rdm_singles(RdmArgs a) {
       const uint64_t os = o < nopp ? __ldg(opp + o) : 0ull;
       double v = o < nopp ? __ldg(rb + o) * __ldg(rk + o) : 0.0;
       v = sdev::flip(v, (__popcll(os & mask) ^ (code >> 31)) & 1u);
-      const uint32_t hi = (uint32_t)__double2hiint(v) & 0x7fffffffu;
-      const uint32_t top = __reduce_max_sync(0xffffffffu, hi ? hi : (__double2loint(v) ? 1u : 0u));
+      const uint32_t hi = (uint32_t)__double2hiint(v) & 0x7fffffffu, key = hi ? hi : (__double2loint(v) ? 1u : 0u);
+      const uint32_t top = __reduce_max_sync(0xffffffffu, key);
       if (top == 0u) continue;  // all zero
+      const uint32_t low = __reduce_min_sync(0xffffffffu, key - 1u) + 1u;  // of the nonzeros
       const int ex = fx::exponent_of(top, true);
-      const bool fixed = ex != fx::kBad;
-      const long long f = fixed ? fx::from_double(v, fx::kVBits - ex) : __double_as_longlong(v);
+      const bool fixed = ex != fx::kBad && (top >> 20) - (low >> 20) <= 60u;
+      Wide57 f{(unsigned long long)__double_as_longlong(v), 0ull};
+      if (fixed) f = two_words(v, fx::kVBits - ex);
       __syncwarp();
-      sv[warp][lane] = make_ulonglong2((unsigned long long)f, os);
+      sv[warp][lane] = make_ulonglong2(f.hi, os);
+      svl[warp][lane] = f.lo;
       __syncwarp();
       if (fixed) {
-        long long a0 = 0, a1 = 0, as = 0;  // 32 terms of 57 bits
+        long long a0 = 0, a1 = 0, as = 0, b0 = 0, b1 = 0, bs = 0;  // 32 terms of 57 bits
 #pragma unroll 8
         for (int i = 0; i < 32; ++i) {
           const ulonglong2 x = sv[warp][i];
-          const long long t = (long long)x.x;
+          const long long t = (long long)x.x, l = (long long)svl[warp][i];
           as += t;
-          a0 += (x.y >> lane & 1ull) ? t : 0ll;
-          if (L > 32) a1 += (x.y >> (lane + 32) & 1ull) ? t : 0ll;
+          bs += l;
+          if (x.y >> lane & 1ull) {
+            a0 += t;
+            b0 += l;
+          }
+          if (L > 32 && (x.y >> (lane + 32) & 1ull)) {
+            a1 += t;
+            b1 += l;
+          }
         }
-        const double unit = scalbn(1.0, ex - fx::kVBits);
-        ssum = fma((double)as, unit, ssum);
-        u0 = fma((double)a0, unit, u0);
-        if (L > 32) u1 = fma((double)a1, unit, u1);
+        const double unit = scalbn(1.0, ex - fx::kVBits), low_unit = unit * 0x1p-57;
+        ssum += fma((double)as, unit, (double)bs * low_unit);
+        u0 += fma((double)a0, unit, (double)b0 * low_unit);
+        if (L > 32) u1 += fma((double)a1, unit, (double)b1 * low_unit);
       } else {
         for (int i = 0; i < 32; ++i) {
           const ulonglong2 x = sv[warp][i];

@@ -14,7 +14,8 @@ import pytest
 
 from golden_io import max_rel
 from oracle.oracle import Oracle
-from sbd_gb300.engine import MIXED, Engine, TPBProblem
+from sbd_gb300.engine import TPBProblem
+from sbd_gb300.engine import MIXED, Engine
 from sbd_gb300.generators import make_problem
 
 torch = pytest.importorskip("torch")

@@ -45,3 +45,44 @@ def test_rdms_against_oracle(engine, norb, na, nb, nocc):
     W[prob.ndet // 2] = np.nan
     assert np.isnan(p.rdm(W)[0]).any()
     p.close()
+
+
+@pytest.mark.parametrize("decades", [0, 6, 12])
+@pytest.mark.parametrize("norb,na,nb,nocc", [(12, 97, 150, 4), (40, 90, 61, 13)])
+def test_elements_of_wide_vectors(engine, norb, na, nb, nocc, decades):
+    """The sums of the same-spin singles over the spectators that have an orbital q,
+    which are the whole of two[s, 1 - s][a, q, i, q]: each to the bound of its own k
+    terms (2^-53 each in the products and in the sum, here and in the reference),
+    with weights over that many decades on the strings of each spin."""
+    prob = make_problem(norb, nocc, nocc, na, nb, seed=na + nb)
+    o = Oracle.from_problem(prob)
+    rng = np.random.default_rng(decades)
+    W = (rng.normal(size=(na, nb)) * 10.0 ** rng.uniform(-decades, 0, (na, 1))
+         * 10.0 ** rng.uniform(-decades, 0, (1, nb)))
+    p = TPBProblem.from_problem(engine, prob)
+    p.build_tables()
+    one, two = p.rdm(W.ravel())
+    ro, rt = o.correlation(W.ravel())
+    L = norb
+    one, ro = (np.asarray(x).reshape(2, L, L) for x in (one, ro))  # [s][a][i]
+    two, rt = (np.asarray(x).reshape(4, L, L, L, L) for x in (two, rt))  # [s1 + 2 s2][d][c][b][a]
+    bits = np.arange(L, dtype=np.uint64)
+    for s, t, x, other in ((0, o.ta, np.abs(W), prob.bstr), (1, o.tb, np.abs(W).T, prob.astr)):
+        occ = ((other.astype(np.uint64)[:, None] >> bits) & np.uint64(1)).astype(float)
+        n = int(t.off_s[-1])
+        bra = np.repeat(np.arange(len(x)), np.diff(t.off_s[:len(x) + 1].astype(np.int64)))
+        ket, move = t.ket_s[:n].astype(np.int64), np.asarray(t.cran_s[:2 * n]).reshape(-1, 2) // 2
+        size, count = np.zeros((L, L, L)), np.zeros((L, L))  # [i][a][q], [i][a]
+        for b, k, (i, a) in zip(bra, ket, move):
+            size[i, a] += (x[b] * x[k]) @ occ
+            count[i, a] += len(occ)
+        i, a, q = np.nonzero(size)
+        for blk, got in ((s + 2 * (1 - s), lambda y: y[q, i, q, a]), ((1 - s) + 2 * s, lambda y: y[i, q, a, q])):
+            err = np.abs(got(two[blk]) - got(rt[blk]))
+            assert (err <= 4 * (count[i, a] + 4) * 2.0 ** -53 * size[i, a, q]).all()
+        i, a = np.nonzero(count)
+        total = np.zeros((L, L))
+        for b, k, (ii, aa) in zip(bra, ket, move):
+            total[ii, aa] += x[b] @ x[k]
+        assert (np.abs(one[s, a, i] - ro[s, a, i]) <= 4 * (count[i, a] + 4) * 2.0 ** -53 * total[i, a]).all()
+    p.close()
