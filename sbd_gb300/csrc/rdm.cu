@@ -398,8 +398,17 @@ void rdm_ab(Problem &p, const RdmArgs &a, cudaStream_t s) {
   const int L = a.L;
   const size_t L2 = (size_t)L * L;
   const size_t words = 4 * (p.A.ns / kAbPairs + L2) + 4 * L2;
-  // counts and cursors of both spins, chunks and types, sorted singles
-  unsigned char *ws = (unsigned char *)workspace(p, WS_RED2, 16 * L2 + 4 * words + 8 * (p.A.ns + p.B.ns) + 64);
+  // counts and cursors of both spins, chunks and types, sorted singles: kept with the
+  // problem, or for this call alone where a budget has no room for them
+  struct Buffer {
+    Ctx *c;
+    void *tmp = nullptr;
+    ~Buffer() { tmp_free(c, tmp); }
+  } buffer{p.ctx};
+  const size_t bytes = 16 * L2 + 4 * words + 8 * (p.A.ns + p.B.ns) + 64, have = p.ws_bytes[WS_RED2];
+  if (p.ctx->budget && bytes > have && p.ctx->in_use - have + bytes > p.ctx->budget)
+    buffer.tmp = tmp_alloc(p.ctx, bytes);
+  unsigned char *ws = (unsigned char *)(buffer.tmp ? buffer.tmp : workspace(p, WS_RED2, bytes));
   uint32_t *count = (uint32_t *)ws, *next = count + 2 * L2;
   uint4 *lists = (uint4 *)(ws + ((16 * L2 + 15) & ~(size_t)15));
   uint2 *pa = (uint2 *)((unsigned char *)lists + 4 * words), *pb = pa + p.A.ns;

@@ -12,6 +12,7 @@ import pytest
 
 from oracle.oracle import Oracle
 from sbd_gb300.engine import TPBProblem
+from sbd_gb300.engine import Engine
 from sbd_gb300.generators import make_problem
 
 torch = pytest.importorskip("torch")
@@ -86,3 +87,27 @@ def test_elements_of_wide_vectors(engine, norb, na, nb, nocc, decades):
             total[ii, aa] += x[b] @ x[k]
         assert (np.abs(one[s, a, i] - ro[s, a, i]) <= 4 * (count[i, a] + 4) * 2.0 ** -53 * total[i, a]).all()
     p.close()
+
+
+def test_density_matrices_within_a_budget():
+    """The sorted singles, which the earlier kernels did without, take no room of a
+    budget that has none left."""
+    prob = make_problem(16, 5, 5, 1500, 30, seed=7)
+    W = np.random.default_rng(0).normal(size=prob.ndet)
+    e = Engine(0)
+    p = TPBProblem.from_problem(e, prob)
+    p.build_tables()
+    one, two = p.rdm(W)
+    used = e.bytes_in_use
+    singles = sum(p.table_counts(s)[0] for s in (0, 1))
+    p.close()
+    e.close()
+    e = Engine(0, hbm_budget=used - 4 * singles)
+    p = TPBProblem.from_problem(e, prob)
+    p.build_tables()
+    for _ in range(2):
+        a, b = p.rdm(W)
+        assert _close(a, one) and _close(b, two)
+    assert e.bytes_in_use <= used - 4 * singles
+    p.close()
+    e.close()
