@@ -11,14 +11,14 @@ diagonal resident, starting from the lowest diagonal entries).
   e2e   : solves/s through the C ABI with host buffers: upload strings and
           integrals, build tables and diagonal, solve, copy both Ritz vectors
           back -- every step
-  roofline : the sigma operator (transpose + alpha sweep + beta sweep), whose
-          per-product device time is recorded with CUDA events on its launch
-          stream during the timed region; algorithmic bytes per product are
-          24*N + 8*nnz_off (read C and hii, write sigma, one 8-byte C read per
-          off-diagonal element).  roofline.fp64 gives the same product against
-          the measured FP64 FMA rate (one FMA per nonzero): the roof of the
-          FP64 kernels; the fixed-point ones (k_slab) add in integers and may
-          pass it
+  roofline : the sigma operator, whose per-product device time is recorded with
+          CUDA events on its launch stream during the timed region.  Fixed-point
+          kernels (k_slab): three integer multiply-adds per nonzero against their
+          measured rate, the bytes of the vectors (24*N) against HBM beside.  FP64
+          kernels: 24*N + 8*nnz_off bytes (read C and hii, write sigma, one 8-byte
+          C read per off-diagonal element) against HBM.  roofline.fp64 gives the
+          product against the measured FP64 FMA rate (one FMA per nonzero), the roof
+          of the FP64 kernels alone
   cpu_baseline : the CPU oracle port of the reference's TRADMODE sigma (OpenMP,
           all host cores) timed on a bounded sample of alpha rows and scaled to
           the solve's sigma count
@@ -147,6 +147,53 @@ def measure_fp64_rates(device: int) -> dict:
     if rc != 0:
         raise RuntimeError(f"FP64 rate probe failed ({rc})")
     return {"dfma_tflops": a.value, "dmma_tflops": b.value}
+
+
+def measure_imad_rate(device: int) -> float:
+    """10^12 integer multiply-adds (32 x 32 + 64 bits) a second, from the same library."""
+    import ctypes as C
+    from sbd_gb300 import build
+    L = C.CDLL(build.RATES_LIB)
+    L.sbdgb_measure_imad_rate.argtypes = [C.c_int, C.POINTER(C.c_double)]
+    a = C.c_double()
+    rc = L.sbdgb_measure_imad_rate(device, C.byref(a))
+    if rc != 0:
+        raise RuntimeError(f"integer rate probe failed ({rc})")
+    return a.value
+
+
+def sigma_roofline(tiles, sigma_ms, N, nnz_off, bytes_sigma, peak, peak_kind, traffic, local) -> dict:
+    """What bounds a product, against the measured roof.  The FP64 kernels: bytes with
+    one read of C per nonzero against HBM, and one FMA per nonzero against the FP64
+    pipe.  The fixed-point ones read C from shared memory and spend three integer
+    multiply-adds per nonzero; for them the bytes are those of the vectors alone, and
+    the ratio with a read per nonzero is kept beside under a name of its own."""
+    t = sigma_ms * 1e-3
+    rates = measure_fp64_rates(local)
+    fp64 = 2.0 * (nnz_off + N) / t / 1e12
+    fp64 = {"unit": "TFLOP/s", "achieved": fp64, "peak": rates["dfma_tflops"], "frac": fp64 / rates["dfma_tflops"],
+            "peak_kind": "measured FP64 FMA pipe (bench_csrc/rates.cu)",
+            "fp64_tensor_peak": rates["dmma_tflops"], "flops": "2 x (nnz_off + N) per sigma"}
+    achieved = bytes_sigma / t / 1e9
+    shape = tiles.get("beta_shape")
+    if shape != "slab":
+        return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                "traffic": traffic,
+                "kernel": ("sigma operator (fused k_sigma_alpha)" if shape == "fused"
+                           else "sigma operator (k_transpose + k_sigma_alpha + k_sigma_beta)"),
+                "algorithmic_bytes": bytes_sigma, "peak_kind": f"{peak_kind} hbm_gbs", "fp64": fp64}
+    imad, vectors = measure_imad_rate(local), 24 * N
+    mads = 3.0 * nnz_off / t / 1e12
+    return {"bound": "integer multiply-adds", "achieved": mads, "peak": imad, "unit": "10^12/s", "frac": mads / imad,
+            "traffic": traffic, "kernel": "sigma operator (k_slab + k_slab_ab)",
+            "peak_kind": "measured 32 x 32 + 64-bit multiply-adds (bench_csrc/rates.cu)",
+            "multiply_adds": "3 x nnz_off per sigma",
+            "hbm": {"unit": "GB/s", "bytes": vectors, "achieved": vectors / t / 1e9, "peak": peak,
+                    "frac": vectors / t / 1e9 / peak, "peak_kind": f"{peak_kind} hbm_gbs",
+                    "what": "C, hii and sigma once each"},
+            "read_per_nonzero": {"unit": "GB/s", "bytes": bytes_sigma, "rate": achieved,
+                                 "what": "the same and 8 bytes of C per nonzero, from shared memory here: no bound"},
+            "fp64": fp64}
 
 
 def measure_fp64_overlap(device: int) -> dict:
@@ -554,12 +601,7 @@ def run_gpu(args):
     t_max = max_over_ranks(dist, t_rank)
     value = ws * args.steps / t_max
     sigma_ms_per = sigma_ms / max(ncalls, 1)
-    achieved = bytes_sigma / (sigma_ms_per * 1e-3) / 1e9
     peak, peak_kind = peaks()
-    # one FMA per off-diagonal element and per diagonal element against the measured
-    # FP64 FMA rate, the roof of the FP64 kernels (k_slab adds in integers)
-    rates = measure_fp64_rates(local)
-    fp64_achieved = 2.0 * (nnz_off + N) / (sigma_ms_per * 1e-3) / 1e12
     tiles = p.tuning(3)  # the solver's products: FP64 in the block ordering
 
     # mixed-precision form on the same problem (reported beside the FP64 headline)
@@ -674,17 +716,7 @@ def run_gpu(args):
             "sigma_products_per_solve": float(np.mean(nsig)),
             "sigma_ms": sigma_ms_per,
             "sigma_tiles": tiles,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": traffic,
-                         "kernel": ("sigma operator (k_slab + k_slab_ab)" if tiles.get("beta_shape") == "slab"
-                                    else "sigma operator (fused k_sigma_alpha)" if tiles.get("beta_shape") == "fused"
-                                    else "sigma operator (k_transpose + k_sigma_alpha + k_sigma_beta)"),
-                         "algorithmic_bytes": bytes_sigma, "peak_kind": f"{peak_kind} hbm_gbs",
-                         "fp64": {"unit": "TFLOP/s", "achieved": fp64_achieved, "peak": rates["dfma_tflops"],
-                                  "frac": fp64_achieved / rates["dfma_tflops"],
-                                  "peak_kind": "measured FP64 FMA pipe (bench_csrc/rates.cu)",
-                                  "fp64_tensor_peak": rates["dmma_tflops"],
-                                  "flops": "2 x (nnz_off + N) per sigma"}},
+            "roofline": sigma_roofline(tiles, sigma_ms_per, N, nnz_off, bytes_sigma, peak, peak_kind, traffic, local),
             "mixed_precision": mixed,
             "config3_sigma": config3,
             "serving": serving,

@@ -162,7 +162,9 @@ int sbdgb_sigma_mixed_block(sbdgb_problem *p, const float *Wk_dev, float *Wb_dev
  * the row length and alignment allow it (one row per CTA of 512 threads
  * otherwise) or 1 = one row per CTA of 1024 threads;
  * shape_b = 7 (reported, not settable) means the fixed-point kernels
- * (sigma_slab.cu), taken without timing where a row has more than 8 nonzeros.
+ * (sigma_slab.cu), taken without timing where a row has at least 14 nonzeros and
+ * each spin 256 strings, or a row 100 nonzeros (double-float in the block ordering:
+ * 100 only), and their shared memory and tables fit;
  * precision 6 reads the FP64 sweeps that solves from init 0 or 2 keep to where the
  * other block-ordering products (3) go by the fixed-point kernels.
  * The first product of each precision tunes (and synchronises), so make it

@@ -6,8 +6,9 @@
 // projections to the FP64 tensor path would pay.
 //
 // A benchmark utility, not part of the engine: built into its own library
-// (libsbdgb_rates.so) that only bench.py loads, to state the FP64 roof the
-// sigma kernels are measured against.  Returns 0 on success, 3 on a CUDA error.
+// (libsbdgb_rates.so) that only bench.py loads, to state the FP64 and integer
+// roofs the sigma kernels are measured against.  Returns 0 on success, 3 on a CUDA
+// error.
 #include <cuda_runtime.h>
 
 namespace {
@@ -65,7 +66,59 @@ __global__ void __launch_bounds__(kRateThreads) k_rate_both(double *out) {
   if (s == 12345.0) out[blockIdx.x] = s;
 }
 
+// 32 x 32 + 64-bit integer multiply-adds, what the fixed-point sigma kernels add
+// their terms with; one operand changes each time, so that no product is kept.
+__global__ void __launch_bounds__(kRateThreads) k_rate_imad(double *out) {
+  int a[8], b = (int)threadIdx.x * 40503 + 12345;
+  long long c[8] = {};
+  for (int u = 0; u < 8; ++u) a[u] = b + 77 * u;
+  for (int i = 0; i < kRateIters; ++i) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      c[u] += (long long)a[u] * b;
+      a[u] ^= i;
+    }
+  }
+  long long s = 0;
+  for (int u = 0; u < 8; ++u) s ^= c[u];
+  if (s == 12345) out[blockIdx.x] = (double)s;
+}
+
 }  // namespace
+
+// 10^12 integer multiply-adds a second, after one untimed run.  Returns 0, or 3 on
+// a CUDA error.
+extern "C" int sbdgb_measure_imad_rate(int device, double *tera_per_s) {
+  if (!tera_per_s) return 1;
+  int sms = 0;
+  if (cudaSetDevice(device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    cudaGetLastError();
+    return 3;
+  }
+  const int blocks = sms * 8;
+  double *out = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  float ms = 0.f;
+  int rc = 0;
+  if (cudaMalloc(&out, sizeof(double) * blocks) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
+      cudaEventCreate(&e1) != cudaSuccess)
+    rc = 3;
+  for (int rep = 0; rep < 2 && rc == 0; ++rep) {
+    cudaEventRecord(e0, 0);
+    k_rate_imad<<<blocks, kRateThreads>>>(out);
+    cudaEventRecord(e1, 0);
+    if (cudaEventSynchronize(e1) != cudaSuccess) rc = 3;
+    cudaEventElapsedTime(&ms, e0, e1);
+  }
+  if (rc == 0 && cudaGetLastError() != cudaSuccess) rc = 3;
+  if (rc == 0) *tera_per_s = (double)blocks * kRateThreads * kRateIters * 8 / (ms * 1e-3) / 1e12;
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  if (out) cudaFree(out);
+  cudaGetLastError();
+  return rc;
+}
 
 // Milliseconds of the FMA loop, the MMA loop and the interleaved loop (same
 // work as both), each after one untimed run.  Returns 0, or 3 on a CUDA error.

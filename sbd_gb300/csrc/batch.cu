@@ -1235,12 +1235,11 @@ void batch_davidson(Ctx &c, Problem **ps, int count, const sbdgb_davidson_opts &
       SBDGB_CUDA(cudaMemcpyAsync(dptr, ptr.data(), sizeof(void *) * ptr.size(), cudaMemcpyHostToDevice, s));
       SBDGB_CUDA(cudaMemcpyAsync(dn, n.data(), sizeof(uint32_t) * count, cudaMemcpyHostToDevice, s));
       const SlabBatchState st{&dS->active, &dS->from, &dS->to, sizeof(BState), dptr, dptr + count, dn};
-      const int nvec = mixed ? nseed : k;  // the FP64 phase of the mixed form starts on nseed vectors
-      slab_batch_plan<double>(slab64, &c, ps, a64.data(), count, st, nvec, s);
+      slab_batch_plan<double>(slab64, &c, ps, a64.data(), count, st, nseed, s);  // it starts on nseed vectors
       SlabBatchState sf = st;
       sf.V = dptr + 2 * count;
       sf.HV = dptr + 3 * count;
-      if (mixed) slab_batch_plan<float>(slab32, &c, ps, a32.data(), count, sf, k, s);
+      slab_batch_plan<float>(slab32, &c, ps, a32.data(), count, sf, k, s);
     }
     SBDGB_CUDA(cudaMemcpyAsync(dP, hp.data(), sizeof(BProb) * count, cudaMemcpyHostToDevice, s));
     SBDGB_CUDA(cudaMemcpyAsync(dch, chunks.data(), sizeof(Chunk) * nch, cudaMemcpyHostToDevice, s));

@@ -12,8 +12,8 @@
 // low x low are added exactly, so a sum's value does not depend on the order of
 // its terms.  A term's error is that of the two conversions (2^-56 of the
 // largest |x| of the sum, 2^-58 of the largest |v|) and the product left out
-// (2^-59 of the largest |x| times the largest |v|, of either sign); an FP64
-// sum's is 2^-53 of each partial sum.
+// (2^-59 of the largest |x| times the largest |v|, of either sign; 2^-58 where v is
+// a sum of two); an FP64 sum's is 2^-53 of each partial sum.
 #pragma once
 
 #include <cuda_runtime.h>

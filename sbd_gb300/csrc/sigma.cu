@@ -33,7 +33,7 @@
 // an alpha-beta element costs two popcounts.
 //
 // The mixed form (T = float) stores C, sigma and the table values in FP32,
-// forms each pair-list sum in FP32 and adds it to an FP64 accumulator per
+// forms each pair-list sum in FP32 and adds it to a float-float accumulator per
 // element; the FP64 form (T = double) accumulates every product in FP64.
 #include <algorithm>
 #include <type_traits>
@@ -835,10 +835,12 @@ inline double nnz_per_row(const Problem &p) {
 // row, 40 and 55, 28 and 49; 1580 x 890, 16.6, 126 and 111, 104 and 95).  With
 // few strings of one spin their CTAs are few or their staging serves few columns
 // (3517 x 108, 64 a row, 196 and 223; 3070 x 180, 58, FP32 116 and 130), which
-// 100 a row outweigh (1914 x 225, 207 a row, 610 and 274).  In the block
+// 100 a row outweigh, however few they are (1914 x 225, 207 a row, 610 and 274;
+// FP64, more than 200 a row: 3000 x 3, 232 and 124; 5 x 10000, 909 and 149; 4000 x 2,
+// 535 and 49; 495 x 1, 63 and 15).  In the block
 // ordering the double-float sweeps are not bound by phases and win up to about
 // 100 (ms, sweeps and slab: 2011 x 1703, 58 a row, 0.47 and 0.53; 6000 x 6000,
-// 78, 3.9 and 4.5; 800 x 800, 605, 1.33 and 0.71).
+// 78, 3.9 and 4.5; 800 x 800, 1007, 1.33 and 0.71).
 // Where a form's kernels need more shared memory than there is, it keeps the others.
 template <typename T, bool kB>
 bool slab_pays(const Problem &p) {
