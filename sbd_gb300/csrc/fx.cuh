@@ -1,9 +1,9 @@
 // Fixed-point arithmetic for FP64 sums of products.
 //
 // On this GPU an FP64 multiply-add issues at 2 per clock and SM, a 32 x 32 ->
-// 64-bit integer multiply-add at 32 (measured 1.97 and 28.6).  A sum over a pair
-// list whose operands are integers on a common scale takes three of the latter
-// per term:
+// 64-bit integer multiply-add at 32 of unsigned operands (measured 1.97 and 29.4;
+// signed ones, which these are, 19.0 as compiled).  A sum over a pair list whose
+// operands are integers on a common scale takes three of the latter per term:
 //
 //   X = round(x 2^(55 - ex)), |x| < 2^ex for every x of the sum
 //   V = round(v 2^(57 - ev)),  |v| < 2^ev for every v of the table

@@ -4,16 +4,17 @@
 //
 // What bounds it.  The kernels of sigma.cu spend one FP64 multiply-add per
 // nonzero and keep the FP64 pipe (2 a clock and SM) 89-91% busy.  Here a
-// nonzero costs three 32 x 32 + 64-bit integer multiply-adds (fx.cuh; 32 a
+// nonzero costs three 32 x 32 + 64-bit integer multiply-adds (fx.cuh; 19 a
 // clock and SM), and its gather comes from shared memory instead of L2.  ncu on
-// the beta sweep of 3274 x 3935 strings (norb 24, 245 pairs a row): L1 data
-// pipe 79%, integer multiply-adds near 70% of their rate, shared loads at 1.2
-// wavefronts per 8 lanes.
+// 3274 x 3935 strings (norb 24, 245 pairs a row), alpha sweep, alpha x beta, beta
+// sweep: L1 data pipe 74, 85 and 70% busy, the pipe of the multiply-adds 70, 56 and
+// 67%, shared loads at 1.24, 1.70 and 1.22 wavefronts per 8 lanes, FP64 pipe at most
+// 4%.
 //
 // Measured (one product in the reference's convention, ms; FP64 kernels, here):
-// norb 12, 161 x 187: 0.374, 0.084; norb 16, 800 x 800: 1.91, 0.70; norb 24,
-// 3274 x 3935: 18.8, 8.2 (sweeps 2.1 and 1.8, alpha x beta 4.4); norb 36, 6000 x
-// 6000: 6.4, 3.6 (1.4, 1.4 and 0.9).  Error against FP64 sums of the
+// norb 12, 161 x 187: 0.374, 0.091; norb 16, 800 x 800: 1.91, 0.72; norb 24,
+// 3274 x 3935: 18.3, 8.2 (sweeps 1.8 and 2.1, alpha x beta 4.2); norb 36, 6000 x
+// 6000: 6.6, 3.8 (1.4, 1.4 and 0.9).  Error against FP64 sums of the
 // off-diagonal part kept apart from the diagonal (2-norm): 0.7-1.1e-16, where
 // the FP64 kernels have 3e-16 to 1.3e-15.
 //

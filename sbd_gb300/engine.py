@@ -310,7 +310,9 @@ class TPBProblem:
         return wb
 
     def tuning(self, precision: int = FP64) -> dict:
-        """Sigma tile shapes chosen by the autotuner and the candidates' timings (ms)."""
+        """Sigma tile shapes chosen by the autotuner and the candidates' timings (ms).
+        precision: FP64, FP32 or double-float, + 3 in the solvers' block ordering; 6 = the
+        FP64 sweeps kept beside the fixed-point kernels ("slab")."""
         a, b = C.c_int(-1), C.c_int(-1)
         ma, mb = (C.c_float * 4)(), (C.c_float * 4)()
         self.engine.check(self.lib.sbdgb_problem_tuning(self.h, precision, C.byref(a), C.byref(b), ma, mb, 4))

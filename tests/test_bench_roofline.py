@@ -26,5 +26,5 @@ def test_fp64_kernels(rates):
 
 @pytest.mark.gpu
 def test_measured_integer_rate():
-    """Between a quarter and twice 32 a clock and SM (152 SMs at 2.07 GHz)."""
-    assert 2.5 < bench.measure_imad_rate(0) < 20.0
+    """Between a half and one and a quarter of 32 a clock and SM (152 SMs at 2.07 GHz)."""
+    assert 5.0 < bench.measure_imad_rate(0) < 12.6
