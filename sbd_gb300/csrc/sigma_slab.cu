@@ -543,10 +543,13 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
 
 // ---- the same sweep in FP32 -------------------------------------------------------
 //
-// FP32 vectors and table values, FP32 products and list sums; a lane's two list sums,
-// the diagonal and what sigma holds are added in float-float as in the kernels of
-// sigma.cu, and the launches' results in FP32 (as there where the alpha x beta pairs
-// or the beta sweep have a launch of their own).  Four columns of a row are 16
+// FP32 vectors and table values, FP32 products and list sums; in a caller's product a
+// lane's two list sums, the diagonal and what sigma holds are added in float-float as
+// in the kernels of sigma.cu, and the launches' results in FP32 (as there where the
+// alpha x beta pairs or the beta sweep have a launch of their own).  In a solve's
+// FP32 phase, whose result the double-float or FP64 phase refines, the two lists
+// share a register (the sign of an eigenvector comes from its roundings: 1e-15 of
+// the integrals turns 17% of a batch's vectors around, in any of these kernels).  Four columns of a row are 16
 // bytes.  Bound: the L1 data pipe (3 bytes of table and 4 of shared memory a
 // term at K = 8).  gridDim.z vectors at once.
 struct SlabArgsF {
@@ -561,7 +564,8 @@ struct SlabArgsF {
   const uint64_t *rowstr, *colmask;
   uint32_t n, m, nb;
   int npair, eta, add, diag;
-  int vec;  // rows of S start on 16-byte boundaries
+  int join;  // the two lists' sums are added in float-float
+  int vec;   // rows of S start on 16-byte boundaries
   uint32_t parts;
 };
 
@@ -688,8 +692,8 @@ __device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__
     float singles[K];
 #pragma unroll
     for (int c = 0; c < K; ++c) {
-      singles[c] = acc[c];
-      acc[c] = 0.f;
+      singles[c] = a.join ? acc[c] : 0.f;
+      acc[c] = a.join ? 0.f : acc[c];
     }
     slab_list_f32<K, false>(acc, t.ket_d, a.val_d, ldg(t.off_d + sl), ldg(t.off_d + sl + 1), lane,
                             reinterpret_cast<const char *>(X), xplane, nullptr, 0u);
@@ -699,7 +703,7 @@ __device__ __forceinline__ void slab_cta_f32(const SlabArgsF &a, const float *__
 #pragma unroll
       for (int c = 0; c < K; ++c) {
         if (c0 + c >= a.m) break;
-        acc[c] += singles[c];
+        if (a.join) acc[c] += singles[c];
         if (a.eta) acc[c] = flip(acc[c], parity((unsigned long long)(str & ldg(a.colmask + c0 + c))));
         if (!whole) S[element(c)] = acc[c];
       }
@@ -1714,7 +1718,7 @@ void launch_slab(const Problem &p, const Args<T> &x, int add, int diag, int eta,
 }
 
 template <bool kAlpha>
-SlabArgsF slab_args_f32(const Problem &p, const Args<float> &x, int add, int diag, int eta) {
+SlabArgsF slab_args_f32(const Problem &p, const Args<float> &x, int add, int diag, int eta, int join) {
   constexpr int sp = kAlpha ? 0 : 1;
   SlabArgsF a{};
   a.hii_df = x.hii_df;
@@ -1733,6 +1737,7 @@ SlabArgsF slab_args_f32(const Problem &p, const Args<float> &x, int add, int dia
   a.eta = eta;
   a.add = add;
   a.diag = diag;
+  a.join = join;
   a.parts = 1;
   return a;
 }
@@ -1740,7 +1745,7 @@ SlabArgsF slab_args_f32(const Problem &p, const Args<float> &x, int add, int dia
 template <bool kAlpha>
 void launch_slab_f32(const Problem &p, const Args<float> &x, const float *const *C, float *const *S, int nvec, int add,
                      int diag, int eta, cudaStream_t s) {
-  SlabArgsF a = slab_args_f32<kAlpha>(p, x, add, diag, eta);
+  SlabArgsF a = slab_args_f32<kAlpha>(p, x, add, diag, eta, eta);  // (the solvers: the block ordering)
   a.vec = p.nb % 4 == 0;
   for (int v = 0; v < nvec; ++v) {
     a.C[v] = C[v];
@@ -1899,8 +1904,8 @@ void slab_batch_plan(SlabBatch &b, Ctx *c, Problem **ps, const sdev::Args<T> *ar
   for (int i = 0; i < count; ++i) {
     const Problem &p = *ps[i];
     if constexpr (kF32) {
-      sa.push_back(slab_args_f32<true>(p, args[i], 0, 0, 1));
-      sb.push_back(slab_args_f32<false>(p, args[i], 1, 1, 1));
+      sa.push_back(slab_args_f32<true>(p, args[i], 0, 0, 1, 0));
+      sb.push_back(slab_args_f32<false>(p, args[i], 1, 1, 1, 0));
       ab.push_back(slab_ab_args_f32(p, args[i], 1));
     } else {
       sa.push_back(slab_args<double, true>(p, args[i], 0, 0, 1, 0));
