@@ -125,9 +125,10 @@ int sbdgb_diag_terms(sbdgb_problem *p, double *hii_out);
  * Where the fixed-point kernels are taken (shape_b = 7 below) the terms of a sum
  * are added exactly on one scale: an element of Wk is held to 2^-56 of the largest
  * of its sum's (one row or column of Wk), a matrix element to 2^-58 of the largest
- * of its spin's.  A row or column of Wk whose nonzeros lie too far apart for that
- * (more than 9 binary orders below the largest on average, or any more than 36), or
- * that is not finite or beyond 2^+-800, is summed in FP64 instead. */
+ * of its spin's (2^-45 where both spins move: rows of Wk share a scale there).  A row
+ * or column of Wk whose nonzeros lie too far apart for that (more than 9 binary
+ * orders below the largest on average, or any more than 36), rows that do not share a
+ * scale, and what is not finite or beyond 2^+-800, are summed in FP64 instead. */
 int sbdgb_sigma(sbdgb_problem *p, const double *Wk_dev, double *Wb_dev, int accumulate, void *stream);
 /* Mixed-precision sigma: FP32 vectors, FP32 products and pair-list sums, a
  * float-float accumulator per element (an FP32 sum and the rounding errors of

@@ -78,7 +78,7 @@ constexpr uint32_t kSlabMaxPair = 1u << 12;  // pair index bits
 // by 1e-15; with 3 decades no element is off by more than the FP64 sums' worst, and
 // the norm of the error is a fifth of theirs.  So a column (ket row) goes by
 // floating-point sums where its nonzeros lie on average more than kWide binary
-// orders below its largest, or any more than kTiny.  (3 decades of weights and
+// orders below its largest, or any more than kTiny (kRows: below).  (3 decades of weights and
 // normal variates: 7 orders on average, 8.4 at most, hardly one beyond 36; 4
 // decades: 8.9.)
 template <typename T>
@@ -93,7 +93,7 @@ struct Format<double> {
   static __device__ __forceinline__ int2 raw(double x) { return make_int2(__double2loint(x), __double2hiint(x)); }
   static __device__ __forceinline__ double of(int2 v) { return __hiloint2double(v.y, v.x); }
   static constexpr int kField = 20;  // key >> kField: the exponent's field
-  static constexpr int kWide = 9, kTiny = 36;
+  static constexpr int kWide = 9, kTiny = 36, kRows = 13;
   static __device__ __forceinline__ double table(int lo, int hi) { return __hiloint2double(hi, lo); }
   static __device__ __forceinline__ int2 parts(int2 v, int ex) {
     return fx::vector_parts((uint32_t)v.x, (uint32_t)v.y, ex);
@@ -111,7 +111,7 @@ struct Format<dfloat> {
   static __device__ __forceinline__ int2 raw(dfloat x) { return make_int2(__float_as_int(x.lo), __float_as_int(x.hi)); }
   static __device__ __forceinline__ dfloat of(int2 v) { return dfloat(__int_as_float(v.y), __int_as_float(v.x)); }
   static constexpr int kField = 23;
-  static constexpr int kWide = 15, kTiny = 42;  // five bits fewer to keep than in FP64
+  static constexpr int kWide = 15, kTiny = 42, kRows = 19;  // five bits fewer to keep than in FP64
   // An FP64 table value: 24 bits in hi, the other 29 in lo (no FP64 instruction).
   static __device__ __forceinline__ dfloat table(int lo, int hi) {
     const int e = (hi >> 20) & 0x7ff, sign = hi & (int)0x80000000;
@@ -757,7 +757,8 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab_f32(SlabArgsF a) {
 //
 // The ket rows of a batch have scales of their own (2^e_g); the batch's is the
 // largest, and the (P|Q) values of a smaller row are scaled down by the
-// difference.
+// difference (in a caller's product kRows binary orders at most: floating-point
+// sums beyond; 3 decades of weights make 10).
 // kSum: the row's sums stay in shared memory until the last batch; otherwise
 // each batch's go to sigma at once (rows with a batch or two; less shared
 // memory, so more CTAs an SM).
@@ -835,7 +836,7 @@ __device__ __forceinline__ void slab_ab_cta(const SlabAbArgs<T> &a, const T *__r
     if (a.guard) {
 #pragma unroll
       for (int g = 0; g < G; ++g)
-        fixed = fixed && !Spread<T>::wide(skey[g]) && (e[g] == fx::kZero || es - e[g] <= F::kTiny);
+        fixed = fixed && !Spread<T>::wide(skey[g]) && (e[g] == fx::kZero || es - e[g] <= F::kRows);
     }
     if (fixed) {  // to fixed point, in place: each thread the columns that it staged
 #pragma unroll

@@ -288,7 +288,7 @@ def test_elements_of_wide_vectors(engine, norb, na, nb, nocc, kind):
     c = torch.tensor(x, device="cuda")
     s = _sigma(p, c)
     assert p.tuning(0)["beta_shape"] == SLAB
-    assert (np.abs(s.cpu().numpy() - ref) / size).max() <= 2 * k * 2.0 ** -53
+    assert (np.abs(s.cpu().numpy() - ref) <= 2 * k * 2.0 ** -53 * size).all()
     assert torch.equal(_sigma(p, c), s)
     hi = c.float()
     pair = torch.stack([hi, (c - hi.double()).float()], dim=-1).contiguous()
@@ -332,3 +332,35 @@ def test_a_budget_holds_what_it_held_without_the_tables(norb, na, nb, nocc):
     e = Engine(0, hbm_budget=1 << 36)  # with room for the tables
     assert calls(e, False)[1] == SLAB
     e.close()
+
+
+@pytest.mark.parametrize("norb,na,nb,nocc", [(24, 300, 280, 8), (16, 60, 300, 5)])
+def test_ket_rows_of_different_scales(engine, norb, na, nb, nocc):
+    """Every other alpha string 2^-35 below its neighbours, on the beta strings that
+    those do not have, so that each row and column holds one scale and the rows of an
+    alpha x beta batch two.  Every element to its terms' FP64 roundings (as above) and
+    those of the matrix elements, at most 2^-45 of the largest (2^-39 in double-float)
+    of each kind, whose scale may be eight times the largest off the diagonal."""
+    prob, p = _problem(engine, norb, nocc, nocc, na, nb, seed=na + nb)
+    H = Oracle.from_problem(prob).hamiltonian()
+    off = H.copy()
+    off.setdiag(0.0)
+    C = np.random.default_rng(nb).uniform(0.5, 1.0, (na, nb))
+    C[::2, 1::2] = 0.0
+    C[1::2, ::2] = 0.0
+    C[1::2] *= 2.0 ** -35
+    x = C.ravel()
+    ref, size, k = H @ x, abs(H) @ np.abs(x), np.diff(H.indptr).max() + 8
+    table = 8 * np.abs(off.data).max() * ((off != 0) @ np.abs(x))
+    c = torch.tensor(x, device="cuda")
+    s = _sigma(p, c)
+    assert p.tuning(0)["beta_shape"] == SLAB
+    assert (np.abs(s.cpu().numpy() - ref) <= 2 * k * 2.0 ** -53 * size + 2.0 ** -45 * table).all()
+    hi = c.float()
+    pair = torch.stack([hi, (c - hi.double()).float()], dim=-1).contiguous()
+    y = torch.empty_like(pair)
+    p.sigma_df_device(pair.data_ptr(), y.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    err = np.abs(y.double().sum(-1).cpu().numpy() - ref)
+    assert (err <= 2 * k * 2.0 ** -46 * size + 2.0 ** -39 * table + 1e-38).all()
+    p.close()
