@@ -96,6 +96,16 @@ __global__ void __launch_bounds__(kT) k_rdm_singles(RdmArgs a) {
     const int oi = code & 0xff, oa = (code >> 8) & 0xff;
     const double *rb = Wr + (size_t)bra * nopp, *rk = Wr + (size_t)ket * nopp;
     double u0 = 0.0, u1 = 0.0, ssum = 0.0;  // orbitals lane and lane + 32, and all
+    if (!two) {  // s alone, each lane its spectators
+#pragma unroll 4
+      for (uint32_t o = lane; o < nopp; o += 32) {
+        const uint32_t ph = (__popcll(__ldg(opp + o) & mask) ^ (code >> 31)) & 1u;
+        ssum += sdev::flip(__ldg(rb + o) * __ldg(rk + o), ph);
+      }
+      for (int d = 16; d > 0; d >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, d);
+      if (lane == 0) atomicAdd(&a.one[(size_t)S * L * L + oi + (size_t)L * oa], ssum);
+      continue;
+    }
     for (uint32_t o0 = 0; o0 < nopp; o0 += 32) {
       const uint32_t o = o0 + lane;
       const uint64_t os = o < nopp ? __ldg(opp + o) : 0ull;
@@ -145,7 +155,6 @@ __global__ void __launch_bounds__(kT) k_rdm_singles(RdmArgs a) {
       }
     }
     if (lane == 0) atomicAdd(&a.one[(size_t)S * L * L + oi + (size_t)L * oa], ssum);
-    if (!two) continue;
     const uint64_t bs = same[bra];
     double *blk = a.two + (size_t)(3 * S) * L * L * L * L;  // s1 = s2 = S
     double *b1 = a.two + (size_t)(S + 2 * (1 - S)) * L * L * L * L;
