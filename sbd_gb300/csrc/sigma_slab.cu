@@ -549,9 +549,9 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab(SlabArgs<T> a) {
 // alpha x beta pairs or the beta sweep have a launch of their own).  In a solve's
 // FP32 phase, whose result the double-float or FP64 phase refines, the two lists
 // share a register (the sign of an eigenvector comes from its roundings: 1e-15 of
-// the integrals turns 17% of a batch's vectors around, in any of these kernels).  Four columns of a row are 16
-// bytes.  Bound: the L1 data pipe (3 bytes of table and 4 of shared memory a
-// term at K = 8).  gridDim.z vectors at once.
+// the integrals turns 17% of a batch's vectors around, in any of these kernels).
+// Four columns of a row are 16 bytes.  Bound: the L1 data pipe (3 bytes of table and
+// 4 of shared memory a term at K = 8).  gridDim.z vectors at once.
 struct SlabArgsF {
   const float *C[4];
   float *S[4];
